@@ -159,6 +159,24 @@ void gemm_swiglu(const Tensor& a, const Tensor& b, Tensor& d, const OptTensor& s
                                              cur_stream()),
               "gemm_swiglu: arguments not served");
 }
+bool gemm_mlp_in(const Tensor& a, const Tensor& b, Tensor& act, const OptTensor& gu, const OptTensor& status) {
+  check_bf16(a, "gemm_mlp_in a"); check_bf16(b, "gemm_mlp_in b"); check_bf16(act, "gemm_mlp_in act");
+  TORCH_CHECK(a.dim() == 2 && b.dim() == 2 && act.dim() == 2 && a.stride(1) == 1 && b.stride(1) == 1 && act.stride(1) == 1, "gemm_mlp_in: 2-D");
+  const int64_t M = a.size(0), K = a.size(1), F = act.size(1);
+  TORCH_CHECK(b.size(0) == 2 * F && b.size(1) == K && act.size(0) == M, "gemm_mlp_in: b must be the stacked [2F, K] gate/up weight");
+  TORCH_CHECK(a.stride(0) % 8 == 0 && b.stride(0) % 8 == 0 && (reinterpret_cast<uintptr_t>(a.data_ptr()) & 15) == 0 &&
+              (reinterpret_cast<uintptr_t>(b.data_ptr()) & 15) == 0, "gemm_mlp_in: operand rows must be 16-byte aligned");
+  long long ldgu = 0;
+  if (gu.has_value() && gu->defined()) {
+    check_bf16(*gu, "gemm_mlp_in gu");
+    TORCH_CHECK(gu->dim() == 2 && gu->size(0) == M && gu->size(1) == 2 * F && gu->stride(1) == 1, "gemm_mlp_in: gu [M, 2F]");
+    ldgu = gu->stride(0);
+  }
+  if (status.has_value() && status->defined()) check_i32(*status, "gemm_mlp_in status");
+  const c10::cuda::CUDAGuard guard(a.device());
+  return agrpo::launch_gemm_mlp_in(a.data_ptr(), a.stride(0), b.data_ptr(), b.stride(0), act.data_ptr(), act.stride(0), opt_ptr<void>(gu), ldgu,
+                                   (int)M, (int)F, (int)K, opt_ptr<int>(status), num_sms(), cur_stream());
+}
 void embedding_bwd(const Tensor& ids, const Tensor& dout, Tensor& dtable) {
   check_i32(ids, "ids"); check_bf16(dout, "dout"); check_f32(dtable, "dtable");
   TORCH_CHECK(dtable.is_contiguous() && dout.is_contiguous(), "embedding_bwd layout");
@@ -912,6 +930,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("decode_layers_counter_words", &decode_layers_counter_words);
   m.def("gemm_swiglu", &gemm_swiglu, py::arg("a"), py::arg("b"), py::arg("d"), py::arg("ss_in") = py::none(), py::arg("eps") = 1e-6,
         py::arg("status") = py::none(), NOGIL);
+  m.def("gemm_mlp_in", &gemm_mlp_in, py::arg("a"), py::arg("b"), py::arg("act"), py::arg("gu") = py::none(), py::arg("status") = py::none(), NOGIL);
   m.def("rmsnorm_fwd", &rmsnorm_fwd, py::arg("x"), py::arg("w"), py::arg("y"), py::arg("rstd") = py::none(),
         py::arg("eps") = 1e-6, NOGIL);
   m.def("rmsnorm_bwd", &rmsnorm_bwd, py::arg("dy"), py::arg("x"), py::arg("w"), py::arg("rstd"), py::arg("dx"),

@@ -3,7 +3,7 @@
 #include "../common/tensormap.h"
 #include "../launchers.h"
 #include "../launchers_layers.h"
-#include "gemm_tcgen05.cuh"
+#include "gemm_pair.cuh"
 #include "layer_ops.cuh"
 
 namespace agrpo {
@@ -17,7 +17,7 @@ struct DytResidualEpilogue {
   long long ldh;
   DytNorm<__nv_bfloat16> n1, n2;
   float a1, a2;
-  int bn;                // column tile of the kernel
+  int bn;                // columns that a warp converts per tile
   float xn[32];          // residual of the next 32 columns, read ahead
 
   // 32 residual values of one row; columns past N (a multiple of 8) are not read
@@ -76,14 +76,15 @@ void launch_gemm_dyt_bf16(const void* a, long long lda, const void* b, long long
     return;
   const int tiles_m = (M + kGemmBM - 1) / kGemmBM;
   const int cands[3] = {256, 128, 64};
-  int BN = 32;
-  for (int bn : cands)
+  const bool pair = pair_serves(M, num_sms);
+  int BN = pair ? pair_pick_bn(M, N, false, num_sms) : 32;
+  if (!pair) for (int bn : cands)
     if ((long long)tiles_m * ((N + bn - 1) / bn) >= 120) {
       BN = bn;
       break;
     }
   const CUtensorMap ta = make_tmap_2d(a, K, M, lda, 64, kGemmBM);
-  const CUtensorMap tb = make_tmap_2d(b, K, N, ldb, 64, BN);
+  const CUtensorMap tb = make_tmap_2d(b, K, N, ldb, 64, pair ? BN / 2 : BN);
   GemmShape p;
   p.M = M; p.N = N; p.K = K;
   p.group_n = 1;
@@ -97,8 +98,12 @@ void launch_gemm_dyt_bf16(const void* a, long long lda, const void* b, long long
   e.n1 = {(P)n1.w, (P)n1.b, (P)n1.alpha};
   e.n2 = {(P)n2.w, (P)n2.b, (P)n2.alpha};
   e.a1 = e.a2 = 0.f;
-  e.bn = BN;
-  if (BN == 256) gemm_launch<256, false, false>(ta, tb, p, e, num_sms, s);
+  e.bn = pair ? BN / 2 : BN;
+  if (pair) {
+    if (BN == 256) gemm_pair_launch<256, false, false>(ta, tb, p, e, num_sms, s);
+    else if (BN == 192) gemm_pair_launch<192, false, false>(ta, tb, p, e, num_sms, s);
+    else gemm_pair_launch<128, false, false>(ta, tb, p, e, num_sms, s);
+  } else if (BN == 256) gemm_launch<256, false, false>(ta, tb, p, e, num_sms, s);
   else if (BN == 128) gemm_launch<128, false, false>(ta, tb, p, e, num_sms, s);
   else if (BN == 64) gemm_launch<64, false, false>(ta, tb, p, e, num_sms, s);
   else gemm_launch<32, false, false>(ta, tb, p, e, num_sms, s);

@@ -2,7 +2,7 @@
 // mixer and feed-forward to the residual stream and prepares the next block's inputs.
 #include "../common/tensormap.h"
 #include "../launchers.h"
-#include "gemm_tcgen05.cuh"
+#include "gemm_pair.cuh"
 #include "parallel_block.cuh"
 
 namespace agrpo {
@@ -36,7 +36,7 @@ struct ProjEpilogue {
 
 struct ResidualEpilogue {
   ResidualOut o;
-  int bn;
+  int bn;        // columns that a warp converts per tile
   float sq;
   float xn[32];  // residual of the next 32 columns, read ahead
 
@@ -93,6 +93,16 @@ struct SplitEpilogue {
 };
 
 template <class Epi>
+void launch_pair_tiles(const void* a, long long lda, int a_cols, const void* b, long long ldb, const GemmShape& p, const Epi& e, int BN,
+                       int num_sms, cudaStream_t s) {
+  const CUtensorMap ta = make_tmap_2d(a, a_cols, p.M, lda, 64, kGemmBM);
+  const CUtensorMap tb = make_tmap_2d(b, p.K, p.N, ldb, 64, BN / 2);
+  if (BN == 256) gemm_pair_launch<256, false, false>(ta, tb, p, e, num_sms, s);
+  else if (BN == 192) gemm_pair_launch<192, false, false>(ta, tb, p, e, num_sms, s);
+  else gemm_pair_launch<128, false, false>(ta, tb, p, e, num_sms, s);
+}
+
+template <class Epi>
 void launch_tiles(const void* a, long long lda, int a_cols, const void* b, long long ldb, const GemmShape& p, const Epi& e, int BN, int num_sms,
                   cudaStream_t s) {
   const CUtensorMap ta = make_tmap_2d(a, a_cols, p.M, lda, 64, kGemmBM);
@@ -126,7 +136,9 @@ void launch_gemm_parallel_proj(const ParallelProjArgs& a, int num_sms, cudaStrea
   e.o = out;
   e.rs = 1.f;
   e.sq = e.sk = 0.f;
-  launch_tiles(a.h, a.lda, a.n2 > 0 ? a.a2 + a.K : a.K, a.w, a.ldw, p, e, pick_bn(p), num_sms, s);
+  const int a_cols = a.n2 > 0 ? a.a2 + a.K : a.K;
+  if (pair_serves(a.M, num_sms)) launch_pair_tiles(a.h, a.lda, a_cols, a.w, a.ldw, p, e, pair_pick_bn(p.M, p.N, false, num_sms, p.n1), num_sms, s);
+  else launch_tiles(a.h, a.lda, a_cols, a.w, a.ldw, p, e, pick_bn(p), num_sms, s);
 }
 
 void launch_gemm_residual(const ResidualArgs& a, int num_sms, cudaStream_t s) {
@@ -140,6 +152,12 @@ void launch_gemm_residual(const ResidualArgs& a, int num_sms, cudaStream_t s) {
   ResidualEpilogue e;
   e.o = out;
   e.sq = 0.f;
+  if (pair_serves(a.M, num_sms)) {
+    const int bn = pair_pick_bn(p.M, p.N, false, num_sms);
+    e.bn = bn / 2;
+    launch_pair_tiles(a.a, a.lda, a.K, a.w, a.ldw, p, e, bn, num_sms, s);
+    return;
+  }
   e.bn = pick_bn(p);
   launch_tiles(a.a, a.lda, a.K, a.w, a.ldw, p, e, e.bn, num_sms, s);
 }

@@ -85,40 +85,6 @@ struct SkParams {
     if (p.trace != nullptr && blockIdx.x == 0 && blockIdx.y == 0) p.trace[slot] = clock64(); \
   } while (0)
 
-__device__ __forceinline__ uint32_t cluster_ctarank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ uint32_t mapa_shared(uint32_t addr, uint32_t rank) {
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
-  return r;
-}
-__device__ __forceinline__ void mbar_arrive_remote(uint32_t remote_addr) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(remote_addr) : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait_cluster(uint64_t* bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t"
-      ".reg .pred P;\n\t"
-      "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 P, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, P;\n\t"
-      "}\n"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-__device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity) {
-  if (mbar_try_wait_cluster(bar, parity)) return true;
-  const long long t0 = clock64();
-  while (!mbar_try_wait_cluster(bar, parity)) {
-    if (clock64() - t0 > kWaitBudgetTicks) return false;
-  }
-  return true;
-}
 __device__ __forceinline__ float ld_dsmem_f32(uint32_t addr) {
   float v;
   // no memory clobber: the loads of one reduction step are independent and must be allowed to overlap; ordering
@@ -137,15 +103,6 @@ __device__ __forceinline__ void st_async_f32x4(uint32_t remote_addr, float a, fl
                "f"(a), "f"(b), "f"(c), "f"(d), "r"(remote_bar)
                : "memory");
 }
-__device__ __forceinline__ void fence_cluster_barrier_init() {
-  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-}
-__device__ __forceinline__ void cluster_sync_all() {
-  // only used once at start-up (barrier initialisation must be visible before any remote arrive); the hardware
-  // cluster barrier cannot stall here because every CTA of a cluster is resident and reaches it unconditionally
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-
 // MT row-tiles of 128 per CTA (M <= 128 * MT), BN columns per cluster, S = cluster size = K splits.
 template <int BN, int MT, int STAGES>
 __global__ void __launch_bounds__(kThreads, 1)

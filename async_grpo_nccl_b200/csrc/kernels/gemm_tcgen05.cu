@@ -1,6 +1,7 @@
 // Host launcher for the tcgen05 GEMM (kernel in gemm_tcgen05.cuh).
 #include "../common/tensormap.h"
 #include "../launchers.h"
+#include "gemm_pair.cuh"
 #include "gemm_tcgen05.cuh"
 
 namespace agrpo {
@@ -16,18 +17,52 @@ void dispatch_major(bool a_mn, bool b_mn, const CUtensorMap& ta, const CUtensorM
   return gemm_launch<BN, true, false>(ta, tb, p, e, sms, s, gj);
 }
 
+bool aligned32(const void* p, long long ld, int elem) { return (reinterpret_cast<uintptr_t>(p) & 31) == 0 && (ld * elem) % 32 == 0; }
+
+template <int BN, class Epi>
+void dispatch_pair_major(bool a_mn, bool b_mn, const CUtensorMap& ta, const CUtensorMap& tb, const GemmShape& p, const Epi& e, int sms,
+                         cudaStream_t s) {
+  if (!a_mn && !b_mn) return gemm_pair_launch<BN, false, false>(ta, tb, p, e, sms, s);
+  if (!a_mn && b_mn) return gemm_pair_launch<BN, false, true>(ta, tb, p, e, sms, s);
+  if (a_mn && b_mn) return gemm_pair_launch<BN, true, true>(ta, tb, p, e, sms, s);
+  return gemm_pair_launch<BN, true, false>(ta, tb, p, e, sms, s);
+}
+template <bool F32, bool AUX>
+void dispatch_pair(int BN, bool a_mn, bool b_mn, const CUtensorMap& ta, const CUtensorMap& tb, const GemmShape& p, PairStoreEpilogue<F32, AUX> e,
+                   int sms, cudaStream_t s) {
+  e.bn = BN / 2;
+  if (BN == 256) return dispatch_pair_major<256>(a_mn, b_mn, ta, tb, p, e, sms, s);
+  if (BN == 192) return dispatch_pair_major<192>(a_mn, b_mn, ta, tb, p, e, sms, s);
+  return dispatch_pair_major<128>(a_mn, b_mn, ta, tb, p, e, sms, s);
+}
+template <bool F32, bool AUX>
+PairStoreEpilogue<F32, AUX> pair_store(void* d, long long ldd, const void* bias, const void* aux, long long ld_aux) {
+  PairStoreEpilogue<F32, AUX> e;
+  e.D = d;
+  e.ldd = ldd;
+  e.bias = reinterpret_cast<const __nv_bfloat16*>(bias);
+  e.aux = aux;
+  e.lda = ld_aux;
+  return e;
+}
+
 template <class Gather>
 void launch_gemm_impl(const void* a, long long lda, const void* b, long long ldb, void* d, long long ldd, int M, int N,
                       int K, bool a_mn, bool b_mn, const void* bias, float alpha, bool out_fp32, bool accumulate,
                       int* status, int num_sms, cudaStream_t stream, const void* residual, long long ldr,
                       const Gather& gj) {
+  // CTA pairs wherever the rows fill more than one tile and the epilogue's 32-byte accesses are aligned. The plain kernel keeps
+  // what a pair does not serve and launches that carry a gather job.
+  const bool wide = aligned32(d, ldd, out_fp32 ? 4 : 2) && N % (out_fp32 ? 8 : 16) == 0 && (reinterpret_cast<uintptr_t>(bias) & 15) == 0 &&
+                    (residual == nullptr || (!out_fp32 && aligned32(residual, ldr, 2)));
+  const bool pair = !Gather::kEnabled && wide && alpha == 1.f && !(accumulate && !out_fp32) && pair_serves(M, num_sms);
   // Widest column tile that still yields about one work item per SM; the 64 / 32 wide tiles serve
   // skinny decode-time GEMMs (K-major operands only) where the weight stream must be spread over all SMs.
   const int tiles_m = (M + kGemmBM - 1) / kGemmBM;
   const bool plain = !a_mn && !b_mn;
   const int cands[4] = {256, 128, 64, 32};
-  int BN = plain ? 32 : 128;
-  for (int i = 0; i < (plain ? 4 : 2); ++i) {
+  int BN = pair ? pair_pick_bn(M, N, b_mn, num_sms) : plain ? 32 : 128;
+  for (int i = 0; !pair && i < (plain ? 4 : 2); ++i) {
     const int bn = cands[i];
     if ((long long)tiles_m * ((N + bn - 1) / bn) >= 120) {
       BN = bn;
@@ -37,7 +72,7 @@ void launch_gemm_impl(const void* a, long long lda, const void* b, long long ldb
   CUtensorMap ta, tb;
   if (!a_mn) ta = make_tmap_2d(a, K, M, lda, 64, kGemmBM);
   else       ta = make_tmap_2d(a, M, K, lda, 64, 64);
-  if (!b_mn) tb = make_tmap_2d(b, K, N, ldb, 64, BN);
+  if (!b_mn) tb = make_tmap_2d(b, K, N, ldb, 64, pair ? BN / 2 : BN);
   else       tb = make_tmap_2d(b, N, K, ldb, 64, 64);
   GemmShape p;
   p.M = M; p.N = N; p.K = K;
@@ -52,6 +87,14 @@ void launch_gemm_impl(const void* a, long long lda, const void* b, long long ldb
   e.alpha = alpha;
   e.out_fp32 = out_fp32 ? 1 : 0;
   e.accumulate = accumulate ? 1 : 0;
+  if (pair) {
+    if (out_fp32) {
+      if (accumulate) dispatch_pair(BN, a_mn, b_mn, ta, tb, p, pair_store<true, true>(d, ldd, bias, d, ldd), num_sms, stream);
+      else dispatch_pair(BN, a_mn, b_mn, ta, tb, p, pair_store<true, false>(d, ldd, bias, nullptr, 0), num_sms, stream);
+    } else if (residual != nullptr) dispatch_pair(BN, a_mn, b_mn, ta, tb, p, pair_store<false, true>(d, ldd, bias, residual, ldr), num_sms, stream);
+    else dispatch_pair(BN, a_mn, b_mn, ta, tb, p, pair_store<false, false>(d, ldd, bias, nullptr, 0), num_sms, stream);
+    return;
+  }
   if (BN == 256) dispatch_major<256>(a_mn, b_mn, ta, tb, p, e, num_sms, stream, gj);
   else if (BN == 128) dispatch_major<128>(a_mn, b_mn, ta, tb, p, e, num_sms, stream, gj);
   else if (BN == 64) gemm_launch<64, false, false>(ta, tb, p, e, num_sms, stream, gj);
@@ -168,10 +211,49 @@ bool launch_gemm_rs_bf16(const void* a, long long lda, const void* b, long long 
   return true;
 }
 
+namespace {
+// act = silu(gate) * up in one launch of CTA pairs; false when they do not serve the shape.
+template <bool BF16>
+bool launch_pair_swiglu(const void* a, long long lda, const void* b, long long ldb, void* d, long long ldd, void* gu, long long ldgu, int M,
+                        int F, int K, const long long* ss_in, float eps, int* status, int num_sms, cudaStream_t stream) {
+  if (!pair_serves(M, num_sms) || F % 16 != 0 || !aligned32(d, ldd, 2) || (gu != nullptr && !aligned32(gu, ldgu, 2))) return false;
+  // two 128-wide halves where that fills the pairs, else 64-wide ones (a tile of half the width takes about 0.6 of the time)
+  const int pairs = num_sms / 2;
+  const auto waves = [&](int half) { return (pair_num_items(M, (F + half - 1) / half, 1) + pairs - 1) / pairs; };
+  const int BN = 0.6f * (float)waves(64) < (float)waves(128) ? 128 : 256;
+  const CUtensorMap ta = make_tmap_2d(a, K, M, lda, 64, kGemmBM);
+  const CUtensorMap tb = make_tmap_2d(b, K, 2 * F, ldb, 64, BN / 2);
+  GemmShape p;
+  p.M = M; p.N = 2 * ((F + BN / 2 - 1) / (BN / 2)) * (BN / 2); p.K = K;
+  p.group_n = 1;
+  p.status = status;
+  p.dual_b = F;
+  PairSwigluEpilogue<BF16> e;
+  e.D = reinterpret_cast<__nv_bfloat16*>(d);
+  e.ldd = ldd;
+  e.gu = reinterpret_cast<__nv_bfloat16*>(gu);
+  e.ldgu = ldgu;
+  e.F = F;
+  e.ss_in = ss_in;
+  e.inv_k = 1.f / (float)K;
+  e.eps = eps;
+  e.rs = 1.f;
+  if (BN == 256) gemm_pair_launch<256, false, false>(ta, tb, p, e, num_sms, stream);
+  else gemm_pair_launch<128, false, false>(ta, tb, p, e, num_sms, stream);
+  return true;
+}
+}  // namespace
+
+bool launch_gemm_mlp_in(const void* a, long long lda, const void* b, long long ldb, void* act, long long ldact, void* gu, long long ldgu,
+                        int M, int F, int K, int* status, int num_sms, cudaStream_t stream) {
+  return M > 0 && launch_pair_swiglu<true>(a, lda, b, ldb, act, ldact, gu, ldgu, M, F, K, nullptr, 0.f, status, num_sms, stream);
+}
+
 // act[M, F] = silu(rs * (a . Wg^T)) * (rs * (a . Wu^T)) with b = [Wg; Wu] stacked ([2F, K], the fused gate/up weight).
 bool launch_gemm_swiglu_bf16(const void* a, long long lda, const void* b, long long ldb, void* d, long long ldd, int M, int F,
                              int K, const long long* ss_in, float eps, int* status, int num_sms, cudaStream_t stream) {
   if (F % 8 != 0 || M <= 0 || F <= 0) return false;
+  if (launch_pair_swiglu<false>(a, lda, b, ldb, d, ldd, nullptr, 0, M, F, K, ss_in, eps, status, num_sms, stream)) return true;
   const int tiles_m = (M + kGemmBM - 1) / kGemmBM;
   const int BN = ((long long)tiles_m * ((2 * F + 127) / 128) >= 120) ? 128 : 64;
   const CUtensorMap ta = make_tmap_2d(a, K, M, lda, 64, kGemmBM);

@@ -16,7 +16,7 @@
 
 #include "../common/tensormap.h"
 #include "../launchers.h"
-#include "gemm_tcgen05.cuh"
+#include "gemm_pair.cuh"
 
 namespace agrpo {
 
@@ -107,15 +107,13 @@ struct LmDlogitsEpilogue {
       d[i] = gs * (((col0 + i == label) ? 1.f : 0.f) - p);
     }
     __nv_bfloat16* dst = dz + (long long)row * ld + col0;
-    if (col0 + 32 <= N && ((reinterpret_cast<uintptr_t>(dst) & 15) == 0)) {
+    if (col0 + 32 <= N && ((reinterpret_cast<uintptr_t>(dst) & 31) == 0)) {
 #pragma unroll
-      for (int i = 0; i < 32; i += 8) {
-        uint4 o;
-        o.x = pack_bf16x2(d[i], d[i + 1]);
-        o.y = pack_bf16x2(d[i + 2], d[i + 3]);
-        o.z = pack_bf16x2(d[i + 4], d[i + 5]);
-        o.w = pack_bf16x2(d[i + 6], d[i + 7]);
-        *reinterpret_cast<uint4*>(dst + i) = o;
+      for (int i = 0; i < 32; i += 16) {
+        uint32_t o[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) o[j] = pack_bf16x2(d[i + 2 * j], d[i + 2 * j + 1]);
+        st_global_32b(dst + i, o);
       }
     } else {
       for (int i = 0; i < 32; ++i)
@@ -258,7 +256,8 @@ void launch_lmhead_logprob(const void* hidden, long long ldh, const void* weight
   const int tiles_n = (V + kLmBN - 1) / kLmBN;
   const int groups = (tiles_n + group_n - 1) / group_n;
   const CUtensorMap ta = make_tmap_2d(hidden, H, T, ldh, 64, kGemmBM);
-  const CUtensorMap tb = make_tmap_2d(weight, H, V, ldw, 64, kLmBN);
+  const bool pair = pair_serves(T, num_sms);
+  const CUtensorMap tb = make_tmap_2d(weight, H, V, ldw, 64, pair ? kLmBN / 2 : kLmBN);
   GemmShape p;
   p.M = T; p.N = V; p.K = H;
   p.group_n = group_n;
@@ -271,7 +270,8 @@ void launch_lmhead_logprob(const void* hidden, long long ldh, const void* weight
   e.part_sz = partials + 2 * (size_t)groups * T;
   e.label_logit = label_logit;
   e.m = 0.f; e.s = 0.f; e.sz = 0.f; e.label = -1;
-  gemm_launch<kLmBN, false, false>(ta, tb, p, e, num_sms, stream);
+  if (pair) gemm_pair_launch<kLmBN, false, false, 4>(ta, tb, p, e, num_sms, stream);
+  else gemm_launch<kLmBN, false, false>(ta, tb, p, e, num_sms, stream);
   lmhead_combine_kernel<<<(T + 255) / 256, 256, 0, stream>>>(e.part_m, e.part_s, e.part_sz, label_logit, labels, groups, T,
                                                             logp, entropy, lse);
   check_cuda(cudaGetLastError(), "lmhead_combine");
@@ -302,7 +302,8 @@ void launch_lmhead_backward(const void* hidden, long long ldh, const void* weigh
     const __nv_bfloat16* wc = reinterpret_cast<const __nv_bfloat16*>(weight) + (long long)v0 * ldw;
     // 1. dlogits chunk [T, vc] (recompute logits tile on tcgen05, transform in the epilogue)
     {
-      const CUtensorMap tb = make_tmap_2d(wc, H, vc, ldw, 64, kLmBN);
+      const bool pair = pair_serves(T, num_sms);
+      const CUtensorMap tb = make_tmap_2d(wc, H, vc, ldw, 64, pair ? kLmBN / 2 : kLmBN);
       GemmShape p;
       p.M = T; p.N = vc; p.K = H;
       p.group_n = 1;
@@ -316,7 +317,8 @@ void launch_lmhead_backward(const void* hidden, long long ldh, const void* weigh
       e.dz = reinterpret_cast<__nv_bfloat16*>(dz_chunk);
       e.ld = chunk_cols;
       e.lse_r = 0.f; e.g_r = 0.f; e.label = -1;
-      gemm_launch<kLmBN, false, false>(ta, tb, p, e, num_sms, stream);
+      if (pair) gemm_pair_launch<kLmBN, false, false>(ta, tb, p, e, num_sms, stream);
+      else gemm_launch<kLmBN, false, false>(ta, tb, p, e, num_sms, stream);
     }
     // 2. dH += dZ . W_chunk        (A = dZ [T, vc] K-major, B = W_chunk as [N = H, K = vc], MN-major)
     launch_gemm_bf16(dz_chunk, chunk_cols, wc, ldw, dh_acc, H, T, H, vc, false, true, nullptr, 1.f, true, ci > 0, status,

@@ -126,6 +126,10 @@ void launch_scatter_add_f32(float* src, long long n, long long unit_rel, const S
 // The gather alone, for a unit with no GEMM to ride on.
 bool launch_unit_gather(const GatherArgs& g, int n_ctas, int* status, cudaStream_t stream);
 
+// The same for training and prompts: act[M, F] = silu(g) * u from bf16-rounded projections, which gu (optional, [M, 2F])
+// receives. Returns false (nothing launched) for shapes it does not serve: a plain product and swiglu_fwd give the same bits.
+bool launch_gemm_mlp_in(const void* a, long long lda, const void* b, long long ldb, void* act, long long ldact, void* gu, long long ldgu,
+                        int M, int F, int K, int* status, int num_sms, cudaStream_t stream);
 // Fused gate/up projection + SwiGLU (+ folded RMSNorm row scale, ss_in = row sums of squares of a, may be nullptr):
 // b is the stacked [2F, K] weight, d the [M, F] activation.
 bool launch_gemm_swiglu_bf16(const void* a, long long lda, const void* b, long long ldb, void* d, long long ldd, int M, int F,

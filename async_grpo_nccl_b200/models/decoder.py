@@ -179,6 +179,22 @@ class NativeDecoder:
             self.C.gemm_bf16(dy, x, sink.view(name), True, True, None, 1.0, True, self.status, None)
         self.launches += 1
 
+    def _mlp_in(self, h: torch.Tensor, w: torch.Tensor, keep: bool) -> Tuple[Optional[torch.Tensor], torch.Tensor]:
+        """(gate / up projections if they are to be kept for the backward pass, SwiGLU activation): one launch, or the plain
+        GEMM (which carries the prefetch of sharded weights) and the elementwise kernel, with the same bits."""
+        T, F = h.shape[0], self.cfg.intermediate_size
+        act = self._new(T, F)
+        gu = self._new(T, 2 * F) if keep else None
+        if self.weights is None and self.C.gemm_mlp_in(h, w, act, gu, self.status):
+            self.launches += 1
+            return gu, act
+        if gu is None:
+            gu = self._new(T, 2 * F)
+        self._gemm(h, w, gu)
+        self.C.swiglu_fwd(gu, act)
+        self.launches += 1
+        return gu, act
+
     def _new(self, *shape, dtype=torch.bfloat16):
         return torch.empty(shape, dtype=dtype, device=self.dev)
 
@@ -210,13 +226,10 @@ class NativeDecoder:
         h2 = self._new(T, cfg.hidden_size)
         rstd2 = self._new(T, dtype=torch.float32)
         C.rmsnorm_fwd(x1, self.w(p + "ln2"), h2, rstd2, cfg.rms_norm_eps)
-        gu = self._new(T, 2 * cfg.intermediate_size)
-        self._gemm(h2, self.w(p + "wgu"), gu)
-        act = self._new(T, cfg.intermediate_size)
-        C.swiglu_fwd(gu, act)
+        gu, act = self._mlp_in(h2, self.w(p + "wgu"), save is not None)
         x2 = self._new(T, cfg.hidden_size)
         self._gemm(act, self.w(p + "wd"), x2, residual=x1)
-        self.launches += 6
+        self.launches += 5
         if save is not None:
             save.update(x=x, h1=h1, rstd1=rstd1, qkv=qkv, attn=attn, lse=lse, x1=x1, h2=h2, rstd2=rstd2, gu=gu, act=act)
         return x2
@@ -253,13 +266,10 @@ class NativeDecoder:
         self._gemm(attn_s, self.w(p + "wo"), x1, residual=x)
         h2 = self._new(Ts, cfg.hidden_size)
         C.rmsnorm_fwd(x1, self.w(p + "ln2"), h2, None, cfg.rms_norm_eps)
-        gu = self._new(Ts, 2 * cfg.intermediate_size)
-        self._gemm(h2, self.w(p + "wgu"), gu)
-        act = self._new(Ts, cfg.intermediate_size)
-        C.swiglu_fwd(gu, act)
+        _, act = self._mlp_in(h2, self.w(p + "wgu"), False)
         x2 = self._new(Ts, cfg.hidden_size)
         self._gemm(act, self.w(p + "wd"), x2, residual=x1)
-        self.launches += 12
+        self.launches += 11
         return x2
 
     def _layer_bwd(self, i: int, dx: torch.Tensor, s: dict, batch: PackedBatch, cos_t, sin_t, sink: GradSink):
