@@ -221,21 +221,35 @@ struct LmSampleEpilogue {
       s *= (m == -INFINITY) ? 0.f : __expf(m - cm);
       m = cm;
     }
+    // The 32 perturbed values first, without a branch between them: with the greedy test and the running maximum inside one loop
+    // every column waited for the one before: 16 rows x 151936 columns took 176 us, now 100 (the weights alone need 71).
+    float v[32];
+    if (greedy) {
+      // the cap is monotonic: the best raw logit is the best capped one, without the ties that saturation rounds to
+#pragma unroll
+      for (int i = 0; i < 32; ++i) v[i] = col0 + i < N ? __uint_as_float(r[i]) : z[i];
+    } else {
+#pragma unroll
+      for (int i = 0; i < 32; ++i) {
+        const uint32_t h = hash_u32(hash_u32((uint32_t)(col0 + i) ^ seed_lo) + seed_hi);
+        const float u = ((float)(h >> 8) + 0.5f) * (1.0f / 16777216.0f);  // (0, 1)
+        v[i] = z[i] - __logf(-__logf(u));
+      }
+    }
+    float top = -INFINITY;
 #pragma unroll
     for (int i = 0; i < 32; ++i) {
       s += __expf(z[i] - m);
-      // the cap is monotonic: the best raw logit is the best capped one, without the ties that saturation rounds to
-      float v = greedy && col0 + i < N ? __uint_as_float(r[i]) : z[i];
-      if (!greedy) {
-        const uint32_t h = hash_u32(hash_u32((uint32_t)(col0 + i) ^ seed_lo) + seed_hi);
-        const float u = ((float)(h >> 8) + 0.5f) * (1.0f / 16777216.0f);  // (0, 1)
-        v += -__logf(-__logf(u));
-      }
-      if (v > best) {
-        best = v;
-        best_z = z[i];
-        best_idx = col0 + i;
-      }
+      top = fmaxf(top, v[i]);
+    }
+    if (top > best) {
+      best = top;
+#pragma unroll
+      for (int i = 31; i >= 0; --i)  // the first column that holds the maximum
+        if (v[i] == top) {
+          best_z = z[i];
+          best_idx = col0 + i;
+        }
     }
   }
   __device__ __forceinline__ void item_end(int row, int M, int, int group) {
