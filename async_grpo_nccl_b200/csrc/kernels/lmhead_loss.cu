@@ -14,6 +14,8 @@
 //             dH and dW tcgen05 GEMMs.
 #include <cuda_bf16.h>
 
+#include <algorithm>
+
 #include "../common/tensormap.h"
 #include "../launchers.h"
 #include "gemm_pair.cuh"
@@ -297,8 +299,11 @@ void launch_lmhead_backward(const void* hidden, long long ldh, const void* weigh
                             cudaStream_t stream) {
   if (T == 0) return;
   const CUtensorMap ta = make_tmap_2d(hidden, H, T, ldh, 64, kGemmBM);
-  for (int v0 = 0, ci = 0; v0 < V; v0 += chunk_cols, ++ci) {
-    const int vc = (V - v0) < chunk_cols ? (V - v0) : chunk_cols;
+  // Equal chunks, as few as the buffer allows: a short last one would pay for a whole pass over dH.
+  const int chunks = (V + chunk_cols - 1) / chunk_cols;
+  const int step = std::min(chunk_cols, ((V + chunks - 1) / chunks + 255) / 256 * 256);
+  for (int v0 = 0, ci = 0; v0 < V; v0 += step, ++ci) {
+    const int vc = (V - v0) < step ? (V - v0) : step;
     const __nv_bfloat16* wc = reinterpret_cast<const __nv_bfloat16*>(weight) + (long long)v0 * ldw;
     // 1. dlogits chunk [T, vc] (recompute logits tile on tcgen05, transform in the epilogue)
     {

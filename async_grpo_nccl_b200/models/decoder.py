@@ -356,6 +356,13 @@ class NativeDecoder:
         self.launches += 2
         return logp, ent
 
+    def _vocab_chunk(self, T: int) -> int:
+        """Columns of the dlogits buffer. A wide chunk reads and writes the fp32 dH sum seldom and fills the pairs' waves; at most
+        1 GiB is spent on it unless ``lmhead_chunk`` asks for more."""
+        if self.lmhead_chunk < 4096:
+            return self.lmhead_chunk
+        return max(self.lmhead_chunk, min(15360, (1 << 29) // max(T, 1) // 256 * 256))
+
     def forward_backward(self, batch: PackedBatch, lc: LossConfig, loss_scale: float, sink: GradSink) -> torch.Tensor:
         """One microbatch: forward, fused loss, full backward into ``sink``. Returns the device stats vector
         (sums over valid tokens, see ops.reference.LOSS_STAT_NAMES). The scalar loss is
@@ -382,7 +389,7 @@ class NativeDecoder:
         ref = batch.ref_logprobs if (lc.kl_beta > 0 and batch.has_ref) else None
         C.grpo_token_loss(logp, batch.old_logprobs, ref, batch.advantages, batch.labels, ent, batch.old_entropies,
                           lc.clip_low, lc.clip_high, lc.clip_ratio_c, lc.kl_beta, loss_scale / n_valid, dlogp, stats)
-        chunk = min(self.lmhead_chunk, (V + 255) // 256 * 256)
+        chunk = min(self._vocab_chunk(T), (V + 255) // 256 * 256)
         dz = self._new(T, chunk)
         dh_acc = self._new(T, cfg.hidden_size, dtype=torch.float32)
         C.lmhead_backward(hn, wl, batch.labels, lse, dlogp, lc.temperature, dz, dh_acc, sink.view(wl_name), self.status)
