@@ -54,6 +54,23 @@ inline T* opt_ptr(const OptTensor& t) {
   return (t.has_value() && t->defined()) ? reinterpret_cast<T*>(t->data_ptr()) : nullptr;
 }
 
+// Rotary tables of a kernel that rotates on the way; off without `pos`.
+inline agrpo::AttnRope rope_args(const OptTensor& pos, const OptTensor& cos_t, const OptTensor& sin_t, int64_t T, int64_t D) {
+  agrpo::AttnRope r;
+  if (!pos.has_value() || !pos->defined()) return r;
+  TORCH_CHECK(cos_t.has_value() && sin_t.has_value(), "rope: tables");
+  check_i32(*pos, "rope pos"); check_f32(*cos_t, "rope cos"); check_f32(*sin_t, "rope sin");
+  TORCH_CHECK(pos->numel() == T && pos->is_contiguous() && cos_t->dim() == 2 && cos_t->size(1) == D / 2 && cos_t->size(0) > 0 &&
+              cos_t->is_contiguous() && sin_t->is_contiguous() && sin_t->sizes() == cos_t->sizes() &&
+              (reinterpret_cast<uintptr_t>(cos_t->data_ptr()) & 15) == 0 && (reinterpret_cast<uintptr_t>(sin_t->data_ptr()) & 15) == 0,
+              "rope: pos [T], tables [max_pos, D / 2]");
+  r.pos = pos->data_ptr<int>();
+  r.cos_t = cos_t->data_ptr<float>();
+  r.sin_t = sin_t->data_ptr<float>();
+  r.max_pos = (int)cos_t->size(0);
+  return r;
+}
+
 void gemm_bf16(const Tensor& a, const Tensor& b, Tensor& d, bool a_mn, bool b_mn, const OptTensor& bias, double alpha,
                bool accumulate, const OptTensor& status, const OptTensor& residual) {
   check_bf16(a, "gemm a");
@@ -158,6 +175,26 @@ void gemm_swiglu(const Tensor& a, const Tensor& b, Tensor& d, const OptTensor& s
                                              (int)F, (int)K, opt_i64(ss_in), (float)eps, opt_ptr<int>(status), num_sms(),
                                              cur_stream()),
               "gemm_swiglu: arguments not served");
+}
+bool gemm_qkv_rope(const Tensor& a, const Tensor& b, Tensor& qkv, const OptTensor& bias, const Tensor& pos, const Tensor& cos_t,
+                   const Tensor& sin_t, int64_t rot_heads, int64_t head_dim, const OptTensor& status) {
+  check_bf16(a, "gemm_qkv_rope a"); check_bf16(b, "gemm_qkv_rope b"); check_bf16(qkv, "gemm_qkv_rope qkv");
+  TORCH_CHECK(a.dim() == 2 && b.dim() == 2 && qkv.dim() == 2 && a.stride(1) == 1 && b.stride(1) == 1 && qkv.stride(1) == 1, "gemm_qkv_rope: 2-D");
+  const int64_t M = a.size(0), K = a.size(1), N = b.size(0);
+  TORCH_CHECK(b.size(1) == K && qkv.size(0) == M && qkv.size(1) == N && rot_heads * head_dim <= N, "gemm_qkv_rope: shapes");
+  TORCH_CHECK(a.stride(0) % 8 == 0 && b.stride(0) % 8 == 0 && (reinterpret_cast<uintptr_t>(a.data_ptr()) & 15) == 0 &&
+              (reinterpret_cast<uintptr_t>(b.data_ptr()) & 15) == 0, "gemm_qkv_rope: operand rows must be 16-byte aligned");
+  if (bias.has_value() && bias->defined()) {
+    check_bf16(*bias, "gemm_qkv_rope bias");
+    TORCH_CHECK(bias->numel() == N && bias->is_contiguous(), "gemm_qkv_rope: bias [N]");
+  }
+  if (status.has_value() && status->defined()) check_i32(*status, "gemm_qkv_rope status");
+  if (M == 0) return true;
+  const agrpo::AttnRope rope = rope_args(pos, cos_t, sin_t, M, head_dim);
+  const c10::cuda::CUDAGuard guard(a.device());
+  return agrpo::launch_gemm_qkv_rope(a.data_ptr(), a.stride(0), b.data_ptr(), b.stride(0), qkv.data_ptr(), qkv.stride(0), (int)M, (int)N,
+                                     (int)K, opt_ptr<void>(bias), rope, (int)rot_heads, (int)head_dim, opt_ptr<int>(status), num_sms(),
+                                     cur_stream());
 }
 bool gemm_mlp_in(const Tensor& a, const Tensor& b, Tensor& act, const OptTensor& gu, const OptTensor& status) {
   check_bf16(a, "gemm_mlp_in a"); check_bf16(b, "gemm_mlp_in b"); check_bf16(act, "gemm_mlp_in act");
@@ -286,7 +323,7 @@ void attn_varlen_fwd(const Tensor& qkv, Tensor& out, const OptTensor& lse, const
 // dqkv: [T, (Hq + 2*Hkv) * D] receives dq | dk | dv. delta [Hq, T] and dq_acc [T, Hq*D] are fp32 scratch.
 void attn_varlen_bwd(const Tensor& qkv, const Tensor& out, const Tensor& dout, const Tensor& lse, Tensor& delta,
                      Tensor& dq_acc, Tensor& dqkv, const Tensor& tiles, int64_t Hq, int64_t Hkv, int64_t D,
-                     double softmax_scale, const OptTensor& status) {
+                     double softmax_scale, const OptTensor& status, const OptTensor& pos, const OptTensor& cos_t, const OptTensor& sin_t) {
   check_bf16(qkv, "qkv"); check_bf16(out, "out"); check_bf16(dout, "dout"); check_bf16(dqkv, "dqkv");
   check_f32(lse, "lse"); check_f32(delta, "delta"); check_f32(dq_acc, "dq_acc"); check_i32(tiles, "tiles");
   const int64_t T = qkv.size(0), C = (Hq + 2 * Hkv) * D;
@@ -299,6 +336,7 @@ void attn_varlen_bwd(const Tensor& qkv, const Tensor& out, const Tensor& dout, c
   TORCH_CHECK(tiles.is_contiguous() && tiles.dim() == 2 && tiles.size(1) == 4, "attn_bwd: tiles [n,4]");
   TORCH_CHECK((reinterpret_cast<uintptr_t>(tiles.data_ptr()) & 15) == 0, "attn_bwd: tile table must be 16-byte aligned");
   TORCH_CHECK(qkv.stride(0) % 8 == 0 && dout.stride(0) % 8 == 0 && dqkv.stride(0) % 8 == 0, "attn_bwd: pitches");
+  const agrpo::AttnRope rope = rope_args(pos, cos_t, sin_t, T, D);
   const c10::cuda::CUDAGuard guard(qkv.device());
   agrpo::launch_attn_varlen_bwd(qkv.data_ptr(), qkv.stride(0), (int)C, qkv.data_ptr(), qkv.stride(0), (int)C, qkv.data_ptr(),
                                 qkv.stride(0), (int)C, 0, (int)(Hq * D), (int)((Hq + Hkv) * D), out.data_ptr(), out.stride(0),
@@ -306,7 +344,7 @@ void attn_varlen_bwd(const Tensor& qkv, const Tensor& out, const Tensor& dout, c
                                 dq_acc.data_ptr<float>(), dqkv.data_ptr(), dqkv.stride(0), dqkv.data_ptr(), dqkv.stride(0),
                                 (int)(Hq * D), dqkv.data_ptr(), dqkv.stride(0), (int)((Hq + Hkv) * D), tiles.data_ptr<int>(),
                                 (int)tiles.size(0), (int)T, (int)Hq, (int)Hkv, (int)D, (float)softmax_scale,
-                                opt_ptr<int>(status), cur_stream());
+                                opt_ptr<int>(status), cur_stream(), rope);
 }
 
 int64_t lmhead_num_groups(int64_t V, int64_t T) { return agrpo::lmhead_num_groups((int)V, (int)T); }
@@ -930,6 +968,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("decode_layers_counter_words", &decode_layers_counter_words);
   m.def("gemm_swiglu", &gemm_swiglu, py::arg("a"), py::arg("b"), py::arg("d"), py::arg("ss_in") = py::none(), py::arg("eps") = 1e-6,
         py::arg("status") = py::none(), NOGIL);
+  m.def("gemm_qkv_rope", &gemm_qkv_rope, py::arg("a"), py::arg("b"), py::arg("qkv"), py::arg("bias"), py::arg("pos"), py::arg("cos_t"),
+        py::arg("sin_t"), py::arg("rot_heads"), py::arg("head_dim"), py::arg("status") = py::none(), NOGIL);
   m.def("gemm_mlp_in", &gemm_mlp_in, py::arg("a"), py::arg("b"), py::arg("act"), py::arg("gu") = py::none(), py::arg("status") = py::none(), NOGIL);
   m.def("rmsnorm_fwd", &rmsnorm_fwd, py::arg("x"), py::arg("w"), py::arg("y"), py::arg("rstd") = py::none(),
         py::arg("eps") = 1e-6, NOGIL);
@@ -944,7 +984,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         py::arg("Hq"), py::arg("Hkv"), py::arg("D"), py::arg("softmax_scale"), py::arg("status") = py::none(), NOGIL);
   m.def("attn_varlen_bwd", &attn_varlen_bwd, py::arg("qkv"), py::arg("out"), py::arg("dout"), py::arg("lse"),
         py::arg("delta"), py::arg("dq_acc"), py::arg("dqkv"), py::arg("tiles"), py::arg("Hq"), py::arg("Hkv"), py::arg("D"),
-        py::arg("softmax_scale"), py::arg("status") = py::none(), NOGIL);
+        py::arg("softmax_scale"), py::arg("status") = py::none(), py::arg("pos") = py::none(), py::arg("cos_t") = py::none(),
+        py::arg("sin_t") = py::none(), NOGIL);
   m.def("lmhead_num_groups", &lmhead_num_groups);
   m.def("grpo_num_loss_stats", &grpo_num_loss_stats);
   m.def("lmhead_logprob", &lmhead_logprob, py::arg("hidden"), py::arg("weight"), py::arg("labels"), py::arg("temperature"),

@@ -10,19 +10,26 @@
 //   dV  += P^T dO         dK  += dS^T Q                 (A operand read back from tensor memory)
 //   dQ   = dS K                                         (dS^T staged in shared memory, MN-major)
 // dK / dV leave as bf16 once per CTA; dQ partial tiles are added to an fp32 accumulator with vector
-// reductions and converted by attn_bwd_finalize_dq.
+// reductions and converted by attn_bwd_finalize_dq. Where rotary embedding came before the attention,
+// both take its transpose along on the way out.
+//
+// A step is a chain (S and dP, then the softmax gradient, then three products, then the read-out of dQ), and the
+// 512 columns leave no room for a second tile, so its length is what counts: eight warps share the
+// elementwise part, two per lane quarter with 64 queries each. P^T and dS^T of a warp stay inside the
+// columns that it read S^T and dP^T from (queries 64.. at column 64), so the two need not wait for each other.
 #include <cuda_bf16.h>
 
 #include "../common/ptx.cuh"
 #include "../common/tensormap.h"
 #include "../launchers.h"
+#include "rope.cuh"
 
 namespace agrpo {
 
 namespace {
 
 constexpr int kT = 128;  // tile edge (keys per CTA, queries per step)
-constexpr int kBwdThreads = 192;
+constexpr int kBwdThreads = 320;
 
 struct AttnBwdParams {
   const int4* tiles;  // {seq_start, seq_len, k0, unused}
@@ -36,6 +43,7 @@ struct AttnBwdParams {
   int T, Hq, group;
   int q_col0, k_col0, v_col0;
   float scale, scale_log2;
+  AttnRope rope;      // transposed rotation of dK, off when pos == nullptr
   int* status;
 };
 
@@ -97,10 +105,10 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     mbar_init(&q_empty[1], 1);
     mbar_init(do_full, 1);
     mbar_init(sdp_full, 1);
-    mbar_init(pds_ready, 4);
+    mbar_init(pds_ready, 8);
     mbar_init(dv_done, 1);
     mbar_init(dq_full, 1);
-    mbar_init(dq_read, 4);
+    mbar_init(dq_read, 8);
     fence_mbar_init();
   }
   if (warp == 1) {
@@ -184,13 +192,13 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         // dV += P^T dO   (A: P^T packed bf16 in R1, B: dO as [N = D, K = queries], MN-major)
 #pragma unroll
         for (int k = 0; k < kT / 16; ++k)
-          tc_mma_f16_ts(tmem_dV, tmem_R1 + k * 8, umma_smem_desc(aDO + k * 2048, kChunkBytes, 1024), kIdescKV,
+          tc_mma_f16_ts(tmem_dV, tmem_R1 + (k & 3) * 8 + (k >> 2) * 64, umma_smem_desc(aDO + k * 2048, kChunkBytes, 1024), kIdescKV,
                         (it > 0 || k > 0) ? 1u : 0u);
         tc_commit(dv_done);
         // dK += dS^T Q
 #pragma unroll
         for (int k = 0; k < kT / 16; ++k)
-          tc_mma_f16_ts(tmem_dK, tmem_R2 + k * 8, umma_smem_desc(aQ + k * 2048, kChunkBytes, 1024), kIdescKV,
+          tc_mma_f16_ts(tmem_dK, tmem_R2 + (k & 3) * 8 + (k >> 2) * 64, umma_smem_desc(aQ + k * 2048, kChunkBytes, 1024), kIdescKV,
                         (it > 0 || k > 0) ? 1u : 0u);
         tc_commit(&q_empty[s]);
         // dQ = dS K      (A: dS^T tile in shared memory read MN-major, B: K as [N = D, K = keys], MN-major)
@@ -202,8 +210,10 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       }
     }
   } else {
-    // Compute warps: thread = one key row (P^T / dS^T) and, for the dQ read-out, one query row.
+    // Compute warps: thread = one key row and half of the queries (P^T / dS^T); for the dQ read-out, one query row and half
+    // of its columns.
     const int quarter = warp & 3;
+    const int part = (warp - 2) >> 2;
     const int r = quarter * 32 + lane;
     const int kj = k0 + r;
     const uint32_t lane_off = static_cast<uint32_t>(quarter * 32) << 16;
@@ -217,10 +227,10 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         const int qi = q0 + r;
         const bool valid = qi < seq_len;
         const long long idx = (long long)head * p.T + seq_start + qi;
-        sLse[b * kT + r] = valid ? p.lse[idx] * 1.4426950408889634f : INFINITY;
-        sDelta[b * kT + r] = valid ? p.delta[idx] : 0.f;
+        if (part == 0) sLse[b * kT + r] = valid ? p.lse[idx] * 1.4426950408889634f : INFINITY;
+        else sDelta[b * kT + r] = valid ? p.delta[idx] : 0.f;
       }
-      named_bar_sync(1, 128);
+      named_bar_sync(1, 256);
       if (!mbar_wait(sdp_full, it & 1)) {
         report_status(p.status, kStatusWaitTmemFullTimeout);
         ok = false;
@@ -229,7 +239,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       tc_fence_after();
       const bool diag = (qt == 0);
 #pragma unroll 1
-      for (int c = 0; c < kT / 32; ++c) {
+      for (int c = part * 2; c < part * 2 + 2; ++c) {
         uint32_t sv[32], dp[32];
         tmem_ld_32x32(tmem_R1 + lane_off + c * 32, sv);
         tmem_ld_32x32(tmem_R2 + lane_off + c * 32, dp);
@@ -251,8 +261,9 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           pk[i / 2] = pack_bf16x2(p0, p1);
           dsk[i / 2] = pack_bf16x2(d0, d1);
         }
-        tmem_st_32x16(tmem_R1 + lane_off + c * 16, pk);
-        tmem_st_32x16(tmem_R2 + lane_off + c * 16, dsk);
+        const uint32_t pcol = lane_off + part * 64 + (c & 1) * 16;
+        tmem_st_32x16(tmem_R1 + pcol, pk);
+        tmem_st_32x16(tmem_R2 + pcol, dsk);
         // dS^T row r, queries [32c, 32c+32) into the 128-byte-swizzled [keys x queries] tile.
         uint8_t* rowp = sDS + (c >> 1) * kChunkBytes + r * 128;
 #pragma unroll
@@ -278,7 +289,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         const bool valid = qi < seq_len;
         float* dst = p.dq_acc + ((long long)seq_start + qi) * ((long long)p.Hq * D) + (long long)head * D;
 #pragma unroll 1
-        for (int c = 0; c < D / 32; ++c) {
+        for (int c = part * (D / 64); c < (part + 1) * (D / 64); ++c) {
           uint32_t o[32];
           tmem_ld_32x32(tmem_R1 + lane_off + c * 32, o);
           tc_wait_ld();
@@ -298,26 +309,40 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       // The last dq_full wait also covered the final dV / dK MMAs (commits are cumulative).
       const bool valid = kj < seq_len;
       const long long t = (long long)seq_start + kj;
-      __nv_bfloat16* dvp = p.dv + t * p.ld_dv + p.dv_col0 + (long long)kv_head * D;
-      __nv_bfloat16* dkp = p.dk + t * p.ld_dk + p.dk_col0 + (long long)kv_head * D;
+      // the warps of part 0 write dV, those of part 1 dK, whose columns i and D / 2 + i rotate together
+      const auto store32 = [](__nv_bfloat16* dst, const float (&v)[32]) {
+#pragma unroll
+        for (int i = 0; i < 32; i += 8) {
+          uint4 w;
+          w.x = pack_bf16x2(v[i], v[i + 1]);
+          w.y = pack_bf16x2(v[i + 2], v[i + 3]);
+          w.z = pack_bf16x2(v[i + 4], v[i + 5]);
+          w.w = pack_bf16x2(v[i + 6], v[i + 7]);
+          *reinterpret_cast<uint4*>(dst + i) = w;
+        }
+      };
+      __nv_bfloat16* out = part == 0 ? p.dv + t * p.ld_dv + p.dv_col0 + (long long)kv_head * D : p.dk + t * p.ld_dk + p.dk_col0 + (long long)kv_head * D;
+      const uint32_t acc = (part == 0 ? tmem_dV : tmem_dK) + lane_off;
 #pragma unroll 1
-      for (int c = 0; c < 2 * D / 32; ++c) {
-        const bool is_k = c >= D / 32;
-        const int cc = is_k ? c - D / 32 : c;
-        uint32_t o[32];
-        tmem_ld_32x32((is_k ? tmem_dK : tmem_dV) + lane_off + cc * 32, o);
+      for (int c = 0; c < D / 64; ++c) {
+        uint32_t lo[32], hi[32];
+        tmem_ld_32x32(acc + c * 32, lo);
+        tmem_ld_32x32(acc + D / 2 + c * 32, hi);
         tc_wait_ld();
         if (valid) {
-          __nv_bfloat16* dst = (is_k ? dkp : dvp) + cc * 32;
+          float x1[32], x2[32];
 #pragma unroll
-          for (int i = 0; i < 32; i += 8) {
-            uint4 w;
-            w.x = pack_bf16x2(__uint_as_float(o[i]), __uint_as_float(o[i + 1]));
-            w.y = pack_bf16x2(__uint_as_float(o[i + 2]), __uint_as_float(o[i + 3]));
-            w.z = pack_bf16x2(__uint_as_float(o[i + 4]), __uint_as_float(o[i + 5]));
-            w.w = pack_bf16x2(__uint_as_float(o[i + 6]), __uint_as_float(o[i + 7]));
-            *reinterpret_cast<uint4*>(dst + i) = w;
+          for (int i = 0; i < 32; ++i) {
+            x1[i] = __uint_as_float(lo[i]);
+            x2[i] = __uint_as_float(hi[i]);
           }
+          if (part == 1 && p.rope.pos != nullptr) {
+            const long long row = p.rope.row(t) * (D / 2) + c * 32;
+#pragma unroll
+            for (int i = 0; i < 32; ++i) rope_rotate(x1[i], x2[i], p.rope.cos_t[row + i], -p.rope.sin_t[row + i]);
+          }
+          store32(out + c * 32, x1);
+          store32(out + D / 2 + c * 32, x2);
         }
       }
     }
@@ -351,18 +376,30 @@ __global__ void attn_bwd_delta_kernel(const __nv_bfloat16* __restrict__ o, const
   if (lane == 0) delta[(long long)h * T + t] = acc;
 }
 
-// dq (bf16, pitch ld, first `cols` columns of each row) = dq_acc (fp32 [T, cols]).
-__global__ void attn_bwd_finalize_dq_kernel(const float* __restrict__ acc, __nv_bfloat16* __restrict__ dq, long long T,
-                                            int cols, long long ld) {
-  const long long total = T * (cols / 4);
+// dq (bf16, pitch ld, first Hq * D columns of each row) = dq_acc (fp32 [T, Hq * D]), rotated back where `rope` says so: a thread
+// converts four columns of each half of a head.
+__global__ void attn_bwd_finalize_dq_kernel(const float* __restrict__ acc, __nv_bfloat16* __restrict__ dq, long long T, int Hq, int D,
+                                            long long ld, const AttnRope rope) {
+  const int per_head = D / 8;
+  const long long total = T * Hq * per_head;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-    const long long t = i / (cols / 4);
-    const int c = (int)(i % (cols / 4)) * 4;
-    const float4 v = *reinterpret_cast<const float4*>(acc + t * cols + c);
-    uint2 w;
-    w.x = pack_bf16x2(v.x, v.y);
-    w.y = pack_bf16x2(v.z, v.w);
-    *reinterpret_cast<uint2*>(dq + t * ld + c) = w;
+    const int j = (int)(i % per_head) * 4;
+    const long long th = i / per_head;
+    const long long t = th / Hq;
+    const int col = (int)(th % Hq) * D + j;
+    float4 a = __ldcs(reinterpret_cast<const float4*>(acc + t * Hq * D + col));
+    float4 b = __ldcs(reinterpret_cast<const float4*>(acc + t * Hq * D + col + D / 2));
+    if (rope.pos != nullptr) {
+      const long long row = rope.row(t) * (D / 2) + j;
+      const float4 c = *reinterpret_cast<const float4*>(rope.cos_t + row), s = *reinterpret_cast<const float4*>(rope.sin_t + row);
+      rope_rotate(a.x, b.x, c.x, -s.x);
+      rope_rotate(a.y, b.y, c.y, -s.y);
+      rope_rotate(a.z, b.z, c.z, -s.z);
+      rope_rotate(a.w, b.w, c.w, -s.w);
+    }
+    __nv_bfloat16* d = dq + t * ld + col;
+    *reinterpret_cast<uint2*>(d) = make_uint2(pack_bf16x2(a.x, a.y), pack_bf16x2(a.z, a.w));
+    *reinterpret_cast<uint2*>(d + D / 2) = make_uint2(pack_bf16x2(b.x, b.y), pack_bf16x2(b.z, b.w));
   }
 }
 
@@ -384,7 +421,7 @@ void launch_attn_varlen_bwd(const void* q, long long ldq, int q_cols, const void
                             long long ldo, const void* dout, long long lddo, const float* lse, float* delta, float* dq_acc,
                             void* dq, long long ld_dq, void* dk, long long ld_dk, int dk_col0, void* dv, long long ld_dv,
                             int dv_col0, const int* tiles, int n_tiles, int T, int Hq, int Hkv, int D, float softmax_scale,
-                            int* status, cudaStream_t s) {
+                            int* status, cudaStream_t s, const AttnRope& rope) {
   if (n_tiles == 0 || T == 0) return;
   if (D != 64 && D != 128) throw std::runtime_error("attn_varlen_bwd: head_dim must be 64 or 128");
   {
@@ -417,14 +454,15 @@ void launch_attn_varlen_bwd(const void* q, long long ldq, int q_cols, const void
   p.v_col0 = v_col0;
   p.scale = softmax_scale;
   p.scale_log2 = softmax_scale * 1.4426950408889634f;
+  p.rope = rope;
   p.status = status;
   if (D == 128) launch_bwd_t<128>(tq, tk, tv, tdo, p, n_tiles, Hkv, s);
   else          launch_bwd_t<64>(tq, tk, tv, tdo, p, n_tiles, Hkv, s);
   {
-    const long long work = (long long)T * (Hq * D / 4);
+    const long long work = (long long)T * (Hq * D / 8);
     long long blocks = (work + 255) / 256;
     if (blocks > 148 * 16) blocks = 148 * 16;
-    attn_bwd_finalize_dq_kernel<<<(unsigned)blocks, 256, 0, s>>>(dq_acc, (__nv_bfloat16*)dq, T, Hq * D, ld_dq);
+    attn_bwd_finalize_dq_kernel<<<(unsigned)blocks, 256, 0, s>>>(dq_acc, (__nv_bfloat16*)dq, T, Hq, D, ld_dq, rope);
     check_cuda(cudaGetLastError(), "attn_bwd_finalize_dq");
   }
 }

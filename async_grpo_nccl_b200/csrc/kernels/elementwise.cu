@@ -6,6 +6,7 @@
 
 #include "../common/ptx.cuh"
 #include "../launchers.h"
+#include "rope.cuh"
 
 namespace agrpo {
 
@@ -238,26 +239,46 @@ __global__ void colsum_kernel(const __nv_bfloat16* __restrict__ a, const __nv_bf
 // RoPE (rotate-half convention) applied in place to the q and k heads of a fused qkv row.
 // cos/sin tables are fp32 [max_pos, D/2]. sign = +1 forward, -1 backward (transpose rotation).
 // ------------------------------------------------------------------------------------------------
+// A thread rotates V column pairs (V = 4: 8-byte accesses; 1 where pitch, head size or address do not allow that).
+template <int V>
 __global__ void rope_kernel(__nv_bfloat16* __restrict__ qkv, const int* __restrict__ pos,
                             const float* __restrict__ cos_t, const float* __restrict__ sin_t, int T, int n_rot_heads,
                             int D, long long row_pitch, int max_pos, float sign) {
-  const int half = D / 2;
-  const long long total = (long long)T * n_rot_heads * half;
+  const int half = D / 2, per_head = half / V;
+  const long long total = (long long)T * n_rot_heads * per_head;
   for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
        idx += (long long)gridDim.x * blockDim.x) {
-    const int i = (int)(idx % half);
-    const long long th = idx / half;
+    const int i = (int)(idx % per_head) * V;
+    const long long th = idx / per_head;
     const int h = (int)(th % n_rot_heads);
     const int t = (int)(th / n_rot_heads);
     int p = pos[t];
     p = p < 0 ? 0 : (p >= max_pos ? max_pos - 1 : p);
-    const float c = cos_t[(size_t)p * half + i];
-    const float s = sin_t[(size_t)p * half + i] * sign;
-    __nv_bfloat16* base = qkv + (size_t)t * row_pitch + (size_t)h * D;
-    const float x1 = __bfloat162float(base[i]);
-    const float x2 = __bfloat162float(base[i + half]);
-    base[i] = __float2bfloat16(x1 * c - x2 * s);
-    base[i + half] = __float2bfloat16(x2 * c + x1 * s);
+    const float* ct = cos_t + (size_t)p * half + i;
+    const float* st = sin_t + (size_t)p * half + i;
+    __nv_bfloat16* base = qkv + (size_t)t * row_pitch + (size_t)h * D + i;
+    __align__(8) __nv_bfloat16 x1[V], x2[V];
+    if constexpr (V == 4) {
+      *reinterpret_cast<uint2*>(x1) = *reinterpret_cast<const uint2*>(base);
+      *reinterpret_cast<uint2*>(x2) = *reinterpret_cast<const uint2*>(base + half);
+    } else {
+      x1[0] = base[0];
+      x2[0] = base[half];
+    }
+#pragma unroll
+    for (int j = 0; j < V; ++j) {
+      float a = __bfloat162float(x1[j]), b = __bfloat162float(x2[j]);
+      rope_rotate(a, b, ct[j], st[j] * sign);
+      x1[j] = __float2bfloat16(a);
+      x2[j] = __float2bfloat16(b);
+    }
+    if constexpr (V == 4) {
+      *reinterpret_cast<uint2*>(base) = *reinterpret_cast<const uint2*>(x1);
+      *reinterpret_cast<uint2*>(base + half) = *reinterpret_cast<const uint2*>(x2);
+    } else {
+      base[0] = x1[0];
+      base[half] = x2[0];
+    }
   }
 }
 
@@ -394,10 +415,13 @@ void launch_colsum(const void* a, float* out, int T, int C, long long lda, cudaS
 void launch_rope(void* qkv, const int* pos, const float* cos_t, const float* sin_t, int T, int n_rot_heads, int D,
                  long long row_pitch, int max_pos, bool backward, cudaStream_t s) {
   if (T == 0) return;
-  const long long work = (long long)T * n_rot_heads * (D / 2);
-  AGRPO_PREFER_SMEM(rope_kernel);
-  rope_kernel<<<grid_for(work, 256), 256, 0, s>>>((__nv_bfloat16*)qkv, pos, cos_t, sin_t, T, n_rot_heads, D, row_pitch,
-                                                  max_pos, backward ? -1.f : 1.f);
+  const bool vec = D % 8 == 0 && row_pitch % 4 == 0 && (reinterpret_cast<uintptr_t>(qkv) & 7) == 0;
+  const long long work = (long long)T * n_rot_heads * (D / 2) / (vec ? 4 : 1);
+  const auto kernel = vec ? rope_kernel<4> : rope_kernel<1>;
+  AGRPO_PREFER_SMEM(rope_kernel<4>);
+  AGRPO_PREFER_SMEM(rope_kernel<1>);
+  kernel<<<grid_for(work, 256), 256, 0, s>>>((__nv_bfloat16*)qkv, pos, cos_t, sin_t, T, n_rot_heads, D, row_pitch, max_pos,
+                                             backward ? -1.f : 1.f);
   check_cuda(cudaGetLastError(), "rope");
 }
 void launch_swiglu_fwd(const void* gu, void* out, int T, int F, cudaStream_t s) {

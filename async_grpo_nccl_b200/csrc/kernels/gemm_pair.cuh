@@ -11,6 +11,7 @@
 // rank 0 is arrived at by the epilogue warps of both. An epilogue functor sees rows and columns exactly as in the plain kernel.
 #pragma once
 #include "gemm_tcgen05.cuh"
+#include "rope.cuh"
 
 namespace agrpo {
 
@@ -154,6 +155,71 @@ struct PairSwigluEpilogue {
     }
   }
 };
+
+// qkv projection with bias and rotary embedding: a warp's 128 columns are one head, whose columns i and 64 + i it reads together.
+// The projection is rounded to bf16 before the rotation: bit for bit a plain product followed by the rotation kernel. Heads of
+// 128 columns, the first `rot_cols` columns rotate, the others (v) are stored as they are; rows of D start on 32 bytes.
+struct PairRopeEpilogue {
+  static constexpr bool kHalves = true;
+  __nv_bfloat16* D;
+  long long ldd;
+  const __nv_bfloat16* bias;  // [N] or nullptr, 16-byte aligned
+  AttnRope rope;
+  int rot_cols;
+  long long table;            // of this thread's row
+
+  __device__ __forceinline__ void item_begin(int row, int M, int) { table = row < M ? rope.row(row) * 64 : 0; }
+  __device__ __forceinline__ void item_end(int, int, int, int) {}
+  // 32 columns at col and 32 at col + 64
+  __device__ __forceinline__ void halves_chunk(int row, int col, const uint32_t (&ra)[32], const uint32_t (&rb)[32], int M, int N) {
+    if (row >= M || col >= N) return;
+    const float* ct = rope.cos_t + table + (col & 63);
+    const float* st = rope.sin_t + table + (col & 63);
+    const bool rotates = col < rot_cols;
+#pragma unroll
+    for (int c = 0; c < 32; c += 16) {
+      uint32_t oa[8], ob[8];
+#pragma unroll
+      for (int j = 0; j < 16; j += 4) {
+        float a[4], b[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          a[k] = __uint_as_float(ra[c + j + k]);
+          b[k] = __uint_as_float(rb[c + j + k]);
+        }
+        if (bias != nullptr) {
+          const uint2 wa = *reinterpret_cast<const uint2*>(bias + col + c + j), wb = *reinterpret_cast<const uint2*>(bias + col + 64 + c + j);
+          const float2 a0 = unpack(wa.x), a1 = unpack(wa.y), b0 = unpack(wb.x), b1 = unpack(wb.y);
+          a[0] += a0.x; a[1] += a0.y; a[2] += a1.x; a[3] += a1.y;
+          b[0] += b0.x; b[1] += b0.y; b[2] += b1.x; b[3] += b1.y;
+        }
+        if (rotates) {
+          const float4 cs = *reinterpret_cast<const float4*>(ct + c + j), sn = *reinterpret_cast<const float4*>(st + c + j);
+          const float cv[4] = {cs.x, cs.y, cs.z, cs.w}, sv[4] = {sn.x, sn.y, sn.z, sn.w};
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            a[k] = __bfloat162float(__float2bfloat16(a[k]));
+            b[k] = __bfloat162float(__float2bfloat16(b[k]));
+            rope_rotate(a[k], b[k], cv[k], sv[k]);
+          }
+        }
+        oa[j / 2] = pack_bf16x2(a[0], a[1]);
+        oa[j / 2 + 1] = pack_bf16x2(a[2], a[3]);
+        ob[j / 2] = pack_bf16x2(b[0], b[1]);
+        ob[j / 2 + 1] = pack_bf16x2(b[2], b[3]);
+      }
+      __nv_bfloat16* d = D + (long long)row * ldd + col + c;
+      st_global_32b(d, oa);
+      st_global_32b(d + 64, ob);
+    }
+  }
+  __device__ __forceinline__ static float2 unpack(uint32_t w) { return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w)); }
+};
+
+template <class Epi, class = void>
+struct EpiHalves { static constexpr bool value = false; };
+template <class Epi>
+struct EpiHalves<Epi, decltype((void)Epi::kHalves)> { static constexpr bool value = Epi::kHalves; };
 
 template <class Epi, class = void>
 struct EpiDual { static constexpr bool value = false; };
@@ -376,6 +442,16 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             tmem_ld_32x32(gate + BN / 2 + c * 32, u);
             tc_wait_ld();
             epi.dual_chunk(row, col + c * 32, g, u, p.M);
+          }
+        } else if constexpr (EpiHalves<Epi>::value) {
+          static_assert(kEpiCols == 128, "a warp's columns are one head");
+#pragma unroll 1
+          for (int c = 0; c < 2; ++c) {
+            uint32_t a[32], b[32];
+            tmem_ld_32x32(taddr + c * 32, a);
+            tmem_ld_32x32(taddr + 64 + c * 32, b);
+            tc_wait_ld();
+            epi.halves_chunk(row, n0 + c * 32, a, b, p.M, n_end);
           }
         } else {
 #pragma unroll 1

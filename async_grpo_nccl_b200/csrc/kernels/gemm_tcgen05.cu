@@ -244,6 +244,27 @@ bool launch_pair_swiglu(const void* a, long long lda, const void* b, long long l
 }
 }  // namespace
 
+bool launch_gemm_qkv_rope(const void* a, long long lda, const void* b, long long ldb, void* qkv, long long ldd, int M, int N, int K,
+                          const void* bias, const AttnRope& rope, int rot_heads, int head_dim, int* status, int num_sms, cudaStream_t stream) {
+  if (head_dim != 128 || N % 128 != 0 || !pair_serves(M, num_sms) || !aligned32(qkv, ldd, 2) || (reinterpret_cast<uintptr_t>(bias) & 15) != 0)
+    return false;
+  const CUtensorMap ta = make_tmap_2d(a, K, M, lda, 64, kGemmBM);
+  const CUtensorMap tb = make_tmap_2d(b, K, N, ldb, 64, 128);
+  GemmShape p;
+  p.M = M; p.N = N; p.K = K;
+  p.group_n = 1;
+  p.status = status;
+  PairRopeEpilogue e;
+  e.D = reinterpret_cast<__nv_bfloat16*>(qkv);
+  e.ldd = ldd;
+  e.bias = reinterpret_cast<const __nv_bfloat16*>(bias);
+  e.rope = rope;
+  e.rot_cols = rot_heads * 128;
+  e.table = 0;
+  gemm_pair_launch<256, false, false>(ta, tb, p, e, num_sms, stream);
+  return true;
+}
+
 bool launch_gemm_mlp_in(const void* a, long long lda, const void* b, long long ldb, void* act, long long ldact, void* gu, long long ldgu,
                         int M, int F, int K, int* status, int num_sms, cudaStream_t stream) {
   return M > 0 && launch_pair_swiglu<true>(a, lda, b, ldb, act, ldact, gu, ldgu, M, F, K, nullptr, 0.f, status, num_sms, stream);

@@ -80,6 +80,20 @@ inline void launch_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_
   check_cuda(cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...), what);
 }
 
+// Rotary tables for kernels that rotate on the way: token t is at position pos[t], clamped to the tables ([max_pos, D / 2], fp32).
+struct AttnRope {
+  const int* pos = nullptr;  // nullptr = off
+  const float* cos_t = nullptr;
+  const float* sin_t = nullptr;
+  int max_pos = 0;
+#ifdef __CUDACC__
+  __device__ __forceinline__ long long row(long long t) const {
+    const int q = pos[t];
+    return q < 0 ? 0 : (q >= max_pos ? max_pos - 1 : q);
+  }
+#endif
+};
+
 // d[M,N] = alpha * A . B^T (+ bias[N]) (+ d). bf16 operands, fp32 accumulation on tcgen05.
 //   a_mn = false: a is [M, K] row-major with pitch lda; a_mn = true: a is [K, M] row-major
 //   b_mn = false: b is [N, K] row-major with pitch ldb; b_mn = true: b is [K, N] row-major
@@ -130,6 +144,10 @@ bool launch_unit_gather(const GatherArgs& g, int n_ctas, int* status, cudaStream
 // receives. Returns false (nothing launched) for shapes it does not serve: a plain product and swiglu_fwd give the same bits.
 bool launch_gemm_mlp_in(const void* a, long long lda, const void* b, long long ldb, void* act, long long ldact, void* gu, long long ldgu,
                         int M, int F, int K, int* status, int num_sms, cudaStream_t stream);
+// qkv projection (+ bias) with rotary embedding of the first rot_heads heads. Returns false (nothing launched) for shapes it does
+// not serve: a plain product and the rotation kernel give the same bits.
+bool launch_gemm_qkv_rope(const void* a, long long lda, const void* b, long long ldb, void* qkv, long long ldd, int M, int N, int K,
+                          const void* bias, const AttnRope& rope, int rot_heads, int head_dim, int* status, int num_sms, cudaStream_t stream);
 // Fused gate/up projection + SwiGLU (+ folded RMSNorm row scale, ss_in = row sums of squares of a, may be nullptr):
 // b is the stacked [2F, K] weight, d the [M, F] activation.
 bool launch_gemm_swiglu_bf16(const void* a, long long lda, const void* b, long long ldb, void* d, long long ldd, int M, int F,
@@ -197,7 +215,7 @@ void launch_attn_varlen_bwd(const void* q, long long ldq, int q_cols, const void
                             long long ldo, const void* dout, long long lddo, const float* lse, float* delta, float* dq_acc,
                             void* dq, long long ld_dq, void* dk, long long ld_dk, int dk_col0, void* dv, long long ld_dv,
                             int dv_col0, const int* tiles, int n_tiles, int T, int Hq, int Hkv, int D, float softmax_scale,
-                            int* status, cudaStream_t s);
+                            int* status, cudaStream_t s, const AttnRope& rope = AttnRope{});
 
 // ---- fused lm_head + GRPO loss (lmhead_loss.cu) ----
 // Number of partial-statistics groups the forward writes for a [T, V] problem.

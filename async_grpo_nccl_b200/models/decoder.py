@@ -179,6 +179,18 @@ class NativeDecoder:
             self.C.gemm_bf16(dy, x, sink.view(name), True, True, None, 1.0, True, self.status, None)
         self.launches += 1
 
+    def _qkv(self, h: torch.Tensor, p: str, qkv: torch.Tensor, pos: torch.Tensor, cos_t: torch.Tensor, sin_t: torch.Tensor) -> None:
+        """Rotated q, k and v of the rows: one launch, or the plain GEMM and the rotation kernel, with the same bits."""
+        cfg = self.cfg
+        rot = cfg.num_attention_heads + cfg.num_key_value_heads
+        w, bias = self.w(p + "wqkv"), self.w(p + "bqkv") if cfg.attention_bias else None
+        if self.weights is None and self.C.gemm_qkv_rope(h, w, qkv, bias, pos, cos_t, sin_t, rot, cfg.head_dim, self.status):
+            self.launches += 1
+            return
+        self._gemm(h, w, qkv, bias=bias)
+        self.C.rope_inplace(qkv, pos, cos_t, sin_t, rot, cfg.head_dim, False)
+        self.launches += 1
+
     def _mlp_in(self, h: torch.Tensor, w: torch.Tensor, keep: bool) -> Tuple[Optional[torch.Tensor], torch.Tensor]:
         """(gate / up projections if they are to be kept for the backward pass, SwiGLU activation): one launch, or the plain
         GEMM (which carries the prefetch of sharded weights) and the elementwise kernel, with the same bits."""
@@ -209,8 +221,7 @@ class NativeDecoder:
         rstd1 = self._new(T, dtype=torch.float32)
         C.rmsnorm_fwd(x, self.w(p + "ln1"), h1, rstd1, cfg.rms_norm_eps)
         qkv = self._new(T, cfg.qkv_dim)
-        self._gemm(h1, self.w(p + "wqkv"), qkv, bias=self.w(p + "bqkv") if cfg.attention_bias else None)
-        C.rope_inplace(qkv, batch.pos, cos_t, sin_t, cfg.num_attention_heads + cfg.num_key_value_heads, cfg.head_dim, False)
+        self._qkv(h1, p, qkv, batch.pos, cos_t, sin_t)
         if kv_write is not None:  # rollout prefill: K/V of every prompt token go to their cache slots
             k_cache, v_cache, slots = kv_write[:3]
             head0 = kv_write[3] if len(kv_write) > 3 else 0  # tensor-parallel engine rank: its share of the kv heads
@@ -229,7 +240,7 @@ class NativeDecoder:
         gu, act = self._mlp_in(h2, self.w(p + "wgu"), save is not None)
         x2 = self._new(T, cfg.hidden_size)
         self._gemm(act, self.w(p + "wd"), x2, residual=x1)
-        self.launches += 5
+        self.launches += 4
         if save is not None:
             save.update(x=x, h1=h1, rstd1=rstd1, qkv=qkv, attn=attn, lse=lse, x1=x1, h2=h2, rstd2=rstd2, gu=gu, act=act)
         return x2
@@ -250,8 +261,7 @@ class NativeDecoder:
         h1 = self._new(Ts, cfg.hidden_size)
         C.rmsnorm_fwd(x, self.w(p + "ln1"), h1, None, cfg.rms_norm_eps)
         qkv_s = self._new(Ts, cfg.qkv_dim)
-        self._gemm(h1, self.w(p + "wqkv"), qkv_s, bias=self.w(p + "bqkv") if cfg.attention_bias else None)
-        C.rope_inplace(qkv_s, pos_s, cos_t, sin_t, Hq + Hkv, D, False)
+        self._qkv(h1, p, qkv_s, pos_s, cos_t, sin_t)
         C.kv_cache_write(qkv_s, slots, k_cache, v_cache, Hq, Hkv, D, self.status, 0)
         qkv = torch.zeros(T, cfg.qkv_dim, dtype=torch.bfloat16, device=x.device)
         qkv.index_copy_(0, sfx, qkv_s)
@@ -269,7 +279,7 @@ class NativeDecoder:
         _, act = self._mlp_in(h2, self.w(p + "wgu"), False)
         x2 = self._new(Ts, cfg.hidden_size)
         self._gemm(act, self.w(p + "wd"), x2, residual=x1)
-        self.launches += 11
+        self.launches += 10
         return x2
 
     def _layer_bwd(self, i: int, dx: torch.Tensor, s: dict, batch: PackedBatch, cos_t, sin_t, sink: GradSink):
@@ -298,16 +308,15 @@ class NativeDecoder:
         delta = self._new(cfg.num_attention_heads, T, dtype=torch.float32)
         dq_acc = self._new(T, cfg.q_dim, dtype=torch.float32)
         C.attn_varlen_bwd(s["qkv"], s["attn"], dattn, s["lse"], delta, dq_acc, dqkv, batch.tiles, cfg.num_attention_heads,
-                          cfg.num_key_value_heads, cfg.head_dim, 1.0 / math.sqrt(cfg.head_dim), self.status)
+                          cfg.num_key_value_heads, cfg.head_dim, 1.0 / math.sqrt(cfg.head_dim), self.status, batch.pos, cos_t, sin_t)
         del dattn, delta, dq_acc
-        C.rope_inplace(dqkv, batch.pos, cos_t, sin_t, cfg.num_attention_heads + cfg.num_key_value_heads, cfg.head_dim, True)
         if cfg.attention_bias:
             C.colsum(dqkv, sink.view(p + "bqkv"))
         dh1 = dh2  # reuse
         self._gemm(dqkv, self.w(p + "wqkv"), dh1, b_mn=True)
         self._wgrad(dqkv, s["h1"], p + "wqkv", sink)
         C.rmsnorm_bwd(dh1, s["x"], self.w(p + "ln1"), s["rstd1"], dx, sink.view(p + "ln1"), True)
-        self.launches += 11
+        self.launches += 10
         sink.unit_done(i + 1)
 
     # ---- public ----

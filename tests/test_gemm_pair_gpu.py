@@ -79,3 +79,27 @@ def test_swiglu_with_row_scale(M, F):
     C.gemm_swiglu(a, w, act, ss, 1e-6, st)
     assert int(st.item()) == 0
     assert rel_err(act.double(), torch.nn.functional.silu(z[:, :F]) * z[:, F:]) < BF16_TOL
+
+
+@pytest.mark.parametrize("M,Hq,Hkv,K", [(129, 1, 1, 64), (300, 2, 1, 200), (777, 12, 2, 256), (128, 2, 1, 64)])
+def test_qkv_with_rotation(M, Hq, Hkv, K):
+    """The bits of the plain GEMM followed by the rotation kernel; a number of heads that ends inside a 256-wide tile, positions
+    past the tables; 128 rows are not served."""
+    C, st = native(), status_word()
+    torch.manual_seed(M)
+    N = (Hq + 2 * Hkv) * 128
+    a = torch.randn(M, K, device=DEV).to(torch.bfloat16)
+    w = torch.randn(N, K, device=DEV).to(torch.bfloat16)
+    bias = torch.randn(N, device=DEV).to(torch.bfloat16)
+    pos = torch.randint(0, 500, (M,), device=DEV, dtype=torch.int32)
+    ang = torch.randn(400, 64, device=DEV)
+    cos_t, sin_t = ang.cos().contiguous(), ang.sin().contiguous()
+    for b in (bias, None):
+        got, want = (torch.zeros(M, N, device=DEV, dtype=torch.bfloat16) for _ in range(2))
+        served = C.gemm_qkv_rope(a, w, got, b, pos, cos_t, sin_t, Hq + Hkv, 128, st)
+        assert served == (M > 128)
+        C.gemm_bf16(a, w, want, False, False, b, 1.0, False, st, None)
+        C.rope_inplace(want, pos, cos_t, sin_t, Hq + Hkv, 128, False)
+        if served:
+            assert torch.equal(got, want)
+    assert int(st.item()) == 0
