@@ -9,8 +9,9 @@
 //   S^T  = K Q^T          dP^T = V dO^T                 (operands from shared memory, TMA-fed)
 //   dV  += P^T dO         dK  += dS^T Q                 (A operand read back from tensor memory)
 //   dQ   = dS K                                         (dS^T staged in shared memory, MN-major)
-// dK / dV leave as bf16 once per CTA; dQ partial tiles are added to an fp32 accumulator with vector
-// reductions and converted by attn_bwd_finalize_dq. Where rotary embedding came before the attention,
+// dK / dV leave as bf16 once per CTA; dQ partial tiles are added to an fp32 accumulator by TMA from the
+// shared memory of dS (whole lines; as 16-byte reductions of single threads, 4096 a step, they were what
+// a step waited for) and converted by attn_bwd_finalize_dq. Where rotary embedding came before the attention,
 // both take its transpose along on the way out.
 //
 // A step is a chain (S and dP, then the softmax gradient, then three products, then the read-out of dQ), and the
@@ -35,7 +36,6 @@ struct AttnBwdParams {
   const int4* tiles;  // {seq_start, seq_len, k0, unused}
   const float* lse;   // [Hq, T]
   const float* delta; // [Hq, T]
-  float* dq_acc;      // [T, Hq*D] fp32, zeroed by the caller
   __nv_bfloat16* dk;  // row pitch ldk, head h at column dk_col0 + h*D
   __nv_bfloat16* dv;
   long long ld_dk, ld_dv;
@@ -47,9 +47,6 @@ struct AttnBwdParams {
   int* status;
 };
 
-__device__ __forceinline__ void red_add_v4(float* addr, float a, float b, float c, float d) {
-  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(addr), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
-}
 __device__ __forceinline__ void named_bar_sync(int id, int count) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(count) : "memory");
 }
@@ -58,7 +55,7 @@ template <int D>
 __global__ void __launch_bounds__(kBwdThreads, 1)
 attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                 const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDO,
-                const AttnBwdParams p) {
+                const __grid_constant__ CUtensorMap tmDQ, const AttnBwdParams p) {
   constexpr int kChunks = D / 64;
   constexpr int kTileBytes = kT * D * 2;
   constexpr int kChunkBytes = kT * 128;     // one 64-column swizzle chunk of a 128-row tile
@@ -285,26 +282,40 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       }
       tc_fence_after();
       {
-        const int qi = q0 + r;
-        const bool valid = qi < seq_len;
-        float* dst = p.dq_acc + ((long long)seq_start + qi) * ((long long)p.Hq * D) + (long long)head * D;
-#pragma unroll 1
-        for (int c = part * (D / 64); c < (part + 1) * (D / 64); ++c) {
-          uint32_t o[32];
-          tmem_ld_32x32(tmem_R1 + lane_off + c * 32, o);
-          tc_wait_ld();
-          if (valid) {
+        constexpr int kMine = D / 64;  // 32-column pieces of dQ that this warp takes out
+        uint32_t o[kMine][32];
 #pragma unroll
-            for (int i = 0; i < 32; i += 4)
-              red_add_v4(dst + c * 32 + i, __uint_as_float(o[i]), __uint_as_float(o[i + 1]), __uint_as_float(o[i + 2]),
-                         __uint_as_float(o[i + 3]));
+        for (int c = 0; c < kMine; ++c) tmem_ld_32x32(tmem_R1 + lane_off + (part * kMine + c) * 32, o[c]);
+        tc_wait_ld();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(dq_read);
+        // dS has been consumed: its tile is the staging area, 32 rows x 128 bytes of it per warp. Rows past the sequence are
+        // zero (their P is), so adding them to what follows changes nothing.
+        uint8_t* buf = sDS + (warp - 2) * 4096;
+        const bool any = q0 + quarter * 32 < seq_len;
+#pragma unroll
+        for (int c = 0; c < kMine; ++c) {
+          if (c > 0) {
+            if (lane == 0) bulk_wait_read<0>();
+            __syncwarp();
+          }
+#pragma unroll
+          for (int u = 0; u < 8; ++u)
+            *reinterpret_cast<uint4*>(buf + lane * 128 + ((u ^ (lane & 7)) << 4)) =
+                make_uint4(o[c][4 * u], o[c][4 * u + 1], o[c][4 * u + 2], o[c][4 * u + 3]);
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0 && any) {
+            tma_reduce_add_2d(&tmDQ, buf, head * D + (part * kMine + c) * 32, seq_start + q0 + quarter * 32);
+            bulk_commit();
           }
         }
+        if (lane == 0) bulk_wait_read<0>();  // the barrier at the top lets every warp write dS again
+        __syncwarp();
       }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(dq_read);
     }
+    if (lane == 0) bulk_wait_all<0>();
     if (ok && n_it > 0) {
       // The last dq_full wait also covered the final dV / dK MMAs (commits are cumulative).
       const bool valid = kj < seq_len;
@@ -405,12 +416,12 @@ __global__ void attn_bwd_finalize_dq_kernel(const float* __restrict__ acc, __nv_
 
 template <int D>
 void launch_bwd_t(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tdo,
-                  const AttnBwdParams& p, int n_tiles, int Hkv, cudaStream_t s) {
+                  const CUtensorMap& tdq, const AttnBwdParams& p, int n_tiles, int Hkv, cudaStream_t s) {
   constexpr int smem = 5 * kT * D * 2 + kT * kT * 2 + 4 * kT * 4 + 128 + 1024;
   auto kernel = attn_bwd_kernel<D>;
   AGRPO_SET_MAX_DYN_SMEM(kernel, smem, "attn_bwd smem attr");
   dim3 grid(Hkv, n_tiles);
-  kernel<<<grid, kBwdThreads, smem, s>>>(tq, tk, tv, tdo, p);
+  kernel<<<grid, kBwdThreads, smem, s>>>(tq, tk, tv, tdo, tdq, p);
   check_cuda(cudaGetLastError(), "attn_bwd launch");
 }
 
@@ -435,11 +446,11 @@ void launch_attn_varlen_bwd(const void* q, long long ldq, int q_cols, const void
   const CUtensorMap tk = make_tmap_2d(k, k_cols, T, ldk, 64, kT);
   const CUtensorMap tv = make_tmap_2d(v, v_cols, T, ldv, 64, kT);
   const CUtensorMap tdo = make_tmap_2d(dout, (uint64_t)Hq * D, T, lddo, 64, kT);
+  const CUtensorMap tdq = make_tmap_2d(dq_acc, (uint64_t)Hq * D, T, (uint64_t)Hq * D, 32, 32, 4);
   AttnBwdParams p;
   p.tiles = reinterpret_cast<const int4*>(tiles);
   p.lse = lse;
   p.delta = delta;
-  p.dq_acc = dq_acc;
   p.dk = reinterpret_cast<__nv_bfloat16*>(dk);
   p.dv = reinterpret_cast<__nv_bfloat16*>(dv);
   p.ld_dk = ld_dk;
@@ -456,8 +467,8 @@ void launch_attn_varlen_bwd(const void* q, long long ldq, int q_cols, const void
   p.scale_log2 = softmax_scale * 1.4426950408889634f;
   p.rope = rope;
   p.status = status;
-  if (D == 128) launch_bwd_t<128>(tq, tk, tv, tdo, p, n_tiles, Hkv, s);
-  else          launch_bwd_t<64>(tq, tk, tv, tdo, p, n_tiles, Hkv, s);
+  if (D == 128) launch_bwd_t<128>(tq, tk, tv, tdo, tdq, p, n_tiles, Hkv, s);
+  else          launch_bwd_t<64>(tq, tk, tv, tdo, tdq, p, n_tiles, Hkv, s);
   {
     const long long work = (long long)T * (Hq * D / 8);
     long long blocks = (work + 255) / 256;
