@@ -176,6 +176,20 @@ void gemm_swiglu(const Tensor& a, const Tensor& b, Tensor& d, const OptTensor& s
                                              cur_stream()),
               "gemm_swiglu: arguments not served");
 }
+bool gemm_swiglu_bwd(const Tensor& dy, const Tensor& w, const Tensor& gu, Tensor& dgu, const OptTensor& status) {
+  check_bf16(dy, "gemm_swiglu_bwd dy"); check_bf16(w, "gemm_swiglu_bwd w"); check_bf16(gu, "gemm_swiglu_bwd gu"); check_bf16(dgu, "gemm_swiglu_bwd dgu");
+  TORCH_CHECK(dy.dim() == 2 && w.dim() == 2 && gu.dim() == 2 && dgu.dim() == 2 && dy.stride(1) == 1 && w.stride(1) == 1 && gu.stride(1) == 1 &&
+              dgu.stride(1) == 1, "gemm_swiglu_bwd: 2-D");
+  const int64_t M = dy.size(0), K = dy.size(1), F = w.size(1);
+  TORCH_CHECK(w.size(0) == K && gu.size(0) == M && gu.size(1) == 2 * F && dgu.sizes() == gu.sizes(), "gemm_swiglu_bwd: shapes");
+  TORCH_CHECK(dy.stride(0) % 8 == 0 && w.stride(0) % 8 == 0 && (reinterpret_cast<uintptr_t>(dy.data_ptr()) & 15) == 0 &&
+              (reinterpret_cast<uintptr_t>(w.data_ptr()) & 15) == 0, "gemm_swiglu_bwd: operand rows must be 16-byte aligned");
+  if (status.has_value() && status->defined()) check_i32(*status, "gemm_swiglu_bwd status");
+  if (M == 0) return true;
+  const c10::cuda::CUDAGuard guard(dy.device());
+  return agrpo::launch_gemm_swiglu_bwd(dy.data_ptr(), dy.stride(0), w.data_ptr(), w.stride(0), gu.data_ptr(), gu.stride(0), dgu.data_ptr(),
+                                       dgu.stride(0), (int)M, (int)F, (int)K, opt_ptr<int>(status), num_sms(), cur_stream());
+}
 bool gemm_qkv_rope(const Tensor& a, const Tensor& b, Tensor& qkv, const OptTensor& bias, const Tensor& pos, const Tensor& cos_t,
                    const Tensor& sin_t, int64_t rot_heads, int64_t head_dim, const OptTensor& status) {
   check_bf16(a, "gemm_qkv_rope a"); check_bf16(b, "gemm_qkv_rope b"); check_bf16(qkv, "gemm_qkv_rope qkv");
@@ -968,6 +982,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("decode_layers_counter_words", &decode_layers_counter_words);
   m.def("gemm_swiglu", &gemm_swiglu, py::arg("a"), py::arg("b"), py::arg("d"), py::arg("ss_in") = py::none(), py::arg("eps") = 1e-6,
         py::arg("status") = py::none(), NOGIL);
+  m.def("gemm_swiglu_bwd", &gemm_swiglu_bwd, py::arg("dy"), py::arg("w"), py::arg("gu"), py::arg("dgu"), py::arg("status") = py::none(), NOGIL);
   m.def("gemm_qkv_rope", &gemm_qkv_rope, py::arg("a"), py::arg("b"), py::arg("qkv"), py::arg("bias"), py::arg("pos"), py::arg("cos_t"),
         py::arg("sin_t"), py::arg("rot_heads"), py::arg("head_dim"), py::arg("status") = py::none(), NOGIL);
   m.def("gemm_mlp_in", &gemm_mlp_in, py::arg("a"), py::arg("b"), py::arg("act"), py::arg("gu") = py::none(), py::arg("status") = py::none(), NOGIL);

@@ -7,6 +7,7 @@
 #include "../common/ptx.cuh"
 #include "../launchers.h"
 #include "rope.cuh"
+#include "swiglu.cuh"
 
 namespace agrpo {
 
@@ -322,12 +323,11 @@ __global__ void swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ gu, const __
       const float2 gf = __bfloat1622float2(g.v[j]);
       const float2 uf = __bfloat1622float2(u.v[j]);
       const float2 df = __bfloat1622float2(d.v[j]);
-      const float s0 = 1.f / (1.f + __expf(-gf.x));
-      const float s1 = 1.f / (1.f + __expf(-gf.y));
-      const float dg0 = df.x * uf.x * s0 * (1.f + gf.x * (1.f - s0));
-      const float dg1 = df.y * uf.y * s1 * (1.f + gf.y * (1.f - s1));
-      dg.v[j] = __floats2bfloat162_rn(dg0, dg1);
-      du.v[j] = __floats2bfloat162_rn(df.x * gf.x * s0, df.y * gf.y * s1);
+      float2 a, b;
+      swiglu_grad(gf.x, uf.x, df.x, a.x, b.x);
+      swiglu_grad(gf.y, uf.y, df.y, a.y, b.y);
+      dg.v[j] = __floats2bfloat162_rn(a.x, a.y);
+      du.v[j] = __floats2bfloat162_rn(b.x, b.y);
     }
     reinterpret_cast<Bf16x8*>(dgu + (size_t)t * 2 * F)[c] = dg;
     reinterpret_cast<Bf16x8*>(dgu + (size_t)t * 2 * F + F)[c] = du;

@@ -12,6 +12,7 @@
 #pragma once
 #include "gemm_tcgen05.cuh"
 #include "rope.cuh"
+#include "swiglu.cuh"
 
 namespace agrpo {
 
@@ -212,6 +213,59 @@ struct PairRopeEpilogue {
       st_global_32b(d, oa);
       st_global_32b(d + 64, ob);
     }
+  }
+  __device__ __forceinline__ static float2 unpack(uint32_t w) { return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w)); }
+};
+
+// Input gradient of the down projection taken on to the gate / up projections: D[m, j] and D[m, F + j] are the gradients of g and u
+// where the product is that of silu(g) * u. The product is rounded to bf16 first: bit for bit a plain product followed by
+// swiglu_bwd. g and u of a warp's next 32 columns are read while the current ones are converted. F is a multiple of 16, rows of
+// gu and D start on 32 bytes.
+struct PairSwigluBwdEpilogue {
+  __nv_bfloat16* D;         // [M, 2F]
+  long long ldd;
+  const __nv_bfloat16* gu;  // [M, 2F]
+  long long ldgu;
+  int F;
+  int bn;                   // columns a warp converts per tile
+  uint32_t g[2][8], u[2][8];
+
+  __device__ __forceinline__ void fetch(int row, int col0, int M) {
+    if (row >= M) return;
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+      if (col0 + i * 16 < F) {
+        const __nv_bfloat16* p = gu + (long long)row * ldgu + col0 + i * 16;
+        ld_global_32b(p, g[i]);
+        ld_global_32b(p + F, u[i]);
+      }
+  }
+  __device__ __forceinline__ void item_begin(int, int, int) {}
+  __device__ __forceinline__ void item_end(int, int, int, int) {}
+  __device__ __forceinline__ void tile_begin(int row, int col0, int M, int) { fetch(row, col0, M); }
+  __device__ __forceinline__ void chunk(int row, int col0, const uint32_t (&r)[32], int M, int N) {
+    uint32_t dg[2][8], du[2][8];
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const uint32_t d2 = pack_bf16x2(__uint_as_float(r[i * 16 + 2 * j]), __uint_as_float(r[i * 16 + 2 * j + 1]));
+        const float2 gf = unpack(g[i][j]), uf = unpack(u[i][j]), df = unpack(d2);
+        float2 a, b;
+        swiglu_grad(gf.x, uf.x, df.x, a.x, b.x);
+        swiglu_grad(gf.y, uf.y, df.y, a.y, b.y);
+        dg[i][j] = pack_bf16x2(a.x, a.y);
+        du[i][j] = pack_bf16x2(b.x, b.y);
+      }
+    if (col0 % bn + 32 < bn) fetch(row, col0 + 32, M);
+    if (row >= M) return;
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+      if (col0 + i * 16 < N) {
+        __nv_bfloat16* d = D + (long long)row * ldd + col0 + i * 16;
+        st_global_32b(d, dg[i]);
+        st_global_32b(d + F, du[i]);
+      }
   }
   __device__ __forceinline__ static float2 unpack(uint32_t w) { return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w)); }
 };

@@ -27,6 +27,12 @@ void dispatch_pair_major(bool a_mn, bool b_mn, const CUtensorMap& ta, const CUte
   if (a_mn && b_mn) return gemm_pair_launch<BN, true, true>(ta, tb, p, e, sms, s);
   return gemm_pair_launch<BN, true, false>(ta, tb, p, e, sms, s);
 }
+template <bool A_MN, bool B_MN, class Epi>
+void dispatch_pair_width(int BN, const CUtensorMap& ta, const CUtensorMap& tb, const GemmShape& p, const Epi& e, int sms, cudaStream_t s) {
+  if (BN == 256) return gemm_pair_launch<256, A_MN, B_MN>(ta, tb, p, e, sms, s);
+  if (BN == 192) return gemm_pair_launch<192, A_MN, B_MN>(ta, tb, p, e, sms, s);
+  return gemm_pair_launch<128, A_MN, B_MN>(ta, tb, p, e, sms, s);
+}
 template <bool F32, bool AUX>
 void dispatch_pair(int BN, bool a_mn, bool b_mn, const CUtensorMap& ta, const CUtensorMap& tb, const GemmShape& p, PairStoreEpilogue<F32, AUX> e,
                    int sms, cudaStream_t s) {
@@ -243,6 +249,27 @@ bool launch_pair_swiglu(const void* a, long long lda, const void* b, long long l
   return true;
 }
 }  // namespace
+
+bool launch_gemm_swiglu_bwd(const void* dy, long long lddy, const void* w, long long ldw, const void* gu, long long ldgu, void* dgu,
+                            long long lddgu, int M, int F, int K, int* status, int num_sms, cudaStream_t stream) {
+  if (!pair_serves(M, num_sms) || F % 16 != 0 || !aligned32(gu, ldgu, 2) || !aligned32(dgu, lddgu, 2)) return false;
+  const int BN = pair_pick_bn(M, F, true, num_sms);
+  const CUtensorMap ta = make_tmap_2d(dy, K, M, lddy, 64, kGemmBM);
+  const CUtensorMap tb = make_tmap_2d(w, F, K, ldw, 64, 64);
+  GemmShape p;
+  p.M = M; p.N = F; p.K = K;
+  p.group_n = 1;
+  p.status = status;
+  PairSwigluBwdEpilogue e;
+  e.D = reinterpret_cast<__nv_bfloat16*>(dgu);
+  e.ldd = lddgu;
+  e.gu = reinterpret_cast<const __nv_bfloat16*>(gu);
+  e.ldgu = ldgu;
+  e.F = F;
+  e.bn = BN / 2;
+  dispatch_pair_width<false, true>(BN, ta, tb, p, e, num_sms, stream);
+  return true;
+}
 
 bool launch_gemm_qkv_rope(const void* a, long long lda, const void* b, long long ldb, void* qkv, long long ldd, int M, int N, int K,
                           const void* bias, const AttnRope& rope, int rot_heads, int head_dim, int* status, int num_sms, cudaStream_t stream) {

@@ -144,6 +144,11 @@ bool launch_unit_gather(const GatherArgs& g, int n_ctas, int* status, cudaStream
 // receives. Returns false (nothing launched) for shapes it does not serve: a plain product and swiglu_fwd give the same bits.
 bool launch_gemm_mlp_in(const void* a, long long lda, const void* b, long long ldb, void* act, long long ldact, void* gu, long long ldgu,
                         int M, int F, int K, int* status, int num_sms, cudaStream_t stream);
+// Gradients of the gate / up projections ([M, 2F]) from the gradient dy [M, K] of the MLP's output: the input gradient of the down
+// projection w [K, F] and the SwiGLU backward in one launch. Returns false (nothing launched) for shapes it does not serve: a
+// plain product and swiglu_bwd give the same bits.
+bool launch_gemm_swiglu_bwd(const void* dy, long long lddy, const void* w, long long ldw, const void* gu, long long ldgu, void* dgu,
+                            long long lddgu, int M, int F, int K, int* status, int num_sms, cudaStream_t stream);
 // qkv projection (+ bias) with rotary embedding of the first rot_heads heads. Returns false (nothing launched) for shapes it does
 // not serve: a plain product and the rotation kernel give the same bits.
 bool launch_gemm_qkv_rope(const void* a, long long lda, const void* b, long long ldb, void* qkv, long long ldd, int M, int N, int K,

@@ -289,12 +289,17 @@ class NativeDecoder:
         p = f"layers.{i}."
         self._enter_unit(i + 1, i if i > 0 else None)
         # ---- MLP ----
-        dact = self._new(T, cfg.intermediate_size)
-        self._gemm(dx, self.w(p + "wd"), dact, b_mn=True)
-        self._wgrad(dx, s["act"], p + "wd", sink)
         dgu = self._new(T, 2 * cfg.intermediate_size)
-        C.swiglu_bwd(s["gu"], dact, dgu)
-        del dact
+        wd = self.w(p + "wd")
+        if self.weights is None and C.gemm_swiglu_bwd(dx, wd, s["gu"], dgu, self.status):
+            self.launches += 1
+        else:  # the same bits; sharded weights prefetch with the plain GEMM
+            dact = self._new(T, cfg.intermediate_size)
+            self._gemm(dx, wd, dact, b_mn=True)
+            C.swiglu_bwd(s["gu"], dact, dgu)
+            self.launches += 1
+            del dact
+        self._wgrad(dx, s["act"], p + "wd", sink)
         dh2 = self._new(T, cfg.hidden_size)
         self._gemm(dgu, self.w(p + "wgu"), dh2, b_mn=True)
         self._wgrad(dgu, s["h2"], p + "wgu", sink)
@@ -316,7 +321,7 @@ class NativeDecoder:
         self._gemm(dqkv, self.w(p + "wqkv"), dh1, b_mn=True)
         self._wgrad(dqkv, s["h1"], p + "wqkv", sink)
         C.rmsnorm_bwd(dh1, s["x"], self.w(p + "ln1"), s["rstd1"], dx, sink.view(p + "ln1"), True)
-        self.launches += 10
+        self.launches += 9
         sink.unit_done(i + 1)
 
     # ---- public ----

@@ -103,3 +103,24 @@ def test_qkv_with_rotation(M, Hq, Hkv, K):
         if served:
             assert torch.equal(got, want)
     assert int(st.item()) == 0
+
+
+# F = 264: no 32-byte rows; 128 rows: not served
+@pytest.mark.parametrize("M,F,K", [(129, 16, 64), (300, 528, 200), (1500, 8960, 64), (128, 272, 64), (200, 264, 64)])
+def test_swiglu_backward(M, F, K):
+    """The bits of the plain GEMM followed by the elementwise kernel."""
+    C, st = native(), status_word()
+    torch.manual_seed(M + F)
+    dy = torch.randn(M, K, device=DEV).to(torch.bfloat16)
+    w = torch.randn(K, F, device=DEV).to(torch.bfloat16)
+    gu = (3 * torch.randn(M, 2 * F, device=DEV)).to(torch.bfloat16)
+    gu[0, ::3], gu[0, 1::3] = 100.0, -100.0  # saturated gates
+    got, want = (torch.zeros(M, 2 * F, device=DEV, dtype=torch.bfloat16) for _ in range(2))
+    dact = torch.empty(M, F, device=DEV, dtype=torch.bfloat16)
+    served = C.gemm_swiglu_bwd(dy, w, gu, got, st)
+    assert served == (M > 128 and F % 16 == 0)
+    C.gemm_bf16(dy, w, dact, False, True, None, 1.0, False, st, None)
+    C.swiglu_bwd(gu, dact, want)
+    if served:
+        assert torch.equal(got, want)
+    assert int(st.item()) == 0
