@@ -2,7 +2,11 @@
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/extension.h>
+#include <algorithm>
+#include <cmath>
 #include <cstdlib>
+#include <tuple>
+#include <vector>
 
 #include <pybind11/numpy.h>
 #include <pybind11/stl.h>
@@ -359,6 +363,181 @@ void attn_varlen_bwd(const Tensor& qkv, const Tensor& out, const Tensor& dout, c
                                 (int)(Hq * D), dqkv.data_ptr(), dqkv.stride(0), (int)((Hq + Hkv) * D), tiles.data_ptr<int>(),
                                 (int)tiles.size(0), (int)T, (int)Hq, (int)Hkv, (int)D, (float)softmax_scale,
                                 opt_ptr<int>(status), cur_stream(), rope);
+}
+
+// ---- a whole decoder layer per call -------------------------------------------------------------------------------------------
+// Small batches are bound by the host: a layer is 8 launches forward and 14 backward of a few microseconds each, and issuing them
+// one by one from Python, with an allocation and a view for each tensor, took about 150 us a layer. Here a layer is one call and
+// its activations are one allocation.
+struct LayerArgs {
+  const uint16_t* params;            // flat bf16 parameters
+  int64_t ln1, wqkv, bqkv, wo, ln2, wgu, wd;  // element offsets; bqkv < 0: none
+  int T, H, Hq, Hkv, D, F;
+  float eps;
+  int qd() const { return Hq * D; }
+  int qkv() const { return (Hq + 2 * Hkv) * D; }
+  const void* w(int64_t off) const { return off < 0 ? nullptr : params + off; }
+};
+LayerArgs layer_args(const Tensor& params, const std::vector<int64_t>& offs, const std::vector<int64_t>& dims, double eps, const Tensor& x) {
+  check_bf16(params, "layer params"); check_bf16(x, "layer x");
+  TORCH_CHECK(params.is_contiguous() && offs.size() == 7 && dims.size() == 5, "layer: flat parameters, 7 offsets, 5 sizes");
+  LayerArgs a;
+  a.params = reinterpret_cast<const uint16_t*>(params.data_ptr());
+  a.ln1 = offs[0]; a.wqkv = offs[1]; a.bqkv = offs[2]; a.wo = offs[3]; a.ln2 = offs[4]; a.wgu = offs[5]; a.wd = offs[6];
+  a.H = (int)dims[0]; a.Hq = (int)dims[1]; a.Hkv = (int)dims[2]; a.D = (int)dims[3]; a.F = (int)dims[4];
+  a.eps = (float)eps;
+  TORCH_CHECK(x.dim() == 2 && x.is_contiguous() && x.size(1) == a.H, "layer: x [T, H]");
+  a.T = (int)x.size(0);
+  const int64_t n = params.numel(), H = a.H;
+  const int64_t ends[7] = {a.ln1 + H, a.wqkv + H * a.qkv(), a.bqkv < 0 ? 0 : a.bqkv + a.qkv(), a.wo + H * a.qd(), a.ln2 + H, a.wgu + 2 * H * a.F, a.wd + H * a.F};
+  for (int i = 0; i < 7; ++i) TORCH_CHECK(ends[i] <= n && (i == 2 || offs[i] >= 0) && (offs[i] < 0 || offs[i] % 8 == 0), "layer: offset of tensor ", i);
+  TORCH_CHECK(a.H % 8 == 0 && a.F % 8 == 0 && a.qd() % 8 == 0 && (reinterpret_cast<uintptr_t>(a.params) & 15) == 0, "layer: rows of 16 bytes");
+  return a;
+}
+void check_tiles(const Tensor& tiles) {
+  check_i32(tiles, "layer tiles");
+  TORCH_CHECK(tiles.is_contiguous() && tiles.dim() == 2 && tiles.size(1) == 4 && (reinterpret_cast<uintptr_t>(tiles.data_ptr()) & 15) == 0, "layer: tiles [n, 4]");
+}
+// Parts of one allocation, each on a 256-byte boundary.
+struct Carve {
+  int64_t size = 0;
+  int64_t add(int64_t bytes) {
+    const int64_t at = size;
+    size += (bytes + 255) / 256 * 256;
+    return at;
+  }
+};
+struct LayerSlab {
+  int64_t h1, qkv, attn, x1, h2, act, gu, rstd1, rstd2, lse, size;
+  LayerSlab(const LayerArgs& a, bool keep) {
+    Carve c;
+    const int64_t T = a.T;
+    h1 = c.add(T * a.H * 2); qkv = c.add(T * a.qkv() * 2); attn = c.add(T * a.qd() * 2); x1 = c.add(T * a.H * 2); h2 = c.add(T * a.H * 2);
+    act = c.add(T * a.F * 2); rstd1 = c.add(T * 4); rstd2 = c.add(T * 4); lse = c.add(T * a.Hq * 4);
+    gu = c.add(keep ? T * 2 * a.F * 2 : 0);
+    size = c.size;
+  }
+};
+
+// One layer forward: (output, activations for layer_bwd, launches). `k_cache` given: k and v of every token also go to `slots` of
+// the paged cache (kv heads [kv_head0, kv_head0 + heads of the cache)).
+std::tuple<Tensor, Tensor, int64_t> layer_fwd(const Tensor& params, const std::vector<int64_t>& offs, const std::vector<int64_t>& dims, double eps,
+                                              const Tensor& x, const Tensor& pos, const Tensor& tiles, const Tensor& cos_t, const Tensor& sin_t,
+                                              const Tensor& status, bool keep, const OptTensor& slots, const OptTensor& k_cache,
+                                              const OptTensor& v_cache, int64_t kv_head0) {
+  const LayerArgs a = layer_args(params, offs, dims, eps, x);
+  check_tiles(tiles); check_i32(status, "layer status");
+  const c10::cuda::CUDAGuard guard(x.device());
+  const int T = a.T, H = a.H, Q = a.qd(), QKV = a.qkv(), F = a.F, sms = num_sms();
+  const agrpo::AttnRope rope = rope_args(pos, cos_t, sin_t, T, a.D);
+  Tensor out = at::empty({T, H}, x.options());
+  const LayerSlab s(a, keep);
+  Tensor slab = at::empty({s.size}, x.options().dtype(torch::kUInt8));
+  if (T == 0) return {out, slab, 0};
+  uint8_t* b = slab.data_ptr<uint8_t>();
+  const auto f32 = [&](int64_t o) { return reinterpret_cast<float*>(b + o); };
+  int* st = status.data_ptr<int>();
+  const cudaStream_t cs = cur_stream();
+  int64_t launches = 7;
+  agrpo::launch_rmsnorm_fwd(x.data_ptr(), a.w(a.ln1), b + s.h1, f32(s.rstd1), T, H, a.eps, cs);
+  if (!agrpo::launch_gemm_qkv_rope(b + s.h1, H, a.w(a.wqkv), H, b + s.qkv, QKV, T, QKV, H, a.w(a.bqkv), rope, a.Hq + a.Hkv, a.D, st, sms, cs)) {
+    agrpo::launch_gemm_bf16(b + s.h1, H, a.w(a.wqkv), H, b + s.qkv, QKV, T, QKV, H, false, false, a.w(a.bqkv), 1.f, false, false, st, sms, cs);
+    agrpo::launch_rope(b + s.qkv, rope.pos, rope.cos_t, rope.sin_t, T, a.Hq + a.Hkv, a.D, QKV, rope.max_pos, false, cs);
+    ++launches;
+  }
+  if (k_cache.has_value() && k_cache->defined()) {
+    const Tensor& k = *k_cache;
+    TORCH_CHECK(slots.has_value() && v_cache.has_value(), "layer: slots and v_cache");
+    check_i32(*slots, "slots"); check_bf16(k, "k_cache"); check_bf16(*v_cache, "v_cache");
+    TORCH_CHECK(slots->numel() == T && k.dim() == 4 && k.is_contiguous() && v_cache->is_contiguous() && v_cache->sizes() == k.sizes() && kv_head0 >= 0 &&
+                k.size(1) + kv_head0 <= a.Hkv && k.size(3) == a.D, "layer: cache [blocks, kv heads of this rank, block size, D]");
+    agrpo::launch_kv_cache_write(b + s.qkv, QKV, (int)((a.Hq + kv_head0) * a.D), (int)((a.Hq + a.Hkv + kv_head0) * a.D), slots->data_ptr<int>(),
+                                 k.data_ptr(), v_cache->data_ptr(), T, (int)k.size(1), a.D, (int)k.size(2), (int)k.size(0), st, cs);
+    ++launches;
+  }
+  agrpo::launch_attn_varlen_fwd(b + s.qkv, QKV, QKV, b + s.qkv, QKV, QKV, b + s.qkv, QKV, QKV, 0, Q, (a.Hq + a.Hkv) * a.D, b + s.attn, Q, f32(s.lse),
+                                tiles.data_ptr<int>(), (int)tiles.size(0), T, a.Hq, a.Hkv, a.D, (float)(1.0 / std::sqrt((double)a.D)), st, cs);
+  agrpo::launch_gemm_bf16(b + s.attn, Q, a.w(a.wo), Q, b + s.x1, H, T, H, Q, false, false, nullptr, 1.f, false, false, st, sms, cs, x.data_ptr(), H);
+  agrpo::launch_rmsnorm_fwd(b + s.x1, a.w(a.ln2), b + s.h2, f32(s.rstd2), T, H, a.eps, cs);
+  if (!agrpo::launch_gemm_mlp_in(b + s.h2, H, a.w(a.wgu), H, b + s.act, F, keep ? b + s.gu : nullptr, 2 * F, T, F, H, st, sms, cs)) {
+    Tensor tmp;
+    void* gu = b + s.gu;
+    if (!keep) {
+      tmp = at::empty({(int64_t)T * 2 * F}, x.options());
+      gu = tmp.data_ptr();
+    }
+    agrpo::launch_gemm_bf16(b + s.h2, H, a.w(a.wgu), H, gu, 2 * F, T, 2 * F, H, false, false, nullptr, 1.f, false, false, st, sms, cs);
+    agrpo::launch_swiglu_fwd(gu, b + s.act, T, F, cs);
+    ++launches;
+  }
+  agrpo::launch_gemm_bf16(b + s.act, F, a.w(a.wd), F, out.data_ptr(), H, T, H, F, false, false, nullptr, 1.f, false, false, st, sms, cs, b + s.x1, H);
+  return {out, slab, launches};
+}
+
+// One layer backward from what layer_fwd kept; dx (gradient of the output) becomes the gradient of x, weight gradients are added
+// to the flat fp32 buffer `grads`. Returns the launches.
+int64_t layer_bwd(const Tensor& params, Tensor& grads, const std::vector<int64_t>& offs, const std::vector<int64_t>& dims, double eps, Tensor& dx,
+                  const Tensor& x, const Tensor& slab, const Tensor& pos, const Tensor& tiles, const Tensor& cos_t, const Tensor& sin_t,
+                  const Tensor& status) {
+  const LayerArgs a = layer_args(params, offs, dims, eps, x);
+  check_tiles(tiles); check_i32(status, "layer status"); check_f32(grads, "layer grads"); check_bf16(dx, "layer dx");
+  const LayerSlab s(a, true);
+  TORCH_CHECK(grads.is_contiguous() && grads.numel() == params.numel(), "layer: grads are laid out as the parameters");
+  TORCH_CHECK(dx.is_contiguous() && dx.sizes() == x.sizes() && slab.is_cuda() && slab.scalar_type() == torch::kUInt8 && slab.numel() == s.size,
+              "layer: dx [T, H] and the activations of layer_fwd(keep)");
+  if (a.T == 0) return 0;
+  const c10::cuda::CUDAGuard guard(x.device());
+  const int T = a.T, H = a.H, Q = a.qd(), QKV = a.qkv(), F = a.F, sms = num_sms();
+  const agrpo::AttnRope rope = rope_args(pos, cos_t, sin_t, T, a.D);
+  const uint8_t* b = slab.data_ptr<uint8_t>();
+  // the MLP's temporaries are dead when the attention's are written
+  Carve cm, ca;
+  const int64_t m_dgu = cm.add((int64_t)T * 2 * F * 2), m_dact = cm.add(T <= 128 || F % 16 != 0 ? (int64_t)T * F * 2 : 0);
+  const int64_t a_dattn = ca.add((int64_t)T * Q * 2), a_dqkv = ca.add((int64_t)T * QKV * 2), a_delta = ca.add((int64_t)T * a.Hq * 4),
+                a_dq = ca.add((int64_t)T * Q * 4);
+  const int64_t shared = std::max(cm.size, ca.size);
+  Tensor tmp = at::empty({shared + (int64_t)T * H * 2}, x.options().dtype(torch::kUInt8));
+  uint8_t* t = tmp.data_ptr<uint8_t>();
+  uint8_t* dh = t + shared;
+  const auto f32 = [&](int64_t o) { return reinterpret_cast<const float*>(b + o); };
+  const auto g = [&](int64_t off) { return grads.data_ptr<float>() + off; };
+  int* st = status.data_ptr<int>();
+  const cudaStream_t cs = cur_stream();
+  const auto dgrad = [&](const void* dy, int ld, int64_t w, int ldw, void* out, int N, int K) {
+    agrpo::launch_gemm_bf16(dy, ld, a.w(w), ldw, out, N, T, N, K, false, true, nullptr, 1.f, false, false, st, sms, cs);
+  };
+  const auto wgrad = [&](const void* dy, int M, const void* in, int N, int64_t w) {
+    agrpo::launch_gemm_bf16(dy, M, in, N, g(w), N, M, N, T, true, true, nullptr, 1.f, true, true, st, sms, cs);
+  };
+  int64_t launches = 14 + (a.bqkv >= 0 ? 1 : 0);
+  if (!agrpo::launch_gemm_swiglu_bwd(dx.data_ptr(), H, a.w(a.wd), F, b + s.gu, 2 * F, t + m_dgu, 2 * F, T, F, H, st, sms, cs)) {
+    Tensor alone;
+    void* dact = t + m_dact;
+    if (cm.size - m_dact < (int64_t)T * F * 2) {  // a launcher declined for another reason than the shape
+      alone = at::empty({(int64_t)T * F}, x.options());
+      dact = alone.data_ptr();
+    }
+    dgrad(dx.data_ptr(), H, a.wd, F, dact, F, H);
+    agrpo::launch_swiglu_bwd(b + s.gu, dact, t + m_dgu, T, F, cs);
+    ++launches;
+  }
+  wgrad(dx.data_ptr(), H, b + s.act, F, a.wd);
+  dgrad(t + m_dgu, 2 * F, a.wgu, H, dh, H, 2 * F);
+  wgrad(t + m_dgu, 2 * F, b + s.h2, H, a.wgu);
+  agrpo::launch_rmsnorm_bwd(dh, b + s.x1, a.w(a.ln2), f32(s.rstd2), dx.data_ptr(), g(a.ln2), T, H, true, cs);
+  dgrad(dx.data_ptr(), H, a.wo, Q, t + a_dattn, Q, H);
+  wgrad(dx.data_ptr(), H, b + s.attn, Q, a.wo);
+  const uint8_t* qkv = b + s.qkv;
+  uint8_t* dqkv = t + a_dqkv;
+  agrpo::launch_attn_varlen_bwd(qkv, QKV, QKV, qkv, QKV, QKV, qkv, QKV, QKV, 0, Q, (a.Hq + a.Hkv) * a.D, b + s.attn, Q, t + a_dattn, Q, f32(s.lse),
+                                reinterpret_cast<float*>(t + a_delta), reinterpret_cast<float*>(t + a_dq), dqkv, QKV, dqkv, QKV, Q, dqkv, QKV,
+                                (a.Hq + a.Hkv) * a.D, tiles.data_ptr<int>(), (int)tiles.size(0), T, a.Hq, a.Hkv, a.D, (float)(1.0 / std::sqrt((double)a.D)), st, cs,
+                                rope);
+  if (a.bqkv >= 0) agrpo::launch_colsum(dqkv, g(a.bqkv), T, QKV, QKV, cs);
+  dgrad(dqkv, QKV, a.wqkv, H, dh, H, QKV);
+  wgrad(dqkv, QKV, b + s.h1, H, a.wqkv);
+  agrpo::launch_rmsnorm_bwd(dh, x.data_ptr(), a.w(a.ln1), f32(s.rstd1), dx.data_ptr(), g(a.ln1), T, H, true, cs);
+  return launches;
 }
 
 int64_t lmhead_num_groups(int64_t V, int64_t T) { return agrpo::lmhead_num_groups((int)V, (int)T); }
@@ -982,6 +1161,11 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("decode_layers_counter_words", &decode_layers_counter_words);
   m.def("gemm_swiglu", &gemm_swiglu, py::arg("a"), py::arg("b"), py::arg("d"), py::arg("ss_in") = py::none(), py::arg("eps") = 1e-6,
         py::arg("status") = py::none(), NOGIL);
+  m.def("layer_fwd", &layer_fwd, py::arg("params"), py::arg("offs"), py::arg("dims"), py::arg("eps"), py::arg("x"), py::arg("pos"),
+        py::arg("tiles"), py::arg("cos_t"), py::arg("sin_t"), py::arg("status"), py::arg("keep"), py::arg("slots") = py::none(),
+        py::arg("k_cache") = py::none(), py::arg("v_cache") = py::none(), py::arg("kv_head0") = 0, NOGIL);
+  m.def("layer_bwd", &layer_bwd, py::arg("params"), py::arg("grads"), py::arg("offs"), py::arg("dims"), py::arg("eps"), py::arg("dx"),
+        py::arg("x"), py::arg("slab"), py::arg("pos"), py::arg("tiles"), py::arg("cos_t"), py::arg("sin_t"), py::arg("status"), NOGIL);
   m.def("gemm_swiglu_bwd", &gemm_swiglu_bwd, py::arg("dy"), py::arg("w"), py::arg("gu"), py::arg("dgu"), py::arg("status") = py::none(), NOGIL);
   m.def("gemm_qkv_rope", &gemm_qkv_rope, py::arg("a"), py::arg("b"), py::arg("qkv"), py::arg("bias"), py::arg("pos"), py::arg("cos_t"),
         py::arg("sin_t"), py::arg("rot_heads"), py::arg("head_dim"), py::arg("status") = py::none(), NOGIL);

@@ -135,6 +135,10 @@ class NativeDecoder:
             weights.status = self.status
         self._rope: Optional[Tuple[torch.Tensor, torch.Tensor]] = None
         self.n_stats = int(self.C.grpo_num_loss_stats())
+        # resident parameters: a layer is one native call (offsets of its tensors in the flat buffer)
+        self._dims = [cfg.hidden_size, cfg.num_attention_heads, cfg.num_key_value_heads, cfg.head_dim, cfg.intermediate_size]
+        self._offs = [[layout.segments[f"layers.{i}.{n}"].offset if f"layers.{i}.{n}" in layout.segments else -1
+                       for n in ("ln1", "wqkv", "bqkv", "wo", "ln2", "wgu", "wd")] for i in range(cfg.num_hidden_layers)]
         self.launches = 0  # kernels of this package launched (bench bookkeeping)
 
     # ---- helpers ----
@@ -214,6 +218,14 @@ class NativeDecoder:
     def _layer_fwd(self, i: int, x: torch.Tensor, batch: PackedBatch, cos_t, sin_t, save: Optional[dict],
                    kv_write: Optional[tuple] = None, next_unit: Optional[int] = None):
         cfg, C = self.cfg, self.C
+        if self.weights is None:
+            k_cache, v_cache, slots, head0 = (tuple(kv_write) + (0,))[:4] if kv_write is not None else (None, None, None, 0)
+            out, slab, n = C.layer_fwd(self.params, self._offs[i], self._dims, cfg.rms_norm_eps, x, batch.pos, batch.tiles, cos_t, sin_t,
+                                       self.status, save is not None, slots, k_cache, v_cache, head0)
+            self.launches += n
+            if save is not None:
+                save.update(x=x, slab=slab)
+            return out
         T = x.shape[0]
         p = f"layers.{i}."
         self._enter_unit(i + 1, next_unit)
@@ -222,12 +234,6 @@ class NativeDecoder:
         C.rmsnorm_fwd(x, self.w(p + "ln1"), h1, rstd1, cfg.rms_norm_eps)
         qkv = self._new(T, cfg.qkv_dim)
         self._qkv(h1, p, qkv, batch.pos, cos_t, sin_t)
-        if kv_write is not None:  # rollout prefill: K/V of every prompt token go to their cache slots
-            k_cache, v_cache, slots = kv_write[:3]
-            head0 = kv_write[3] if len(kv_write) > 3 else 0  # tensor-parallel engine rank: its share of the kv heads
-            C.kv_cache_write(qkv, slots, k_cache, v_cache, cfg.num_attention_heads, cfg.num_key_value_heads, cfg.head_dim,
-                             self.status, head0)
-            self.launches += 1
         attn = self._new(T, cfg.q_dim)
         lse = self._new(cfg.num_attention_heads, T, dtype=torch.float32)
         C.attn_varlen_fwd(qkv, attn, lse, batch.tiles, cfg.num_attention_heads, cfg.num_key_value_heads, cfg.head_dim,
@@ -285,20 +291,20 @@ class NativeDecoder:
     def _layer_bwd(self, i: int, dx: torch.Tensor, s: dict, batch: PackedBatch, cos_t, sin_t, sink: GradSink):
         """dx (bf16 [T, H]) is the gradient w.r.t. the layer output; it is updated in place to the gradient w.r.t. the input."""
         cfg, C = self.cfg, self.C
+        if self.weights is None:
+            self.launches += C.layer_bwd(self.params, sink.flat, self._offs[i], self._dims, cfg.rms_norm_eps, dx, s["x"], s["slab"], batch.pos,
+                                         batch.tiles, cos_t, sin_t, self.status)
+            sink.unit_done(i + 1)
+            return
         T = dx.shape[0]
         p = f"layers.{i}."
         self._enter_unit(i + 1, i if i > 0 else None)
         # ---- MLP ----
         dgu = self._new(T, 2 * cfg.intermediate_size)
-        wd = self.w(p + "wd")
-        if self.weights is None and C.gemm_swiglu_bwd(dx, wd, s["gu"], dgu, self.status):
-            self.launches += 1
-        else:  # the same bits; sharded weights prefetch with the plain GEMM
-            dact = self._new(T, cfg.intermediate_size)
-            self._gemm(dx, wd, dact, b_mn=True)
-            C.swiglu_bwd(s["gu"], dact, dgu)
-            self.launches += 1
-            del dact
+        dact = self._new(T, cfg.intermediate_size)
+        self._gemm(dx, self.w(p + "wd"), dact, b_mn=True)
+        C.swiglu_bwd(s["gu"], dact, dgu)
+        del dact
         self._wgrad(dx, s["act"], p + "wd", sink)
         dh2 = self._new(T, cfg.hidden_size)
         self._gemm(dgu, self.w(p + "wgu"), dh2, b_mn=True)
@@ -321,7 +327,7 @@ class NativeDecoder:
         self._gemm(dqkv, self.w(p + "wqkv"), dh1, b_mn=True)
         self._wgrad(dqkv, s["h1"], p + "wqkv", sink)
         C.rmsnorm_bwd(dh1, s["x"], self.w(p + "ln1"), s["rstd1"], dx, sink.view(p + "ln1"), True)
-        self.launches += 9
+        self.launches += 10
         sink.unit_done(i + 1)
 
     # ---- public ----
