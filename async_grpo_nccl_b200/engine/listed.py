@@ -194,15 +194,19 @@ class ListedEngine(RolloutEngine):
             self._apply_table_updates({"upd_slot": u[:, 0].tolist(), "upd_index": u[:, 1].tolist(), "upd_block": u[:, 2].tolist()})
         for step in self._portions([(s, p, t) for _, s, p, t, _ in segs]):
             buf = self._forward(step)
-            t0 = 0
+            t0, picked, owners = 0, [], []
             for slot, past, toks in step:
                 n_entry, _, past0, _, want = next(e for e in segs if e[1] == slot)
                 rows = [t0 + past0 + w - past for w in want if past <= past0 + w < past + len(toks)]
                 if rows:
-                    z = self.dec.logits(self.dec.hidden(buf, torch.tensor(rows, device=self.dev)))
-                    out[n_entry] = torch.cat([out[n_entry], z]) if n_entry in out else z
+                    picked += rows
+                    owners.append((n_entry, len(rows)))
                 self.h_lens[slot] = past + len(toks)
                 t0 += len(toks)
+            if picked:  # one pass over the output matrix for the rows of all entries
+                z = self.dec.logits(self.dec.hidden(buf, torch.tensor(picked, device=self.dev)))
+                for (n_entry, _), part in zip(owners, z.split([n for _, n in owners])):
+                    out[n_entry] = torch.cat([out[n_entry], part]) if n_entry in out else part
         if dec:
             active = np.asarray([d[1] for d in dec], dtype=np.int64)
             feed = torch.tensor([[d[1] for d in dec], [int(d[3][0]) for d in dec]], dtype=torch.int64).pin_memory().to(self.dev, non_blocking=True)
@@ -212,9 +216,12 @@ class ListedEngine(RolloutEngine):
             self._stage_decode(active, none, none, none)
             B = min(self.max_seqs, (int(active.max()) + 32) // 32 * 32)
             self._decode_layers(B, self._choose_splits(B, len(dec), int(self.h_lens[active].max())))
-            for n_entry, slot, _, _, want in dec:
-                if want:
-                    out[n_entry] = self.dec.logits(self.dec.hidden(self.b_buf, slice(slot, slot + 1))).expand(len(want), -1)
+            asked = [i for i, d in enumerate(dec) if d[4]]
+            if asked:
+                rows = feed[0] if len(asked) == len(dec) else feed[0].index_select(0, torch.tensor(asked, device=self.dev))
+                z = self.dec.logits(self.dec.hidden(self.b_buf, rows))
+                for j, i in enumerate(asked):
+                    out[dec[i][0]] = z[j:j + 1].expand(len(dec[i][4]), -1)
         self.launches += self.dec.launches
         self.dec.launches = 0
         if not out:
