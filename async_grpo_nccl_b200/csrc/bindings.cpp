@@ -398,6 +398,12 @@ void check_tiles(const Tensor& tiles) {
   check_i32(tiles, "layer tiles");
   TORCH_CHECK(tiles.is_contiguous() && tiles.dim() == 2 && tiles.size(1) == 4 && (reinterpret_cast<uintptr_t>(tiles.data_ptr()) & 15) == 0, "layer: tiles [n, 4]");
 }
+// Programmatic dependent launch for the launches of a scope: the prologue of a kernel overlaps the tail of the one before.
+struct PdlScope {
+  bool before = agrpo::pdl_flag();
+  PdlScope() { agrpo::pdl_flag() = true; }
+  ~PdlScope() { agrpo::pdl_flag() = before; }
+};
 // Parts of one allocation, each on a 256-byte boundary.
 struct Carve {
   int64_t size = 0;
@@ -438,6 +444,7 @@ std::tuple<Tensor, Tensor, int64_t> layer_fwd(const Tensor& params, const std::v
   const auto f32 = [&](int64_t o) { return reinterpret_cast<float*>(b + o); };
   int* st = status.data_ptr<int>();
   const cudaStream_t cs = cur_stream();
+  const PdlScope pdl;
   int64_t launches = 7;
   agrpo::launch_rmsnorm_fwd(x.data_ptr(), a.w(a.ln1), b + s.h1, f32(s.rstd1), T, H, a.eps, cs);
   if (!agrpo::launch_gemm_qkv_rope(b + s.h1, H, a.w(a.wqkv), H, b + s.qkv, QKV, T, QKV, H, a.w(a.bqkv), rope, a.Hq + a.Hkv, a.D, st, sms, cs)) {
@@ -509,6 +516,7 @@ int64_t layer_bwd(const Tensor& params, Tensor& grads, const std::vector<int64_t
   const auto wgrad = [&](const void* dy, int M, const void* in, int N, int64_t w) {
     agrpo::launch_gemm_bf16(dy, M, in, N, g(w), N, M, N, T, true, true, nullptr, 1.f, true, true, st, sms, cs);
   };
+  const PdlScope pdl;
   int64_t launches = 14 + (a.bqkv >= 0 ? 1 : 0);
   if (!agrpo::launch_gemm_swiglu_bwd(dx.data_ptr(), H, a.w(a.wd), F, b + s.gu, 2 * F, t + m_dgu, 2 * F, T, F, H, st, sms, cs)) {
     Tensor alone;

@@ -115,6 +115,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  pdl_wait();
+  pdl_launch();
   const uint32_t tmem_base = *tmem_slot;
   const uint32_t tmem_R1 = tmem_base;        // S^T -> P^T (bf16) -> dQ
   const uint32_t tmem_R2 = tmem_base + 128;  // dP^T -> dS^T (bf16)
@@ -370,6 +372,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 // delta[h, t] = sum_d dO[t, h, d] * O[t, h, d]; one warp per (t, h).
 __global__ void attn_bwd_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ d_o,
                                       float* __restrict__ delta, int T, int Hq, int D, long long ldo, long long lddo) {
+  pdl_wait();
+  pdl_launch();
   const long long w = blockIdx.x * (long long)(blockDim.x >> 5) + (threadIdx.x >> 5);
   if (w >= (long long)T * Hq) return;
   const int lane = threadIdx.x & 31;
@@ -391,6 +395,8 @@ __global__ void attn_bwd_delta_kernel(const __nv_bfloat16* __restrict__ o, const
 // converts four columns of each half of a head.
 __global__ void attn_bwd_finalize_dq_kernel(const float* __restrict__ acc, __nv_bfloat16* __restrict__ dq, long long T, int Hq, int D,
                                             long long ld, const AttnRope rope) {
+  pdl_wait();
+  pdl_launch();
   const int per_head = D / 8;
   const long long total = T * Hq * per_head;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
@@ -421,8 +427,7 @@ void launch_bwd_t(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMa
   auto kernel = attn_bwd_kernel<D>;
   AGRPO_SET_MAX_DYN_SMEM(kernel, smem, "attn_bwd smem attr");
   dim3 grid(Hkv, n_tiles);
-  kernel<<<grid, kBwdThreads, smem, s>>>(tq, tk, tv, tdo, tdq, p);
-  check_cuda(cudaGetLastError(), "attn_bwd launch");
+  launch_kernel(kernel, grid, dim3(kBwdThreads), smem, s, "attn_bwd launch", tq, tk, tv, tdo, tdq, p);
 }
 
 }  // namespace
@@ -437,9 +442,8 @@ void launch_attn_varlen_bwd(const void* q, long long ldq, int q_cols, const void
   if (D != 64 && D != 128) throw std::runtime_error("attn_varlen_bwd: head_dim must be 64 or 128");
   {
     const long long warps = (long long)T * Hq;
-    attn_bwd_delta_kernel<<<(unsigned)((warps + 7) / 8), 256, 0, s>>>((const __nv_bfloat16*)out, (const __nv_bfloat16*)dout,
-                                                                     delta, T, Hq, D, ldo, lddo);
-    check_cuda(cudaGetLastError(), "attn_bwd_delta");
+    launch_kernel(attn_bwd_delta_kernel, dim3((unsigned)((warps + 7) / 8)), dim3(256), 0, s, "attn_bwd_delta", (const __nv_bfloat16*)out,
+                  (const __nv_bfloat16*)dout, delta, T, Hq, D, ldo, lddo);
   }
   check_cuda(cudaMemsetAsync(dq_acc, 0, (size_t)T * Hq * D * sizeof(float), s), "attn_bwd dq memset");
   const CUtensorMap tq = make_tmap_2d(q, q_cols, T, ldq, 64, kT);
@@ -473,8 +477,8 @@ void launch_attn_varlen_bwd(const void* q, long long ldq, int q_cols, const void
     const long long work = (long long)T * (Hq * D / 8);
     long long blocks = (work + 255) / 256;
     if (blocks > 148 * 16) blocks = 148 * 16;
-    attn_bwd_finalize_dq_kernel<<<(unsigned)blocks, 256, 0, s>>>(dq_acc, (__nv_bfloat16*)dq, T, Hq, D, ld_dq, rope);
-    check_cuda(cudaGetLastError(), "attn_bwd_finalize_dq");
+    launch_kernel(attn_bwd_finalize_dq_kernel, dim3((unsigned)blocks), dim3(256), 0, s, "attn_bwd_finalize_dq", (const float*)dq_acc,
+                  (__nv_bfloat16*)dq, (long long)T, Hq, D, ld_dq, rope);
   }
 }
 

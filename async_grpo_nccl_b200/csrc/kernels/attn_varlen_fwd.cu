@@ -83,6 +83,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  pdl_wait();
+  pdl_launch();
   const uint32_t tmem_base = *tmem_slot;
   const uint32_t tmem_S = tmem_base;
   const uint32_t tmem_O = tmem_base + 128;
@@ -285,8 +287,7 @@ void launch_fwd_t(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMa
   auto kernel = attn_fwd_kernel<D>;
   AGRPO_SET_MAX_DYN_SMEM(kernel, smem, "attn_fwd smem attr");
   dim3 grid(Hq, n_tiles);
-  kernel<<<grid, kAttnThreads, smem, s>>>(tq, tk, tv, p);
-  check_cuda(cudaGetLastError(), "attn_fwd launch");
+  launch_kernel(kernel, grid, dim3(kAttnThreads), smem, s, "attn_fwd launch", tq, tk, tv, p);
 }
 
 }  // namespace

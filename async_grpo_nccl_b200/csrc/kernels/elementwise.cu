@@ -150,6 +150,8 @@ __global__ void rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __
 __global__ void rmsnorm_bwd_dx_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
                                       const __nv_bfloat16* __restrict__ w, const float* __restrict__ rstd_in,
                                       __nv_bfloat16* __restrict__ dx, int T, int H, int accumulate) {
+  pdl_wait();
+  pdl_launch();
   const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (row >= T) return;
   const int lane = threadIdx.x & 31;
@@ -198,6 +200,8 @@ __global__ void rmsnorm_bwd_dx_kernel(const __nv_bfloat16* __restrict__ dy, cons
 __global__ void colsum_kernel(const __nv_bfloat16* __restrict__ a, const __nv_bfloat16* __restrict__ b,
                               const float* __restrict__ rscale, float* __restrict__ out, int T, int C, long long lda,
                               int rows_per_block) {
+  pdl_wait();
+  pdl_launch();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int c = blockIdx.x * 64 + lane * 2;
   const int r0 = blockIdx.y * rows_per_block;
@@ -393,24 +397,21 @@ void launch_rmsnorm_fwd(const void* x, const void* w, void* y, float* rstd, int 
 void launch_rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* rstd, void* dx, float* dw, int T,
                         int H, bool accumulate_dx, cudaStream_t s) {
   if (T == 0) return;
-  rmsnorm_bwd_dx_kernel<<<(T + 7) / 8, 256, 0, s>>>((const __nv_bfloat16*)dy, (const __nv_bfloat16*)x,
-                                                    (const __nv_bfloat16*)w, rstd, (__nv_bfloat16*)dx, T, H,
-                                                    accumulate_dx ? 1 : 0);
-  check_cuda(cudaGetLastError(), "rmsnorm_bwd_dx");
+  launch_kernel(rmsnorm_bwd_dx_kernel, dim3((T + 7) / 8), dim3(256), 0, s, "rmsnorm_bwd_dx", (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x,
+                (const __nv_bfloat16*)w, rstd, (__nv_bfloat16*)dx, T, H, accumulate_dx ? 1 : 0);
   if (dw != nullptr) {
     const int rows_per_block = 256;
     dim3 grid((H + 63) / 64, (T + rows_per_block - 1) / rows_per_block);
-    colsum_kernel<<<grid, 256, 0, s>>>((const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, rstd, dw, T, H, H,
-                                       rows_per_block);
-    check_cuda(cudaGetLastError(), "rmsnorm_bwd_dw");
+    launch_kernel(colsum_kernel, grid, dim3(256), 0, s, "rmsnorm_bwd_dw", (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, rstd, dw, T, H,
+                  (long long)H, rows_per_block);
   }
 }
 void launch_colsum(const void* a, float* out, int T, int C, long long lda, cudaStream_t s) {
   if (T == 0) return;
   const int rows_per_block = 256;
   dim3 grid((C + 63) / 64, (T + rows_per_block - 1) / rows_per_block);
-  colsum_kernel<<<grid, 256, 0, s>>>((const __nv_bfloat16*)a, nullptr, nullptr, out, T, C, lda, rows_per_block);
-  check_cuda(cudaGetLastError(), "colsum");
+  launch_kernel(colsum_kernel, grid, dim3(256), 0, s, "colsum", (const __nv_bfloat16*)a, (const __nv_bfloat16*)nullptr, (const float*)nullptr, out,
+                T, C, lda, rows_per_block);
 }
 void launch_rope(void* qkv, const int* pos, const float* cos_t, const float* sin_t, int T, int n_rot_heads, int D,
                  long long row_pitch, int max_pos, bool backward, cudaStream_t s) {
