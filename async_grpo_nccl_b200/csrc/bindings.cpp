@@ -356,13 +356,15 @@ void attn_varlen_bwd(const Tensor& qkv, const Tensor& out, const Tensor& dout, c
   TORCH_CHECK(qkv.stride(0) % 8 == 0 && dout.stride(0) % 8 == 0 && dqkv.stride(0) % 8 == 0, "attn_bwd: pitches");
   const agrpo::AttnRope rope = rope_args(pos, cos_t, sin_t, T, D);
   const c10::cuda::CUDAGuard guard(qkv.device());
+  Tensor dkv;
+  if (agrpo::attn_bwd_pieces((int)tiles.size(0), (int)Hq, (int)Hkv) > 1) dkv = at::empty({T, 2 * Hkv * D}, dq_acc.options());
   agrpo::launch_attn_varlen_bwd(qkv.data_ptr(), qkv.stride(0), (int)C, qkv.data_ptr(), qkv.stride(0), (int)C, qkv.data_ptr(),
                                 qkv.stride(0), (int)C, 0, (int)(Hq * D), (int)((Hq + Hkv) * D), out.data_ptr(), out.stride(0),
                                 dout.data_ptr(), dout.stride(0), lse.data_ptr<float>(), delta.data_ptr<float>(),
                                 dq_acc.data_ptr<float>(), dqkv.data_ptr(), dqkv.stride(0), dqkv.data_ptr(), dqkv.stride(0),
                                 (int)(Hq * D), dqkv.data_ptr(), dqkv.stride(0), (int)((Hq + Hkv) * D), tiles.data_ptr<int>(),
                                 (int)tiles.size(0), (int)T, (int)Hq, (int)Hkv, (int)D, (float)softmax_scale,
-                                opt_ptr<int>(status), cur_stream(), rope);
+                                opt_ptr<int>(status), cur_stream(), rope, dkv.defined() ? dkv.data_ptr<float>() : nullptr);
 }
 
 // ---- a whole decoder layer per call -------------------------------------------------------------------------------------------
@@ -502,6 +504,8 @@ int64_t layer_bwd(const Tensor& params, Tensor& grads, const std::vector<int64_t
   const int64_t m_dgu = cm.add((int64_t)T * 2 * F * 2), m_dact = cm.add(T <= 128 || F % 16 != 0 ? (int64_t)T * F * 2 : 0);
   const int64_t a_dattn = ca.add((int64_t)T * Q * 2), a_dqkv = ca.add((int64_t)T * QKV * 2), a_delta = ca.add((int64_t)T * a.Hq * 4),
                 a_dq = ca.add((int64_t)T * Q * 4);
+  const bool spread = agrpo::attn_bwd_pieces((int)tiles.size(0), a.Hq, a.Hkv) > 1;
+  const int64_t a_dkv = ca.add(spread ? (int64_t)T * 2 * a.Hkv * a.D * 4 : 0);
   const int64_t shared = std::max(cm.size, ca.size);
   Tensor tmp = at::empty({shared + (int64_t)T * H * 2}, x.options().dtype(torch::kUInt8));
   uint8_t* t = tmp.data_ptr<uint8_t>();
@@ -540,7 +544,8 @@ int64_t layer_bwd(const Tensor& params, Tensor& grads, const std::vector<int64_t
   agrpo::launch_attn_varlen_bwd(qkv, QKV, QKV, qkv, QKV, QKV, qkv, QKV, QKV, 0, Q, (a.Hq + a.Hkv) * a.D, b + s.attn, Q, t + a_dattn, Q, f32(s.lse),
                                 reinterpret_cast<float*>(t + a_delta), reinterpret_cast<float*>(t + a_dq), dqkv, QKV, dqkv, QKV, Q, dqkv, QKV,
                                 (a.Hq + a.Hkv) * a.D, tiles.data_ptr<int>(), (int)tiles.size(0), T, a.Hq, a.Hkv, a.D, (float)(1.0 / std::sqrt((double)a.D)), st, cs,
-                                rope);
+                                rope, spread ? reinterpret_cast<float*>(t + a_dkv) : nullptr);
+  if (spread) launches += 2;
   if (a.bqkv >= 0) agrpo::launch_colsum(dqkv, g(a.bqkv), T, QKV, QKV, cs);
   dgrad(dqkv, QKV, a.wqkv, H, dh, H, QKV);
   wgrad(dqkv, QKV, b + s.h1, H, a.wqkv);

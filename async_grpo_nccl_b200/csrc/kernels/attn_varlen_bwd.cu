@@ -14,6 +14,9 @@
 // a step waited for) and converted by attn_bwd_finalize_dq. Where rotary embedding came before the attention,
 // both take its transpose along on the way out.
 //
+// Where one CTA per (key tile, kv head) would leave SMs idle or waiting for the longest one, the group's
+// query heads are dealt to several CTAs, which add their dK / dV up in an fp32 accumulator like dQ.
+//
 // A step is a chain (S and dP, then the softmax gradient, then three products, then the read-out of dQ), and the
 // 512 columns leave no room for a second tile, so its length is what counts: eight warps share the
 // elementwise part, two per lane quarter with 64 queries each. P^T and dS^T of a warp stay inside the
@@ -40,7 +43,8 @@ struct AttnBwdParams {
   __nv_bfloat16* dv;
   long long ld_dk, ld_dv;
   int dk_col0, dv_col0;
-  int T, Hq, group;
+  int T, Hq, Hkv, group;
+  int pieces;         // CTAs that share the query heads of a (key tile, kv head); > 1: dK / dV go to the fp32 accumulator
   int q_col0, k_col0, v_col0;
   float scale, scale_log2;
   AttnRope rope;      // transposed rotation of dK, off when pos == nullptr
@@ -55,7 +59,7 @@ template <int D>
 __global__ void __launch_bounds__(kBwdThreads, 1)
 attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                 const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDO,
-                const __grid_constant__ CUtensorMap tmDQ, const AttnBwdParams p) {
+                const __grid_constant__ CUtensorMap tmDQ, const __grid_constant__ CUtensorMap tmDKV, const AttnBwdParams p) {
   constexpr int kChunks = D / 64;
   constexpr int kTileBytes = kT * D * 2;
   constexpr int kChunkBytes = kT * 128;     // one 64-column swizzle chunk of a 128-row tile
@@ -87,12 +91,13 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 11);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int kv_head = blockIdx.x;
+  const int kv_head = blockIdx.x / p.pieces, piece = blockIdx.x - kv_head * p.pieces;
+  const int head0 = kv_head * p.group + piece * p.group / p.pieces;  // first of this CTA's query heads
   // The table is sorted for the forward pass (heaviest query tile first); the heaviest key tile is the last.
   const int4 tile = p.tiles[gridDim.y - 1 - blockIdx.y];
   const int seq_start = tile.x, seq_len = tile.y, k0 = tile.z;
   const int n_q = (seq_len - k0 + kT - 1) / kT;
-  const int n_it = n_q * p.group;
+  const int n_it = n_q * ((piece + 1) * p.group / p.pieces - piece * p.group / p.pieces);
 
   if (threadIdx.x == 0) {
     mbar_init(kv_full, 1);
@@ -133,7 +138,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       }
       for (int it = 0; it < n_it; ++it) {
         const int hg = it / n_q, qt = it - hg * n_q;
-        const int head = kv_head * p.group + hg;
+        const int head = head0 + hg;
         const int row = seq_start + k0 + qt * kT;
         const int s = it & 1;
         if (it >= 2 && !mbar_wait(&q_empty[s], ((it >> 1) - 1) & 1)) {
@@ -219,7 +224,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     bool ok = true;
     for (int it = 0; it < n_it; ++it) {
       const int hg = it / n_q, qt = it - hg * n_q;
-      const int head = kv_head * p.group + hg;
+      const int head = head0 + hg;
       const int q0 = k0 + qt * kT;
       const int b = it & 1;
       {
@@ -320,6 +325,31 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     if (lane == 0) bulk_wait_all<0>();
     if (ok && n_it > 0) {
       // The last dq_full wait also covered the final dV / dK MMAs (commits are cumulative).
+      if (p.pieces > 1) {
+        // rows past the sequence are zero here too; the staging pieces of this warp are free (bulk_wait_all)
+        uint8_t* buf = sDS + (warp - 2) * 4096;
+        const int y = seq_start + k0 + quarter * 32;
+        if (k0 + quarter * 32 < seq_len) {
+#pragma unroll 1
+          for (int c = 0; c < D / 32; ++c) {
+            uint32_t o[32];
+            tmem_ld_32x32((part == 0 ? tmem_dV : tmem_dK) + lane_off + c * 32, o);
+            tc_wait_ld();
+            if (lane == 0) bulk_wait_read<0>();
+            __syncwarp();
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+              *reinterpret_cast<uint4*>(buf + lane * 128 + ((u ^ (lane & 7)) << 4)) = make_uint4(o[4 * u], o[4 * u + 1], o[4 * u + 2], o[4 * u + 3]);
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) {
+              tma_reduce_add_2d(&tmDKV, buf, ((part == 0 ? p.Hkv : 0) + kv_head) * D + c * 32, y);
+              bulk_commit();
+            }
+          }
+          if (lane == 0) bulk_wait_all<0>();
+        }
+      } else {
       const bool valid = kj < seq_len;
       const long long t = (long long)seq_start + kj;
       // the warps of part 0 write dV, those of part 1 dK, whose columns i and D / 2 + i rotate together
@@ -358,6 +388,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           store32(out + D / 2 + c * 32, x2);
         }
       }
+      }
     }
   }
 
@@ -391,21 +422,21 @@ __global__ void attn_bwd_delta_kernel(const __nv_bfloat16* __restrict__ o, const
   if (lane == 0) delta[(long long)h * T + t] = acc;
 }
 
-// dq (bf16, pitch ld, first Hq * D columns of each row) = dq_acc (fp32 [T, Hq * D]), rotated back where `rope` says so: a thread
-// converts four columns of each half of a head.
-__global__ void attn_bwd_finalize_dq_kernel(const float* __restrict__ acc, __nv_bfloat16* __restrict__ dq, long long T, int Hq, int D,
-                                            long long ld, const AttnRope rope) {
+// out (bf16, pitch ld, `heads` heads) = acc (fp32, pitch lda), rotated back where `rope` says so: a thread converts four columns of
+// each half of a head.
+__global__ void attn_bwd_finalize_kernel(const float* __restrict__ acc, long long lda, __nv_bfloat16* __restrict__ out, long long ld, long long T,
+                                         int heads, int D, const AttnRope rope) {
   pdl_wait();
   pdl_launch();
   const int per_head = D / 8;
-  const long long total = T * Hq * per_head;
+  const long long total = T * heads * per_head;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
     const int j = (int)(i % per_head) * 4;
     const long long th = i / per_head;
-    const long long t = th / Hq;
-    const int col = (int)(th % Hq) * D + j;
-    float4 a = __ldcs(reinterpret_cast<const float4*>(acc + t * Hq * D + col));
-    float4 b = __ldcs(reinterpret_cast<const float4*>(acc + t * Hq * D + col + D / 2));
+    const long long t = th / heads;
+    const int col = (int)(th % heads) * D + j;
+    float4 a = __ldcs(reinterpret_cast<const float4*>(acc + t * lda + col));
+    float4 b = __ldcs(reinterpret_cast<const float4*>(acc + t * lda + col + D / 2));
     if (rope.pos != nullptr) {
       const long long row = rope.row(t) * (D / 2) + j;
       const float4 c = *reinterpret_cast<const float4*>(rope.cos_t + row), s = *reinterpret_cast<const float4*>(rope.sin_t + row);
@@ -414,30 +445,46 @@ __global__ void attn_bwd_finalize_dq_kernel(const float* __restrict__ acc, __nv_
       rope_rotate(a.z, b.z, c.z, -s.z);
       rope_rotate(a.w, b.w, c.w, -s.w);
     }
-    __nv_bfloat16* d = dq + t * ld + col;
+    __nv_bfloat16* d = out + t * ld + col;
     *reinterpret_cast<uint2*>(d) = make_uint2(pack_bf16x2(a.x, a.y), pack_bf16x2(a.z, a.w));
     *reinterpret_cast<uint2*>(d + D / 2) = make_uint2(pack_bf16x2(b.x, b.y), pack_bf16x2(b.z, b.w));
   }
 }
+void finalize(const float* acc, long long lda, void* out, long long ld, int T, int heads, int D, const AttnRope& rope, cudaStream_t s) {
+  const long long blocks = ((long long)T * heads * (D / 8) + 255) / 256;
+  launch_kernel(attn_bwd_finalize_kernel, dim3((unsigned)(blocks < 148 * 16 ? blocks : 148 * 16)), dim3(256), 0, s, "attn_bwd_finalize", acc, lda,
+                (__nv_bfloat16*)out, ld, (long long)T, heads, D, rope);
+}
 
 template <int D>
 void launch_bwd_t(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tdo,
-                  const CUtensorMap& tdq, const AttnBwdParams& p, int n_tiles, int Hkv, cudaStream_t s) {
+                  const CUtensorMap& tdq, const CUtensorMap& tdkv, const AttnBwdParams& p, int n_tiles, int Hkv, cudaStream_t s) {
   constexpr int smem = 5 * kT * D * 2 + kT * kT * 2 + 4 * kT * 4 + 128 + 1024;
   auto kernel = attn_bwd_kernel<D>;
   AGRPO_SET_MAX_DYN_SMEM(kernel, smem, "attn_bwd smem attr");
-  dim3 grid(Hkv, n_tiles);
-  launch_kernel(kernel, grid, dim3(kBwdThreads), smem, s, "attn_bwd launch", tq, tk, tv, tdo, tdq, p);
+  dim3 grid(Hkv * p.pieces, n_tiles);
+  launch_kernel(kernel, grid, dim3(kBwdThreads), smem, s, "attn_bwd launch", tq, tk, tv, tdo, tdq, tdkv, p);
 }
 
 }  // namespace
+
+// CTAs over which the query heads of a (key tile, kv head) are dealt: enough for about four CTAs per SM, so that the longest of them
+// (all query tiles of the longest sequence) is a small part of an SM's share. 12 query and 2 kv heads, us with one and with several
+// pieces: one sequence of 759 tokens 210 -> 70, 11 sequences of up to 8575 2486 -> 2293, 19 of 330 145 -> 138; 820 CTAs (28 and 4
+// heads, 25415 tokens) gain nothing from a second piece (2557 and 2577).
+int attn_bwd_pieces(int n_tiles, int Hq, int Hkv) {
+  const long long ctas = (long long)n_tiles * Hkv;
+  if (ctas <= 0) return 1;
+  const long long want = (4 * 148 + ctas - 1) / ctas, group = Hq / Hkv;
+  return (int)(want < 1 ? 1 : want < group ? want : group);
+}
 
 void launch_attn_varlen_bwd(const void* q, long long ldq, int q_cols, const void* k, long long ldk, int k_cols,
                             const void* v, long long ldv, int v_cols, int q_col0, int k_col0, int v_col0, const void* out,
                             long long ldo, const void* dout, long long lddo, const float* lse, float* delta, float* dq_acc,
                             void* dq, long long ld_dq, void* dk, long long ld_dk, int dk_col0, void* dv, long long ld_dv,
                             int dv_col0, const int* tiles, int n_tiles, int T, int Hq, int Hkv, int D, float softmax_scale,
-                            int* status, cudaStream_t s, const AttnRope& rope) {
+                            int* status, cudaStream_t s, const AttnRope& rope, float* dkv_acc) {
   if (n_tiles == 0 || T == 0) return;
   if (D != 64 && D != 128) throw std::runtime_error("attn_varlen_bwd: head_dim must be 64 or 128");
   {
@@ -446,11 +493,14 @@ void launch_attn_varlen_bwd(const void* q, long long ldq, int q_cols, const void
                   (const __nv_bfloat16*)dout, delta, T, Hq, D, ldo, lddo);
   }
   check_cuda(cudaMemsetAsync(dq_acc, 0, (size_t)T * Hq * D * sizeof(float), s), "attn_bwd dq memset");
+  const int pieces = dkv_acc != nullptr ? attn_bwd_pieces(n_tiles, Hq, Hkv) : 1;
+  if (pieces > 1) check_cuda(cudaMemsetAsync(dkv_acc, 0, (size_t)T * 2 * Hkv * D * sizeof(float), s), "attn_bwd dkv memset");
   const CUtensorMap tq = make_tmap_2d(q, q_cols, T, ldq, 64, kT);
   const CUtensorMap tk = make_tmap_2d(k, k_cols, T, ldk, 64, kT);
   const CUtensorMap tv = make_tmap_2d(v, v_cols, T, ldv, 64, kT);
   const CUtensorMap tdo = make_tmap_2d(dout, (uint64_t)Hq * D, T, lddo, 64, kT);
   const CUtensorMap tdq = make_tmap_2d(dq_acc, (uint64_t)Hq * D, T, (uint64_t)Hq * D, 32, 32, 4);
+  const CUtensorMap tdkv = pieces > 1 ? make_tmap_2d(dkv_acc, 2ull * Hkv * D, T, 2ull * Hkv * D, 32, 32, 4) : tdq;
   AttnBwdParams p;
   p.tiles = reinterpret_cast<const int4*>(tiles);
   p.lse = lse;
@@ -463,7 +513,9 @@ void launch_attn_varlen_bwd(const void* q, long long ldq, int q_cols, const void
   p.dv_col0 = dv_col0;
   p.T = T;
   p.Hq = Hq;
+  p.Hkv = Hkv;
   p.group = Hq / Hkv;
+  p.pieces = pieces;
   p.q_col0 = q_col0;
   p.k_col0 = k_col0;
   p.v_col0 = v_col0;
@@ -471,14 +523,12 @@ void launch_attn_varlen_bwd(const void* q, long long ldq, int q_cols, const void
   p.scale_log2 = softmax_scale * 1.4426950408889634f;
   p.rope = rope;
   p.status = status;
-  if (D == 128) launch_bwd_t<128>(tq, tk, tv, tdo, tdq, p, n_tiles, Hkv, s);
-  else          launch_bwd_t<64>(tq, tk, tv, tdo, tdq, p, n_tiles, Hkv, s);
-  {
-    const long long work = (long long)T * (Hq * D / 8);
-    long long blocks = (work + 255) / 256;
-    if (blocks > 148 * 16) blocks = 148 * 16;
-    launch_kernel(attn_bwd_finalize_dq_kernel, dim3((unsigned)blocks), dim3(256), 0, s, "attn_bwd_finalize_dq", (const float*)dq_acc,
-                  (__nv_bfloat16*)dq, (long long)T, Hq, D, ld_dq, rope);
+  if (D == 128) launch_bwd_t<128>(tq, tk, tv, tdo, tdq, tdkv, p, n_tiles, Hkv, s);
+  else          launch_bwd_t<64>(tq, tk, tv, tdo, tdq, tdkv, p, n_tiles, Hkv, s);
+  finalize(dq_acc, (long long)Hq * D, dq, ld_dq, T, Hq, D, rope, s);
+  if (pieces > 1) {
+    finalize(dkv_acc, 2ll * Hkv * D, reinterpret_cast<__nv_bfloat16*>(dk) + dk_col0, ld_dk, T, Hkv, D, rope, s);
+    finalize(dkv_acc + Hkv * D, 2ll * Hkv * D, reinterpret_cast<__nv_bfloat16*>(dv) + dv_col0, ld_dv, T, Hkv, D, AttnRope{}, s);
   }
 }
 
