@@ -8,7 +8,8 @@
 //
 // Roles per CTA as in the plain kernel (TMA warp, MMA warp, epilogue warps); only rank 0 issues MMAs. `full` barriers live
 // in rank 0 and count the bytes of both CTAs; commits release the stage and publish the accumulator in both CTAs; `tempty` of
-// rank 0 is arrived at by the epilogue warps of both. An epilogue functor sees rows and columns exactly as in the plain kernel.
+// rank 0 is arrived at by the epilogue warps of both. An epilogue functor sees rows and columns exactly as in the plain kernel: the
+// two warps of a lane quarter share the columns of a tile, or, where an epilogue sums over them (kWholeTiles), take tiles in turn.
 #pragma once
 #include "gemm_tcgen05.cuh"
 #include "rope.cuh"
@@ -276,6 +277,11 @@ template <class Epi>
 struct EpiHalves<Epi, decltype((void)Epi::kHalves)> { static constexpr bool value = Epi::kHalves; };
 
 template <class Epi, class = void>
+struct EpiWholeTiles { static constexpr bool value = false; };
+template <class Epi>
+struct EpiWholeTiles<Epi, decltype((void)Epi::kWholeTiles)> { static constexpr bool value = Epi::kWholeTiles; };
+
+template <class Epi, class = void>
 struct EpiDual { static constexpr bool value = false; };
 template <class Epi>
 struct EpiDual<Epi, decltype((void)Epi::kDual)> { static constexpr bool value = Epi::kDual; };
@@ -284,7 +290,8 @@ struct EpiDual<Epi, decltype((void)Epi::kDual)> { static constexpr bool value = 
 // columns (measured at 31287 x 1536 x 8960: 546, 591, 638 us; a 192-wide MN-major tile of B is loaded as 256 columns and takes
 // 0.86), so a narrower tile pays where it saves a wave: at 6223 x 1536 x 8960 the 150 tiles of 256 columns need 3 waves of 74
 // pairs (153 us), 200 tiles of 192 columns need 3 cheaper ones (124 us); 1536 x 1536 x 31287 is 36 tiles (218 us) or 72 (130 us).
-inline int pair_pick_bn(int M, int N, bool b_mn, int num_sms, int n1 = 0) {
+// A width is a multiple of `unit`.
+inline int pair_pick_bn(int M, int N, bool b_mn, int num_sms, int n1 = 0, int unit = 1) {
   const int pairs = num_sms / 2 > 0 ? num_sms / 2 : 1;
   const int cands[3] = {256, 192, 128};
   const float cost[3] = {1.f, b_mn ? 0.86f : 0.80f, 0.60f};
@@ -292,6 +299,7 @@ inline int pair_pick_bn(int M, int N, bool b_mn, int num_sms, int n1 = 0) {
   float best_t = 0.f;
   for (int i = 0; i < 3; ++i) {
     const int bn = cands[i];
+    if (bn % unit != 0) continue;
     const int tiles_n = n1 > 0 ? (n1 + bn - 1) / bn + (N - n1 + bn - 1) / bn : (N + bn - 1) / bn;
     const int items = pair_num_items(M, tiles_n, 1);
     const float t = (float)((items + pairs - 1) / pairs) * cost[i];
@@ -326,7 +334,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   constexpr int kStages = S::kStages;
   constexpr uint32_t kTmemCols = BN > 128 ? 512 : 256;
   constexpr int kTmemBuf = kTmemCols / 2;  // columns from one accumulator to the other
-  constexpr int kEpiCols = BN / (EW / 4);   // columns of a tile that one epilogue warp converts
+  constexpr bool kWhole = EpiWholeTiles<Epi>::value;
+  static_assert(!kWhole || EW == 8, "two warps per lane quarter, one per accumulator");
+  constexpr int kEpiCols = kWhole ? BN : BN / (EW / 4);  // columns of a tile that one epilogue warp converts
   constexpr uint32_t kIdesc = umma_idesc_bf16(kPairBM, BN, A_MN ? 1 : 0, B_MN ? 1 : 0);
 
   extern __shared__ uint8_t smem_raw[];
@@ -354,7 +364,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(&tfull_bar[b], 1);
-      mbar_init(&tempty_bar[b], 2 * EW);  // the epilogue warps of both CTAs
+      mbar_init(&tempty_bar[b], kWhole ? EW : 2 * EW);  // the epilogue warps of both CTAs
     }
     fence_mbar_init();
     fence_cluster_barrier_init();
@@ -466,12 +476,19 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   } else {
     // ------------------------------ Epilogue ------------------------------
     const int quarter = warp & 3;
-    const int part = (warp - 2) >> 2;  // which kEpiCols columns of a tile
+    const int turn = (warp - 2) >> 2;
+    const int part = kWhole ? 0 : turn;  // which kEpiCols columns of a tile
     int local = 0;
     bool ok = true;
     for (int item = my_pair; item < num_items && ok; item += stride) {
       int tm, tn0, count;
       pair_item_coords(item, tiles_m, tiles_n, p.group_n, tm, tn0, count);
+      if constexpr (kWhole) {  // an item is one tile
+        if ((local & 1) != turn) {
+          ++local;
+          continue;
+        }
+      }
       const int row = tm * kPairBM + rank * kGemmBM + quarter * 32 + lane;
       epi.item_begin(row, p.M, p.N);
       for (int t = 0; t < count; ++t, ++local) {

@@ -9,8 +9,14 @@ namespace agrpo {
 
 namespace {
 
+// The row sums of squares go out as fixed-point numbers, so that their order does not matter; within `sum_cols` columns (the plain
+// kernel's column tile) they are added in fp32, column after column. A kernel of another tile width keeps to the same groups: the
+// row scales that follow, and with them every later layer, do not depend on which kernel ran. SUMS (CTA pairs): a warp takes whole tiles.
+template <bool SUMS>
 struct ProjEpilogue {
+  static constexpr bool kWholeTiles = SUMS;
   ProjOut o;
+  int sum_cols;
   float rs, sq, sk;
 
   __device__ __forceinline__ void item_begin(int row, int M, int) {
@@ -28,14 +34,23 @@ struct ProjEpilogue {
         o.store8(row, col0 + c, v, sq, sk);
       }
     }
+    if constexpr (SUMS) {
+      if ((col0 + 32) % sum_cols == 0) {
+        o.add_stats(row, sq, sk);
+        sq = sk = 0.f;
+      }
+    }
   }
   __device__ __forceinline__ void item_end(int row, int M, int, int) {
     if (row < M) o.add_stats(row, sq, sk);
   }
 };
 
+template <bool SUMS>
 struct ResidualEpilogue {
+  static constexpr bool kWholeTiles = SUMS;
   ResidualOut o;
+  int sum_cols;
   int bn;        // columns that a warp converts per tile
   float sq;
   float xn[32];  // residual of the next 32 columns, read ahead
@@ -65,6 +80,12 @@ struct ResidualEpilogue {
 #pragma unroll
         for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[c + i]);
         o.store8(row, col0 + c, xv + c, v, sq);
+      }
+    }
+    if constexpr (SUMS) {
+      if ((col0 + 32) % sum_cols == 0) {
+        o.add_stats(row, sq);
+        sq = 0.f;
       }
     }
   }
@@ -132,13 +153,12 @@ void launch_gemm_parallel_proj(const ParallelProjArgs& a, int num_sms, cudaStrea
   p.status = a.status;
   p.n1 = a.n2 > 0 ? a.n1 : 0;
   p.a2 = a.a2;
-  ProjEpilogue e;
-  e.o = out;
-  e.rs = 1.f;
-  e.sq = e.sk = 0.f;
-  const int a_cols = a.n2 > 0 ? a.a2 + a.K : a.K;
-  if (pair_serves(a.M, num_sms)) launch_pair_tiles(a.h, a.lda, a_cols, a.w, a.ldw, p, e, pair_pick_bn(p.M, p.N, false, num_sms, p.n1), num_sms, s);
-  else launch_tiles(a.h, a.lda, a_cols, a.w, a.ldw, p, e, pick_bn(p), num_sms, s);
+  const int a_cols = a.n2 > 0 ? a.a2 + a.K : a.K, plain_bn = pick_bn(p);
+  if (!pair_serves(a.M, num_sms)) launch_tiles(a.h, a.lda, a_cols, a.w, a.ldw, p, ProjEpilogue<false>{out, 0, 1.f, 0.f, 0.f}, plain_bn, num_sms, s);
+  else if (out.ss_q != nullptr) launch_pair_tiles(a.h, a.lda, a_cols, a.w, a.ldw, p, ProjEpilogue<true>{out, plain_bn, 1.f, 0.f, 0.f},
+                                                  pair_pick_bn(p.M, p.N, false, num_sms, p.n1, plain_bn), num_sms, s);
+  else launch_pair_tiles(a.h, a.lda, a_cols, a.w, a.ldw, p, ProjEpilogue<false>{out, 0, 1.f, 0.f, 0.f},
+                         pair_pick_bn(p.M, p.N, false, num_sms, p.n1), num_sms, s);
 }
 
 void launch_gemm_residual(const ResidualArgs& a, int num_sms, cudaStream_t s) {
@@ -149,17 +169,16 @@ void launch_gemm_residual(const ResidualArgs& a, int num_sms, cudaStream_t s) {
   p.M = a.M; p.N = a.N; p.K = a.K;
   p.group_n = 1;
   p.status = a.status;
-  ResidualEpilogue e;
-  e.o = out;
-  e.sq = 0.f;
-  if (pair_serves(a.M, num_sms)) {
+  const int plain_bn = pick_bn(p);
+  if (!pair_serves(a.M, num_sms)) {
+    launch_tiles(a.a, a.lda, a.K, a.w, a.ldw, p, ResidualEpilogue<false>{out, 0, plain_bn, 0.f, {}}, plain_bn, num_sms, s);
+  } else if (out.ss != nullptr) {
+    const int bn = pair_pick_bn(p.M, p.N, false, num_sms, 0, plain_bn);
+    launch_pair_tiles(a.a, a.lda, a.K, a.w, a.ldw, p, ResidualEpilogue<true>{out, plain_bn, bn, 0.f, {}}, bn, num_sms, s);
+  } else {
     const int bn = pair_pick_bn(p.M, p.N, false, num_sms);
-    e.bn = bn / 2;
-    launch_pair_tiles(a.a, a.lda, a.K, a.w, a.ldw, p, e, bn, num_sms, s);
-    return;
+    launch_pair_tiles(a.a, a.lda, a.K, a.w, a.ldw, p, ResidualEpilogue<false>{out, 0, bn / 2, 0.f, {}}, bn, num_sms, s);
   }
-  e.bn = pick_bn(p);
-  launch_tiles(a.a, a.lda, a.K, a.w, a.ldw, p, e, e.bn, num_sms, s);
 }
 
 void launch_gemm_split_store(const SplitStoreArgs& a, int num_sms, cudaStream_t s) {

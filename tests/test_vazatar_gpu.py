@@ -287,6 +287,64 @@ def test_residual_gemm(M, N, K, accumulate):
     assert float((xd.double().cpu() - ref).abs().max()) < 2e-5
 
 
+def sum_columns(M, n1, n2=0):
+    """Columns whose squares are added in fp32, one after the other: the widest of 256, 128, 64 that gives 120 tiles of 128 rows."""
+    tiles = lambda w: -(-M // 128) * (-(-n1 // w) + -(-n2 // w))
+    return next((w for w in (256, 128, 64) if tiles(w) >= 120), 32)
+
+
+def squares(v, a, b, step, chain):
+    """Fixed-point row sums of the squares of columns [a, b): fp32 with one rounding per operation inside each group of `step`
+    columns, an integer sum of the groups. `chain` columns are added up by themselves first (0: each directly)."""
+    f32 = lambda z: z.astype(np.float32).astype(np.longdouble)
+    total, v = np.zeros(v.shape[0], dtype=np.int64), v.astype(np.longdouble)
+    for g in range(a - a % step, b, step):
+        s = np.zeros(v.shape[0], dtype=np.longdouble)
+        lo, hi = max(a, g), min(b, g + step)
+        for c in range(lo, hi, chain or 1):
+            if chain:
+                part = np.zeros_like(s)
+                for j in range(c, c + chain):
+                    part = f32(v[:, j] * v[:, j] + part)
+                s = f32(s + part)
+            else:
+                s = f32(v[:, c] * v[:, c] + s)
+        total += np.rint(s * 2 ** 30).astype(np.int64)
+    return total
+
+
+# rows and columns for which 32, 64, 128 and 256 columns are one group, the last with a narrower and an incomplete last tile
+@pytest.mark.parametrize("M,N", [(300, 520), (1000, 1024), (2000, 1024), (4000, 1096), (6223, 1536)])
+def test_row_sums_of_the_residual_do_not_depend_on_the_kernel(M, N):
+    C, K = native(), 72
+    gen = torch.Generator().manual_seed(M)
+    a, w, x = rnd(gen, M, K), rnd(gen, N, K), torch.randn(M, N, generator=gen).cuda()
+    ss, st = torch.zeros(M, dtype=torch.int64, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+    C.gemm_residual(dev(a), dev(w), x, True, None, None, None, None, ss, st)
+    rows = torch.randperm(M, generator=gen)[:150]
+    want = squares(x.cpu()[rows].numpy(), 0, N, sum_columns(M, N), 0)
+    assert int(st.item()) == 0 and torch.equal(ss.cpu()[rows], torch.from_numpy(want))
+
+
+@pytest.mark.parametrize("M,n1,n2", [(300, 584, 64), (1000, 840, 200), (2000, 1096, 0), (4000, 1096, 264)])
+def test_row_sums_of_the_projection_do_not_depend_on_the_kernel(M, n1, n2):
+    """Whole numbers, so that the product is exact in fp32; the sums of their squares are rounded."""
+    C, K = native(), 64
+    gen = torch.Generator().manual_seed(M)
+    a, w = (torch.randint(-15, 16, s, generator=gen).double() for s in ((M, 2 * K), (n1 + n2, K)))
+    u = torch.empty(M, n1, device="cuda", dtype=torch.bfloat16)
+    act = torch.empty(M, n2, device="cuda", dtype=torch.bfloat16) if n2 else None
+    st = torch.zeros(1, dtype=torch.int32, device="cuda")
+    sq, sk = (torch.zeros(M, dtype=torch.int64, device="cuda") for _ in range(2))
+    q_end, k_end = n1 // 2 // 8 * 8, n1 - 40
+    C.gemm_parallel_proj(dev(a), dev(w), u, act, None, K, 1e-6, sq, sk, q_end, k_end, st)
+    rows, step = torch.randperm(M, generator=gen)[:150], sum_columns(M, n1, n2)
+    v = (a[rows, :K] @ w[:n1].T).numpy()
+    assert int(st.item()) == 0
+    assert torch.equal(sq.cpu()[rows], torch.from_numpy(squares(v, 0, q_end, step, 8)))
+    assert torch.equal(sk.cpu()[rows], torch.from_numpy(squares(v, q_end, k_end, step, 8)))
+
+
 @pytest.mark.parametrize("M,n1,n2,K", [(3, 16, 8, 64), (100, 96, 32, 640), (200, 112, 64, 512), (300, 32, 128, 200)])
 def test_gemm_with_two_kinds_of_output(M, n1, n2, K):
     C, g = native(), torch.Generator().manual_seed(M)
