@@ -275,6 +275,7 @@ bool launch_gemm_qkv_rope(const void* a, long long lda, const void* b, long long
                           const void* bias, const AttnRope& rope, int rot_heads, int head_dim, int* status, int num_sms, cudaStream_t stream) {
   if (head_dim != 128 || N % 128 != 0 || !pair_serves(M, num_sms) || !aligned32(qkv, ldd, 2) || (reinterpret_cast<uintptr_t>(bias) & 15) != 0)
     return false;
+  if (gemm_skinny_splits(M, N, K, num_sms) > 0) return false;  // the plain product is cut along K: other bits
   const CUtensorMap ta = make_tmap_2d(a, K, M, lda, 64, kGemmBM);
   const CUtensorMap tb = make_tmap_2d(b, K, N, ldb, 64, 128);
   GemmShape p;
@@ -294,7 +295,9 @@ bool launch_gemm_qkv_rope(const void* a, long long lda, const void* b, long long
 
 bool launch_gemm_mlp_in(const void* a, long long lda, const void* b, long long ldb, void* act, long long ldact, void* gu, long long ldgu,
                         int M, int F, int K, int* status, int num_sms, cudaStream_t stream) {
-  return M > 0 && launch_pair_swiglu<true>(a, lda, b, ldb, act, ldact, gu, ldgu, M, F, K, nullptr, 0.f, status, num_sms, stream);
+  // where the plain product is cut along K it has other bits
+  return M > 0 && gemm_skinny_splits(M, 2 * F, K, num_sms) == 0 &&
+         launch_pair_swiglu<true>(a, lda, b, ldb, act, ldact, gu, ldgu, M, F, K, nullptr, 0.f, status, num_sms, stream);
 }
 
 // act[M, F] = silu(rs * (a . Wg^T)) * (rs * (a . Wu^T)) with b = [Wg; Wu] stacked ([2F, K], the fused gate/up weight).

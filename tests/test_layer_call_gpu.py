@@ -1,0 +1,110 @@
+"""A decoder layer as one native call against the same kernels called one by one, bit for bit."""
+import pytest
+import torch
+
+from gpu_util import make_tiles, native, status_word
+
+pytestmark = pytest.mark.gpu
+DEV, EPS = "cuda", 1e-6
+H, HQ, HKV, F = 512, 4, 2, 528
+
+
+class Layer:
+    """Flat parameters of one layer and the inputs of a packed batch; sequences of one tile, so that no sum depends on an order."""
+
+    def __init__(self, lens, D=128, bias=True, seed=0):
+        g = torch.Generator(device=DEV).manual_seed(seed)
+        self.lens, self.D, self.T = lens, D, sum(lens)
+        qd, cols = HQ * D, (HQ + 2 * HKV) * D
+        shapes = dict(ln1=(H,), wqkv=(cols, H), bqkv=(cols,), wo=(H, qd), ln2=(H,), wgu=(2 * F, H), wd=(H, F))
+        if not bias:
+            del shapes["bqkv"]
+        self.offs, n = {}, 0
+        for k, s in shapes.items():
+            self.offs[k] = n
+            n += (torch.Size(s).numel() + 63) // 64 * 64
+        self.shapes = shapes
+        self.params = (torch.randn(n, device=DEV, generator=g) * 0.05).to(torch.bfloat16)
+        for k in ("ln1", "ln2"):
+            self.view(k).add_(1.0)
+        self.grads = torch.randn(n, device=DEV, generator=g)
+        self.x, self.dy = (torch.randn(self.T, H, device=DEV, generator=g).to(torch.bfloat16) for _ in range(2))
+        self.pos = torch.cat([torch.arange(m, dtype=torch.int32) for m in lens]).to(DEV)
+        ang = torch.randn(128, D // 2, device=DEV, generator=g)
+        self.cos, self.sin = ang.cos().contiguous(), ang.sin().contiguous()
+        self.tiles, self.st = make_tiles(lens), status_word()
+        self.dims = [H, HQ, HKV, D, F]
+        self.off_list = [self.offs.get(k, -1) for k in ("ln1", "wqkv", "bqkv", "wo", "ln2", "wgu", "wd")]
+
+    def view(self, k, flat=None):
+        flat = self.params if flat is None else flat
+        return flat[self.offs[k]:self.offs[k] + torch.Size(self.shapes[k]).numel()].view(self.shapes[k])
+
+    def new(self, *shape, dtype=torch.bfloat16):
+        return torch.zeros(shape, device=DEV, dtype=dtype)
+
+    def gemm(self, a, b, out, a_mn=False, b_mn=False, bias=None, accumulate=False, residual=None):
+        native().gemm_bf16(a, b, out, a_mn, b_mn, bias, 1.0, accumulate, self.st, residual)
+        return out
+
+    def forward(self):
+        C, T, D = native(), self.T, self.D
+        w, s = self.view, dict(rstd1=self.new(T, dtype=torch.float32), rstd2=self.new(T, dtype=torch.float32))
+        s["h1"] = self.new(T, H)
+        C.rmsnorm_fwd(self.x, w("ln1"), s["h1"], s["rstd1"], EPS)
+        s["qkv"] = self.gemm(s["h1"], w("wqkv"), self.new(T, (HQ + 2 * HKV) * D), bias=w("bqkv") if "bqkv" in self.offs else None)
+        C.rope_inplace(s["qkv"], self.pos, self.cos, self.sin, HQ + HKV, D, False)
+        s["attn"], s["lse"] = self.new(T, HQ * D), self.new(HQ, T, dtype=torch.float32)
+        C.attn_varlen_fwd(s["qkv"], s["attn"], s["lse"], self.tiles, HQ, HKV, D, D ** -0.5, self.st)
+        s["x1"] = self.gemm(s["attn"], w("wo"), self.new(T, H), residual=self.x)
+        s["h2"] = self.new(T, H)
+        C.rmsnorm_fwd(s["x1"], w("ln2"), s["h2"], s["rstd2"], EPS)
+        s["gu"], s["act"] = self.gemm(s["h2"], w("wgu"), self.new(T, 2 * F)), self.new(T, F)
+        C.swiglu_fwd(s["gu"], s["act"])
+        return self.gemm(s["act"], w("wd"), self.new(T, H), residual=s["x1"]), s
+
+    def backward(self, s, grads):
+        C, T, D = native(), self.T, self.D
+        w, g, dx = self.view, lambda k: self.view(k, grads), self.dy.clone()
+        dact, dgu = self.gemm(dx, w("wd"), self.new(T, F), b_mn=True), self.new(T, 2 * F)
+        C.swiglu_bwd(s["gu"], dact, dgu)
+        self.gemm(dx, s["act"], g("wd"), True, True, accumulate=True)
+        dh = self.gemm(dgu, w("wgu"), self.new(T, H), b_mn=True)
+        self.gemm(dgu, s["h2"], g("wgu"), True, True, accumulate=True)
+        C.rmsnorm_bwd(dh, s["x1"], w("ln2"), s["rstd2"], dx, g("ln2"), True)
+        dattn = self.gemm(dx, w("wo"), self.new(T, HQ * D), b_mn=True)
+        self.gemm(dx, s["attn"], g("wo"), True, True, accumulate=True)
+        dqkv, delta, acc = self.new(T, (HQ + 2 * HKV) * D), self.new(HQ, T, dtype=torch.float32), self.new(T, HQ * D, dtype=torch.float32)
+        C.attn_varlen_bwd(s["qkv"], s["attn"], dattn, s["lse"], delta, acc, dqkv, self.tiles, HQ, HKV, D, D ** -0.5, self.st, self.pos, self.cos, self.sin)
+        if "bqkv" in self.offs:
+            C.colsum(dqkv, g("bqkv"))
+        self.gemm(dqkv, w("wqkv"), dh, b_mn=True)
+        self.gemm(dqkv, s["h1"], g("wqkv"), True, True, accumulate=True)
+        C.rmsnorm_bwd(dh, self.x, w("ln1"), s["rstd1"], dx, g("ln1"), True)
+        return dx
+
+    def call_forward(self, keep, **kw):
+        return native().layer_fwd(self.params, self.off_list, self.dims, EPS, self.x, self.pos, self.tiles, self.cos, self.sin, self.st, keep, **kw)
+
+    def call_backward(self, slab, grads):
+        dx = self.dy.clone()
+        n = native().layer_bwd(self.params, grads, self.off_list, self.dims, EPS, dx, self.x, slab, self.pos, self.tiles, self.cos, self.sin, self.st)
+        return dx, n
+
+
+# one tile of rows; 129 - 256 rows: products with K-major operands are cut along K; more: CTA pairs. Heads of 64 are not rotated in the product
+@pytest.mark.parametrize("lens", [[60], [100, 29], [128, 72], [128, 128], [128, 128, 44]])
+@pytest.mark.parametrize("D,bias", [(128, True), (64, False)])
+def test_layer_call(lens, D, bias):
+    L = Layer(lens, D, bias, seed=sum(lens))
+    want, s = L.forward()
+    got, slab, _ = L.call_forward(True)
+    assert torch.equal(got, want)
+    assert torch.equal(L.call_forward(False)[0], want)
+    g0, g1 = L.grads.clone(), L.grads.clone()
+    want_dx = L.backward(s, g0)
+    dx, _ = L.call_backward(slab, g1)
+    assert int(L.st.item()) == 0
+    assert torch.equal(dx, want_dx)
+    for k in L.shapes:
+        assert torch.equal(L.view(k, g1), L.view(k, g0)), k
