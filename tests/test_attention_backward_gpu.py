@@ -62,3 +62,29 @@ def test_attention_backward_pieces(lens, Hq, Hkv, D):
     # P and dS are bf16 operands (2^-9 each), the result is bf16: a few 2^-9 of the gradient's size
     for a, b in ((0, Hq * D), (Hq * D, (Hq + Hkv) * D), ((Hq + Hkv) * D, cols)):
         assert rel_err(got[:, a:b].double(), x.grad[:, a:b]) < 2e-2
+
+
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+@pytest.mark.parametrize("Hq,Hkv,D", [(2, 2, 128), (2, 2, 64)])
+def test_attention_backward_keeps_sequences_apart(Hq, Hkv, D, bad):
+    """A sequence whose last keys are not finite: the gradients of the sequence after it, whose first rows share its tiles, are
+    bit for bit those without."""
+    C, st = native(), status_word()
+    torch.manual_seed(D)
+    lens, cols = [100, 120], (Hq + 2 * Hkv) * D
+    T, n = sum(lens), lens[0]
+    clean = torch.randn(T, cols, device=DEV).to(torch.bfloat16)
+    dout = torch.randn(T, Hq * D, device=DEV).to(torch.bfloat16)
+    tiles, sc, grads = make_tiles(lens), D ** -0.5, []
+    for poison in (False, True):
+        qkv = clean.clone()
+        if poison:
+            qkv[n - 2, Hq * D:(Hq + Hkv) * D] = bad
+        out, lse = torch.empty_like(dout), torch.empty(Hq, T, device=DEV)
+        C.attn_varlen_fwd(qkv, out, lse, tiles, Hq, Hkv, D, sc, st)
+        delta, acc, got = torch.empty(Hq, T, device=DEV), torch.empty(T, Hq * D, device=DEV), torch.zeros(T, cols, device=DEV, dtype=torch.bfloat16)
+        C.attn_varlen_bwd(qkv, out, dout, lse, delta, acc, got, tiles, Hq, Hkv, D, sc, st)
+        grads.append(got)
+    assert int(st.item()) == 0
+    assert bool(grads[0].isfinite().all()) and not bool(grads[1][:n].isfinite().all())
+    assert torch.equal(grads[1][n:], grads[0][n:])
