@@ -356,15 +356,16 @@ void attn_varlen_bwd(const Tensor& qkv, const Tensor& out, const Tensor& dout, c
   TORCH_CHECK(qkv.stride(0) % 8 == 0 && dout.stride(0) % 8 == 0 && dqkv.stride(0) % 8 == 0, "attn_bwd: pitches");
   const agrpo::AttnRope rope = rope_args(pos, cos_t, sin_t, T, D);
   const c10::cuda::CUDAGuard guard(qkv.device());
+  const int pieces = agrpo::attn_bwd_pieces((int)tiles.size(0), (int)Hq, (int)Hkv, num_sms());
   Tensor dkv;
-  if (agrpo::attn_bwd_pieces((int)tiles.size(0), (int)Hq, (int)Hkv) > 1) dkv = at::empty({T, 2 * Hkv * D}, dq_acc.options());
+  if (pieces > 1) dkv = at::empty({pieces, tiles.size(0), 2 * Hkv, 128, D}, dq_acc.options());
   agrpo::launch_attn_varlen_bwd(qkv.data_ptr(), qkv.stride(0), (int)C, qkv.data_ptr(), qkv.stride(0), (int)C, qkv.data_ptr(),
                                 qkv.stride(0), (int)C, 0, (int)(Hq * D), (int)((Hq + Hkv) * D), out.data_ptr(), out.stride(0),
                                 dout.data_ptr(), dout.stride(0), lse.data_ptr<float>(), delta.data_ptr<float>(),
                                 dq_acc.data_ptr<float>(), dqkv.data_ptr(), dqkv.stride(0), dqkv.data_ptr(), dqkv.stride(0),
                                 (int)(Hq * D), dqkv.data_ptr(), dqkv.stride(0), (int)((Hq + Hkv) * D), tiles.data_ptr<int>(),
                                 (int)tiles.size(0), (int)T, (int)Hq, (int)Hkv, (int)D, (float)softmax_scale,
-                                opt_ptr<int>(status), cur_stream(), rope, dkv.defined() ? dkv.data_ptr<float>() : nullptr);
+                                opt_ptr<int>(status), cur_stream(), rope, pieces, dkv.defined() ? dkv.data_ptr<float>() : nullptr);
 }
 
 // ---- a whole decoder layer per call -------------------------------------------------------------------------------------------
@@ -504,8 +505,8 @@ int64_t layer_bwd(const Tensor& params, Tensor& grads, const std::vector<int64_t
   const int64_t m_dgu = cm.add((int64_t)T * 2 * F * 2), m_dact = cm.add(T <= 128 || F % 16 != 0 ? (int64_t)T * F * 2 : 0);
   const int64_t a_dattn = ca.add((int64_t)T * Q * 2), a_dqkv = ca.add((int64_t)T * QKV * 2), a_delta = ca.add((int64_t)T * a.Hq * 4),
                 a_dq = ca.add((int64_t)T * Q * 4);
-  const bool spread = agrpo::attn_bwd_pieces((int)tiles.size(0), a.Hq, a.Hkv) > 1;
-  const int64_t a_dkv = ca.add(spread ? (int64_t)T * 2 * a.Hkv * a.D * 4 : 0);
+  const int pieces = agrpo::attn_bwd_pieces((int)tiles.size(0), a.Hq, a.Hkv, sms);
+  const int64_t a_dkv = ca.add(pieces > 1 ? (int64_t)pieces * tiles.size(0) * 2 * a.Hkv * 128 * a.D * 4 : 0);
   const int64_t shared = std::max(cm.size, ca.size);
   Tensor tmp = at::empty({shared + (int64_t)T * H * 2}, x.options().dtype(torch::kUInt8));
   uint8_t* t = tmp.data_ptr<uint8_t>();
@@ -544,8 +545,8 @@ int64_t layer_bwd(const Tensor& params, Tensor& grads, const std::vector<int64_t
   agrpo::launch_attn_varlen_bwd(qkv, QKV, QKV, qkv, QKV, QKV, qkv, QKV, QKV, 0, Q, (a.Hq + a.Hkv) * a.D, b + s.attn, Q, t + a_dattn, Q, f32(s.lse),
                                 reinterpret_cast<float*>(t + a_delta), reinterpret_cast<float*>(t + a_dq), dqkv, QKV, dqkv, QKV, Q, dqkv, QKV,
                                 (a.Hq + a.Hkv) * a.D, tiles.data_ptr<int>(), (int)tiles.size(0), T, a.Hq, a.Hkv, a.D, (float)(1.0 / std::sqrt((double)a.D)), st, cs,
-                                rope, spread ? reinterpret_cast<float*>(t + a_dkv) : nullptr);
-  if (spread) launches += 2;
+                                rope, pieces, pieces > 1 ? reinterpret_cast<float*>(t + a_dkv) : nullptr);
+  if (pieces > 1) ++launches;
   if (a.bqkv >= 0) agrpo::launch_colsum(dqkv, g(a.bqkv), T, QKV, QKV, cs);
   dgrad(dqkv, QKV, a.wqkv, H, dh, H, QKV);
   wgrad(dqkv, QKV, b + s.h1, H, a.wqkv);
@@ -553,6 +554,7 @@ int64_t layer_bwd(const Tensor& params, Tensor& grads, const std::vector<int64_t
   return launches;
 }
 
+int64_t attn_bwd_pieces(int64_t n_tiles, int64_t Hq, int64_t Hkv) { return agrpo::attn_bwd_pieces((int)n_tiles, (int)Hq, (int)Hkv, num_sms()); }
 int64_t lmhead_num_groups(int64_t V, int64_t T) { return agrpo::lmhead_num_groups((int)V, (int)T); }
 int64_t grpo_num_loss_stats() { return agrpo::grpo_num_loss_stats(); }
 
@@ -1198,6 +1200,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         py::arg("delta"), py::arg("dq_acc"), py::arg("dqkv"), py::arg("tiles"), py::arg("Hq"), py::arg("Hkv"), py::arg("D"),
         py::arg("softmax_scale"), py::arg("status") = py::none(), py::arg("pos") = py::none(), py::arg("cos_t") = py::none(),
         py::arg("sin_t") = py::none(), NOGIL);
+  m.def("attn_bwd_pieces", &attn_bwd_pieces);
   m.def("lmhead_num_groups", &lmhead_num_groups);
   m.def("grpo_num_loss_stats", &grpo_num_loss_stats);
   m.def("lmhead_logprob", &lmhead_logprob, py::arg("hidden"), py::arg("weight"), py::arg("labels"), py::arg("temperature"),

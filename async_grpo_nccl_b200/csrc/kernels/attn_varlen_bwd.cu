@@ -11,11 +11,12 @@
 //   dQ   = dS K                                         (dS^T staged in shared memory, MN-major)
 // dK / dV leave as bf16 once per CTA; dQ partial tiles are added to an fp32 accumulator by TMA from the
 // shared memory of dS (whole lines; as 16-byte reductions of single threads, 4096 a step, they were what
-// a step waited for) and converted by attn_bwd_finalize_dq. Where rotary embedding came before the attention,
+// a step waited for) and converted by attn_bwd_finalize_kernel. Where rotary embedding came before the attention,
 // both take its transpose along on the way out.
 //
 // Where one CTA per (key tile, kv head) would leave SMs idle or waiting for the longest one, the group's
-// query heads are dealt to several CTAs, which add their dK / dV up in an fp32 accumulator like dQ.
+// query heads are dealt to several CTAs. Each stores its fp32 dK / dV, and a second kernel adds them up in order: unlike dQ, whose
+// tiles arrive in any order, dK and dV repeat bit for bit. Only rows of the tiles are written.
 //
 // A step is a chain (S and dP, then the softmax gradient, then three products, then the read-out of dQ), and the
 // 512 columns leave no room for a second tile, so its length is what counts: eight warps share the
@@ -44,7 +45,8 @@ struct AttnBwdParams {
   long long ld_dk, ld_dv;
   int dk_col0, dv_col0;
   int T, Hq, Hkv, group;
-  int pieces;         // CTAs that share the query heads of a (key tile, kv head); > 1: dK / dV go to the fp32 accumulator
+  int pieces;         // CTAs that share the query heads of a (key tile, kv head)
+  float* dkv;         // pieces > 1: dK / dV go here (part_offset)
   int q_col0, k_col0, v_col0;
   float scale, scale_log2;
   AttnRope rope;      // transposed rotation of dK, off when pos == nullptr
@@ -55,11 +57,18 @@ __device__ __forceinline__ void named_bar_sync(int id, int count) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(count) : "memory");
 }
 
+// Where the 32 rows `quarter` of a tile and head (K's heads, then V's) of one piece start: [D / 4 column groups][32 rows][4 columns],
+// the order in which a warp reads them from tensor memory.
+template <int D>
+__device__ __forceinline__ long long part_offset(int piece, int n_tiles, int tile, int Hkv, int head, int quarter) {
+  return ((((long long)piece * n_tiles + tile) * 2 * Hkv + head) * 4 + quarter) * (32 * D);
+}
+
 template <int D>
 __global__ void __launch_bounds__(kBwdThreads, 1)
 attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                 const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDO,
-                const __grid_constant__ CUtensorMap tmDQ, const __grid_constant__ CUtensorMap tmDKV, const AttnBwdParams p) {
+                const __grid_constant__ CUtensorMap tmDQ, const AttnBwdParams p) {
   constexpr int kChunks = D / 64;
   constexpr int kTileBytes = kT * D * 2;
   constexpr int kChunkBytes = kT * 128;     // one 64-column swizzle chunk of a 128-row tile
@@ -94,7 +103,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   const int kv_head = blockIdx.x / p.pieces, piece = blockIdx.x - kv_head * p.pieces;
   const int head0 = kv_head * p.group + piece * p.group / p.pieces;  // first of this CTA's query heads
   // The table is sorted for the forward pass (heaviest query tile first); the heaviest key tile is the last.
-  const int4 tile = p.tiles[gridDim.y - 1 - blockIdx.y];
+  const int tile_idx = gridDim.y - 1 - blockIdx.y;
+  const int4 tile = p.tiles[tile_idx];
   const int seq_start = tile.x, seq_len = tile.y, k0 = tile.z;
   const int n_q = (seq_len - k0 + kT - 1) / kT;
   const int n_it = n_q * ((piece + 1) * p.group / p.pieces - piece * p.group / p.pieces);
@@ -330,33 +340,22 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     if (lane == 0) bulk_wait_all<0>();
     if (ok && n_it > 0) {
       // The last dq_full wait also covered the final dV / dK MMAs (commits are cumulative).
-      if (p.pieces > 1) {
-        // rows past the sequence are zero here too; the staging pieces of this warp are free (bulk_wait_all)
-        uint8_t* buf = sDS + (warp - 2) * 4096;
-        const int y = seq_start + k0 + quarter * 32;
-        if (k0 + quarter * 32 < seq_len) {
-#pragma unroll 1
-          for (int c = 0; c < D / 32; ++c) {
-            uint32_t o[32];
-            tmem_ld_32x32((part == 0 ? tmem_dV : tmem_dK) + lane_off + c * 32, o);
-            tc_wait_ld();
-            if (lane == 0) bulk_wait_read<0>();
-            __syncwarp();
-#pragma unroll
-            for (int u = 0; u < 8; ++u)
-              *reinterpret_cast<uint4*>(buf + lane * 128 + ((u ^ (lane & 7)) << 4)) = make_uint4(o[4 * u], o[4 * u + 1], o[4 * u + 2], o[4 * u + 3]);
-            fence_proxy_async_smem();
-            __syncwarp();
-            if (lane == 0) {
-              tma_reduce_add_2d(&tmDKV, buf, ((part == 0 ? p.Hkv : 0) + kv_head) * D + c * 32, y);
-              bulk_commit();
-            }
-          }
-          if (lane == 0) bulk_wait_all<0>();
-        }
-      } else {
       const bool valid = kj < seq_len;
       const long long t = (long long)seq_start + kj;
+      const uint32_t acc = (part == 0 ? tmem_dV : tmem_dK) + lane_off;
+      if (p.pieces > 1) {
+        float* out = p.dkv + part_offset<D>(piece, gridDim.y, tile_idx, p.Hkv, (part == 0 ? p.Hkv : 0) + kv_head, quarter) + lane * 4;
+#pragma unroll 1
+        for (int c = 0; c < D / 32; ++c) {
+          uint32_t o[32];
+          tmem_ld_32x32(acc + c * 32, o);
+          tc_wait_ld();
+          if (valid) {
+#pragma unroll
+            for (int i = 0; i < 32; i += 4) *reinterpret_cast<uint4*>(out + (c * 8 + i / 4) * 128) = make_uint4(o[i], o[i + 1], o[i + 2], o[i + 3]);
+          }
+        }
+      } else {
       // the warps of part 0 write dV, those of part 1 dK, whose columns i and D / 2 + i rotate together
       const auto store32 = [](__nv_bfloat16* dst, const float (&v)[32]) {
 #pragma unroll
@@ -370,7 +369,6 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         }
       };
       __nv_bfloat16* out = part == 0 ? p.dv + t * p.ld_dv + p.dv_col0 + (long long)kv_head * D : p.dk + t * p.ld_dk + p.dk_col0 + (long long)kv_head * D;
-      const uint32_t acc = (part == 0 ? tmem_dV : tmem_dK) + lane_off;
 #pragma unroll 1
       for (int c = 0; c < D / 64; ++c) {
         uint32_t lo[32], hi[32];
@@ -455,6 +453,51 @@ __global__ void attn_bwd_finalize_kernel(const float* __restrict__ acc, long lon
     *reinterpret_cast<uint2*>(d + D / 2) = make_uint2(pack_bf16x2(b.x, b.y), pack_bf16x2(b.z, b.w));
   }
 }
+
+// dK and dV (bf16) from the pieces' parts, summed in the order of the pieces, K rotated back where `rope` says so. A block takes one
+// part (32 rows of one tile, blockIdx.z: quarter) of one head (blockIdx.y: the heads of K, then those of V); a thread converts 16
+// columns of each half of a head, so that a warp reads whole lines and writes whole sectors.
+template <int D>
+__global__ void __launch_bounds__(D)
+attn_bwd_finalize_dkv_kernel(const float* __restrict__ acc, int pieces, const int4* __restrict__ tiles, __nv_bfloat16* __restrict__ dk, long long ld_dk,
+                             __nv_bfloat16* __restrict__ dv, long long ld_dv, int Hkv, const AttnRope rope) {
+  pdl_wait();
+  pdl_launch();
+  const int4 tile = tiles[blockIdx.x];
+  const int lane = threadIdx.x & 31, j = (threadIdx.x >> 5) * 16, head = blockIdx.y;  // D / 32 warps of 16 columns each
+  const int kj = tile.z + blockIdx.z * 32 + lane;
+  if (kj >= tile.y) return;
+  const bool is_k = head < Hkv;
+  const long long t = (long long)tile.x + kj;
+  float a[16] = {}, b[16] = {};
+#pragma unroll 2
+  for (int q = 0; q < pieces; ++q) {
+    const float* src = acc + part_offset<D>(q, gridDim.x, blockIdx.x, Hkv, head, blockIdx.z) + lane * 4;
+    float4 x[4], y[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      x[i] = __ldcs(reinterpret_cast<const float4*>(src + (j / 4 + i) * 128));
+      y[i] = __ldcs(reinterpret_cast<const float4*>(src + ((j + D / 2) / 4 + i) * 128));
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      a[4 * i] += x[i].x; a[4 * i + 1] += x[i].y; a[4 * i + 2] += x[i].z; a[4 * i + 3] += x[i].w;
+      b[4 * i] += y[i].x; b[4 * i + 1] += y[i].y; b[4 * i + 2] += y[i].z; b[4 * i + 3] += y[i].w;
+    }
+  }
+  if (is_k && rope.pos != nullptr) {
+    const long long row = rope.row(t) * (D / 2) + j;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) rope_rotate(a[i], b[i], rope.cos_t[row + i], -rope.sin_t[row + i]);
+  }
+  __nv_bfloat16* d = (is_k ? dk + t * ld_dk + head * D : dv + t * ld_dv + (head - Hkv) * D) + j;
+#pragma unroll
+  for (int i = 0; i < 16; i += 8) {
+    *reinterpret_cast<uint4*>(d + i) = make_uint4(pack_bf16x2(a[i], a[i + 1]), pack_bf16x2(a[i + 2], a[i + 3]), pack_bf16x2(a[i + 4], a[i + 5]), pack_bf16x2(a[i + 6], a[i + 7]));
+    *reinterpret_cast<uint4*>(d + D / 2 + i) = make_uint4(pack_bf16x2(b[i], b[i + 1]), pack_bf16x2(b[i + 2], b[i + 3]), pack_bf16x2(b[i + 4], b[i + 5]), pack_bf16x2(b[i + 6], b[i + 7]));
+  }
+}
+
 void finalize(const float* acc, long long lda, void* out, long long ld, int T, int heads, int D, const AttnRope& rope, cudaStream_t s) {
   const long long blocks = ((long long)T * heads * (D / 8) + 255) / 256;
   launch_kernel(attn_bwd_finalize_kernel, dim3((unsigned)(blocks < 148 * 16 ? blocks : 148 * 16)), dim3(256), 0, s, "attn_bwd_finalize", acc, lda,
@@ -463,24 +506,25 @@ void finalize(const float* acc, long long lda, void* out, long long ld, int T, i
 
 template <int D>
 void launch_bwd_t(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tdo,
-                  const CUtensorMap& tdq, const CUtensorMap& tdkv, const AttnBwdParams& p, int n_tiles, int Hkv, cudaStream_t s) {
+                  const CUtensorMap& tdq, const AttnBwdParams& p, int n_tiles, int Hkv, cudaStream_t s) {
   constexpr int smem = 5 * kT * D * 2 + kT * kT * 2 + 4 * kT * 4 + 128 + 1024;
   auto kernel = attn_bwd_kernel<D>;
   AGRPO_SET_MAX_DYN_SMEM(kernel, smem, "attn_bwd smem attr");
   dim3 grid(Hkv * p.pieces, n_tiles);
-  launch_kernel(kernel, grid, dim3(kBwdThreads), smem, s, "attn_bwd launch", tq, tk, tv, tdo, tdq, tdkv, p);
+  launch_kernel(kernel, grid, dim3(kBwdThreads), smem, s, "attn_bwd launch", tq, tk, tv, tdo, tdq, p);
 }
 
 }  // namespace
 
 // CTAs over which the query heads of a (key tile, kv head) are dealt: enough for about four CTAs per SM, so that the longest of them
-// (all query tiles of the longest sequence) is a small part of an SM's share. 12 query and 2 kv heads, us with one and with several
-// pieces: one sequence of 759 tokens 210 -> 70, 11 sequences of up to 8575 2486 -> 2293, 19 of 330 145 -> 138; 820 CTAs (28 and 4
-// heads, 25415 tokens) gain nothing from a second piece (2557 and 2577).
-int attn_bwd_pieces(int n_tiles, int Hq, int Hkv) {
+// (all query tiles of the longest sequence) is a small part of an SM's share. 12 query and 2 kv heads, us with one piece and with as
+// many as this rule says: one sequence of 759 tokens 210 and 66 (6 pieces), of 8000 1988 and 994 (5), 19 of 330 142 and 136 (6), 11 of up
+// to 8575 2492 and 2342 (2); sequences of one length gain less or nothing: 40 of 330 216 and 232 (3), 8 of 4096 2045 and 2058 (2). 824
+// CTAs (28 and 4 heads, 25415 tokens) are left as they are.
+int attn_bwd_pieces(int n_tiles, int Hq, int Hkv, int num_sms) {
   const long long ctas = (long long)n_tiles * Hkv;
   if (ctas <= 0) return 1;
-  const long long want = (4 * 148 + ctas - 1) / ctas, group = Hq / Hkv;
+  const long long want = (4 * num_sms + ctas - 1) / ctas, group = Hq / Hkv;
   return (int)(want < 1 ? 1 : want < group ? want : group);
 }
 
@@ -489,7 +533,7 @@ void launch_attn_varlen_bwd(const void* q, long long ldq, int q_cols, const void
                             long long ldo, const void* dout, long long lddo, const float* lse, float* delta, float* dq_acc,
                             void* dq, long long ld_dq, void* dk, long long ld_dk, int dk_col0, void* dv, long long ld_dv,
                             int dv_col0, const int* tiles, int n_tiles, int T, int Hq, int Hkv, int D, float softmax_scale,
-                            int* status, cudaStream_t s, const AttnRope& rope, float* dkv_acc) {
+                            int* status, cudaStream_t s, const AttnRope& rope, int pieces, float* dkv_acc) {
   if (n_tiles == 0 || T == 0) return;
   if (D != 64 && D != 128) throw std::runtime_error("attn_varlen_bwd: head_dim must be 64 or 128");
   {
@@ -498,14 +542,11 @@ void launch_attn_varlen_bwd(const void* q, long long ldq, int q_cols, const void
                   (const __nv_bfloat16*)dout, delta, T, Hq, D, ldo, lddo);
   }
   check_cuda(cudaMemsetAsync(dq_acc, 0, (size_t)T * Hq * D * sizeof(float), s), "attn_bwd dq memset");
-  const int pieces = dkv_acc != nullptr ? attn_bwd_pieces(n_tiles, Hq, Hkv) : 1;
-  if (pieces > 1) check_cuda(cudaMemsetAsync(dkv_acc, 0, (size_t)T * 2 * Hkv * D * sizeof(float), s), "attn_bwd dkv memset");
   const CUtensorMap tq = make_tmap_2d(q, q_cols, T, ldq, 64, kT);
   const CUtensorMap tk = make_tmap_2d(k, k_cols, T, ldk, 64, kT);
   const CUtensorMap tv = make_tmap_2d(v, v_cols, T, ldv, 64, kT);
   const CUtensorMap tdo = make_tmap_2d(dout, (uint64_t)Hq * D, T, lddo, 64, kT);
   const CUtensorMap tdq = make_tmap_2d(dq_acc, (uint64_t)Hq * D, T, (uint64_t)Hq * D, 32, 32, 4);
-  const CUtensorMap tdkv = pieces > 1 ? make_tmap_2d(dkv_acc, 2ull * Hkv * D, T, 2ull * Hkv * D, 32, 32, 4) : tdq;
   AttnBwdParams p;
   p.tiles = reinterpret_cast<const int4*>(tiles);
   p.lse = lse;
@@ -521,6 +562,7 @@ void launch_attn_varlen_bwd(const void* q, long long ldq, int q_cols, const void
   p.Hkv = Hkv;
   p.group = Hq / Hkv;
   p.pieces = pieces;
+  p.dkv = dkv_acc;
   p.q_col0 = q_col0;
   p.k_col0 = k_col0;
   p.v_col0 = v_col0;
@@ -528,13 +570,12 @@ void launch_attn_varlen_bwd(const void* q, long long ldq, int q_cols, const void
   p.scale_log2 = softmax_scale * 1.4426950408889634f;
   p.rope = rope;
   p.status = status;
-  if (D == 128) launch_bwd_t<128>(tq, tk, tv, tdo, tdq, tdkv, p, n_tiles, Hkv, s);
-  else          launch_bwd_t<64>(tq, tk, tv, tdo, tdq, tdkv, p, n_tiles, Hkv, s);
+  if (D == 128) launch_bwd_t<128>(tq, tk, tv, tdo, tdq, p, n_tiles, Hkv, s);
+  else          launch_bwd_t<64>(tq, tk, tv, tdo, tdq, p, n_tiles, Hkv, s);
   finalize(dq_acc, (long long)Hq * D, dq, ld_dq, T, Hq, D, rope, s);
-  if (pieces > 1) {
-    finalize(dkv_acc, 2ll * Hkv * D, reinterpret_cast<__nv_bfloat16*>(dk) + dk_col0, ld_dk, T, Hkv, D, rope, s);
-    finalize(dkv_acc + Hkv * D, 2ll * Hkv * D, reinterpret_cast<__nv_bfloat16*>(dv) + dv_col0, ld_dv, T, Hkv, D, AttnRope{}, s);
-  }
+  if (pieces > 1)
+    launch_kernel(D == 128 ? attn_bwd_finalize_dkv_kernel<128> : attn_bwd_finalize_dkv_kernel<64>, dim3(n_tiles, 2 * Hkv, 4), dim3(D), 0, s,
+                  "attn_bwd_finalize_dkv", (const float*)dkv_acc, pieces, p.tiles, p.dk + dk_col0, ld_dk, p.dv + dv_col0, ld_dv, Hkv, rope);
 }
 
 }  // namespace agrpo

@@ -220,9 +220,9 @@ void launch_attn_varlen_bwd(const void* q, long long ldq, int q_cols, const void
                             long long ldo, const void* dout, long long lddo, const float* lse, float* delta, float* dq_acc,
                             void* dq, long long ld_dq, void* dk, long long ld_dk, int dk_col0, void* dv, long long ld_dv,
                             int dv_col0, const int* tiles, int n_tiles, int T, int Hq, int Hkv, int D, float softmax_scale,
-                            int* status, cudaStream_t s, const AttnRope& rope = AttnRope{}, float* dkv_acc = nullptr);
-// > 1: dkv_acc (fp32 [T, 2 * Hkv * D] scratch) is needed to spread the work over more CTAs; without it each kv head is one.
-int attn_bwd_pieces(int n_tiles, int Hq, int Hkv);
+                            int* status, cudaStream_t s, const AttnRope& rope = AttnRope{}, int pieces = 1, float* dkv_acc = nullptr);
+// CTAs to spread a kv head's work over; more than one need dkv_acc, fp32 [pieces, n_tiles, 2 * Hkv, 128, D] scratch.
+int attn_bwd_pieces(int n_tiles, int Hq, int Hkv, int num_sms);
 
 // ---- fused lm_head + GRPO loss (lmhead_loss.cu) ----
 // Number of partial-statistics groups the forward writes for a [T, V] problem.

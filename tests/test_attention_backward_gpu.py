@@ -37,7 +37,7 @@ def test_attention_backward_rotates(D):
 # 1 key tile per head: as many CTAs as query heads; 7 heads in 7, in 2 (100 tiles x 4 kv heads) and in 1 piece (600 x 4)
 @pytest.mark.parametrize("lens,Hq,Hkv,D", [([5, 128], 6, 2, 128), ([300, 129, 1], 7, 1, 64), ([128] * 100, 28, 4, 128), ([40] * 600, 28, 4, 64)])
 def test_attention_backward_pieces(lens, Hq, Hkv, D):
-    """Query heads of a group dealt to several CTAs, against fp64; rows outside the sequences' tiles stay as they were."""
+    """Query heads of a group dealt to several CTAs, against fp64; dK and dV repeat bit for bit."""
     C, st = native(), status_word()
     torch.manual_seed(len(lens))
     T, cols, g = sum(lens), (Hq + 2 * Hkv) * D, Hq // Hkv
@@ -50,6 +50,10 @@ def test_attention_backward_pieces(lens, Hq, Hkv, D):
     got = torch.zeros(T, cols, device=DEV, dtype=torch.bfloat16)
     C.attn_varlen_bwd(qkv, out, dout, lse, delta, acc, got, tiles, Hq, Hkv, D, sc, st)
     assert int(st.item()) == 0
+    for _ in range(4):
+        again = torch.zeros_like(got)
+        C.attn_varlen_bwd(qkv, out, dout, lse, delta, acc, again, tiles, Hq, Hkv, D, sc, st)
+        assert torch.equal(again[:, Hq * D:], got[:, Hq * D:])
     x = qkv.double().requires_grad_(True)
     h, o, outs = x.view(T, Hq + 2 * Hkv, D), 0, []
     for n in lens:
@@ -65,26 +69,46 @@ def test_attention_backward_pieces(lens, Hq, Hkv, D):
 
 
 @pytest.mark.parametrize("bad", [float("inf"), float("nan")])
-@pytest.mark.parametrize("Hq,Hkv,D", [(2, 2, 128), (2, 2, 64)])
+@pytest.mark.parametrize("Hq,Hkv,D", [(2, 2, 128), (2, 2, 64), (6, 2, 128), (6, 2, 64)])
 def test_attention_backward_keeps_sequences_apart(Hq, Hkv, D, bad):
-    """A sequence whose last keys are not finite: the gradients of the sequence after it, whose first rows share its tiles, are
-    bit for bit those without."""
+    """A sequence whose last rows are not finite: the gradients of the sequence after it, whose first rows share its tiles, are
+    bit for bit those without, with one CTA per kv head and with several."""
     C, st = native(), status_word()
     torch.manual_seed(D)
     lens, cols = [100, 120], (Hq + 2 * Hkv) * D
     T, n = sum(lens), lens[0]
     clean = torch.randn(T, cols, device=DEV).to(torch.bfloat16)
-    dout = torch.randn(T, Hq * D, device=DEV).to(torch.bfloat16)
+    clean_dout = torch.randn(T, Hq * D, device=DEV).to(torch.bfloat16)
     tiles, sc, grads = make_tiles(lens), D ** -0.5, []
     for poison in (False, True):
-        qkv = clean.clone()
+        qkv, dout = clean.clone(), clean_dout.clone()
         if poison:
-            qkv[n - 2, Hq * D:(Hq + Hkv) * D] = bad
+            qkv[n - 2], dout[n - 2] = bad, bad
         out, lse = torch.empty_like(dout), torch.empty(Hq, T, device=DEV)
         C.attn_varlen_fwd(qkv, out, lse, tiles, Hq, Hkv, D, sc, st)
+        assert (C.attn_bwd_pieces(tiles.shape[0], Hq, Hkv) > 1) == (Hq > Hkv)
         delta, acc, got = torch.empty(Hq, T, device=DEV), torch.empty(T, Hq * D, device=DEV), torch.zeros(T, cols, device=DEV, dtype=torch.bfloat16)
         C.attn_varlen_bwd(qkv, out, dout, lse, delta, acc, got, tiles, Hq, Hkv, D, sc, st)
         grads.append(got)
     assert int(st.item()) == 0
     assert bool(grads[0].isfinite().all()) and not bool(grads[1][:n].isfinite().all())
     assert torch.equal(grads[1][n:], grads[0][n:])
+
+
+@pytest.mark.parametrize("Hq,Hkv", [(2, 2), (6, 2)])
+def test_attention_backward_writes_rows_of_its_tiles(Hq, Hkv):
+    """Rows that belong to no tile: dK and dV stay as they were, with one CTA per kv head and with several."""
+    C, st, D = native(), status_word(), 64
+    torch.manual_seed(Hq)
+    lens, rest = [130, 40], 50
+    T, cols = sum(lens) + rest, (Hq + 2 * Hkv) * D
+    qkv = torch.randn(T, cols, device=DEV).to(torch.bfloat16)
+    dout = torch.randn(T, Hq * D, device=DEV).to(torch.bfloat16)
+    out, lse, tiles = torch.zeros_like(dout), torch.zeros(Hq, T, device=DEV), make_tiles(lens)
+    C.attn_varlen_fwd(qkv, out, lse, tiles, Hq, Hkv, D, D ** -0.5, st)
+    delta, acc = torch.empty(Hq, T, device=DEV), torch.empty(T, Hq * D, device=DEV)
+    got = torch.full((T, cols), 7.0, device=DEV, dtype=torch.bfloat16)
+    C.attn_varlen_bwd(qkv, out, dout, lse, delta, acc, got, tiles, Hq, Hkv, D, D ** -0.5, st)
+    assert int(st.item()) == 0
+    assert bool((got[-rest:, Hq * D:] == 7.0).all()) and bool((got[-rest:, :Hq * D] == 0.0).all())
+    assert not bool((got[:-rest] == 7.0).all(1).any())
