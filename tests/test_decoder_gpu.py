@@ -488,3 +488,27 @@ def test_engine_prefix_cache_hits_do_not_change_tokens():
     eng.add_request("a3", pa, n=1, max_new_tokens=4, temperature=0.0, seed=1, ignore_eos=True)
     eng.run_until_done()
     assert eng.prefix_hit_tokens == 96
+
+
+@pytest.mark.parametrize("n", [2000, 2600])
+def test_training_steps_on_one_long_sequence_come_to_an_end(n):
+    """Many steps in a row; every wait of the kernels is bounded and would show in the status word."""
+    from async_grpo_nccl_b200.models.config import PRESETS
+    from async_grpo_nccl_b200.models.decoder import GradSink, LossConfig, NativeDecoder
+    from async_grpo_nccl_b200.models.layout import ParamLayout
+    from async_grpo_nccl_b200.packing import pack_samples
+    from dataclasses import replace
+
+    cfg = replace(PRESETS["qwen2.5-1.5b"], num_hidden_layers=4)
+    layout = ParamLayout(cfg)
+    flat = torch.empty(layout.total, dtype=torch.bfloat16, device=DEV)
+    layout.init_random_device_(flat, 0)
+    rng = np.random.default_rng(0)
+    batch = pack_samples([{"sample_ids": rng.integers(0, 1000, n).astype(np.int32), "input_len": n // 3, "output_len": n - n // 3, "advantage": 1.0}],
+                         pin=False).to_device(DEV)
+    dec, sink = NativeDecoder(cfg, layout, flat), GradSink(layout, DEV)
+    for _ in range(40):
+        dec.forward_backward(batch, LossConfig(kl_beta=0.0, temperature=1.0), 1.0, sink)
+    torch.cuda.synchronize()
+    dec.check_status()
+    assert bool(sink.flat.isfinite().all())
