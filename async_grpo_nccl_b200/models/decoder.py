@@ -234,6 +234,11 @@ class NativeDecoder:
         C.rmsnorm_fwd(x, self.w(p + "ln1"), h1, rstd1, cfg.rms_norm_eps)
         qkv = self._new(T, cfg.qkv_dim)
         self._qkv(h1, p, qkv, batch.pos, cos_t, sin_t)
+        if kv_write is not None:  # rollout prefill: K/V of every prompt token go to their cache slots
+            k_cache, v_cache, slots, head0 = (tuple(kv_write) + (0,))[:4]  # tensor-parallel engine rank: its share of the kv heads
+            C.kv_cache_write(qkv, slots, k_cache, v_cache, cfg.num_attention_heads, cfg.num_key_value_heads, cfg.head_dim,
+                             self.status, head0)
+            self.launches += 1
         attn = self._new(T, cfg.q_dim)
         lse = self._new(cfg.num_attention_heads, T, dtype=torch.float32)
         C.attn_varlen_fwd(qkv, attn, lse, batch.tiles, cfg.num_attention_heads, cfg.num_key_value_heads, cfg.head_dim,

@@ -1,4 +1,6 @@
-"""A decoder layer as one native call against the same kernels called one by one, bit for bit."""
+"""A decoder layer as one native call against the same kernels called one by one, bit for bit; the decoder over resident parameters
+(one call per layer) and over parameters handed out unit by unit (kernels called one by one)."""
+import numpy as np
 import pytest
 import torch
 
@@ -108,3 +110,54 @@ def test_layer_call(lens, D, bias):
     assert torch.equal(dx, want_dx)
     for k in L.shapes:
         assert torch.equal(L.view(k, g1), L.view(k, g0)), k
+
+
+class Units:
+    """A provider of parameters unit by unit that has all of them at hand."""
+
+    def __init__(self, layout, flat):
+        self.layout, self.flat, self.device, self.status = layout, flat, flat.device, None
+
+    def view(self, name):
+        return self.layout.view(self.flat, name)
+
+    def enter(self, unit, then):
+        return 0
+
+    def wants_ride(self, a, b):
+        return False
+
+
+def decoders(lens):
+    from async_grpo_nccl_b200.models.config import PRESETS
+    from async_grpo_nccl_b200.models.decoder import NativeDecoder
+    from async_grpo_nccl_b200.models.layout import ParamLayout
+    from async_grpo_nccl_b200.packing import pack_samples
+
+    cfg = PRESETS["tiny128"]
+    layout = ParamLayout(cfg)
+    p32 = torch.empty(layout.total)
+    layout.init_random_(p32, 0)
+    flat = p32.to(torch.bfloat16).to(DEV)
+    rng = np.random.default_rng(3)
+    samples = [{"sample_ids": rng.integers(0, cfg.vocab_size, n).astype(np.int32), "input_len": n // 3, "output_len": n - n // 3, "advantage": 1.0}
+               for n in lens]
+    batch = pack_samples(samples, pin=False).to_device(DEV)
+    return cfg, layout, batch, NativeDecoder(cfg, layout, flat), NativeDecoder(cfg, layout, None, weights=Units(layout, flat))
+
+
+def test_prompt_layer_writes_the_cache_with_either_kind_of_parameters():
+    cfg, layout, batch, resident, sharded = decoders([40, 100, 7])
+    T, bs = batch.T, 16
+    blocks = (T + bs - 1) // bs
+    slots = torch.randperm(blocks * bs, generator=torch.Generator().manual_seed(0))[:T].to(torch.int32).to(DEV)
+    x = torch.randn(T, cfg.hidden_size, device=DEV).to(torch.bfloat16)
+    got = []
+    for dec in (resident, sharded):
+        k, v = (torch.full((blocks, cfg.num_key_value_heads, bs, cfg.head_dim), 5.0, device=DEV, dtype=torch.bfloat16) for _ in range(2))
+        cos_t, sin_t = dec.rope_tables(1)
+        out = dec._layer_fwd(0, x, batch, cos_t, sin_t, None, kv_write=(k, v, slots))
+        dec.check_status()
+        got.append((out, k, v))
+    assert all(torch.equal(a, b) for a, b in zip(*got))
+    assert int((got[1][1] != 5.0).any(-1).any(1).sum()) == T
