@@ -369,7 +369,7 @@ void attn_varlen_bwd(const Tensor& qkv, const Tensor& out, const Tensor& dout, c
 }
 
 // ---- a whole decoder layer per call -------------------------------------------------------------------------------------------
-// Small batches are bound by the host: a layer is 8 launches forward and 14 backward of a few microseconds each, and issuing them
+// Small batches are bound by the host: a layer is 7 launches forward and 15 backward of a few microseconds each, and issuing them
 // one by one from Python, with an allocation and a view for each tensor, took about 150 us a layer. Here a layer is one call and
 // its activations are one allocation.
 struct LayerArgs {
@@ -524,7 +524,7 @@ int64_t layer_bwd(const Tensor& params, Tensor& grads, const std::vector<int64_t
   };
   // Launched one after the other, without programmatic dependent launch: with it, training steps on one sequence of 2000 to 2600 tokens
   // came to a stop now and then (up to one in a few dozen), for a cause that has not been found.
-  int64_t launches = 14 + (a.bqkv >= 0 ? 1 : 0);
+  int64_t launches = 15 + (a.bqkv >= 0 ? 1 : 0);
   if (!agrpo::launch_gemm_swiglu_bwd(dx.data_ptr(), H, a.w(a.wd), F, b + s.gu, 2 * F, t + m_dgu, 2 * F, T, F, H, st, sms, cs)) {
     Tensor alone;
     void* dact = t + m_dact;

@@ -251,7 +251,7 @@ class NativeDecoder:
         gu, act = self._mlp_in(h2, self.w(p + "wgu"), save is not None)
         x2 = self._new(T, cfg.hidden_size)
         self._gemm(act, self.w(p + "wd"), x2, residual=x1)
-        self.launches += 4
+        self.launches += 3
         if save is not None:
             save.update(x=x, h1=h1, rstd1=rstd1, qkv=qkv, attn=attn, lse=lse, x1=x1, h2=h2, rstd2=rstd2, gu=gu, act=act)
         return x2
@@ -290,7 +290,7 @@ class NativeDecoder:
         _, act = self._mlp_in(h2, self.w(p + "wgu"), False)
         x2 = self._new(Ts, cfg.hidden_size)
         self._gemm(act, self.w(p + "wd"), x2, residual=x1)
-        self.launches += 10
+        self.launches += 4
         return x2
 
     def _layer_bwd(self, i: int, dx: torch.Tensor, s: dict, batch: PackedBatch, cos_t, sin_t, sink: GradSink):
@@ -332,7 +332,9 @@ class NativeDecoder:
         self._gemm(dqkv, self.w(p + "wqkv"), dh1, b_mn=True)
         self._wgrad(dqkv, s["h1"], p + "wqkv", sink)
         C.rmsnorm_bwd(dh1, s["x"], self.w(p + "ln1"), s["rstd1"], dx, sink.view(p + "ln1"), True)
-        self.launches += 10
+        # SwiGLU, two norms of two kernels, attention with its row products and its conversions (one more for shared kv heads)
+        spread = C.attn_bwd_pieces(batch.tiles.shape[0], cfg.num_attention_heads, cfg.num_key_value_heads) > 1
+        self.launches += 8 + spread + cfg.attention_bias
         sink.unit_done(i + 1)
 
     # ---- public ----
@@ -425,7 +427,7 @@ class NativeDecoder:
         dx = self._new(T, cfg.hidden_size)
         C.rmsnorm_bwd(dhn, x_last, self.w("final_norm"), rstd_f, dx, sink.view("final_norm"), False)
         del dhn
-        self.launches += 8 + 3 * ((V + chunk - 1) // chunk)
+        self.launches += 6 + 3 * ((V + chunk - 1) // chunk)
         for i in reversed(range(cfg.num_hidden_layers)):
             s = saves[i]
             if self.recompute:

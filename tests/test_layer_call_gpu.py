@@ -161,3 +161,28 @@ def test_prompt_layer_writes_the_cache_with_either_kind_of_parameters():
         got.append((out, k, v))
     assert all(torch.equal(a, b) for a, b in zip(*got))
     assert int((got[1][1] != 5.0).any(-1).any(1).sum()) == T
+
+
+def package_kernels(fn):
+    """Kernels of this package that `fn` launches."""
+    from torch.profiler import ProfilerActivity, profile
+
+    with profile(activities=[ProfilerActivity.CUDA]) as p:
+        fn()
+        torch.cuda.synchronize()
+    return sum(e.count for e in p.key_averages() if "agrpo" in e.key)
+
+
+# 60 rows: plain kernels; 200: products cut along K; 400: CTA pairs
+@pytest.mark.parametrize("lens", [[60], [120, 80], [128, 128, 144]])
+def test_launches_are_counted(lens):
+    from async_grpo_nccl_b200.models.decoder import GradSink, LossConfig
+
+    cfg, layout, batch, resident, sharded = decoders(lens)
+    lc, sink = LossConfig(kl_beta=0.0, temperature=1.0), GradSink(layout, DEV)
+    for dec in (resident, sharded):
+        for fn in (lambda: dec.logprobs(batch, 1.0), lambda: dec.forward_backward(batch, lc, 0.5, sink)):
+            fn()
+            before = dec.launches
+            seen = package_kernels(fn)
+            assert dec.launches - before == seen
