@@ -117,6 +117,11 @@ struct LmDlogitsEpilogue {
         for (int j = 0; j < 8; ++j) o[j] = pack_bf16x2(d[i + 2 * j], d[i + 2 * j + 1]);
         st_global_32b(dst + i, o);
       }
+    } else if (col0 + 32 <= N && ((reinterpret_cast<uintptr_t>(dst) & 15) == 0)) {  // a buffer width that is no multiple of 16
+#pragma unroll
+      for (int i = 0; i < 32; i += 8)
+        *reinterpret_cast<uint4*>(dst + i) = make_uint4(pack_bf16x2(d[i], d[i + 1]), pack_bf16x2(d[i + 2], d[i + 3]),
+                                                        pack_bf16x2(d[i + 4], d[i + 5]), pack_bf16x2(d[i + 6], d[i + 7]));
     } else {
       for (int i = 0; i < 32; ++i)
         if (col0 + i < N) dst[i] = __float2bfloat16(d[i]);

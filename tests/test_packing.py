@@ -60,3 +60,14 @@ def test_dummy_and_logprob_packing():
         assert np.array_equal(lp.labels[off:off + L - 1].numpy(), s["sample_ids"][1:])
         assert lp.labels[off + L - 1].item() == -100
         off += L
+
+
+def test_width_of_the_dlogits_buffer():
+    """What the caller asks for is what it gets; else by rows, within 1 GiB and at least 4096 columns."""
+    from async_grpo_nccl_b200.models.decoder import vocab_chunk
+
+    for asked in (256, 3840, 4096, 8192, 15359, 20000):
+        assert vocab_chunk(36000, asked) == asked and vocab_chunk(1, asked) == asked
+    assert vocab_chunk(759) == 15360 and vocab_chunk(0) == 15360
+    assert vocab_chunk(50000) == 10496 and 50000 * vocab_chunk(50000) * 2 <= 1 << 30
+    assert vocab_chunk(400000) == 4096
