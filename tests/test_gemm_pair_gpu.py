@@ -106,7 +106,8 @@ def test_qkv_with_rotation(M, Hq, Hkv, K):
 
 
 # F = 264: no 32-byte rows; 128 rows: not served
-@pytest.mark.parametrize("M,F,K", [(129, 16, 64), (300, 528, 200), (1500, 8960, 64), (128, 272, 64), (200, 264, 64)])
+# 6223 rows x 1536: 192-wide tiles
+@pytest.mark.parametrize("M,F,K", [(129, 16, 64), (300, 528, 200), (1500, 8960, 64), (6223, 1536, 72), (128, 272, 64), (200, 264, 64)])
 def test_swiglu_backward(M, F, K):
     """The bits of the plain GEMM followed by the elementwise kernel."""
     C, st = native(), status_word()

@@ -234,7 +234,8 @@ def test_embedding_and_norms(dtype):
 
 # M, n1, n2, K: split-K and persistent kernels, a second product that starts off the tile grid, widths off the 64 grid
 PROJ = [(1, 64, 64, 512), (7, 192, 40, 520), (100, 576, 1032, 640), (200, 320, 72, 1024), (5, 128, 96, 72), (300, 192, 200, 136), (1000, 2048, 264, 256),
-        (140, 256, 0, 192), (33, 1536, 0, 768)]
+        (140, 256, 0, 192), (33, 1536, 0, 768),
+        (3000, 8000, 960, 72), (6223, 1536, 0, 72)]  # 256 and 192 columns on CTA pairs
 
 
 @pytest.mark.parametrize("M,n1,n2,K", PROJ)
