@@ -20,24 +20,27 @@ constexpr int kDecD = 128;
 constexpr int kDecBlock = 16;
 constexpr int kDecWarps = 4;
 
-__device__ __forceinline__ void cp_async16(void* smem_dst, const void* gsrc) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(smem_dst)), "l"(gsrc) : "memory");
+__device__ __forceinline__ void cp_async16(uint32_t smem_dst, const void* gsrc) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_dst), "l"(gsrc) : "memory");
 }
+__device__ __forceinline__ void cp_async16(void* smem_dst, const void* gsrc) { cp_async16(smem_u32(smem_dst), gsrc); }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
-__device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], const void* smem) {
+__device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], uint32_t smem) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-               : "r"(smem_u32(smem)));
+               : "r"(smem));
 }
-__device__ __forceinline__ void ldmatrix_x4_trans(uint32_t (&r)[4], const void* smem) {
+__device__ __forceinline__ void ldmatrix_x4_trans(uint32_t (&r)[4], uint32_t smem) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-               : "r"(smem_u32(smem)));
+               : "r"(smem));
 }
+__device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], const void* smem) { ldmatrix_x4(r, smem_u32(smem)); }
+__device__ __forceinline__ void ldmatrix_x4_trans(uint32_t (&r)[4], const void* smem) { ldmatrix_x4_trans(r, smem_u32(smem)); }
 __device__ __forceinline__ void mma_16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
                                           uint32_t b1) {
   asm volatile(
@@ -67,32 +70,100 @@ struct DecodeParams {
   int* tickets;             // [B, Hkv] zero-initialised arrival counters, or nullptr: the last split CTA to finish merges
 };
 
-// Shared-memory tile of one 16-token block: 16 rows x 256 bytes, 16-byte chunk c of row r stored at c ^ (r & 7).
-__device__ __forceinline__ uint8_t* tile_chunk(uint8_t* tile, int row, int chunk) {
+// Shared-memory tile of one 16-token block: 16 rows x 256 bytes, 16-byte chunk c of row r stored at c ^ (r & 7). Tiles start on
+// 256 bytes, so that chunk c ^ d of a row is at the address of chunk c with d << 4 flipped.
+__device__ __forceinline__ uint32_t tile_chunk(uint32_t tile, int row, int chunk) {
   return tile + row * 256 + ((chunk ^ (row & 7)) << 4);
 }
 
-// 128 threads (4 warps) work on one (split, kv head, sequence) item; `dsm` is 64 KB of shared memory that they own for
-// the duration of the call, `warp` in [0, 4) and `tid` in [0, 128) index the caller's threads, `s_last` is one shared
-// int. Threads synchronise on named barrier 1 (128 threads), so the function may be called by a subset of a larger CTA.
-// Returns true in every thread of the CTA that produced the final output row group (splits == 1, or the last split).
+// 128 threads (4 warps) work on one (split, kv head, sequence) item; `dsm` is shared memory that they own for the duration of
+// the call, `warp` in [0, 4) and `tid` in [0, 128) index the caller's threads. Threads synchronise on named barrier 1 (128
+// threads), so the function may be called by a subset of a larger CTA; a caller that loops over items synchronises between them.
 __device__ __forceinline__ void dec_bar_sync() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
 
 // STAGES = K/V blocks a warp keeps in shared memory (one being consumed, STAGES - 1 in flight): dsm must hold
 // 4 * STAGES * 8 KB. A decode item is a chain of block loads, so its time is (blocks per warp) x (load latency) /
 // (loads in flight).
-template <int STAGES>
-__device__ __forceinline__ bool paged_decode_attend(const DecodeParams& p, int split, int kvh, int b, uint8_t* dsm, int warp,
-                                                    int tid, int* s_last) {
+// `cache_off`: elements from the caches' start to this layer's. `p` is best a kernel parameter: as a local struct it takes
+// 30 registers.
+// Asks for this item's first pages to be brought into L2: at most 256 KB, so that the items of a long context do not push one
+// another (and the weights) out again before they are read.
+__device__ __forceinline__ void paged_decode_prefetch(const DecodeParams& p, long long cache_off, int split, int kvh, int b, int tid) {
+  const int n_blocks = (p.seq_lens[b] + kDecBlock - 1) / kDecBlock;
+  const int blk_begin = (int)((long long)n_blocks * split / p.splits);
+  const int blk_end = (int)((long long)n_blocks * (split + 1) / p.splits);
+  if (tid < 32 && blk_begin + tid < blk_end) {
+    const int page = p.block_tables[(long long)b * p.max_blocks + blk_begin + tid];
+    if (page < 0 || page >= p.num_cache_blocks) return;  // reported by the loads themselves
+    const long long at = cache_off + ((long long)page * p.Hkv + kvh) * kDecBlock * kDecD;
+    bulk_prefetch_l2(p.k_cache + at, kDecBlock * kDecD * 2);
+    bulk_prefetch_l2(p.v_cache + at, kDecBlock * kDecD * 2);
+  }
+}
+
+// ready() returns once the query row and the newest token's cache row are visible to the calling warp. The first blocks of older
+// tokens are requested before it: they do not depend on this layer.
+// emit(g, d, acc, M, L): weighted sum, maximum and denominator of head g at dim d over this split's tokens.
+template <int STAGES, class Ready, class Emit>
+__device__ __forceinline__ void paged_decode_partial(const DecodeParams& p, long long cache_off, int split, int kvh, int b,
+                                                     uint8_t* dsm, int warp, int tid, Ready&& ready, Emit&& emit) {
   const int lane = tid & 31;
-  dec_bar_sync();  // a caller that loops over items: the previous item's merge has finished reading the staging area
   const int seq_len = p.seq_lens[b];
   const int n_blocks = (seq_len + kDecBlock - 1) / kDecBlock;
   const int blk_begin = (int)((long long)n_blocks * split / p.splits);
   const int blk_end = (int)((long long)n_blocks * (split + 1) / p.splits);
   // per-warp staging: STAGES x (K tile 4 KB + V tile 4 KB)
-  uint8_t* wbuf = dsm + warp * (STAGES * 8192);
+  const uint32_t wbuf = smem_u32(dsm) + warp * (STAGES * 8192);
   const int* table = p.block_tables + (long long)b * p.max_blocks;
+
+  // Tile j of this warp: K (even j) or V (odd j) of its block j / 2, in slot j % (2 STAGES).
+  constexpr int kSlots = 2 * STAGES;
+  const int my0 = blk_begin + warp;
+  const int n_mine = my0 < blk_end ? (blk_end - my0 + kDecWarps - 1) / kDecWarps : 0;
+  // Lane k holds the cache block of this warp's block 32 n + k: a load of the table in front of every tile is an L2 round trip
+  // in the chain (600 cycles where acquires keep emptying the L1).
+  int pages = 0;
+  auto load_pages = [&](int first) {
+    const int blk = my0 + (first + lane) * kDecWarps;
+    pages = blk < blk_end ? table[blk] : 0;
+    if (pages < 0 || pages >= p.num_cache_blocks) {
+      report_status(p.status, kStatusBadIndex);
+      pages = 0;
+    }
+  };
+  load_pages(0);
+  // tile j, whose block is one of the 32 that `pages` holds
+  auto issue_tile = [&](int j) {
+    const int phys = __shfl_sync(0xffffffffu, pages, (j >> 1) & 31);
+    const __nv_bfloat16* src = ((j & 1) ? p.v_cache : p.k_cache) + cache_off + ((long long)phys * p.Hkv + kvh) * kDecBlock * kDecD;
+    // 256 chunks of 16 bytes per tile: two rows at a time
+    const uint32_t dst = tile_chunk(wbuf + (j % kSlots) * 4096, lane >> 4, lane & 15);
+    src += lane * 8;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) cp_async16((dst ^ (((2 * i) & 7) << 4)) + i * 512, src + i * 2 * kDecD);
+  };
+
+  // One commit group per tile (empty when there is nothing left to load), so that "at most n groups pending" always names the
+  // same tile. The first 2 STAGES - 1 tiles now: the scores of block i + 1 are computed before block i's values are added
+  // up, so K runs one block ahead of V.
+  bool late = false;  // the newest token's block is among the first ones
+#pragma unroll
+  for (int j = 0; j < kSlots - 1; ++j) {
+    const int blk = my0 + (j >> 1) * kDecWarps;
+    if (blk < blk_end) {
+      if (blk == n_blocks - 1) late = true;
+      else issue_tile(j);
+    }
+    cp_async_commit();
+  }
+  ready();
+  if (late) {
+    const int j0 = (n_blocks - 1 - my0) / kDecWarps * 2;
+    issue_tile(j0);
+    if (j0 + 1 < kSlots - 1) issue_tile(j0 + 1);
+    cp_async_commit();
+    cp_async_wait<0>();
+  }
 
   // Q fragments (A operand, rows = query heads of this kv head, zero above G), pre-scaled later in fp32.
   uint32_t qa[kDecD / 16][2];
@@ -113,52 +184,37 @@ __device__ __forceinline__ bool paged_decode_attend(const DecodeParams& p, int s
   for (int n = 0; n < kDecD / 8; ++n) o[n][0] = o[n][1] = 0.f;
   float m = -INFINITY, l = 0.f;
 
-  auto issue_load = [&](int blk_idx, int stage) {
-    int phys = table[blk_idx];
-    if (phys < 0 || phys >= p.num_cache_blocks) {
-      report_status(p.status, kStatusBadIndex);
-      phys = 0;
-    }
-    const __nv_bfloat16* ksrc = p.k_cache + ((long long)phys * p.Hkv + kvh) * kDecBlock * kDecD;
-    const __nv_bfloat16* vsrc = p.v_cache + ((long long)phys * p.Hkv + kvh) * kDecBlock * kDecD;
-    uint8_t* kt = wbuf + stage * 8192;
-    uint8_t* vt = kt + 4096;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int idx = i * 32 + lane;  // 256 chunks of 16 bytes per tile
-      const int row = idx >> 4, chunk = idx & 15;
-      cp_async16(tile_chunk(kt, row, chunk), ksrc + row * kDecD + chunk * 8);
-      cp_async16(tile_chunk(vt, row, chunk), vsrc + row * kDecD + chunk * 8);
-    }
+  // S = Q K^T of a block's 16 tokens, dims 16 kk .. 16 kk + 15: two n-tiles of 8 tokens.
+  auto k_tile = [&](int i) {
+    return tile_chunk(wbuf + ((2 * i) % kSlots) * 4096, (lane & 7) + ((lane >> 4) << 3), (lane >> 3) & 1);
   };
-
-  // One commit group per loop iteration (empty when there is nothing left to load), so that "at most STAGES - 1 groups
-  // pending" always means: the block about to be consumed has landed.
-  int my = blk_begin + warp;
-#pragma unroll
-  for (int i = 0; i < STAGES - 1; ++i) {
-    if (my + i * kDecWarps < blk_end) issue_load(my + i * kDecWarps, i);
-    cp_async_commit();
-  }
-  int stage = 0;
-  for (; my < blk_end; my += kDecWarps, stage = (stage + 1 == STAGES ? 0 : stage + 1)) {
-    const int nxt = my + (STAGES - 1) * kDecWarps;
-    if (nxt < blk_end) issue_load(nxt, stage == 0 ? STAGES - 1 : stage - 1);
-    cp_async_commit();
-    cp_async_wait<STAGES - 1>();
+  auto score_step = [&](uint32_t kt, int kk, float (&a)[4], float (&b)[4]) {
+    uint32_t kb[4];
+    ldmatrix_x4(kb, kt ^ (kk << 5));
+    mma_16816(a, qa[kk][0], 0u, qa[kk][1], 0u, kb[0], kb[1]);
+    mma_16816(b, qa[kk][0], 0u, qa[kk][1], 0u, kb[2], kb[3]);
+  };
+  float s0[4] = {0.f, 0.f, 0.f, 0.f}, s1[4] = {0.f, 0.f, 0.f, 0.f};
+  if (n_mine > 0) {
+    cp_async_wait<kSlots - 2>();  // K of the first block
     __syncwarp();
-    uint8_t* kt = wbuf + stage * 8192;
-    uint8_t* vt = kt + 4096;
-    // S = Q K^T for 16 tokens: two n-tiles of 8 tokens.
-    float s0[4] = {0.f, 0.f, 0.f, 0.f}, s1[4] = {0.f, 0.f, 0.f, 0.f};
+    const uint32_t kt = k_tile(0);
 #pragma unroll
-    for (int kk = 0; kk < kDecD / 16; ++kk) {
-      uint32_t kb[4];
-      const int row = (lane & 7) + ((lane >> 4) << 3);
-      const int chunk = kk * 2 + ((lane >> 3) & 1);
-      ldmatrix_x4(kb, tile_chunk(kt, row, chunk));
-      mma_16816(s0, qa[kk][0], 0u, qa[kk][1], 0u, kb[0], kb[1]);
-      mma_16816(s1, qa[kk][0], 0u, qa[kk][1], 0u, kb[2], kb[3]);
+    for (int kk = 0; kk < kDecD / 16; ++kk) score_step(kt, kk, s0, s1);
+  }
+  // Live at the start of iteration i: V of block i, K of block i + 1; the slot behind them is refilled, then the one of K i.
+  for (int i = 0; i < n_mine; ++i) {
+    __syncwarp();  // every lane has read K of block i and V of block i - 1
+    const int my = my0 + i * kDecWarps;
+    {
+      const int j = 2 * i + kSlots - 1;  // V of block i + STAGES - 1, K of block i + STAGES
+      if (my + (STAGES - 1) * kDecWarps < blk_end) issue_tile(j);
+      cp_async_commit();
+      if (my + STAGES * kDecWarps < blk_end) {
+        if (((i + STAGES) & 31) == 0) load_pages(i + STAGES);
+        issue_tile(j + 1);
+      }
+      cp_async_commit();
     }
     // scores of head lane/4 for tokens {2i, 2i+1, 8+2i, 9+2i}, i = lane%4
     const int tok0 = my * kDecBlock + (lane & 3) * 2;
@@ -175,7 +231,7 @@ __device__ __forceinline__ bool paged_decode_attend(const DecodeParams& p, int s
     const float base = (m_new == -INFINITY) ? 0.f : m_new;
     float pr[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) pr[i] = exp2f(sc[i] - base);
+    for (int k = 0; k < 4; ++k) pr[k] = exp2f(sc[k] - base);
     float ps = pr[0] + pr[1] + pr[2] + pr[3];
     ps += __shfl_xor_sync(0xffffffffu, ps, 1);
     ps += __shfl_xor_sync(0xffffffffu, ps, 2);
@@ -183,20 +239,21 @@ __device__ __forceinline__ bool paged_decode_attend(const DecodeParams& p, int s
     m = m_new;
     const uint32_t pa0 = pack_bf16x2(pr[0], pr[1]);
     const uint32_t pa2 = pack_bf16x2(pr[2], pr[3]);
+    cp_async_wait<kSlots - 2>();  // up to K of block i + 1
+    __syncwarp();
+    const uint32_t kt = k_tile(i + 1);
+    const uint32_t vt = tile_chunk(wbuf + ((2 * i + 1) % kSlots) * 4096, (lane & 7) + (((lane >> 3) & 1) << 3), lane >> 4);
 #pragma unroll
-    for (int n = 0; n < kDecD / 8; ++n) {
-      o[n][0] *= alpha;
-      o[n][1] *= alpha;
-    }
-    // O += P V : V^T fragments through transposing ldmatrix, two n-tiles (16 dims) per instruction.
+    for (int k = 0; k < 4; ++k) s0[k] = s1[k] = 0.f;
+    // O += P V of this block (V^T fragments through transposing ldmatrix, two n-tiles of 8 dims per instruction) between the
+    // steps of the next block's scores, which are a chain. After the last block those are computed from a stale tile and unused.
 #pragma unroll
     for (int n2 = 0; n2 < kDecD / 16; ++n2) {
       uint32_t vb[4];
-      const int row = (lane & 7) + (((lane >> 3) & 1) << 3);
-      const int chunk = n2 * 2 + (lane >> 4);
-      ldmatrix_x4_trans(vb, tile_chunk(vt, row, chunk));
-      float c0[4] = {o[n2 * 2][0], o[n2 * 2][1], 0.f, 0.f};
-      float c1[4] = {o[n2 * 2 + 1][0], o[n2 * 2 + 1][1], 0.f, 0.f};
+      ldmatrix_x4_trans(vb, vt ^ (n2 << 5));
+      score_step(kt, n2, s0, s1);
+      float c0[4] = {o[n2 * 2][0] * alpha, o[n2 * 2][1] * alpha, 0.f, 0.f};
+      float c1[4] = {o[n2 * 2 + 1][0] * alpha, o[n2 * 2 + 1][1] * alpha, 0.f, 0.f};
       mma_16816(c0, pa0, 0u, pa2, 0u, vb[0], vb[1]);
       mma_16816(c1, pa0, 0u, pa2, 0u, vb[2], vb[3]);
       o[n2 * 2][0] = c0[0];
@@ -204,7 +261,6 @@ __device__ __forceinline__ bool paged_decode_attend(const DecodeParams& p, int s
       o[n2 * 2 + 1][0] = c1[0];
       o[n2 * 2 + 1][1] = c1[1];
     }
-    __syncwarp();
   }
 
   // Merge the four warps through shared memory (reusing the staging area after everyone is done).
@@ -216,8 +272,7 @@ __device__ __forceinline__ bool paged_decode_attend(const DecodeParams& p, int s
 #pragma unroll
     for (int n = 0; n < kDecD / 8; ++n) {
       const int d = n * 8 + (lane & 3) * 2;
-      mo[(warp * 8 + g) * kDecD + d] = o[n][0];
-      mo[(warp * 8 + g) * kDecD + d + 1] = o[n][1];
+      *reinterpret_cast<float2*>(mo + (warp * 8 + g) * kDecD + d) = make_float2(o[n][0], o[n][1]);
     }
     if ((lane & 3) == 0) {
       mml[(warp * 8 + g) * 2] = m;
@@ -225,19 +280,33 @@ __device__ __forceinline__ bool paged_decode_attend(const DecodeParams& p, int s
     }
   }
   dec_bar_sync();
-  for (int idx = tid; idx < p.G * kDecD; idx += kDecWarps * 32) {
-    const int g = idx / kDecD, d = idx % kDecD;
-    float M = -INFINITY;
+  static_assert(kDecD == kDecWarps * 32, "a thread per output dim");
+  float acc[8], M[8], L[8];
 #pragma unroll
-    for (int w = 0; w < kDecWarps; ++w) M = fmaxf(M, mml[(w * 8 + g) * 2]);
-    float L = 0.f, acc = 0.f;
+  for (int g = 0; g < 8; ++g) {  // heads above G (rows of zeros) too: independent of one another, nothing is emitted between the loads
+    M[g] = -INFINITY;
+#pragma unroll
+    for (int w = 0; w < kDecWarps; ++w) M[g] = fmaxf(M[g], mml[(w * 8 + g) * 2]);
+    L[g] = acc[g] = 0.f;
 #pragma unroll
     for (int w = 0; w < kDecWarps; ++w) {
       const float mw = mml[(w * 8 + g) * 2];
-      const float wgt = (mw == -INFINITY) ? 0.f : exp2f(mw - M);
-      L += mml[(w * 8 + g) * 2 + 1] * wgt;
-      acc += mo[(w * 8 + g) * kDecD + d] * wgt;
+      const float wgt = (mw == -INFINITY) ? 0.f : exp2f(mw - M[g]);
+      L[g] += mml[(w * 8 + g) * 2 + 1] * wgt;
+      acc[g] += mo[(w * 8 + g) * kDecD + tid] * wgt;
     }
+  }
+#pragma unroll
+  for (int g = 0; g < 8; ++g)
+    if (g < p.G) emit(g, tid, acc[g], M[g], L[g]);
+}
+
+// The item as the stand-alone kernel runs it: partial sums to memory, the last split of a (sequence, kv head) merges.
+// `s_last` is one shared int.
+template <int STAGES, class Ready>
+__device__ __forceinline__ void paged_decode_attend(const DecodeParams& p, int split, int kvh, int b, uint8_t* dsm, int warp,
+                                                    int tid, int* s_last, Ready&& ready) {
+  paged_decode_partial<STAGES>(p, 0, split, kvh, b, dsm, warp, tid, ready, [&](int g, int d, float acc, float M, float L) {
     if (p.splits == 1) {
       p.out[(long long)b * p.ldo + (long long)(kvh * p.G + g) * kDecD + d] = __float2bfloat16(L > 0.f ? acc / L : 0.f);
     } else {
@@ -248,10 +317,9 @@ __device__ __forceinline__ bool paged_decode_attend(const DecodeParams& p, int s
         p.part_ml[base * 2 + 1] = L;
       }
     }
-  }
+  });
   // Split-KV merge without a second kernel: every split CTA of a (sequence, kv head) takes a ticket after its
   // partials are visible device-wide; the one that draws the last ticket merges all of them and re-arms the counter.
-  bool final_writer = p.splits == 1;
   if (p.splits > 1 && p.tickets != nullptr) {
     __threadfence();
     dec_bar_sync();
@@ -263,7 +331,6 @@ __device__ __forceinline__ bool paged_decode_attend(const DecodeParams& p, int s
     }
     dec_bar_sync();
     if (*s_last) {
-      final_writer = true;
       __threadfence();
       // four output dims per thread (16-byte loads of the partial outputs), eight splits at a time with all their loads
       // issued before the first use: they are L2 round trips, and the merging CTA is on the step's critical path
@@ -305,7 +372,6 @@ __device__ __forceinline__ bool paged_decode_attend(const DecodeParams& p, int s
       }
     }
   }
-  return final_writer;
 }
 
 }  // namespace

@@ -17,10 +17,17 @@
 //   (W' = weight with the RMSNorm weight folded into its columns, rs = 1 / rms of the row.)
 //
 // Work item of a GEMM phase = (128-feature tile, K split). Every item writes its fp32 partial tile to a scratch slot
-// (L2-resident), bumps the tile's arrival counter, waits (bounded) until all S splits of the tile have arrived, then
-// reduces ITS share of the batch rows over the S partials in a fixed order and applies the epilogue: the reduction is
-// spread over all CTAs and its result does not depend on arrival order. A global counter `done` counts finished shares;
-// the activation producer of the next phase waits for the count that says the whole phase is complete.
+// (L2-resident) and reduces ITS share of the batch rows over the S partials in a fixed order, then applies the epilogue: the
+// reduction is spread over all CTAs and its result does not depend on arrival order. Partials are handed over without a flag
+// (kNotYet in decode_sync.cuh): fence, arrival counter and load cost three L2 round trips where polling the data costs
+// one. A gate / up tile that is not split along K goes from the accumulator to the activation without leaving the CTA. The
+// splits of an attention item are merged the same way, heads dealt to the splits. A global counter `done` counts finished
+// shares; the activation producer and the compute warps wait for the count that says that the phase before is complete, the
+// latter so that row statistics and residuals are in registers when the accumulator is. Attention has warps of its own: in one
+// loop with the epilogues its registers spill, and local memory is slow here, since every acquire empties the L1.
+//
+// Bound by the chain of hand-offs, not by bytes. 28 layers of 1536 / 8960, a step: 16 rows x 2048 tokens 1.66 ms with arrival
+// counters and attention in the compute warps, 1.49 ms so; 32 rows x 1024 tokens 1.65 and 1.47 (weights alone: 0.48).
 //
 // Every wait is bounded; a wait that runs out records a status code, makes the CTA leave through its normal exit (TMEM
 // freed) and the other CTAs follow as soon as they see the status word.
@@ -36,11 +43,11 @@ namespace agrpo {
 
 namespace {
 
-constexpr int kMegaThreads = 256;
+constexpr int kMegaThreads = 384;  // weights, activations, products, watcher; four compute warps; four attention warps
 constexpr int kFT = 128;                    // features per item (MMA M)
 constexpr int kMBK = 64;                    // K per stage
 constexpr int kWStage = kFT * kMBK * 2;     // 16 KB
-constexpr int kMaxGroups = 512;             // arrival counters per GEMM phase
+constexpr int kCounterWords = 4;
 
 struct MegaPhase {
   int n_groups;  // feature tiles
@@ -51,7 +58,7 @@ struct MegaPhase {
 struct MegaParams {
   int L, B, H, Q, QD, F, Hq, Hkv, grid;
   MegaPhase ph[4];
-  int att_groups, splits;
+  int att_items, splits;  // att_items: rows x kv heads x splits
   unsigned int per_layer;  // `done` increments per layer
   __nv_bfloat16 *x, *x1, *qkv, *attn, *act;
   const __nv_bfloat16* bqkv;
@@ -67,11 +74,8 @@ struct MegaParams {
   __nv_bfloat16* cache;
   long long cache_layer_stride, cache_v_off;
   int num_cache_blocks;
-  float scale_log2;
-  float *part_o, *part_ml;
-  int* att_tickets;
+  DecodeParams att;
   float* partials;
-  unsigned int* arrive;  // [4][kMaxGroups] monotonic arrival counters
   unsigned int* done;
   int* status;
   long long* trace;  // optional: clock64 stamps of CTA 0 in layer trace_layer (32 slots), nullptr = off
@@ -105,20 +109,132 @@ struct MegaCfg {
   static constexpr int kXStage = BT * kMBK * 2;
   static constexpr int kNSW = 7;
   static constexpr int kXA = 98304;  // activation ring; the attention phase stages K/V tiles here (3 blocks per warp)
-  static constexpr int kAttStages = 3;
   static constexpr int kNSX = (kXA / kXStage) > 8 ? 8 : (kXA / kXStage);
   static constexpr int kAcc = 2;
   static constexpr uint32_t kTmemCols = (kAcc * BT) < 32 ? 32 : (kAcc * BT);
-  static constexpr int kSmem = kNSW * kWStage + kXA + 1024 /* barriers */ + 1024 /* alignment */;
+  static constexpr int kEx = 2 * 2 * 16 * 64 * 4;  // gate / up exchange: two turns of 16 rows x 64 features each way
+  static constexpr int kSmem = kNSW * kWStage + kXA + kEx + 1024 /* barriers */ + 1024 /* alignment */;
+  // rows of a share that a warp reduces at a time, and partials of a row requested at a time
+  static constexpr int kRU = BT <= 32 ? 1 : 2;
+  static constexpr int kNS = BT <= 32 ? 12 : 4;
 };
 
 // What the roles of one CTA share.
 struct MegaShared {
   uint64_t full_w[8], empty_w[8], full_x[8], empty_x[8], tmem_full[2], tmem_empty[2], xa_bar;
   uint32_t tmem_slot;
-  int s_last;
+  unsigned int seen;     // the value of `done` that this CTA has observed
+  unsigned int xa_free;  // layers whose qkv products have read all that they need from the activation ring
   int abort;
 };
+
+constexpr int kAttStages = 3;
+
+// Polls until every value of `t` that is wanted has arrived; load(k) and wanted(k) of value k, arrived(value). False when the
+// wait ran out.
+template <class T, int N, class Load, class Wanted, class Arrived>
+__device__ __forceinline__ bool gather_handoff(T (&t)[N], const int* status, Load&& load, Wanted&& wanted, Arrived&& arrived) {
+  uint32_t missing = 0;
+#pragma unroll
+  for (int k = 0; k < N; ++k)
+    if (wanted(k)) t[k] = load(k);
+#pragma unroll
+  for (int k = 0; k < N; ++k)
+    if (wanted(k) && !arrived(t[k])) missing |= 1u << k;
+  bool ok = true;
+  if (missing != 0) {
+    const long long t0 = clock64();
+    int it = 0;
+    do {
+#pragma unroll
+      for (int k = 0; k < N; ++k)
+        if (missing >> k & 1) t[k] = load(k);
+#pragma unroll
+      for (int k = 0; k < N; ++k)
+        if ((missing >> k & 1) && arrived(t[k])) missing &= ~(1u << k);
+      if ((++it & 31) == 0 && (status_set(status) || clock64() - t0 > kWaitBudgetTicks)) {
+        report_status(const_cast<int*>(status), kStatusBarrierTimeout);
+        ok = false;
+        break;
+      }
+    } while (missing != 0);
+  }
+  __syncwarp();
+  return ok;
+}
+
+// One attention item: this split's share of the tokens of (sequence b, kv head kvh), then, with several splits, heads split,
+// split + splits, ... merged over all of them, one warp a head, four dims a lane. False in the lanes whose wait ran out.
+__device__ __forceinline__ bool mega_attention_item(const DecodeParams& dp, long long cache_off, int split, int kvh, int b, uint8_t* xa,
+                                                    int cw, int tid, const unsigned int* seen, unsigned int qkv_done, long long* trace) {
+  const int lane = tid & 31;
+  const int splits = dp.splits;
+  const long long slot0 = ((long long)b * dp.Hkv + kvh) * splits * 8;
+  bool ok = true;
+  paged_decode_partial<kAttStages>(
+      dp, cache_off, split, kvh, b, xa, cw, tid,
+      [&] {
+        if (!wait_seen(seen, qkv_done, dp.status)) {
+          report_status(dp.status, kStatusPeerFlagTimeout);
+          ok = false;
+        }
+        __syncwarp();
+        if (trace != nullptr && tid == 0) trace[24] = clock64();
+      },
+      [&](int g, int d, float a, float M, float L) {
+        if (splits == 1) {
+          dp.out[(long long)b * dp.ldo + (long long)(kvh * dp.G + g) * kDecD + d] = __float2bfloat16(L > 0.f ? a / L : 0.f);
+        } else {
+          const long long s = slot0 + split * 8 + g;
+          st_handoff(dp.part_o + s * kDecD + d, a);
+          if (d == 0) {
+            st_handoff(dp.part_ml + s * 2, M);
+            st_handoff(dp.part_ml + s * 2 + 1, L);
+          }
+        }
+      });
+  if (trace != nullptr && tid == 0) trace[27] = clock64();
+  if (splits == 1) return ok;
+  for (int g = split + splits * cw; g < dp.G; g += splits * 4) {
+    float M = -INFINITY, L = 0.f;
+    float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int s0 = 0; s0 < splits; s0 += 8) {
+      struct Part {
+        float4 o;
+        float2 ml;
+      } v[8];
+      auto po = [&](int k) { return reinterpret_cast<float4*>(dp.part_o + (slot0 + (s0 + k) * 8 + g) * kDecD) + lane; };
+      auto pm = [&](int k) { return reinterpret_cast<float2*>(dp.part_ml + (slot0 + (s0 + k) * 8 + g) * 2); };
+      ok = gather_handoff(v, dp.status, [&](int k) { return Part{ld_handoff4(po(k)), ld_handoff2(pm(k))}; },
+                          [&](int k) { return s0 + k < splits; },
+                          [](const Part& t) { return has_arrived(t.o) && has_arrived(t.ml.x) && has_arrived(t.ml.y); }) && ok;
+      float Mn = M;
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        if (s0 + j < splits) {
+          clear_handoff4(po(j));
+          if (lane == 0) clear_handoff2(pm(j));
+          Mn = fmaxf(Mn, v[j].ml.x);
+        }
+      const float keep = (M == -INFINITY) ? 0.f : exp2f(M - Mn);
+      L *= keep;
+      a.x *= keep; a.y *= keep; a.z *= keep; a.w *= keep;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        if (s0 + j >= splits) continue;
+        const float w = (v[j].ml.x == -INFINITY) ? 0.f : exp2f(v[j].ml.x - Mn);
+        L += v[j].ml.y * w;
+        a.x += v[j].o.x * w; a.y += v[j].o.y * w; a.z += v[j].o.z * w; a.w += v[j].o.w * w;
+      }
+      M = Mn;
+    }
+    uint2 o;  // the expression of the stand-alone kernel: both paths give the same bits
+    o.x = pack_bf16x2(L > 0.f ? a.x / L : 0.f, L > 0.f ? a.y / L : 0.f);
+    o.y = pack_bf16x2(L > 0.f ? a.z / L : 0.f, L > 0.f ? a.w / L : 0.f);
+    *reinterpret_cast<uint2*>(dp.out + (long long)b * dp.ldo + (long long)(kvh * dp.G + g) * kDecD + 4 * lane) = o;
+  }
+  return ok;
+}
 
 template <int BT>
 __global__ void __launch_bounds__(kMegaThreads, 1)
@@ -134,7 +250,8 @@ decode_layers_kernel(const __grid_constant__ CUtensorMap tmWqkv, const __grid_co
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* w_ring = smem;
   uint8_t* xa = smem + NSW * kWStage;
-  MegaShared* sh = reinterpret_cast<MegaShared*>(xa + Cfg::kXA);
+  float* ex = reinterpret_cast<float*>(xa + Cfg::kXA);
+  MegaShared* sh = reinterpret_cast<MegaShared*>(xa + Cfg::kXA + Cfg::kEx);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int cta = blockIdx.x, G = p.grid;
@@ -148,11 +265,12 @@ decode_layers_kernel(const __grid_constant__ CUtensorMap tmWqkv, const __grid_co
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(&sh->tmem_full[a], 1);
-      mbar_init(&sh->tmem_empty[a], 1);
+      mbar_init(&sh->tmem_empty[a], 4);  // the compute warps
     }
     mbar_init(&sh->xa_bar, 128);
-    sh->s_last = 0;
     sh->abort = 0;
+    sh->seen = 0;
+    sh->xa_free = 0;
     fence_mbar_init();
   }
   if (warp == 3) {
@@ -163,305 +281,258 @@ decode_layers_kernel(const __grid_constant__ CUtensorMap tmWqkv, const __grid_co
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = sh->tmem_slot;
-
   // done-counter value at which the inputs of GEMM phase ph of layer l are complete
   auto target = [&](int l, int ph) -> unsigned int {
     unsigned int t = (unsigned int)l * p.per_layer;
-    if (ph >= 1) t += (unsigned int)(p.ph[0].n_groups * p.ph[0].S) + (unsigned int)p.att_groups;
+    if (ph >= 1) t += (unsigned int)(p.ph[0].n_groups * p.ph[0].S) + (unsigned int)p.att_items;
     if (ph >= 2) t += (unsigned int)(p.ph[1].n_groups * p.ph[1].S);
     if (ph >= 3) t += (unsigned int)(p.ph[2].n_groups * p.ph[2].S);
     return t;
   };
 
-  if (warp == 0) {
-    // ================= weight producer: never waits for another CTA =================
-    // Two cursors walk the same sequence of weight tiles (layer, phase, item, K block): `ld` issues the TMA loads into
-    // the shared-memory ring, `pf` runs prefetch_tiles ahead of it and only asks for the tiles to be brought into L2.
-    // The ring alone covers a few microseconds of streaming; the L2 window keeps HBM busy through the attention phase
-    // and the hand-offs between phases, when the ring is full and nobody consumes it.
-    if (elect_one()) {
-      struct Cur {
-        int l, ph, item, kb, kb1, ft;
-      };
-      auto seek = [&](Cur& c) -> bool {  // first K block of the item at (l, ph, item), or of the next one that exists
-        while (c.l < p.L) {
-          const int S = p.ph[c.ph].S, nkb = p.ph[c.ph].num_kb;
-          if (c.item < p.ph[c.ph].n_groups * S) {
-            c.ft = c.item / S;
-            const int ks = c.item - c.ft * S;
-            c.kb = (int)((long long)nkb * ks / S);
-            c.kb1 = (int)((long long)nkb * (ks + 1) / S);
-            if (c.kb < c.kb1) return true;
-            c.item += G;
-            continue;
+  // Registers at launch: 384 x 168. What the four single-thread roles do not need goes to the attention warps, whose loop
+  // spills at 168 (96 + 168 + 240 = 3 x 168).
+  if (warp < 4) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 96;");
+    if (warp == 0) {
+      // ================= weight producer: never waits for another CTA =================
+      // Two cursors walk the same sequence of weight tiles (layer, phase, item, K block): `ld` issues the TMA loads into
+      // the shared-memory ring, `pf` runs prefetch_tiles ahead of it and only asks for the tiles to be brought into L2.
+      // The ring alone covers a few microseconds of streaming; the L2 window keeps HBM busy through the attention phase
+      // and the hand-offs between phases, when the ring is full and nobody consumes it.
+      if (elect_one()) {
+        struct Cur {
+          int l, ph, item, kb, kb1, ft;
+        };
+        auto seek = [&](Cur& c) -> bool {  // first K block of the item at (l, ph, item), or of the next one that exists
+          while (c.l < p.L) {
+            const int S = p.ph[c.ph].S, nkb = p.ph[c.ph].num_kb;
+            if (c.item < p.ph[c.ph].n_groups * S) {
+              c.ft = c.item / S;
+              const int ks = c.item - c.ft * S;
+              c.kb = (int)((long long)nkb * ks / S);
+              c.kb1 = (int)((long long)nkb * (ks + 1) / S);
+              if (c.kb < c.kb1) return true;
+              c.item += G;
+              continue;
+            }
+            c.item = cta;
+            if (++c.ph == 4) {
+              c.ph = 0;
+              ++c.l;
+            }
           }
-          c.item = cta;
-          if (++c.ph == 4) {
-            c.ph = 0;
-            ++c.l;
+          return false;
+        };
+        auto step = [&](Cur& c) -> bool {
+          if (++c.kb < c.kb1) return true;
+          c.item += G;
+          return seek(c);
+        };
+        auto tmap = [&](int ph) { return ph == 0 ? &tmWqkv : ph == 1 ? &tmWo : ph == 2 ? &tmWgu : &tmWd; };
+        Cur ld{0, 0, cta, 0, 0, 0}, pf{0, 0, cta, 0, 0, 0};
+        bool ld_on = seek(ld), pf_on = seek(pf);
+        int ahead = 0;
+        int st = 0;
+        uint32_t par = 0;
+        bool ok = true;
+        while (ld_on) {
+          while (pf_on && ahead < p.prefetch_tiles) {
+            if (pf.ph == 2) {
+              tma_prefetch_l2_3d(tmap(2), pf.kb * kMBK, pf.ft * 64, pf.l);
+              tma_prefetch_l2_3d(tmap(2), pf.kb * kMBK, p.F + pf.ft * 64, pf.l);
+            } else {
+              tma_prefetch_l2_3d(tmap(pf.ph), pf.kb * kMBK, pf.ft * kFT, pf.l);
+            }
+            pf_on = step(pf);
+            ++ahead;
           }
-        }
-        return false;
-      };
-      auto step = [&](Cur& c) -> bool {
-        if (++c.kb < c.kb1) return true;
-        c.item += G;
-        return seek(c);
-      };
-      auto tmap = [&](int ph) { return ph == 0 ? &tmWqkv : ph == 1 ? &tmWo : ph == 2 ? &tmWgu : &tmWd; };
-      Cur ld{0, 0, cta, 0, 0, 0}, pf{0, 0, cta, 0, 0, 0};
-      bool ld_on = seek(ld), pf_on = seek(pf);
-      int ahead = 0;
-      int st = 0;
-      uint32_t par = 0;
-      bool ok = true;
-      while (ld_on) {
-        while (pf_on && ahead < p.prefetch_tiles) {
-          if (pf.ph == 2) {
-            tma_prefetch_l2_3d(tmap(2), pf.kb * kMBK, pf.ft * 64, pf.l);
-            tma_prefetch_l2_3d(tmap(2), pf.kb * kMBK, p.F + pf.ft * 64, pf.l);
+          if (!mbar_wait_s(&sh->empty_w[st], par ^ 1, p.status)) {
+            report_status(p.status, kStatusWaitEmptyTimeout);
+            ok = false;
+            break;
+          }
+          uint8_t* dst = w_ring + st * kWStage;
+          mbar_expect_tx(&sh->full_w[st], kWStage);
+          if (ld.ph == 2) {  // 64 gate features on MMA rows 0..63, the matching 64 up features on rows 64..127
+            tma_load_3d(dst, tmap(2), &sh->full_w[st], ld.kb * kMBK, ld.ft * 64, ld.l);
+            tma_load_3d(dst + 64 * kMBK * 2, tmap(2), &sh->full_w[st], ld.kb * kMBK, p.F + ld.ft * 64, ld.l);
           } else {
-            tma_prefetch_l2_3d(tmap(pf.ph), pf.kb * kMBK, pf.ft * kFT, pf.l);
+            tma_load_3d(dst, tmap(ld.ph), &sh->full_w[st], ld.kb * kMBK, ld.ft * kFT, ld.l);
           }
-          pf_on = step(pf);
-          ++ahead;
+          if (++st == NSW) {
+            st = 0;
+            par ^= 1;
+          }
+          ld_on = step(ld);
+          --ahead;
         }
-        if (!mbar_wait_s(&sh->empty_w[st], par ^ 1, p.status)) {
-          report_status(p.status, kStatusWaitEmptyTimeout);
-          ok = false;
-          break;
-        }
-        uint8_t* dst = w_ring + st * kWStage;
-        mbar_expect_tx(&sh->full_w[st], kWStage);
-        if (ld.ph == 2) {  // 64 gate features on MMA rows 0..63, the matching 64 up features on rows 64..127
-          tma_load_3d(dst, tmap(2), &sh->full_w[st], ld.kb * kMBK, ld.ft * 64, ld.l);
-          tma_load_3d(dst + 64 * kMBK * 2, tmap(2), &sh->full_w[st], ld.kb * kMBK, p.F + ld.ft * 64, ld.l);
-        } else {
-          tma_load_3d(dst, tmap(ld.ph), &sh->full_w[st], ld.kb * kMBK, ld.ft * kFT, ld.l);
-        }
-        if (++st == NSW) {
-          st = 0;
-          par ^= 1;
-        }
-        ld_on = step(ld);
-        --ahead;
+        if (!ok) sh->abort = 1;
       }
-      if (!ok) sh->abort = 1;
-    }
-  } else if (warp == 1) {
-    // ================= activation producer: waits for the phase that writes its operand =================
-    if (elect_one()) {
-      int st = 0;
-      uint32_t par = 0;
-      bool ok = true;
-      for (int l = 0; l < p.L && ok; ++l) {
-        for (int ph = 0; ph < 4 && ok; ++ph) {
-          const CUtensorMap* tm = ph == 0 ? &tmX : ph == 1 ? &tmAttn : ph == 2 ? &tmX1 : &tmAct;
-          const int S = p.ph[ph].S, nkb = p.ph[ph].num_kb, n_items = p.ph[ph].n_groups * S;
-          if (ph == 1) {
-            // the attention phase used this ring's memory through the generic proxy: its threads fenced and arrived
-            if (!mbar_wait_s(&sh->xa_bar, (uint32_t)(l & 1), p.status)) {
-              report_status(p.status, kStatusBarrierTimeout);
-              ok = false;
-              break;
-            }
-          }
-          bool waited = (l == 0 && ph == 0);
-          for (int item = cta; item < n_items && ok; item += G) {
-            if (!waited) {
-              if (!wait_counter(p.done, target(l, ph), p.status)) {
-                report_status(p.status, kStatusPeerFlagTimeout);
-                ok = false;
-                break;
+    } else if (warp == 1) {
+      // ================= activation producer: waits for the phase that writes its operand =================
+      if (elect_one()) {
+        int st = 0;
+        uint32_t par = 0;
+        bool ok = true;
+        // Layer whose attention phase lies between this CTA's last load and the next, -1 if none. A CTA without work items never
+        // waits for xa_bar: its compute warps may be several phases of that barrier ahead.
+        int staged = -1;
+        for (int l = 0; l < p.L && ok; ++l) {
+          for (int ph = 0; ph < 4 && ok; ++ph) {
+            const CUtensorMap* tm = ph == 0 ? &tmX : ph == 1 ? &tmAttn : ph == 2 ? &tmX1 : &tmAct;
+            const int S = p.ph[ph].S, nkb = p.ph[ph].num_kb, n_items = p.ph[ph].n_groups * S;
+            if (ph == 1) staged = l;
+            bool waited = (l == 0 && ph == 0);
+            for (int item = cta; item < n_items && ok; item += G) {
+              if (!waited) {
+                if (!wait_seen(&sh->seen, target(l, ph), p.status)) {
+                  report_status(p.status, kStatusPeerFlagTimeout);
+                  ok = false;
+                  break;
+                }
+                fence_proxy_async_all();  // other SMs wrote the operand with ordinary stores; TMA reads it
+                waited = true;
               }
-              fence_proxy_async_all();  // other SMs wrote the operand with ordinary stores; TMA reads it
-              waited = true;
-            }
-            const int ft = item / S, ks = item - ft * S;
-            const int kb0 = (int)((long long)nkb * ks / S), kb1 = (int)((long long)nkb * (ks + 1) / S);
-            for (int kb = kb0; kb < kb1; ++kb) {
-              if (!mbar_wait_s(&sh->empty_x[st], par ^ 1, p.status)) {
-                report_status(p.status, kStatusWaitEmptyTimeout);
-                ok = false;
-                break;
+              if (staged >= 0) {
+                // the attention phase used this ring's memory through the generic proxy: its threads fenced and arrived
+                if (!mbar_wait_s(&sh->xa_bar, (uint32_t)(staged & 1), p.status)) {
+                  report_status(p.status, kStatusBarrierTimeout);
+                  ok = false;
+                  break;
+                }
+                staged = -1;
               }
-              mbar_expect_tx(&sh->full_x[st], Cfg::kXStage);
-              tma_load_2d(xa + st * Cfg::kXStage, tm, &sh->full_x[st], kb * kMBK, 0);
-              if (++st == NSX) {
-                st = 0;
-                par ^= 1;
+              const int ft = item / S, ks = item - ft * S;
+              const int kb0 = (int)((long long)nkb * ks / S), kb1 = (int)((long long)nkb * (ks + 1) / S);
+              for (int kb = kb0; kb < kb1; ++kb) {
+                if (!mbar_wait_s(&sh->empty_x[st], par ^ 1, p.status)) {
+                  report_status(p.status, kStatusWaitEmptyTimeout);
+                  ok = false;
+                  break;
+                }
+                mbar_expect_tx(&sh->full_x[st], Cfg::kXStage);
+                tma_load_2d(xa + st * Cfg::kXStage, tm, &sh->full_x[st], kb * kMBK, 0);
+                if (++st == NSX) {
+                  st = 0;
+                  par ^= 1;
+                }
               }
             }
           }
         }
+        if (!ok) sh->abort = 1;
       }
-      if (!ok) sh->abort = 1;
-    }
-  } else if (warp == 2) {
-    // ================= MMA issuer =================
-    if (elect_one()) {
-      int sw = 0, sx = 0, acc = 0;
-      uint32_t pw = 0, px = 0, pa = 0;
-      bool ok = true;
-      for (int l = 0; l < p.L && ok; ++l) {
-        for (int ph = 0; ph < 4 && ok; ++ph) {
-          const int S = p.ph[ph].S, nkb = p.ph[ph].num_kb, n_items = p.ph[ph].n_groups * S;
-          for (int item = cta; item < n_items && ok; item += G) {
-            const int ft = item / S, ks = item - ft * S;
-            const int kb0 = (int)((long long)nkb * ks / S), kb1 = (int)((long long)nkb * (ks + 1) / S);
-            if (!mbar_wait_s(&sh->tmem_empty[acc], pa ^ 1, p.status)) {
-              report_status(p.status, kStatusWaitTmemEmptyTimeout);
-              ok = false;
-              break;
-            }
-            tc_fence_after();
-            const uint32_t d_addr = tmem_base + (uint32_t)(acc * BT);
-            for (int kb = kb0; kb < kb1; ++kb) {
-              if (!mbar_wait_s(&sh->full_w[sw], pw, p.status) || !mbar_wait_s(&sh->full_x[sx], px, p.status)) {
-                report_status(p.status, kStatusWaitFullTimeout);
+    } else if (warp == 2) {
+      // ================= MMA issuer =================
+      if (elect_one()) {
+        int sw = 0, sx = 0, acc = 0;
+        uint32_t pw = 0, px = 0, pa = 0;
+        bool ok = true;
+        for (int l = 0; l < p.L && ok; ++l) {
+          for (int ph = 0; ph < 4 && ok; ++ph) {
+            const int S = p.ph[ph].S, nkb = p.ph[ph].num_kb, n_items = p.ph[ph].n_groups * S;
+            for (int item = cta; item < n_items && ok; item += G) {
+              const int ft = item / S, ks = item - ft * S;
+              const int kb0 = (int)((long long)nkb * ks / S), kb1 = (int)((long long)nkb * (ks + 1) / S);
+              if (!mbar_wait_s(&sh->tmem_empty[acc], pa ^ 1, p.status)) {
+                report_status(p.status, kStatusWaitTmemEmptyTimeout);
                 ok = false;
                 break;
               }
               tc_fence_after();
-              if (kb == kb0) MEGA_STAMP(ph * 6 + 0);
-              if (kb == kb0 && ph == 1) MEGA_STAMP_ALL(2);
-              if (kb == kb0 && ph == 0) MEGA_STAMP_ALL(3);
-              const uint32_t sa = smem_u32(w_ring + sw * kWStage);
-              const uint32_t sb = smem_u32(xa + sx * Cfg::kXStage);
+              const uint32_t d_addr = tmem_base + (uint32_t)(acc * BT);
+              for (int kb = kb0; kb < kb1; ++kb) {
+                if (!mbar_wait_s(&sh->full_w[sw], pw, p.status) || !mbar_wait_s(&sh->full_x[sx], px, p.status)) {
+                  report_status(p.status, kStatusWaitFullTimeout);
+                  ok = false;
+                  break;
+                }
+                tc_fence_after();
+                if (kb == kb0) MEGA_STAMP(ph * 6 + 0);
+                if (kb == kb0 && ph == 1) MEGA_STAMP_ALL(2);
+                if (kb == kb0 && ph == 0) MEGA_STAMP_ALL(3);
+                const uint32_t sa = smem_u32(w_ring + sw * kWStage);
+                const uint32_t sb = smem_u32(xa + sx * Cfg::kXStage);
 #pragma unroll
-              for (int k = 0; k < kMBK / 16; ++k)
-                tc_mma_f16(d_addr, umma_smem_desc(sa + k * 32, 16, 1024), umma_smem_desc(sb + k * 32, 16, 1024), kIdesc,
-                           (kb > kb0 || k > 0) ? 1u : 0u);
-              tc_commit(&sh->empty_w[sw]);
-              tc_commit(&sh->empty_x[sx]);
-              if (++sw == NSW) {
-                sw = 0;
-                pw ^= 1;
+                for (int k = 0; k < kMBK / 16; ++k)
+                  tc_mma_f16(d_addr, umma_smem_desc(sa + k * 32, 16, 1024), umma_smem_desc(sb + k * 32, 16, 1024), kIdesc,
+                             (kb > kb0 || k > 0) ? 1u : 0u);
+                tc_commit(&sh->empty_w[sw]);
+                tc_commit(&sh->empty_x[sx]);
+                if (++sw == NSW) {
+                  sw = 0;
+                  pw ^= 1;
+                }
+                if (++sx == NSX) {
+                  sx = 0;
+                  px ^= 1;
+                }
               }
-              if (++sx == NSX) {
-                sx = 0;
-                px ^= 1;
+              if (!ok) break;
+              tc_commit(&sh->tmem_full[acc]);
+              MEGA_STAMP(ph * 6 + 1);
+              if (++acc == Cfg::kAcc) {
+                acc = 0;
+                pa ^= 1;
               }
             }
-            if (!ok) break;
-            tc_commit(&sh->tmem_full[acc]);
-            MEGA_STAMP(ph * 6 + 1);
-            if (++acc == Cfg::kAcc) {
-              acc = 0;
-              pa ^= 1;
+          }
+        }
+        if (!ok) sh->abort = 1;
+      }
+    } else if (warp == 3) {
+      // ================= watcher: the only thread of the CTA that polls the global counter =================
+      if (elect_one()) {
+        bool ok = true;
+        for (int l = 0; l < p.L && ok; ++l) {
+          for (int step = 0; step < 5 && ok; ++step) {  // inputs of qkv, attention, o, gate / up, down
+            const unsigned int want = step == 1 ? (unsigned int)l * p.per_layer + (unsigned int)(p.ph[0].n_groups * p.ph[0].S)
+                                                : target(l, step == 0 ? 0 : step - 1);
+            if (!wait_counter(p.done, want, p.status)) {
+              report_status(p.status, kStatusPeerFlagTimeout);
+              ok = false;
+            } else {
+              st_release_cta(&sh->seen, want);
             }
           }
         }
       }
-      if (!ok) sh->abort = 1;
     }
-  } else if (warp >= 4) {
-    // ================= compute warps: GEMM reductions + epilogues, attention =================
+  } else if (warp < 8) {
+    // ================= compute warps: GEMM reductions + epilogues =================
     const int cw = warp - 4;             // TMEM lane quarter (warp % 4)
     const int tid = threadIdx.x - 128;   // 0..127
     const uint32_t lane_off = static_cast<uint32_t>(cw * 32) << 16;
     int acc = 0;
     uint32_t pa = 0;
+    bool fail = false;  // this warp's; all compute warps leave together at the next group_bar_or
     bool ok = true;
     const int B = p.B;
-
-    DecodeParams dp;
-    dp.q = p.qkv;
-    dp.ldq = p.Q;
-    dp.q_col0 = 0;
-    dp.block_tables = p.block_tables;
-    dp.seq_lens = p.seq_lens;
-    dp.max_blocks = p.max_blocks;
-    dp.Hq = p.Hq;
-    dp.Hkv = p.Hkv;
-    dp.G = p.Hq / p.Hkv;
-    dp.scale_log2 = p.scale_log2;
-    dp.splits = p.splits;
-    dp.out = p.attn;
-    dp.ldo = p.QD;
-    dp.part_o = p.part_o;
-    dp.part_ml = p.part_ml;
-    dp.num_cache_blocks = p.num_cache_blocks;
-    dp.status = p.status;
-    dp.tickets = p.att_tickets;
+    auto wait_done = [&](unsigned int want) {
+      if (!wait_seen(&sh->seen, want, p.status)) {
+        report_status(p.status, kStatusPeerFlagTimeout);
+        fail = true;
+      }
+      __syncwarp();
+    };
 
     for (int l = 0; l < p.L && ok; ++l) {
       __nv_bfloat16* k_cache = p.cache + (long long)l * p.cache_layer_stride;
       __nv_bfloat16* v_cache = k_cache + p.cache_v_off;
       if (tid == 0) MEGA_STAMP(26);
       for (int ph = 0; ph < 4 && ok; ++ph) {
-        if (ph == 1) {
-          // ---------------- attention over the paged cache ----------------
-          if (tid == 0) {
-            if (!wait_counter(p.done, (unsigned int)l * p.per_layer + (unsigned int)(p.ph[0].n_groups * p.ph[0].S), p.status)) {
-              report_status(p.status, kStatusPeerFlagTimeout);
-              sh->abort = 1;
-            }
-          }
-          dec_bar_sync();
-          if (sh->abort) {
-            ok = false;
-            break;
-          }
-          if (tid == 0) MEGA_STAMP(24);
-          if (tid == 0) MEGA_STAMP_ALL(0);
-          dp.k_cache = k_cache;
-          dp.v_cache = v_cache;
-          const int n_att = p.att_groups * p.splits;
-          for (int it = cta; it < n_att; it += G) {
-            const int split = it % p.splits;
-            const int rest = it / p.splits;
-            const int kvh = rest % p.Hkv, b = rest / p.Hkv;
-            if (p.seq_lens[b] <= 0) {
-              // an idle row (a free slot inside the batch): nothing to attend to, its output is never used
-              if (split == 0 && tid == 0) red_release_gpu_add(p.done, 1u);
-              continue;
-            }
-            const bool fin = paged_decode_attend<Cfg::kAttStages>(dp, split, kvh, b, xa, cw, tid, &sh->s_last);
-            if (fin) {
-              dec_bar_sync();  // every thread's output stores are issued
-              if (tid == 0) {
-                __threadfence();
-                red_release_gpu_add(p.done, 1u);
-              }
-            }
-          }
-          fence_proxy_async_smem();   // the activation ring is handed back to TMA
-          mbar_arrive(&sh->xa_bar);
-          if (tid == 0) MEGA_STAMP(25);
-          if (tid == 0) MEGA_STAMP_ALL(1);
-        }
         // ---------------- GEMM items of this phase ----------------
         const int S = p.ph[ph].S, n_items = p.ph[ph].n_groups * S;
+        bool waited = l == 0 && ph == 0;
         for (int item = cta; item < n_items && ok; item += G) {
           const int grp = item / S, ks = item - grp * S;
-          bool have_acc = true;
-          if (!mbar_wait_s(&sh->tmem_full[acc], pa, p.status)) {
-            report_status(p.status, kStatusWaitTmemFullTimeout);
-            sh->abort = 1;  // read by every compute thread after the barriers below: they all leave together
-            have_acc = false;
-          }
-          tc_fence_after();
-          if (tid == 0) MEGA_STAMP(ph * 6 + 2);
-          float* slot = p.partials + (size_t)item * (BT * kFT);
-          if (have_acc) {
-#pragma unroll 1
-            for (int c = 0; c < BT / 32; ++c) {
-              if (c * 32 >= B) break;  // padding rows
-              uint32_t r[32];
-              tmem_ld_32x32(tmem_base + lane_off + (uint32_t)(acc * BT + c * 32), r);
-              tc_wait_ld();
-#pragma unroll
-              for (int i = 0; i < 32; ++i)
-                if (c * 32 + i < B) __stcg(slot + (size_t)(c * 32 + i) * kFT + cw * 32 + lane, __uint_as_float(r[i]));
-            }
-          }
-          tc_fence_before();
-          // Row statistics, lengths and the residual of my first rows do not depend on the other splits: request them now,
-          // they arrive while this CTA waits for the tile's other splits.
+          if (!waited) wait_done(target(l, ph));
+          waited = true;
           const int r0 = (int)((long long)B * ks / S), r1 = (int)((long long)B * (ks + 1) / S);
-          constexpr int RU = 4;
+          constexpr int RU = Cfg::kRU, NS = Cfg::kNS;
           const int b_first = r0 + cw * RU;
+          // Row statistics, lengths and the residual of this warp's first rows: requested while the product still runs.
           sumsq_t m_ss[RU];
           int m_len[RU];
           float4 m_rr[RU], m_cs[RU], m_sn[RU];
@@ -498,35 +569,69 @@ decode_layers_kernel(const __grid_constant__ CUtensorMap tmWqkv, const __grid_co
               }
             }
           };
-          load_meta(b_first);
-          // the CTA barrier orders every thread's partial stores before the release below (cumulative at GPU scope)
-          dec_bar_sync();
-          if (tid == 0) {
-            mbar_arrive(&sh->tmem_empty[acc]);
-            unsigned int* ctr = p.arrive + ph * kMaxGroups + grp;
-            red_release_gpu_add(ctr, 1u);
-            MEGA_STAMP(ph * 6 + 3);
-            if (!wait_counter(ctr, (unsigned int)S * (unsigned int)(l + 1), p.status)) {
-              report_status(p.status, kStatusBarrierTimeout);
-              sh->abort = 1;
+          const bool direct = ph == 2 && S == 1;
+          // direct: statistics of rows 32 c + lane
+          auto row_scale = [&](int c) {
+            const int b = c * 32 + lane;
+            return b < B ? rsqrtf(sumsq_from_fixed(ld_sumsq_l2(p.ss + (size_t)(2 * l + 1) * p.ss_stride + b)) * p.inv_h + p.eps) : 0.f;
+          };
+          float rs_next = 0.f;
+          if (direct) rs_next = row_scale(0);
+          else load_meta(b_first);
+          if (!mbar_wait_s(&sh->tmem_full[acc], pa, p.status)) {
+            report_status(p.status, kStatusWaitTmemFullTimeout);
+            fail = true;
+          }
+          tc_fence_after();
+          if (tid == 0) MEGA_STAMP(ph * 6 + 2);
+          float* slot = p.partials + (size_t)item * (BT * kFT);
+#pragma unroll 1
+          for (int c = 0; c < BT / 32; ++c) {
+            if (c * 32 >= B) break;  // padding rows
+            uint32_t r[32];
+            tmem_ld_32x32(tmem_base + lane_off + (uint32_t)(acc * BT + c * 32), r);
+            tc_wait_ld();
+            if (!direct) {
+#pragma unroll
+              for (int i = 0; i < 32; ++i)
+                if (c * 32 + i < B) st_handoff(slot + (size_t)(c * 32 + i) * kFT + cw * 32 + lane, __uint_as_float(r[i]));
+              continue;
+            }
+            // Warps 0 and 1 hold the gate features, 2 and 3 the up features. The former finish the even rows, the latter the
+            // odd ones: each gives away the half that it does not finish. Two buffers in turn, so one barrier a turn is enough.
+            const bool up = cw >= 2;
+            const float rs_mine = rs_next;
+            if ((c + 1) * 32 < B) rs_next = row_scale(c + 1);
+            float* give = ex + ((c & 1) * 2 + (up ? 1 : 0)) * (16 * 64) + (cw & 1) * 32 + lane;
+            const float* take = ex + ((c & 1) * 2 + (up ? 0 : 1)) * (16 * 64) + (cw & 1) * 32 + lane;
+#pragma unroll
+            for (int i = 0; i < 16; ++i) give[i * 64] = __uint_as_float(up ? r[2 * i] : r[2 * i + 1]);
+            asm volatile("bar.sync 2, 128;" ::: "memory");
+            __nv_bfloat16* dst = p.act + (size_t)(c * 32 + (up ? 1 : 0)) * p.F + grp * 64 + (cw & 1) * 32 + lane;
+#pragma unroll
+            for (int i0 = 0; i0 < 16; i0 += 4) {
+              if (c * 32 + 2 * i0 >= B) break;
+#pragma unroll
+              for (int i = i0; i < i0 + 4; ++i) {
+                const float rs = __shfl_sync(0xffffffffu, rs_mine, 2 * i + (up ? 1 : 0));
+                const float mine = __uint_as_float(up ? r[2 * i + 1] : r[2 * i]), theirs = take[i * 64];
+                const float g = (up ? theirs : mine) * rs, u = (up ? mine : theirs) * rs;
+                const __nv_bfloat16 o = __float2bfloat16(g / (1.f + __expf(-g)) * u);
+                if (c * 32 + 2 * i + (up ? 1 : 0) < B) dst[(size_t)(2 * i) * p.F] = o;
+              }
             }
           }
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&sh->tmem_empty[acc]);
+          if (tid == 0) MEGA_STAMP(ph * 6 + 3);
           if (++acc == Cfg::kAcc) {
             acc = 0;
             pa ^= 1;
           }
-          dec_bar_sync();
-          if (sh->abort) {
-            ok = false;
-            break;
-          }
-          if (tid == 0) MEGA_STAMP(ph * 6 + 4);
           // ---- my share of the rows: reduce over the S partials, epilogue ----
-          const float* gbase = p.partials + (size_t)(grp * S) * (BT * kFT);
-          // Four rows per warp pass. Everything a row needs from memory (its S partials, statistics, residual, rotary
-          // table entries, cache slot) is requested before the first use, so that the L2 round trips of the four rows
-          // and of the splits overlap instead of adding up.
-          for (int b0 = b_first; b0 < r1; b0 += 4 * RU) {
+          float* gbase = p.partials + (size_t)(grp * S) * (BT * kFT);
+          for (int b0 = b_first; !direct && b0 < r1; b0 += 4 * RU) {
             if (b0 != b_first) load_meta(b0);
             float4 v[RU];
             bool on[RU];
@@ -535,20 +640,20 @@ decode_layers_kernel(const __grid_constant__ CUtensorMap tmWqkv, const __grid_co
               on[j] = b0 + j < r1;
               v[j] = make_float4(0.f, 0.f, 0.f, 0.f);
             }
-            for (int s = 0; s < S; s += 2) {
-              float4 t0[RU], t1[RU];
-              const bool two = s + 1 < S;
+            for (int s0 = 0; s0 < S; s0 += NS) {
+              float4 t[NS * RU];  // split s0 + k / RU of row b0 + k % RU
+              auto src = [&](int k) { return reinterpret_cast<float4*>(gbase + ((size_t)(s0 + k / RU) * BT + b0 + k % RU) * kFT) + lane; };
+              auto wanted = [&](int k) { return s0 + k / RU < S && b0 + k % RU < r1; };
+              if (!gather_handoff(t, p.status, [&](int k) { return ld_handoff4(src(k)); }, wanted, [](const float4& w) { return has_arrived(w); }))
+                fail = true;
+              if (tid == 0) MEGA_STAMP(ph * 6 + 4);
 #pragma unroll
-              for (int j = 0; j < RU; ++j) {
-                const float4* src = reinterpret_cast<const float4*>(gbase + ((size_t)s * BT + (on[j] ? b0 + j : r0)) * kFT) + lane;
-                t0[j] = __ldcg(src);
-                t1[j] = two ? __ldcg(src + (size_t)BT * kFT / 4) : make_float4(0.f, 0.f, 0.f, 0.f);
-              }
-#pragma unroll
-              for (int j = 0; j < RU; ++j) {  // fixed order: split s, then split s + 1
-                v[j].x += t0[j].x; v[j].y += t0[j].y; v[j].z += t0[j].z; v[j].w += t0[j].w;
-                v[j].x += t1[j].x; v[j].y += t1[j].y; v[j].z += t1[j].z; v[j].w += t1[j].w;
-              }
+              for (int k = 0; k < NS * RU; ++k)
+                if (wanted(k)) {  // fixed order over the splits
+                  clear_handoff4(src(k));
+                  float4& w = v[k % RU];
+                  w.x += t[k].x; w.y += t[k].y; w.z += t[k].z; w.w += t[k].w;
+                }
             }
             if (ph == 0) {
               const bool is_q = grp < p.Hq, is_k = !is_q && grp < p.Hq + p.Hkv;
@@ -606,20 +711,63 @@ decode_layers_kernel(const __grid_constant__ CUtensorMap tmWqkv, const __grid_co
                 if (!on[j]) continue;
                 const float4 w = make_float4(v[j].x + m_rr[j].x, v[j].y + m_rr[j].y, v[j].z + m_rr[j].z, v[j].w + m_rr[j].w);
                 st_bf16x4(obase + (size_t)(b0 + j) * p.H + grp * kFT + 4 * lane, w);
-                float sq = w.x * w.x + w.y * w.y + w.z * w.z + w.w * w.w;
+                float sq = __fmaf_rn(w.w, w.w, __fmaf_rn(w.z, w.z, __fmaf_rn(w.x, w.x, __fmul_rn(w.y, w.y))));
 #pragma unroll
                 for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
                 if (lane == 0) sumsq_atomic_add(p.ss + (size_t)(2 * l + (ph == 1 ? 1 : 2)) * p.ss_stride + b0 + j, sq);
               }
             }
           }
-          dec_bar_sync();
-          if (tid == 0) {
+          // the barrier orders every thread's stores before the release below (cumulative at GPU scope)
+          ok = !group_bar_or<2>(fail);
+          if (ok && tid == 0) {
             red_release_gpu_add(p.done, 1u);
             MEGA_STAMP(ph * 6 + 5);
           }
         }
+        if (ph == 0 && tid == 0) st_release_cta(&sh->xa_free, (unsigned int)(l + 1));
       }
+    }
+    if (!ok && tid == 0) sh->abort = 1;
+  } else {
+    // ================= attention warps =================
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 240;");
+    const int aw = warp - 8;
+    const int tid = threadIdx.x - 256;
+    bool fail = false, ok = true;
+    for (int l = 0; l < p.L && ok; ++l) {
+      const unsigned int qkv_done = (unsigned int)l * p.per_layer + (unsigned int)(p.ph[0].n_groups * p.ph[0].S);
+      // The K/V blocks are staged in the activation ring: this CTA's products have read all that was in it, and it is not
+      // filled again before xa_bar.
+      for (int it = cta; it < p.att_items; it += G) {
+        const int rest = it / p.splits;
+        paged_decode_prefetch(p.att, (long long)l * p.cache_layer_stride, it % p.splits, rest % p.Hkv, rest / p.Hkv, tid);
+      }
+      if (!wait_seen(&sh->xa_free, (unsigned int)(l + 1), p.status)) {
+        report_status(p.status, kStatusBarrierTimeout);
+        fail = true;
+      }
+      for (int it = cta; it < p.att_items && ok; it += G) {
+        const int split = it % p.splits;
+        const int rest = it / p.splits;
+        const int kvh = rest % p.Hkv, b = rest / p.Hkv;
+        if (p.seq_lens[b] > 0) {
+          if (!mega_attention_item(p.att, (long long)l * p.cache_layer_stride, split, kvh, b, xa, aw, tid, &sh->seen, qkv_done,
+                                   cta == 0 && l == p.trace_layer ? p.trace : nullptr))
+            fail = true;
+        } else if (!wait_seen(&sh->seen, qkv_done, p.status)) {
+          // an idle row (a free slot inside the batch), whose output is never used: it still counts after the qkv phase only
+          report_status(p.status, kStatusPeerFlagTimeout);
+          fail = true;
+        }
+        ok = !group_bar_or<1>(fail);  // every thread's output stores are issued, the staging area is free
+        if (ok && tid == 0) red_release_gpu_add(p.done, 1u);
+      }
+      if (!ok) break;
+      fence_proxy_async_smem();   // the activation ring is handed back to TMA
+      mbar_arrive(&sh->xa_bar);
+      if (tid == 0) MEGA_STAMP(25);
+      if (tid == 0) MEGA_STAMP_ALL(1);
     }
     if (!ok && tid == 0) sh->abort = 1;
   }
@@ -693,8 +841,8 @@ long long decode_layers_scratch_bytes(int rows, int H, int Q, int QD, int F, int
 
 bool decode_layers_supported(int rows, int H, int Q, int QD, int F, int Hq, int Hkv, int head_dim) {
   return rows >= 1 && rows <= 256 && head_dim == 128 && H % 128 == 0 && Q % 128 == 0 && QD % 64 == 0 && F % 64 == 0 &&
-         Q == (Hq + 2 * Hkv) * 128 && QD == Hq * 128 && Hkv > 0 && Hq % Hkv == 0 && Hq / Hkv <= 8 && Q / 128 <= kMaxGroups &&
-         F / 64 <= kMaxGroups && H / 128 <= kMaxGroups;
+         Q == (Hq + 2 * Hkv) * 128 && QD == Hq * 128 && Hkv > 0 && Hq % Hkv == 0 && Hq / Hkv <= 8 && Q / 128 <= 512 &&
+         F / 64 <= 512 && H / 128 <= 512;
 }
 
 void launch_decode_layers(const DecodeLayersArgs& a, cudaStream_t stream) {
@@ -713,9 +861,9 @@ void launch_decode_layers(const DecodeLayersArgs& a, cudaStream_t stream) {
     per_layer += (unsigned int)(groups[i] * p.ph[i].S);
     if ((long long)groups[i] * p.ph[i].S > max_items) max_items = (long long)groups[i] * p.ph[i].S;
   }
-  p.att_groups = a.B * a.Hkv;
   p.splits = a.splits < 1 ? 1 : a.splits;
-  p.per_layer = per_layer + (unsigned int)p.att_groups;
+  p.att_items = a.B * a.Hkv * p.splits;
+  p.per_layer = per_layer + (unsigned int)p.att_items;
   const int BT = a.B <= 32 ? 32 : a.B <= 64 ? 64 : a.B <= 128 ? 128 : 256;
   if (max_items * BT * kFT * 4 > a.partials_bytes) throw std::runtime_error("decode_layers: scratch buffer too small");
   p.x = (__nv_bfloat16*)a.x; p.x1 = (__nv_bfloat16*)a.x1; p.qkv = (__nv_bfloat16*)a.qkv; p.attn = (__nv_bfloat16*)a.attn;
@@ -727,18 +875,30 @@ void launch_decode_layers(const DecodeLayersArgs& a, cudaStream_t stream) {
   p.block_tables = a.block_tables; p.max_blocks = a.max_blocks; p.seq_lens = a.seq_lens;
   p.cache = (__nv_bfloat16*)a.cache; p.cache_layer_stride = a.cache_layer_stride; p.cache_v_off = a.cache_v_off;
   p.num_cache_blocks = a.num_cache_blocks;
-  p.scale_log2 = a.softmax_scale * 1.4426950408889634f;
-  p.part_o = a.part_o; p.part_ml = a.part_ml; p.att_tickets = a.att_tickets;
+  DecodeParams& d = p.att;
+  d.q = p.qkv; d.ldq = a.Q; d.q_col0 = 0;
+  d.k_cache = p.cache; d.v_cache = p.cache + a.cache_v_off;
+  d.block_tables = a.block_tables; d.max_blocks = a.max_blocks; d.seq_lens = a.seq_lens; d.num_cache_blocks = a.num_cache_blocks;
+  d.Hq = a.Hq; d.Hkv = a.Hkv; d.G = a.Hq / a.Hkv; d.splits = p.splits;
+  d.scale_log2 = a.softmax_scale * 1.4426950408889634f;
+  d.out = p.attn; d.ldo = a.QD;
+  d.part_o = a.part_o; d.part_ml = a.part_ml; d.tickets = nullptr;
+  d.status = a.status;
   p.partials = a.partials;
-  p.arrive = a.counters;
-  p.done = a.counters + 4 * kMaxGroups;
+  p.done = a.counters;
   p.status = a.status;
   p.trace = a.trace;
   p.trace_layer = a.trace_layer;
   p.prefetch_tiles = a.prefetch_tiles;
   p.trace_all = a.trace_words >= 32 + 4 * a.num_sms ? 1 : 0;
-  // counters start from zero in every launch (stream-ordered, also inside a captured graph)
-  check_cuda(cudaMemsetAsync(a.counters, 0, (4 * kMaxGroups + 4) * sizeof(unsigned int), stream), "decode_layers counters");
+  // the counter starts from zero and the handed-over buffers from "not yet" in every launch (stream-ordered, also inside a
+  // captured graph)
+  check_cuda(cudaMemsetAsync(a.counters, 0, kCounterWords * sizeof(unsigned int), stream), "decode_layers counters");
+  check_cuda(cudaMemsetAsync(a.partials, 0xff, (size_t)max_items * BT * kFT * 4, stream), "decode_layers partials");
+  if (p.splits > 1) {
+    check_cuda(cudaMemsetAsync(a.part_o, 0xff, (size_t)p.att_items * 8 * kDecD * 4, stream), "decode_layers attention partials");
+    check_cuda(cudaMemsetAsync(a.part_ml, 0xff, (size_t)p.att_items * 8 * 2 * 4, stream), "decode_layers attention partials");
+  }
   CUtensorMap tm[8];
   tm[0] = make_tmap_w3d(a.wqkv, a.H, a.Q, a.L, a.wqkv_stride, kFT);
   tm[1] = make_tmap_w3d(a.wo, a.QD, a.H, a.L, a.wo_stride, kFT);
@@ -756,6 +916,6 @@ void launch_decode_layers(const DecodeLayersArgs& a, cudaStream_t stream) {
   }
 }
 
-int decode_layers_counter_words() { return 4 * kMaxGroups + 4; }
+int decode_layers_counter_words() { return kCounterWords; }
 
 }  // namespace agrpo

@@ -138,11 +138,13 @@ __global__ void rope_kv_write_decode_kernel(__nv_bfloat16* __restrict__ qkv, lon
 
 __global__ void __launch_bounds__(kDecWarps * 32)
 paged_decode_attn_kernel(const DecodeParams p) {
-  extern __shared__ __align__(128) uint8_t dsm[];
+  extern __shared__ __align__(256) uint8_t dsm[];
   __shared__ int s_last;
-  pdl_wait();
-  pdl_launch();
-  paged_decode_attend<2>(p, blockIdx.x, blockIdx.y, blockIdx.z, dsm, threadIdx.x >> 5, threadIdx.x, &s_last);
+  // lengths, tables and the pages of older tokens are older than the kernel before this one
+  paged_decode_attend<2>(p, blockIdx.x, blockIdx.y, blockIdx.z, dsm, threadIdx.x >> 5, threadIdx.x, &s_last, [] {
+    pdl_wait();
+    pdl_launch();
+  });
 }
 
 __global__ void paged_decode_combine_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml, int splits,

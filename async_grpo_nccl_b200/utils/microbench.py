@@ -589,7 +589,7 @@ def bench_decode(args):
         rec = {"bench": "decode_layers_trace", "layer": eng.mega_trace_layer, "unit": "us since the layer's start on CTA 0"}
         for ph, pn in enumerate(["qkv", "o", "gate_up", "down"]):
             rec[pn] = {n: rel(ph * 6 + i) for i, n in enumerate(names)}
-        rec["attention"] = {"inputs_ready": rel(24), "end": rel(25)}
+        rec["attention"] = {"inputs_ready": rel(24), "split_done": rel(27), "end": rel(25)}
         per = t[32:].reshape(-1, 4)
         per = per[per[:, 0] > 0]
         if len(per):
