@@ -127,6 +127,26 @@ void embedding_fwd(const Tensor& ids, const Tensor& table, Tensor& out) {
   agrpo::launch_embedding_fwd(ids.data_ptr<int>(), table.data_ptr(), out.data_ptr(), (int)ids.numel(), (int)table.size(1),
                               (int)table.size(0), cur_stream());
 }
+// idx: rows of x, each below x.size(0) (the packer's output_indices).
+void gather_loss_rows(const Tensor& idx, const Tensor& x, const Tensor& labels, const Tensor& cols, Tensor& xo, Tensor& labels_o, Tensor& cols_o) {
+  check_i32(idx, "idx"); check_bf16(x, "x"); check_bf16(xo, "xo"); check_i32(labels, "labels"); check_i32(labels_o, "labels_o");
+  check_f32(cols, "cols"); check_f32(cols_o, "cols_o");
+  const int64_t n = idx.numel(), T = x.size(0), H = x.size(1);
+  TORCH_CHECK(idx.is_contiguous() && x.is_contiguous() && xo.is_contiguous() && H % 8 == 0 && xo.size(0) == n && xo.size(1) == H, "gather_loss_rows: rows");
+  TORCH_CHECK(labels.is_contiguous() && labels.numel() == T && labels_o.is_contiguous() && labels_o.numel() == n, "gather_loss_rows: labels");
+  TORCH_CHECK(cols.dim() == 2 && cols.size(0) <= 31 && cols.size(1) == T && cols.stride(1) == 1 && cols_o.is_contiguous() &&
+              cols_o.numel() == cols.size(0) * n, "gather_loss_rows: columns");
+  const c10::cuda::CUDAGuard guard(x.device());
+  agrpo::launch_gather_loss_rows(idx.data_ptr<int>(), (int)n, x.data_ptr(), xo.data_ptr(), (int)H, labels.data_ptr<int>(), labels_o.data_ptr<int>(),
+                                 cols.data_ptr<float>(), (int)cols.size(0), cols.stride(0), cols_o.data_ptr<float>(), cur_stream());
+}
+void scatter_rows(const Tensor& idx, const Tensor& x, Tensor& xo) {
+  check_i32(idx, "idx"); check_bf16(x, "x"); check_bf16(xo, "xo");
+  TORCH_CHECK(idx.is_contiguous() && x.is_contiguous() && xo.is_contiguous() && x.size(0) == idx.numel() && x.size(1) == xo.size(1) &&
+              x.size(1) % 8 == 0, "scatter_rows");
+  const c10::cuda::CUDAGuard guard(x.device());
+  agrpo::launch_scatter_rows(idx.data_ptr<int>(), (int)idx.numel(), x.data_ptr(), xo.data_ptr(), (int)x.size(1), cur_stream());
+}
 void embedding_sumsq(const Tensor& ids, const Tensor& table, Tensor& out, Tensor& ss) {
   check_i32(ids, "ids"); check_bf16(table, "table"); check_bf16(out, "out"); check_i64(ss, "ss");
   TORCH_CHECK(table.is_contiguous() && out.is_contiguous() && table.size(1) % 8 == 0, "embedding_sumsq layout");
@@ -1205,6 +1225,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("attn_bwd_pieces", &attn_bwd_pieces);
   m.def("lmhead_num_groups", &lmhead_num_groups);
   m.def("grpo_num_loss_stats", &grpo_num_loss_stats);
+  m.def("gather_loss_rows", &gather_loss_rows, NOGIL);
+  m.def("scatter_rows", &scatter_rows, NOGIL);
   m.def("lmhead_logprob", &lmhead_logprob, py::arg("hidden"), py::arg("weight"), py::arg("labels"), py::arg("temperature"),
         py::arg("partials"), py::arg("label_logit"), py::arg("logp") = py::none(), py::arg("entropy") = py::none(),
         py::arg("lse") = py::none(), py::arg("status") = py::none(), NOGIL);

@@ -107,6 +107,32 @@ __global__ void embedding_bwd_kernel(const int* __restrict__ ids, const __nv_bfl
 }
 
 // ------------------------------------------------------------------------------------------------
+// Rows that carry a loss: row idx[j] of a packed batch to row j of a compact one and back. A warp per row; bound by the rows read
+// and written (28033 of 31287 rows of 1536: 30 us, against the 10 % of four products of 151936 columns that they save).
+// ------------------------------------------------------------------------------------------------
+__global__ void gather_loss_rows_kernel(const int* __restrict__ idx, int n, const __nv_bfloat16* __restrict__ x,
+                                        __nv_bfloat16* __restrict__ xo, int H, const int* __restrict__ labels, int* __restrict__ labels_o,
+                                        const float* __restrict__ f, int nf, long long ldf, float* __restrict__ fo) {
+  const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (row >= n) return;
+  const int lane = threadIdx.x & 31;
+  const long long from = idx[row];
+  const Bf16x8* src = reinterpret_cast<const Bf16x8*>(x + from * H);
+  Bf16x8* dst = reinterpret_cast<Bf16x8*>(xo + (size_t)row * H);
+  for (int i = lane; i < H / 8; i += 32) dst[i] = src[i];
+  if (lane < nf) fo[(size_t)lane * n + row] = f[lane * ldf + from];
+  if (lane == 31) labels_o[row] = labels[from];
+}
+__global__ void scatter_rows_kernel(const int* __restrict__ idx, int n, const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ xo,
+                                    int H) {
+  const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (row >= n) return;
+  const Bf16x8* src = reinterpret_cast<const Bf16x8*>(x + (size_t)row * H);
+  Bf16x8* dst = reinterpret_cast<Bf16x8*>(xo + (size_t)idx[row] * H);
+  for (int i = threadIdx.x & 31; i < H / 8; i += 32) dst[i] = src[i];
+}
+
+// ------------------------------------------------------------------------------------------------
 // RMSNorm: y = x * rstd * w, rstd = rsqrt(mean(x^2) + eps)
 // ------------------------------------------------------------------------------------------------
 __global__ void rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
@@ -368,6 +394,17 @@ void launch_embedding_fwd(const int* ids, const void* table, void* out, int T, i
   AGRPO_PREFER_SMEM(embedding_fwd_kernel);
   embedding_fwd_kernel<<<(T + 7) / 8, 256, 0, s>>>(ids, (const __nv_bfloat16*)table, (__nv_bfloat16*)out, T, H, V);
   check_cuda(cudaGetLastError(), "embedding_fwd");
+}
+void launch_gather_loss_rows(const int* idx, int n, const void* x, void* xo, int H, const int* labels, int* labels_o, const float* f, int nf,
+                             long long ldf, float* fo, cudaStream_t s) {
+  if (n == 0) return;
+  gather_loss_rows_kernel<<<(n + 7) / 8, 256, 0, s>>>(idx, n, (const __nv_bfloat16*)x, (__nv_bfloat16*)xo, H, labels, labels_o, f, nf, ldf, fo);
+  check_cuda(cudaGetLastError(), "gather_loss_rows");
+}
+void launch_scatter_rows(const int* idx, int n, const void* x, void* xo, int H, cudaStream_t s) {
+  if (n == 0) return;
+  scatter_rows_kernel<<<(n + 7) / 8, 256, 0, s>>>(idx, n, (const __nv_bfloat16*)x, (__nv_bfloat16*)xo, H);
+  check_cuda(cudaGetLastError(), "scatter_rows");
 }
 void launch_embedding_sumsq(const int* ids, const void* table, void* out, long long* ss, int n_ss, int ss_stride, int T, int H,
                             int V, cudaStream_t s) {

@@ -184,6 +184,11 @@ int gemm_skinny_splits(int M, int N, int K, int num_sms);
 // ---- bandwidth-bound decoder ops (elementwise.cu); bf16 activations, H and F multiples of 8 ----
 void launch_embedding_fwd(const int* ids, const void* table, void* out, int T, int H, int V, cudaStream_t s);
 void launch_embedding_bwd(const int* ids, const void* dout, float* dtable, int T, int H, int V, cudaStream_t s);
+// Rows idx[0 .. n) of x [*, H] (H a multiple of 8), labels and the nf <= 31 columns f + k * ldf, compact: xo [n, H], labels_o [n],
+// fo [nf, n]. scatter_rows writes row j of x to row idx[j] of xo.
+void launch_gather_loss_rows(const int* idx, int n, const void* x, void* xo, int H, const int* labels, int* labels_o, const float* f, int nf,
+                             long long ldf, float* fo, cudaStream_t s);
+void launch_scatter_rows(const int* idx, int n, const void* x, void* xo, int H, cudaStream_t s);
 // Lookup + ss[0][row] = sum of squares of the row, ss[1..n_ss)[row] = 0. ss is [n_ss, ss_stride] int64: sums of squares
 // in fixed point with 30 fractional bits (value * 2^30), which makes their atomic accumulation order-independent.
 void launch_embedding_sumsq(const int* ids, const void* table, void* out, long long* ss, int n_ss, int ss_stride, int T, int H,

@@ -112,6 +112,11 @@ class GradSink:
         self.flat.zero_()
 
 
+# Work of the output matrix on rows without a loss from which on those rows are left out: 50 us at 1.4 PFLOP/s, twice what the
+# gather, the scatter and their allocations take (a model of 2048 x 512: 1.56 ms an update with all rows, 1.61 without).
+LOSS_ROWS_MIN_FLOPS = 7e10
+
+
 def vocab_chunk(T: int, asked: Optional[int] = None) -> int:
     """Columns of the dlogits buffer of ``T`` rows: what the caller asks for, else 15360 but at most 1 GiB, and at least 4096. A
     wide chunk reads and writes the fp32 dH sum seldom and fills the pairs' waves: 10 chunks of 151936 columns take about 0.8 of
@@ -350,6 +355,19 @@ class NativeDecoder:
     # ---- public ----
     def hidden(self, batch: PackedBatch, saves: Optional[List[dict]] = None) -> Tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
         """Returns (normed final hidden, pre-norm hidden, final rstd)."""
+        x = self._body(batch, saves)
+        hn, rstd = self._final_norm(x)
+        return hn, x, rstd
+
+    def _final_norm(self, x: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor]:
+        hn = torch.empty_like(x)
+        rstd = self._new(x.shape[0], dtype=torch.float32)
+        self.C.rmsnorm_fwd(x, self.w("final_norm"), hn, rstd, self.cfg.rms_norm_eps)
+        self.launches += 1
+        return hn, rstd
+
+    def _body(self, batch: PackedBatch, saves: Optional[List[dict]]) -> torch.Tensor:
+        """Embedding and all layers."""
         cfg, C = self.cfg, self.C
         T = batch.T
         cos_t, sin_t = self.rope_tables()
@@ -367,11 +385,8 @@ class NativeDecoder:
                                 next_unit=i + 2 if i + 1 < n_layers else None)
             if saves is not None and self.recompute:
                 save["x"] = x_in
-        hn = self._new(T, cfg.hidden_size)
-        rstd = self._new(T, dtype=torch.float32)
-        C.rmsnorm_fwd(x, self.w("final_norm"), hn, rstd, cfg.rms_norm_eps)
-        self.launches += 2
-        return hn, x, rstd
+        self.launches += 1
+        return x
 
     def ensure_rope(self, max_pos: int) -> None:
         if self._rope is None or self._rope[0].shape[0] < max_pos:
@@ -401,7 +416,22 @@ class NativeDecoder:
         T = batch.T
         cos_t, sin_t = self.rope_tables()
         saves: List[dict] = []
-        hn, x_last, rstd_f = self.hidden(batch, saves)
+        x_last = self._body(batch, saves)
+        # From the final norm to its gradient only rows with a label take part: prompts and the last row of a sample have none
+        # (a third of the rows where answers are short), and their gradient is zero.
+        labels, advantages, old_logp, old_ent = batch.labels, batch.advantages, batch.old_logprobs, batch.old_entropies
+        ref = batch.ref_logprobs if (lc.kl_beta > 0 and batch.has_ref) else None
+        rows = None
+        # logits twice, two gradients
+        if batch.loss_rows and batch.total_out > 0 and 8.0 * (T - batch.total_out) * cfg.vocab_size * cfg.hidden_size > LOSS_ROWS_MIN_FLOPS:
+            rows, x_all, n = batch.output_indices, x_last, batch.total_out
+            x_last, labels, cols = self._new(n, cfg.hidden_size), self._new(n, dtype=torch.int32), self._new(4, n, dtype=torch.float32)
+            C.gather_loss_rows(rows, x_all, batch.labels, batch.float_buf[:4 * T].view(4, T), x_last, labels, cols)
+            advantages, old_logp, old_ent = cols[0], cols[1], cols[2]
+            ref = cols[3] if ref is not None else None
+            T = n
+            del x_all
+        hn, rstd_f = self._final_norm(x_last)
         wl_name = self.layout.lm_head_name()
         wl = self.w(wl_name)
         V = wl.shape[0]
@@ -411,18 +441,17 @@ class NativeDecoder:
         logp = self._new(T, dtype=torch.float32)
         ent = self._new(T, dtype=torch.float32)
         lse = self._new(T, dtype=torch.float32)
-        C.lmhead_logprob(hn, wl, batch.labels, lc.temperature, partials, ll, logp, ent, lse, self.status)
+        C.lmhead_logprob(hn, wl, labels, lc.temperature, partials, ll, logp, ent, lse, self.status)
         del partials
         stats = torch.zeros(self.n_stats, dtype=torch.float32, device=self.dev)
         dlogp = self._new(T, dtype=torch.float32)
         n_valid = max(1.0, batch.scalars.get("num_output_tokens_non_masked", float(batch.total_out)))
-        ref = batch.ref_logprobs if (lc.kl_beta > 0 and batch.has_ref) else None
-        C.grpo_token_loss(logp, batch.old_logprobs, ref, batch.advantages, batch.labels, ent, batch.old_entropies,
+        C.grpo_token_loss(logp, old_logp, ref, advantages, labels, ent, old_ent,
                           lc.clip_low, lc.clip_high, lc.clip_ratio_c, lc.kl_beta, loss_scale / n_valid, dlogp, stats)
         chunk = min(vocab_chunk(T, self.lmhead_chunk), (V + 255) // 256 * 256)
         dz = self._new(T, chunk)
         dh_acc = self._new(T, cfg.hidden_size, dtype=torch.float32)
-        C.lmhead_backward(hn, wl, batch.labels, lse, dlogp, lc.temperature, dz, dh_acc, sink.view(wl_name), self.status)
+        C.lmhead_backward(hn, wl, labels, lse, dlogp, lc.temperature, dz, dh_acc, sink.view(wl_name), self.status)
         del dz
         dhn = self._new(T, cfg.hidden_size)
         C.cast_f32_bf16(dh_acc, dhn)
@@ -431,6 +460,11 @@ class NativeDecoder:
         C.rmsnorm_bwd(dhn, x_last, self.w("final_norm"), rstd_f, dx, sink.view("final_norm"), False)
         del dhn
         self.launches += 6 + 3 * ((V + chunk - 1) // chunk)
+        if rows is not None:
+            dx_rows, dx = dx, torch.zeros(batch.T, cfg.hidden_size, dtype=torch.bfloat16, device=self.dev)
+            C.scatter_rows(rows, dx_rows, dx)
+            del dx_rows
+            self.launches += 2
         for i in reversed(range(cfg.num_hidden_layers)):
             s = saves[i]
             if self.recompute:

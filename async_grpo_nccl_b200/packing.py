@@ -33,6 +33,8 @@ class PackedBatch:
     scalars: Dict[str, float] = field(default_factory=dict)
     uids: List[Any] = field(default_factory=list)
     dummy: bool = False
+    # output_indices names exactly the rows with a label (not so where a sample has no prompt: its first output has no row)
+    loss_rows: bool = False
 
     def _i(self, start: int, n: int) -> torch.Tensor:
         return self.int_buf[start:start + n]
@@ -93,7 +95,7 @@ class PackedBatch:
         ib = self.int_buf.to(device, non_blocking=non_blocking)
         fb = self.float_buf.to(device, non_blocking=non_blocking)
         return PackedBatch(self.T, self.n, self.total_out, self.n_tiles, ib, fb, self.has_ref, dict(self.scalars),
-                           list(self.uids), self.dummy)
+                           list(self.uids), self.dummy, self.loss_rows)
 
 
 def tiles_offset(T: int, n: int, total_out: int) -> int:
@@ -218,7 +220,7 @@ def pack_samples(samples: Sequence[Dict[str, Any]], pin: bool = True, use_native
         "num_tokens": float(T),
     }
     return PackedBatch(T, n, total_out, n_tiles, int_buf, float_buf, ref is not None, scalars,
-                       [s.get("__uid__") for s in real])
+                       [s.get("__uid__") for s in real], loss_rows=bool(in_lens.min() >= 1))
 
 
 def pack_for_logprob(samples: Sequence[Dict[str, Any]], pin: bool = True) -> PackedBatch:
