@@ -1,5 +1,6 @@
 // Python bindings: tensor checks here, raw-pointer launchers in the .cu files.
 #include <ATen/cuda/CUDAContext.h>
+#include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/extension.h>
 #include <algorithm>
@@ -580,9 +581,31 @@ int64_t attn_bwd_pieces(int64_t n_tiles, int64_t Hq, int64_t Hkv) { return agrpo
 int64_t lmhead_num_groups(int64_t V, int64_t T) { return agrpo::lmhead_num_groups((int)V, (int)T); }
 int64_t grpo_num_loss_stats() { return agrpo::grpo_num_loss_stats(); }
 
+// Kept logits [T, cols]: as many leading columns of the vocabulary (rounded up to 8 where all of them are kept).
+int kept_cols(const OptTensor& logits, int64_t T, int64_t V) {
+  if (!logits.has_value() || !logits->defined()) return 0;
+  check_f32(*logits, "logits");
+  TORCH_CHECK(logits->dim() == 2 && logits->is_contiguous() && logits->size(0) == T && logits->size(1) % 8 == 0 &&
+              logits->size(1) <= (V + 7) / 8 * 8 && (reinterpret_cast<uintptr_t>(logits->data_ptr()) & 31) == 0, "lmhead: logits [T, 8k]");
+  return (int)logits->size(1);
+}
+long long ld_kept(const OptTensor& logits) { return logits.has_value() && logits->defined() ? logits->size(1) : 0; }
+// Columns of [rows, V] fp32 that may be kept from the forward to the backward pass: as many as a quarter of the memory that this
+// process could still get (free on the device, or cached by torch's allocator) holds, in steps of 256.
+int64_t lmhead_keep_columns(int64_t rows, int64_t V) {
+  if (rows <= 0) return 0;
+  const int64_t all = (V + 7) / 8 * 8;
+  if (all * rows * 4 <= (64 << 20)) return all;
+  size_t free_b = 0, total_b = 0;
+  C10_CUDA_CHECK(cudaMemGetInfo(&free_b, &total_b));
+  const auto st = c10::cuda::CUDACachingAllocator::getDeviceStats(c10::cuda::current_device());
+  const int64_t cached = st.reserved_bytes[0].current - st.allocated_bytes[0].current;  // [0]: over all pools
+  const int64_t cols = ((int64_t)free_b + cached) / 4 / (rows * 4);
+  return cols >= all ? all : cols / 256 * 256;
+}
 void lmhead_logprob(const Tensor& hidden, const Tensor& weight, const Tensor& labels, double temperature, Tensor& partials,
                     Tensor& label_logit, const OptTensor& logp, const OptTensor& entropy, const OptTensor& lse,
-                    const OptTensor& status) {
+                    const OptTensor& status, const OptTensor& logits) {
   check_bf16(hidden, "hidden"); check_bf16(weight, "weight"); check_i32(labels, "labels");
   check_f32(partials, "partials"); check_f32(label_logit, "label_logit");
   TORCH_CHECK(hidden.dim() == 2 && weight.dim() == 2 && hidden.stride(1) == 1 && weight.stride(1) == 1, "lmhead: 2-D");
@@ -596,7 +619,7 @@ void lmhead_logprob(const Tensor& hidden, const Tensor& weight, const Tensor& la
   agrpo::launch_lmhead_logprob(hidden.data_ptr(), hidden.stride(0), weight.data_ptr(), weight.stride(0), labels.data_ptr<int>(),
                                (int)T, (int)H, (int)V, (float)temperature, partials.data_ptr<float>(),
                                label_logit.data_ptr<float>(), opt_ptr<float>(logp), opt_ptr<float>(entropy), opt_ptr<float>(lse),
-                               opt_ptr<int>(status), num_sms(), cur_stream());
+                               opt_ptr<float>(logits), ld_kept(logits), kept_cols(logits, T, V), opt_ptr<int>(status), num_sms(), cur_stream());
 }
 
 void grpo_token_loss(const Tensor& logp, const OptTensor& old_logp, const OptTensor& ref_logp, const Tensor& adv,
@@ -616,7 +639,8 @@ void grpo_token_loss(const Tensor& logp, const OptTensor& old_logp, const OptTen
 }
 
 void lmhead_backward(const Tensor& hidden, const Tensor& weight, const Tensor& labels, const Tensor& lse, const Tensor& dlogp,
-                     double temperature, Tensor& dz_chunk, Tensor& dh_acc, const OptTensor& dweight, const OptTensor& status) {
+                     double temperature, Tensor& dz_chunk, Tensor& dh_acc, const OptTensor& dweight, const OptTensor& status,
+                     const OptTensor& logits) {
   check_bf16(hidden, "hidden"); check_bf16(weight, "weight"); check_i32(labels, "labels"); check_f32(lse, "lse");
   check_f32(dlogp, "dlogp"); check_bf16(dz_chunk, "dz_chunk"); check_f32(dh_acc, "dh_acc");
   const int64_t T = hidden.size(0), H = hidden.size(1), V = weight.size(0);
@@ -633,6 +657,7 @@ void lmhead_backward(const Tensor& hidden, const Tensor& weight, const Tensor& l
   agrpo::launch_lmhead_backward(hidden.data_ptr(), hidden.stride(0), weight.data_ptr(), weight.stride(0), labels.data_ptr<int>(),
                                 lse.data_ptr<float>(), dlogp.data_ptr<float>(), (int)T, (int)H, (int)V, (float)temperature,
                                 dz_chunk.data_ptr(), (int)dz_chunk.size(1), dh_acc.data_ptr<float>(), dw, ld_dw,
+                                opt_ptr<float>(logits), ld_kept(logits), kept_cols(logits, T, V),
                                 opt_ptr<int>(status), num_sms(), cur_stream());
 }
 
@@ -1229,13 +1254,14 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("scatter_rows", &scatter_rows, NOGIL);
   m.def("lmhead_logprob", &lmhead_logprob, py::arg("hidden"), py::arg("weight"), py::arg("labels"), py::arg("temperature"),
         py::arg("partials"), py::arg("label_logit"), py::arg("logp") = py::none(), py::arg("entropy") = py::none(),
-        py::arg("lse") = py::none(), py::arg("status") = py::none(), NOGIL);
+        py::arg("lse") = py::none(), py::arg("status") = py::none(), py::arg("logits") = py::none(), NOGIL);
+  m.def("lmhead_keep_columns", &lmhead_keep_columns);
   m.def("grpo_token_loss", &grpo_token_loss, py::arg("logp"), py::arg("old_logp"), py::arg("ref_logp"), py::arg("adv"),
         py::arg("labels"), py::arg("entropy"), py::arg("old_entropy"), py::arg("clip_low"), py::arg("clip_high"),
         py::arg("clip_c"), py::arg("kl_beta"), py::arg("grad_weight"), py::arg("dlogp"), py::arg("stats"), NOGIL);
   m.def("lmhead_backward", &lmhead_backward, py::arg("hidden"), py::arg("weight"), py::arg("labels"), py::arg("lse"),
         py::arg("dlogp"), py::arg("temperature"), py::arg("dz_chunk"), py::arg("dh_acc"), py::arg("dweight") = py::none(),
-        py::arg("status") = py::none(), NOGIL);
+        py::arg("status") = py::none(), py::arg("logits") = py::none(), NOGIL);
   m.def("kv_cache_write", &kv_cache_write, py::arg("qkv"), py::arg("slots"), py::arg("k_cache"), py::arg("v_cache"), py::arg("Hq"),
         py::arg("Hkv"), py::arg("D"), py::arg("status") = py::none(), py::arg("kv_head0") = 0, NOGIL);
   m.def("kv_cache_write_decode", &kv_cache_write_decode, py::arg("qkv"), py::arg("block_tables"), py::arg("seq_lens"),

@@ -9,9 +9,9 @@
 //             per-column-group partials into logprob / entropy / lse per token.
 //   loss    : one elementwise kernel computes the per-token objective, d loss / d logprob and a small
 //             statistics vector (read by the host once per microbatch).
-//   backward: per vocabulary chunk, the GEMM is recomputed with an epilogue that writes
-//             dlogits = g * (onehot - softmax) / temperature as bf16 into a chunk buffer, which feeds the
-//             dH and dW tcgen05 GEMMs.
+//   backward: per vocabulary chunk, dlogits = g * (onehot - softmax) / temperature as bf16 in a chunk buffer, which feeds the
+//             dH and dW tcgen05 GEMMs. Where memory allows, the forward pass has kept its fp32 logits and one
+//             pass over them makes the chunk; else the GEMM is recomputed with that epilogue.
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -26,6 +26,8 @@ namespace {
 
 constexpr int kLmBN = 256;
 
+// KEEP: the logits of columns below keep_cols are stored as well, as the fp32 sums that they are.
+template <bool KEEP>
 struct LmStatsEpilogue {
   const int* labels;   // [T] target token per row, < 0 = masked
   float inv_temp;
@@ -33,6 +35,9 @@ struct LmStatsEpilogue {
   float* part_s;
   float* part_sz;
   float* label_logit;  // [T]
+  float* logits;       // [T, ld_logits], rows on 32 bytes
+  long long ld_logits;
+  int keep_cols;       // a multiple of 8
   // per-thread running state
   float m, s, sz;
   int label;
@@ -45,6 +50,12 @@ struct LmStatsEpilogue {
   }
   __device__ __forceinline__ void chunk(int row, int col0, const uint32_t (&r)[32], int M, int N) {
     if (row >= M || col0 >= N) return;
+    if constexpr (KEEP) {
+      float* dst = logits + (long long)row * ld_logits + col0;
+#pragma unroll
+      for (int i = 0; i < 32; i += 8)
+        if (col0 + i < keep_cols) st_global_32b(dst + i, reinterpret_cast<const uint32_t(&)[8]>(r[i]));
+    }
     float z[32];
     float cm = -INFINITY;
 #pragma unroll
@@ -81,6 +92,39 @@ struct LmStatsEpilogue {
   }
 };
 
+__device__ __forceinline__ float dlogit(float logit, float inv_temp, float lse, float gs, bool is_label) {
+  return gs * ((is_label ? 1.f : 0.f) - __expf(logit * inv_temp - lse));
+}
+
+// dlogits of one chunk from kept logits: a block takes a row, a thread eight columns at a time. Bound by memory: 6 bytes an element
+// where the recomputed product does 2 H operations. An update of 12 samples (8600 rows with a loss, 3584 x 152064): 121 ms with the
+// product, 117 so; 28033 rows of 1536: 179 and 177.
+__global__ void __launch_bounds__(256)
+lmhead_dlogits_kernel(const float* __restrict__ logits, long long ld_logits, const int* __restrict__ labels, const float* __restrict__ lse,
+                      const float* __restrict__ g, float inv_temp, int v0, int vc, __nv_bfloat16* __restrict__ dz, long long ld) {
+  const long long row = blockIdx.x;
+  const float lse_r = lse[row], gs = g[row] * inv_temp;
+  const int label = labels[row] - v0;
+  const float* src = logits + row * ld_logits + v0;
+  __nv_bfloat16* dst = dz + row * ld;
+  for (int c = 8 * threadIdx.x; c < vc; c += 8 * 256) {
+    uint32_t r[8];
+    ld_global_32b(src + c, r);  // columns from vc on, if any, lie within the row's padding
+    uint32_t o[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      o[j] = pack_bf16x2(dlogit(__uint_as_float(r[2 * j]), inv_temp, lse_r, gs, c + 2 * j == label),
+                         dlogit(__uint_as_float(r[2 * j + 1]), inv_temp, lse_r, gs, c + 2 * j + 1 == label));
+    if (c + 8 <= vc) {
+      *reinterpret_cast<uint4*>(dst + c) = make_uint4(o[0], o[1], o[2], o[3]);
+    } else {
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        if (c + j < vc) dst[c + j] = __ushort_as_bfloat16((unsigned short)(o[j / 2] >> (j % 2 * 16)));
+    }
+  }
+}
+
 struct LmDlogitsEpilogue {
   const int* labels;
   const float* lse;    // [T]
@@ -105,8 +149,7 @@ struct LmDlogitsEpilogue {
     const float gs = g_r * inv_temp;
 #pragma unroll
     for (int i = 0; i < 32; ++i) {
-      const float p = __expf(__uint_as_float(r[i]) * inv_temp - lse_r);
-      d[i] = gs * (((col0 + i == label) ? 1.f : 0.f) - p);
+      d[i] = dlogit(__uint_as_float(r[i]), inv_temp, lse_r, gs, col0 + i == label);
     }
     __nv_bfloat16* dst = dz + (long long)row * ld + col0;
     if (col0 + 32 <= N && ((reinterpret_cast<uintptr_t>(dst) & 31) == 0)) {
@@ -278,7 +321,8 @@ static int lmhead_group_n(int V, int T) {
 
 void launch_lmhead_logprob(const void* hidden, long long ldh, const void* weight, long long ldw, const int* labels, int T,
                            int H, int V, float temperature, float* partials, float* label_logit, float* logp,
-                           float* entropy, float* lse, int* status, int num_sms, cudaStream_t stream) {
+                           float* entropy, float* lse, float* logits, long long ld_logits, int keep_cols, int* status, int num_sms,
+                           cudaStream_t stream) {
   if (T == 0) return;
   const int group_n = lmhead_group_n(V, T);
   const int tiles_n = (V + kLmBN - 1) / kLmBN;
@@ -290,18 +334,22 @@ void launch_lmhead_logprob(const void* hidden, long long ldh, const void* weight
   p.M = T; p.N = V; p.K = H;
   p.group_n = group_n;
   p.status = status;
-  LmStatsEpilogue e;
-  e.labels = labels;
-  e.inv_temp = 1.f / temperature;
-  e.part_m = partials;
-  e.part_s = partials + (size_t)groups * T;
-  e.part_sz = partials + 2 * (size_t)groups * T;
-  e.label_logit = label_logit;
-  e.m = 0.f; e.s = 0.f; e.sz = 0.f; e.label = -1;
-  if (pair) gemm_pair_launch<kLmBN, false, false, 4>(ta, tb, p, e, num_sms, stream);
-  else gemm_launch<kLmBN, false, false>(ta, tb, p, e, num_sms, stream);
-  lmhead_combine_kernel<<<(T + 31) / 32, 32 * kCombineWarps, 0, stream>>>(e.part_m, e.part_s, e.part_sz, label_logit, labels, groups, T,
-                                                            logp, entropy, lse);
+  auto product = [&](auto e) {
+    e.labels = labels;
+    e.inv_temp = 1.f / temperature;
+    e.part_m = partials;
+    e.part_s = partials + (size_t)groups * T;
+    e.part_sz = partials + 2 * (size_t)groups * T;
+    e.label_logit = label_logit;
+    e.logits = logits; e.ld_logits = ld_logits; e.keep_cols = keep_cols;
+    e.m = 0.f; e.s = 0.f; e.sz = 0.f; e.label = -1;
+    if (pair) gemm_pair_launch<kLmBN, false, false, 4>(ta, tb, p, e, num_sms, stream);
+    else gemm_launch<kLmBN, false, false>(ta, tb, p, e, num_sms, stream);
+  };
+  if (keep_cols > 0) product(LmStatsEpilogue<true>{});
+  else product(LmStatsEpilogue<false>{});
+  lmhead_combine_kernel<<<(T + 31) / 32, 32 * kCombineWarps, 0, stream>>>(partials, partials + (size_t)groups * T, partials + 2 * (size_t)groups * T,
+                                                            label_logit, labels, groups, T, logp, entropy, lse);
   check_cuda(cudaGetLastError(), "lmhead_combine");
 }
 
@@ -321,8 +369,8 @@ int grpo_num_loss_stats() { return kNumLossStats; }
 
 void launch_lmhead_backward(const void* hidden, long long ldh, const void* weight, long long ldw, const int* labels,
                             const float* lse, const float* dlogp, int T, int H, int V, float temperature, void* dz_chunk,
-                            int chunk_cols, float* dh_acc, float* dweight, long long ld_dw, int* status, int num_sms,
-                            cudaStream_t stream) {
+                            int chunk_cols, float* dh_acc, float* dweight, long long ld_dw, const float* logits, long long ld_logits, int keep_cols,
+                            int* status, int num_sms, cudaStream_t stream) {
   if (T == 0) return;
   const CUtensorMap ta = make_tmap_2d(hidden, H, T, ldh, 64, kGemmBM);
   // Equal chunks, as few as the buffer allows: a short last one would pay for a whole pass over dH.
@@ -331,8 +379,12 @@ void launch_lmhead_backward(const void* hidden, long long ldh, const void* weigh
   for (int v0 = 0, ci = 0; v0 < V; v0 += step, ++ci) {
     const int vc = (V - v0) < step ? (V - v0) : step;
     const __nv_bfloat16* wc = reinterpret_cast<const __nv_bfloat16*>(weight) + (long long)v0 * ldw;
-    // 1. dlogits chunk [T, vc] (recompute logits tile on tcgen05, transform in the epilogue)
-    {
+    // 1. dlogits chunk [T, vc]: from kept logits, or recompute the logits tile on tcgen05 and transform in the epilogue
+    if ((v0 + vc + 7) / 8 * 8 <= keep_cols && (reinterpret_cast<uintptr_t>(dz_chunk) & 15) == 0) {
+      lmhead_dlogits_kernel<<<T, 256, 0, stream>>>(logits, ld_logits, labels, lse, dlogp, 1.f / temperature, v0, vc,
+                                                   reinterpret_cast<__nv_bfloat16*>(dz_chunk), chunk_cols);
+      check_cuda(cudaGetLastError(), "lmhead_dlogits");
+    } else {
       const bool pair = pair_serves(T, num_sms);
       const CUtensorMap tb = make_tmap_2d(wc, H, vc, ldw, 64, pair ? kLmBN / 2 : kLmBN);
       GemmShape p;

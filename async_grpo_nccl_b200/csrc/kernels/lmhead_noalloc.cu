@@ -109,7 +109,7 @@ extern "C" int agrpo_lmhead_logprob_noalloc(const void* hidden_bf16, long long h
   }
   try {
     agrpo::launch_lmhead_logprob(hidden_bf16, hidden_pitch, weight_bf16, weight_pitch, labels, T, H, V, temperature, partials,
-                                 label_logit, logp, entropy, lse, g_status_addr[dev], g_num_sms[dev], s);
+                                 label_logit, logp, entropy, lse, nullptr, 0, 0, g_status_addr[dev], g_num_sms[dev], s);
   } catch (const std::exception& ex) {
     set_msg(err_msg, err_cap, ex.what());
     return AGRPO_NOALLOC_E_CUDA;

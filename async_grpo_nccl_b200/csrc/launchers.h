@@ -237,8 +237,11 @@ int lmhead_num_groups(int V, int T);
 // Outputs (each may be nullptr): logp[t] = z[label] - lse (0 on masked rows), entropy[t], lse[t].
 void launch_lmhead_logprob(const void* hidden, long long ldh, const void* weight, long long ldw, const int* labels, int T,
                            int H, int V, float temperature, float* partials, float* label_logit, float* logp,
-                           float* entropy, float* lse, int* status, int num_sms, cudaStream_t stream);
-// Per-token dual-clip GRPO objective (+ kl_beta * k3 KL against ref_logp), its derivative w.r.t. logp scaled by
+                           float* entropy, float* lse, float* logits, long long ld_logits, int keep_cols, int* status, int num_sms,
+                           cudaStream_t stream);
+// keep_cols > 0: the fp32 logits (before the temperature) of that many leading columns, a multiple of 8 or from V on, also go to
+// logits [T, ld_logits] (rows on 32 bytes, ld_logits >= keep_cols and >= V rounded up to 8 where keep_cols >= V); the backward pass
+// reads them instead of recomputing the product. Per-token dual-clip GRPO objective (+ kl_beta * k3 KL against ref_logp), its derivative w.r.t. logp scaled by
 // grad_weight, and sums over valid tokens in stats[grpo_num_loss_stats()] (atomic adds; zero it first).
 void launch_grpo_token_loss(const float* logp, const float* old_logp, const float* ref_logp, const float* adv,
                             const int* labels, const float* entropy, const float* old_entropy, int T, float clip_low,
@@ -249,8 +252,8 @@ int grpo_num_loss_stats();
 // dz_chunk: bf16 [T, chunk_cols] scratch, chunk_cols a multiple of 256.
 void launch_lmhead_backward(const void* hidden, long long ldh, const void* weight, long long ldw, const int* labels,
                             const float* lse, const float* dlogp, int T, int H, int V, float temperature, void* dz_chunk,
-                            int chunk_cols, float* dh_acc, float* dweight, long long ld_dw, int* status, int num_sms,
-                            cudaStream_t stream);
+                            int chunk_cols, float* dh_acc, float* dweight, long long ld_dw, const float* logits, long long ld_logits, int keep_cols,
+                            int* status, int num_sms, cudaStream_t stream);
 
 // ---- rollout engine (rollout.cu) ----
 // KV cache layout per layer: [num_blocks, Hkv, block_size, D] (K and V separately). slots[t] < 0 skips token t.

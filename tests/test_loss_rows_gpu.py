@@ -51,3 +51,28 @@ def test_sample_without_prompt_keeps_all_rows():
     from async_grpo_nccl_b200.packing import pack_samples
 
     assert not pack_samples(samples([(0, 9), (4, 3)], 2000)).loss_rows
+
+
+# rows below and above one pair tile, a vocabulary that is no multiple of 8, buffers that hold no, some and all of the columns
+@pytest.mark.parametrize("T,H,V,chunk,keep", [(70, 128, 1003, 512, 1008), (300, 256, 2048, 512, 2048), (300, 256, 2048, 512, 1280), (513, 128, 5001, 1024, 2048),
+                                              (129, 64, 264, 256, 256)])
+def test_kept_logits_give_the_same_gradients(T, H, V, chunk, keep):
+    from gpu_util import native, status_word
+
+    C = native()
+    torch.manual_seed(T)
+    h, W = (torch.randn(n, H, device="cuda").mul_(0.3).to(torch.bfloat16) for n in (T, V))
+    labels = torch.randint(0, V, (T,), device="cuda", dtype=torch.int32)
+    labels[::7] = -1
+    dlogp, st = torch.randn(T, device="cuda"), status_word()
+    groups = C.lmhead_num_groups(V, T)
+    got = []
+    for logits in (None, torch.full((T, keep), float("nan"), device="cuda")):
+        f = lambda n: torch.zeros(n, device="cuda")
+        logp, ent, lse = f(T), f(T), f(T)
+        C.lmhead_logprob(h, W, labels, 0.7, f(3 * groups * T), f(T), logp, ent, lse, st, logits)
+        dz, dh, dW = torch.empty(T, chunk, device="cuda", dtype=torch.bfloat16), f(T * H).view(T, H), f(V * H).view(V, H)
+        C.lmhead_backward(h, W, labels, lse, dlogp, 0.7, dz, dh, dW, st, logits)
+        got.append((logp, ent, lse, dh, dW))
+    assert int(st.item()) == 0
+    assert all(torch.equal(a, b) for a, b in zip(*got))
