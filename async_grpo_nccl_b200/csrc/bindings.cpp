@@ -810,10 +810,6 @@ void decode_layers(int64_t L, int64_t B, const Tensor& wqkv0, int64_t wqkv_strid
   a.partials = partials.data_ptr<float>(); a.partials_bytes = partials.numel() * 4;
   a.counters = reinterpret_cast<unsigned int*>(counters.data_ptr<int>());
   a.status = opt_ptr<int>(status);
-  {
-    static const int pf = [] { const char* e = std::getenv("AGRPO_MEGA_PREFETCH"); return e ? std::atoi(e) : 8; }();
-    a.prefetch_tiles = pf;
-  }
   if (trace.has_value() && trace->defined()) {
     check_i64(*trace, "trace");
     TORCH_CHECK(trace->numel() >= 32 && trace->is_contiguous(), "decode_layers: trace [32]");

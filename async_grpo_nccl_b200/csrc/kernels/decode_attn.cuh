@@ -4,6 +4,7 @@
 #include <cuda_bf16.h>
 
 #include "../common/ptx.cuh"
+#include "decode_sync.cuh"
 
 namespace agrpo {
 
@@ -86,21 +87,6 @@ __device__ __forceinline__ void dec_bar_sync() { asm volatile("bar.sync 1, 128;"
 // (loads in flight).
 // `cache_off`: elements from the caches' start to this layer's. `p` is best a kernel parameter: as a local struct it takes
 // 30 registers.
-// Asks for this item's first pages to be brought into L2: at most 256 KB, so that the items of a long context do not push one
-// another (and the weights) out again before they are read.
-__device__ __forceinline__ void paged_decode_prefetch(const DecodeParams& p, long long cache_off, int split, int kvh, int b, int tid) {
-  const int n_blocks = (p.seq_lens[b] + kDecBlock - 1) / kDecBlock;
-  const int blk_begin = (int)((long long)n_blocks * split / p.splits);
-  const int blk_end = (int)((long long)n_blocks * (split + 1) / p.splits);
-  if (tid < 32 && blk_begin + tid < blk_end) {
-    const int page = p.block_tables[(long long)b * p.max_blocks + blk_begin + tid];
-    if (page < 0 || page >= p.num_cache_blocks) return;  // reported by the loads themselves
-    const long long at = cache_off + ((long long)page * p.Hkv + kvh) * kDecBlock * kDecD;
-    bulk_prefetch_l2(p.k_cache + at, kDecBlock * kDecD * 2);
-    bulk_prefetch_l2(p.v_cache + at, kDecBlock * kDecD * 2);
-  }
-}
-
 // ready() returns once the query row and the newest token's cache row are visible to the calling warp. The first blocks of older
 // tokens are requested before it: they do not depend on this layer.
 // emit(g, d, acc, M, L): weighted sum, maximum and denominator of head g at dim d over this split's tokens.
@@ -110,8 +96,8 @@ __device__ __forceinline__ void paged_decode_partial(const DecodeParams& p, long
   const int lane = tid & 31;
   const int seq_len = p.seq_lens[b];
   const int n_blocks = (seq_len + kDecBlock - 1) / kDecBlock;
-  const int blk_begin = (int)((long long)n_blocks * split / p.splits);
-  const int blk_end = (int)((long long)n_blocks * (split + 1) / p.splits);
+  const int blk_begin = share(n_blocks, split, p.splits);
+  const int blk_end = share(n_blocks, split + 1, p.splits);
   // per-warp staging: STAGES x (K tile 4 KB + V tile 4 KB)
   const uint32_t wbuf = smem_u32(dsm) + warp * (STAGES * 8192);
   const int* table = p.block_tables + (long long)b * p.max_blocks;
@@ -147,7 +133,7 @@ __device__ __forceinline__ void paged_decode_partial(const DecodeParams& p, long
   // same tile. The first 2 STAGES - 1 tiles now: the scores of block i + 1 are computed before block i's values are added
   // up, so K runs one block ahead of V.
   bool late = false;  // the newest token's block is among the first ones
-#pragma unroll
+#pragma unroll 1
   for (int j = 0; j < kSlots - 1; ++j) {
     const int blk = my0 + (j >> 1) * kDecWarps;
     if (blk < blk_end) {
@@ -267,6 +253,7 @@ __device__ __forceinline__ void paged_decode_partial(const DecodeParams& p, long
   dec_bar_sync();
   float* mo = reinterpret_cast<float*>(dsm);           // [warps][8][D]
   float* mml = mo + kDecWarps * 8 * kDecD;             // [warps][8][2]
+  float* fin = mml + kDecWarps * 8 * 2;                // [8][8]: weights of the four warps, maximum, denominator
   {
     const int g = lane >> 2;
 #pragma unroll
@@ -280,25 +267,37 @@ __device__ __forceinline__ void paged_decode_partial(const DecodeParams& p, long
     }
   }
   dec_bar_sync();
-  static_assert(kDecD == kDecWarps * 32, "a thread per output dim");
-  float acc[8], M[8], L[8];
+  if (warp == 0) {  // a lane for each of 8 heads x 4 warps
+    const int g = lane >> 2;
+    float M = -INFINITY, L = 0.f, mine = 0.f;
 #pragma unroll
-  for (int g = 0; g < 8; ++g) {  // heads above G (rows of zeros) too: independent of one another, nothing is emitted between the loads
-    M[g] = -INFINITY;
-#pragma unroll
-    for (int w = 0; w < kDecWarps; ++w) M[g] = fmaxf(M[g], mml[(w * 8 + g) * 2]);
-    L[g] = acc[g] = 0.f;
+    for (int w = 0; w < kDecWarps; ++w) M = fmaxf(M, mml[(w * 8 + g) * 2]);
 #pragma unroll
     for (int w = 0; w < kDecWarps; ++w) {
       const float mw = mml[(w * 8 + g) * 2];
-      const float wgt = (mw == -INFINITY) ? 0.f : exp2f(mw - M[g]);
-      L[g] += mml[(w * 8 + g) * 2 + 1] * wgt;
-      acc[g] += mo[(w * 8 + g) * kDecD + tid] * wgt;
+      const float wgt = (mw == -INFINITY) ? 0.f : exp2f(mw - M);
+      L += mml[(w * 8 + g) * 2 + 1] * wgt;
+      if (w == (lane & 3)) mine = wgt;
+    }
+    fin[g * 8 + (lane & 3)] = mine;
+    if ((lane & 3) == 0) {
+      fin[g * 8 + 4] = M;
+      fin[g * 8 + 5] = L;
     }
   }
-#pragma unroll
-  for (int g = 0; g < 8; ++g)
-    if (g < p.G) emit(g, tid, acc[g], M[g], L[g]);
+  dec_bar_sync();
+  static_assert(kDecD == kDecWarps * 32, "a thread per output dim");
+#pragma unroll 2
+  for (int g = 0; g < p.G; ++g) {
+    const float4 wgt = *reinterpret_cast<const float4*>(fin + g * 8);
+    const float2 ml = *reinterpret_cast<const float2*>(fin + g * 8 + 4);
+    float acc = 0.f;
+    acc += mo[g * kDecD + tid] * wgt.x;
+    acc += mo[(8 + g) * kDecD + tid] * wgt.y;
+    acc += mo[(16 + g) * kDecD + tid] * wgt.z;
+    acc += mo[(24 + g) * kDecD + tid] * wgt.w;
+    emit(g, tid, acc, ml.x, ml.y);
+  }
 }
 
 // The item as the stand-alone kernel runs it: partial sums to memory, the last split of a (sequence, kv head) merges.

@@ -26,8 +26,13 @@
 // latter so that row statistics and residuals are in registers when the accumulator is. Attention has warps of its own: in one
 // loop with the epilogues its registers spill, and local memory is slow here, since every acquire empties the L1.
 //
+// The code has to stay small: every role's instructions are needed once a phase, and at 161 KB of them each phase waited for the
+// instruction cache (an epilogue of 1.5 us took 5). So loops that run once a layer are not unrolled, and waits poll in one place.
+//
 // Bound by the chain of hand-offs, not by bytes. 28 layers of 1536 / 8960, a step: 16 rows x 2048 tokens 1.66 ms with arrival
-// counters and attention in the compute warps, 1.49 ms so; 32 rows x 1024 tokens 1.65 and 1.47 (weights alone: 0.48).
+// counters and attention in the compute warps, 1.45 ms so; 32 rows x 1024 tokens 1.65 and 1.42 (weights alone: 0.48). Handing the
+// activations over by value as well (polled by the attention warps) gave 1.44 and 1.43: what it saved in fences it lost to the
+// polls' traffic.
 //
 // Every wait is bounded; a wait that runs out records a status code, makes the CTA leave through its normal exit (TMEM
 // freed) and the other CTAs follow as soon as they see the status word.
@@ -80,7 +85,6 @@ struct MegaParams {
   int* status;
   long long* trace;  // optional: clock64 stamps of CTA 0 in layer trace_layer (32 slots), nullptr = off
   int trace_layer;
-  int prefetch_tiles;  // weight tiles (16 KB) per CTA requested into L2 ahead of the shared-memory ring (0 = off)
   int trace_all;     // also record 4 global-timer stamps per CTA (trace must hold 32 + 4 * grid words)
 };
 
@@ -112,7 +116,7 @@ struct MegaCfg {
   static constexpr int kNSX = (kXA / kXStage) > 8 ? 8 : (kXA / kXStage);
   static constexpr int kAcc = 2;
   static constexpr uint32_t kTmemCols = (kAcc * BT) < 32 ? 32 : (kAcc * BT);
-  static constexpr int kEx = 2 * 2 * 16 * 64 * 4;  // gate / up exchange: two turns of 16 rows x 64 features each way
+  static constexpr int kEx = 32 * kFT * 4;  // gate / up exchange: 32 rows
   static constexpr int kSmem = kNSW * kWStage + kXA + kEx + 1024 /* barriers */ + 1024 /* alignment */;
   // rows of a share that a warp reduces at a time, and partials of a row requested at a time
   static constexpr int kRU = BT <= 32 ? 1 : 2;
@@ -137,27 +141,23 @@ __device__ __forceinline__ bool gather_handoff(T (&t)[N], const int* status, Loa
   uint32_t missing = 0;
 #pragma unroll
   for (int k = 0; k < N; ++k)
-    if (wanted(k)) t[k] = load(k);
-#pragma unroll
-  for (int k = 0; k < N; ++k)
-    if (wanted(k) && !arrived(t[k])) missing |= 1u << k;
+    if (wanted(k)) missing |= 1u << k;
   bool ok = true;
-  if (missing != 0) {
-    const long long t0 = clock64();
-    int it = 0;
-    do {
+  const long long t0 = clock64();
+  int it = 0;
+#pragma unroll 1
+  while (missing != 0) {  // one copy of the loads
 #pragma unroll
-      for (int k = 0; k < N; ++k)
-        if (missing >> k & 1) t[k] = load(k);
+    for (int k = 0; k < N; ++k)
+      if (missing >> k & 1) t[k] = load(k);
 #pragma unroll
-      for (int k = 0; k < N; ++k)
-        if ((missing >> k & 1) && arrived(t[k])) missing &= ~(1u << k);
-      if ((++it & 31) == 0 && (status_set(status) || clock64() - t0 > kWaitBudgetTicks)) {
-        report_status(const_cast<int*>(status), kStatusBarrierTimeout);
-        ok = false;
-        break;
-      }
-    } while (missing != 0);
+    for (int k = 0; k < N; ++k)
+      if ((missing >> k & 1) && arrived(t[k])) missing &= ~(1u << k);
+    if ((++it & 31) == 0 && (status_set(status) || clock64() - t0 > kWaitBudgetTicks)) {
+      report_status(const_cast<int*>(status), kStatusBarrierTimeout);
+      ok = false;
+      break;
+    }
   }
   __syncwarp();
   return ok;
@@ -296,76 +296,42 @@ decode_layers_kernel(const __grid_constant__ CUtensorMap tmWqkv, const __grid_co
     asm volatile("setmaxnreg.dec.sync.aligned.u32 96;");
     if (warp == 0) {
       // ================= weight producer: never waits for another CTA =================
-      // Two cursors walk the same sequence of weight tiles (layer, phase, item, K block): `ld` issues the TMA loads into
-      // the shared-memory ring, `pf` runs prefetch_tiles ahead of it and only asks for the tiles to be brought into L2.
-      // The ring alone covers a few microseconds of streaming; the L2 window keeps HBM busy through the attention phase
-      // and the hand-offs between phases, when the ring is full and nobody consumes it.
+      // Tiles in the order in which the products use them (layer, phase, item, K block), limited only by the depth of the ring. (Asking
+      // for tiles further on to be brought into L2 costs more than it gives: 8 tiles ahead 1.47 ms a step of 16 rows, none 1.44.)
       if (elect_one()) {
-        struct Cur {
-          int l, ph, item, kb, kb1, ft;
-        };
-        auto seek = [&](Cur& c) -> bool {  // first K block of the item at (l, ph, item), or of the next one that exists
-          while (c.l < p.L) {
-            const int S = p.ph[c.ph].S, nkb = p.ph[c.ph].num_kb;
-            if (c.item < p.ph[c.ph].n_groups * S) {
-              c.ft = c.item / S;
-              const int ks = c.item - c.ft * S;
-              c.kb = (int)((long long)nkb * ks / S);
-              c.kb1 = (int)((long long)nkb * (ks + 1) / S);
-              if (c.kb < c.kb1) return true;
-              c.item += G;
-              continue;
-            }
-            c.item = cta;
-            if (++c.ph == 4) {
-              c.ph = 0;
-              ++c.l;
-            }
-          }
-          return false;
-        };
-        auto step = [&](Cur& c) -> bool {
-          if (++c.kb < c.kb1) return true;
-          c.item += G;
-          return seek(c);
-        };
-        auto tmap = [&](int ph) { return ph == 0 ? &tmWqkv : ph == 1 ? &tmWo : ph == 2 ? &tmWgu : &tmWd; };
-        Cur ld{0, 0, cta, 0, 0, 0}, pf{0, 0, cta, 0, 0, 0};
-        bool ld_on = seek(ld), pf_on = seek(pf);
-        int ahead = 0;
         int st = 0;
         uint32_t par = 0;
         bool ok = true;
-        while (ld_on) {
-          while (pf_on && ahead < p.prefetch_tiles) {
-            if (pf.ph == 2) {
-              tma_prefetch_l2_3d(tmap(2), pf.kb * kMBK, pf.ft * 64, pf.l);
-              tma_prefetch_l2_3d(tmap(2), pf.kb * kMBK, p.F + pf.ft * 64, pf.l);
-            } else {
-              tma_prefetch_l2_3d(tmap(pf.ph), pf.kb * kMBK, pf.ft * kFT, pf.l);
+#pragma unroll 1
+        for (int l = 0; l < p.L && ok; ++l) {
+#pragma unroll 1
+          for (int ph = 0; ph < 4 && ok; ++ph) {
+            const CUtensorMap* map = ph == 0 ? &tmWqkv : ph == 1 ? &tmWo : ph == 2 ? &tmWgu : &tmWd;
+            const int S = p.ph[ph].S, nkb = p.ph[ph].num_kb, n_items = p.ph[ph].n_groups * S;
+#pragma unroll 1
+            for (int item = cta; item < n_items && ok; item += G) {
+              const int ft = item / S, ks = item - ft * S;
+              const int row = ft * (ph == 2 ? 64 : kFT);
+              const int kb1 = share(nkb, ks + 1, S);
+#pragma unroll 1
+              for (int kb = share(nkb, ks, S); kb < kb1; ++kb) {
+                if (!mbar_wait_s(&sh->empty_w[st], par ^ 1, p.status)) {
+                  report_status(p.status, kStatusWaitEmptyTimeout);
+                  ok = false;
+                  break;
+                }
+                uint8_t* dst = w_ring + st * kWStage;
+                mbar_expect_tx(&sh->full_w[st], kWStage);
+                // gate / up: 64 gate features on MMA rows 0..63 (the map's box), the matching 64 up features on rows 64..127
+                tma_load_3d(dst, map, &sh->full_w[st], kb * kMBK, row, l);
+                if (ph == 2) tma_load_3d(dst + 64 * kMBK * 2, map, &sh->full_w[st], kb * kMBK, p.F + row, l);
+                if (++st == NSW) {
+                  st = 0;
+                  par ^= 1;
+                }
+              }
             }
-            pf_on = step(pf);
-            ++ahead;
           }
-          if (!mbar_wait_s(&sh->empty_w[st], par ^ 1, p.status)) {
-            report_status(p.status, kStatusWaitEmptyTimeout);
-            ok = false;
-            break;
-          }
-          uint8_t* dst = w_ring + st * kWStage;
-          mbar_expect_tx(&sh->full_w[st], kWStage);
-          if (ld.ph == 2) {  // 64 gate features on MMA rows 0..63, the matching 64 up features on rows 64..127
-            tma_load_3d(dst, tmap(2), &sh->full_w[st], ld.kb * kMBK, ld.ft * 64, ld.l);
-            tma_load_3d(dst + 64 * kMBK * 2, tmap(2), &sh->full_w[st], ld.kb * kMBK, p.F + ld.ft * 64, ld.l);
-          } else {
-            tma_load_3d(dst, tmap(ld.ph), &sh->full_w[st], ld.kb * kMBK, ld.ft * kFT, ld.l);
-          }
-          if (++st == NSW) {
-            st = 0;
-            par ^= 1;
-          }
-          ld_on = step(ld);
-          --ahead;
         }
         if (!ok) sh->abort = 1;
       }
@@ -404,7 +370,7 @@ decode_layers_kernel(const __grid_constant__ CUtensorMap tmWqkv, const __grid_co
                 staged = -1;
               }
               const int ft = item / S, ks = item - ft * S;
-              const int kb0 = (int)((long long)nkb * ks / S), kb1 = (int)((long long)nkb * (ks + 1) / S);
+              const int kb0 = share(nkb, ks, S), kb1 = share(nkb, ks + 1, S);
               for (int kb = kb0; kb < kb1; ++kb) {
                 if (!mbar_wait_s(&sh->empty_x[st], par ^ 1, p.status)) {
                   report_status(p.status, kStatusWaitEmptyTimeout);
@@ -434,7 +400,7 @@ decode_layers_kernel(const __grid_constant__ CUtensorMap tmWqkv, const __grid_co
             const int S = p.ph[ph].S, nkb = p.ph[ph].num_kb, n_items = p.ph[ph].n_groups * S;
             for (int item = cta; item < n_items && ok; item += G) {
               const int ft = item / S, ks = item - ft * S;
-              const int kb0 = (int)((long long)nkb * ks / S), kb1 = (int)((long long)nkb * (ks + 1) / S);
+              const int kb0 = share(nkb, ks, S), kb1 = share(nkb, ks + 1, S);
               if (!mbar_wait_s(&sh->tmem_empty[acc], pa ^ 1, p.status)) {
                 report_status(p.status, kStatusWaitTmemEmptyTimeout);
                 ok = false;
@@ -529,7 +495,7 @@ decode_layers_kernel(const __grid_constant__ CUtensorMap tmWqkv, const __grid_co
           const int grp = item / S, ks = item - grp * S;
           if (!waited) wait_done(target(l, ph));
           waited = true;
-          const int r0 = (int)((long long)B * ks / S), r1 = (int)((long long)B * (ks + 1) / S);
+          const int r0 = share(B, ks, S), r1 = share(B, ks + 1, S);
           constexpr int RU = Cfg::kRU, NS = Cfg::kNS;
           const int b_first = r0 + cw * RU;
           // Row statistics, lengths and the residual of this warp's first rows: requested while the product still runs.
@@ -577,62 +543,62 @@ decode_layers_kernel(const __grid_constant__ CUtensorMap tmWqkv, const __grid_co
           };
           float rs_next = 0.f;
           if (direct) rs_next = row_scale(0);
-          else load_meta(b_first);
-          if (!mbar_wait_s(&sh->tmem_full[acc], pa, p.status)) {
-            report_status(p.status, kStatusWaitTmemFullTimeout);
-            fail = true;
-          }
-          tc_fence_after();
-          if (tid == 0) MEGA_STAMP(ph * 6 + 2);
-          float* slot = p.partials + (size_t)item * (BT * kFT);
+          float* gbase = p.partials + (size_t)(grp * S) * (BT * kFT);
+          // The first pass begins before the product is complete (at least one, also for a warp without rows); one copy of the code.
 #pragma unroll 1
-          for (int c = 0; c < BT / 32; ++c) {
-            if (c * 32 >= B) break;  // padding rows
-            uint32_t r[32];
-            tmem_ld_32x32(tmem_base + lane_off + (uint32_t)(acc * BT + c * 32), r);
-            tc_wait_ld();
-            if (!direct) {
+          for (int b0 = b_first; b0 == b_first || b0 < r1; b0 += 4 * RU) {
+            if (!direct) load_meta(b0);
+            if (b0 == b_first) {
+              if (!mbar_wait_s(&sh->tmem_full[acc], pa, p.status)) {
+                report_status(p.status, kStatusWaitTmemFullTimeout);
+                fail = true;
+              }
+              tc_fence_after();
+              if (tid == 0) MEGA_STAMP(ph * 6 + 2);
+              float* slot = p.partials + (size_t)item * (BT * kFT);
+#pragma unroll 1
+              for (int c = 0; c < BT / 32; ++c) {
+                if (c * 32 >= B) break;  // padding rows
+                uint32_t r[32];
+                tmem_ld_32x32(tmem_base + lane_off + (uint32_t)(acc * BT + c * 32), r);
+                tc_wait_ld();
+                if (!direct) {
 #pragma unroll
-              for (int i = 0; i < 32; ++i)
-                if (c * 32 + i < B) st_handoff(slot + (size_t)(c * 32 + i) * kFT + cw * 32 + lane, __uint_as_float(r[i]));
-              continue;
-            }
-            // Warps 0 and 1 hold the gate features, 2 and 3 the up features. The former finish the even rows, the latter the
-            // odd ones: each gives away the half that it does not finish. Two buffers in turn, so one barrier a turn is enough.
-            const bool up = cw >= 2;
-            const float rs_mine = rs_next;
-            if ((c + 1) * 32 < B) rs_next = row_scale(c + 1);
-            float* give = ex + ((c & 1) * 2 + (up ? 1 : 0)) * (16 * 64) + (cw & 1) * 32 + lane;
-            const float* take = ex + ((c & 1) * 2 + (up ? 0 : 1)) * (16 * 64) + (cw & 1) * 32 + lane;
+                  for (int i = 0; i < 32; ++i)
+                    if (c * 32 + i < B) st_handoff(slot + (size_t)(c * 32 + i) * kFT + cw * 32 + lane, __uint_as_float(r[i]));
+                  continue;
+                }
+                // Warps 0 and 1 hold the gate features, 2 and 3 the up features: through shared memory, then a warp takes every fourth
+                // row, a lane two features.
+                const float rs_mine = rs_next;
+                if (c + 1 < BT / 32 && (c + 1) * 32 < B) rs_next = row_scale(c + 1);
+                if (c > 0) asm volatile("bar.sync 2, 128;" ::: "memory");
 #pragma unroll
-            for (int i = 0; i < 16; ++i) give[i * 64] = __uint_as_float(up ? r[2 * i] : r[2 * i + 1]);
-            asm volatile("bar.sync 2, 128;" ::: "memory");
-            __nv_bfloat16* dst = p.act + (size_t)(c * 32 + (up ? 1 : 0)) * p.F + grp * 64 + (cw & 1) * 32 + lane;
-#pragma unroll
-            for (int i0 = 0; i0 < 16; i0 += 4) {
-              if (c * 32 + 2 * i0 >= B) break;
-#pragma unroll
-              for (int i = i0; i < i0 + 4; ++i) {
-                const float rs = __shfl_sync(0xffffffffu, rs_mine, 2 * i + (up ? 1 : 0));
-                const float mine = __uint_as_float(up ? r[2 * i + 1] : r[2 * i]), theirs = take[i * 64];
-                const float g = (up ? theirs : mine) * rs, u = (up ? mine : theirs) * rs;
-                const __nv_bfloat16 o = __float2bfloat16(g / (1.f + __expf(-g)) * u);
-                if (c * 32 + 2 * i + (up ? 1 : 0) < B) dst[(size_t)(2 * i) * p.F] = o;
+                for (int i = 0; i < 32; ++i) ex[i * kFT + cw * 32 + lane] = __uint_as_float(r[i]);
+                asm volatile("bar.sync 2, 128;" ::: "memory");
+#pragma unroll 2
+                for (int i = cw; i < 32; i += 4) {
+                  const int row = c * 32 + i;
+                  if (row >= B) break;
+                  const float rs = __shfl_sync(0xffffffffu, rs_mine, i);
+                  const float2 gv = *reinterpret_cast<const float2*>(ex + i * kFT + 2 * lane);
+                  const float2 uv = *reinterpret_cast<const float2*>(ex + i * kFT + 64 + 2 * lane);
+                  const float g0 = gv.x * rs, g1 = gv.y * rs;
+                  *reinterpret_cast<uint32_t*>(p.act + (size_t)row * p.F + grp * 64 + 2 * lane) =
+                      pack_bf16x2(g0 / (1.f + __expf(-g0)) * (uv.x * rs), g1 / (1.f + __expf(-g1)) * (uv.y * rs));
+                }
+              }
+              tc_fence_before();
+              __syncwarp();
+              if (lane == 0) mbar_arrive(&sh->tmem_empty[acc]);
+              if (tid == 0) MEGA_STAMP(ph * 6 + 3);
+              if (++acc == Cfg::kAcc) {
+                acc = 0;
+                pa ^= 1;
               }
             }
-          }
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&sh->tmem_empty[acc]);
-          if (tid == 0) MEGA_STAMP(ph * 6 + 3);
-          if (++acc == Cfg::kAcc) {
-            acc = 0;
-            pa ^= 1;
-          }
-          // ---- my share of the rows: reduce over the S partials, epilogue ----
-          float* gbase = p.partials + (size_t)(grp * S) * (BT * kFT);
-          for (int b0 = b_first; !direct && b0 < r1; b0 += 4 * RU) {
-            if (b0 != b_first) load_meta(b0);
+            if (direct || b0 >= r1) break;
+            // ---- my share of the rows: reduce over the S partials, epilogue ----
             float4 v[RU];
             bool on[RU];
 #pragma unroll
@@ -739,10 +705,6 @@ decode_layers_kernel(const __grid_constant__ CUtensorMap tmWqkv, const __grid_co
       const unsigned int qkv_done = (unsigned int)l * p.per_layer + (unsigned int)(p.ph[0].n_groups * p.ph[0].S);
       // The K/V blocks are staged in the activation ring: this CTA's products have read all that was in it, and it is not
       // filled again before xa_bar.
-      for (int it = cta; it < p.att_items; it += G) {
-        const int rest = it / p.splits;
-        paged_decode_prefetch(p.att, (long long)l * p.cache_layer_stride, it % p.splits, rest % p.Hkv, rest / p.Hkv, tid);
-      }
       if (!wait_seen(&sh->xa_free, (unsigned int)(l + 1), p.status)) {
         report_status(p.status, kStatusBarrierTimeout);
         fail = true;
@@ -889,7 +851,6 @@ void launch_decode_layers(const DecodeLayersArgs& a, cudaStream_t stream) {
   p.status = a.status;
   p.trace = a.trace;
   p.trace_layer = a.trace_layer;
-  p.prefetch_tiles = a.prefetch_tiles;
   p.trace_all = a.trace_words >= 32 + 4 * a.num_sms ? 1 : 0;
   // the counter starts from zero and the handed-over buffers from "not yet" in every launch (stream-ordered, also inside a
   // captured graph)

@@ -9,6 +9,10 @@ namespace agrpo {
 
 namespace {
 
+// Where part i of n begins when `total` is cut into n parts. In 32 bits: a 64-bit division is 2 KB of code, and there were fourteen
+// in the persistent kernel. total * n stays far below 2^32 for K blocks, rows and the cache blocks of a sequence.
+__device__ __forceinline__ int share(int total, int i, int n) { return (int)((unsigned)total * (unsigned)i / (unsigned)n); }
+
 __device__ __forceinline__ unsigned int ld_acquire_gpu(const unsigned int* p) {
   unsigned int v;
   asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
