@@ -590,17 +590,20 @@ int kept_cols(const OptTensor& logits, int64_t T, int64_t V) {
   return (int)logits->size(1);
 }
 long long ld_kept(const OptTensor& logits) { return logits.has_value() && logits->defined() ? logits->size(1) : 0; }
-// Columns of [rows, V] fp32 that may be kept from the forward to the backward pass: as many as a quarter of the memory that this
-// process could still get (free on the device, or cached by torch's allocator) holds, in steps of 256.
-int64_t lmhead_keep_columns(int64_t rows, int64_t V) {
+// Columns of [rows, V] fp32 that may be kept from the forward to the backward pass of a step that takes about `reserve` bytes besides.
+// All of them if torch's allocator holds enough unused memory for both, as it does from the second step of a kind on; else as many as
+// a quarter of what this process could get beyond `reserve` holds, in steps of 256. The device is only asked in the second case:
+// on a machine with other users cudaMemGetInfo takes 0.1 to 100 ms.
+int64_t lmhead_keep_columns(int64_t rows, int64_t V, double reserve) {
   if (rows <= 0) return 0;
-  const int64_t all = (V + 7) / 8 * 8;
-  if (all * rows * 4 <= (64 << 20)) return all;
-  size_t free_b = 0, total_b = 0;
-  C10_CUDA_CHECK(cudaMemGetInfo(&free_b, &total_b));
+  const int64_t all = (V + 7) / 8 * 8, need = all * rows * 4;
+  if (need <= (64 << 20)) return all;
   const auto st = c10::cuda::CUDACachingAllocator::getDeviceStats(c10::cuda::current_device());
   const int64_t cached = st.reserved_bytes[0].current - st.allocated_bytes[0].current;  // [0]: over all pools
-  const int64_t cols = ((int64_t)free_b + cached) / 4 / (rows * 4);
+  if (cached >= need + (int64_t)(0.6 * reserve)) return all;  // `reserve` is an estimate from above
+  size_t free_b = 0, total_b = 0;
+  C10_CUDA_CHECK(cudaMemGetInfo(&free_b, &total_b));
+  const int64_t cols = std::max<int64_t>(0, (int64_t)free_b + cached - (int64_t)reserve) / 4 / (rows * 4);
   return cols >= all ? all : cols / 256 * 256;
 }
 void lmhead_logprob(const Tensor& hidden, const Tensor& weight, const Tensor& labels, double temperature, Tensor& partials,

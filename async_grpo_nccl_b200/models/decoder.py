@@ -366,6 +366,13 @@ class NativeDecoder:
         self.launches += 1
         return hn, rstd
 
+    def _activation_bytes(self, T: int) -> float:
+        """What a training step of T rows holds at its peak besides kept logits, roughly and from above."""
+        cfg = self.cfg
+        layer = 2.0 * T * (5 * cfg.hidden_size + cfg.qkv_dim + cfg.q_dim + 3 * cfg.intermediate_size)
+        layers = 2.0 * T * cfg.hidden_size * cfg.num_hidden_layers + 2 * layer if self.recompute else layer * cfg.num_hidden_layers
+        return 1.25 * (layers + layer) + 2.0 * T * vocab_chunk(T, self.lmhead_chunk)
+
     def _body(self, batch: PackedBatch, saves: Optional[List[dict]]) -> torch.Tensor:
         """Embedding and all layers."""
         cfg, C = self.cfg, self.C
@@ -416,14 +423,22 @@ class NativeDecoder:
         T = batch.T
         cos_t, sin_t = self.rope_tables()
         saves: List[dict] = []
-        x_last = self._body(batch, saves)
         # From the final norm to its gradient only rows with a label take part: prompts and the last row of a sample have none
-        # (a third of the rows where answers are short), and their gradient is zero.
+        # (a third of the rows where answers are short), and their gradient is zero. Work that is saved: logits twice, two gradients.
+        compact = (batch.loss_rows and batch.total_out > 0
+                   and 8.0 * (T - batch.total_out) * cfg.vocab_size * cfg.hidden_size > LOSS_ROWS_MIN_FLOPS)
+        # The backward pass needs the logits again: kept in fp32 (31287 x 151936: 19 GB) they are read once, 2 ms, instead of
+        # recomputed, 10 ms. Columns that do not fit into the memory that the activations leave are recomputed. They come first: a
+        # step then finds the block that the step before gave back whole, where a request behind the activations would find it
+        # split and ask the device for another (20 ms).
+        n_head = batch.total_out if compact else T
+        keep = int(C.lmhead_keep_columns(n_head, cfg.vocab_size, self._activation_bytes(T)))
+        logits = self._new(n_head, keep, dtype=torch.float32) if keep > 0 else None
+        x_last = self._body(batch, saves)
         labels, advantages, old_logp, old_ent = batch.labels, batch.advantages, batch.old_logprobs, batch.old_entropies
         ref = batch.ref_logprobs if (lc.kl_beta > 0 and batch.has_ref) else None
         rows = None
-        # logits twice, two gradients
-        if batch.loss_rows and batch.total_out > 0 and 8.0 * (T - batch.total_out) * cfg.vocab_size * cfg.hidden_size > LOSS_ROWS_MIN_FLOPS:
+        if compact:
             rows, x_all, n = batch.output_indices, x_last, batch.total_out
             x_last, labels, cols = self._new(n, cfg.hidden_size), self._new(n, dtype=torch.int32), self._new(4, n, dtype=torch.float32)
             C.gather_loss_rows(rows, x_all, batch.labels, batch.float_buf[:4 * T].view(4, T), x_last, labels, cols)
@@ -444,10 +459,6 @@ class NativeDecoder:
         chunk = min(vocab_chunk(T, self.lmhead_chunk), (V + 255) // 256 * 256)
         dz = self._new(T, chunk)
         dh_acc = self._new(T, cfg.hidden_size, dtype=torch.float32)
-        # The backward pass needs the logits again: kept in fp32 (31287 x 151936: 19 GB) they are read once, 2 ms, instead of
-        # recomputed, 10 ms. Columns that do not fit into a quarter of the free memory are recomputed.
-        keep = int(C.lmhead_keep_columns(T, V))
-        logits = self._new(T, keep, dtype=torch.float32) if keep > 0 else None
         C.lmhead_logprob(hn, wl, labels, lc.temperature, partials, ll, logp, ent, lse, self.status, logits)
         del partials
         stats = torch.zeros(self.n_stats, dtype=torch.float32, device=self.dev)
