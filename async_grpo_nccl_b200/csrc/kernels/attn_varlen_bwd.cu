@@ -53,6 +53,27 @@ struct AttnBwdParams {
   int* status;
 };
 
+// Two fp32 operations an instruction, each rounded as the single one.
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  float2 d;
+  asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmov.b64 z, {%6, %7};\n\t"
+      "fma.rn.f32x2 x, x, y, z;\n\tmov.b64 {%0, %1}, x;\n\t}"
+      : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return d;
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  float2 d;
+  asm("{\n\t.reg .b64 x, y;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tadd.rn.f32x2 x, x, y;\n\tmov.b64 {%0, %1}, x;\n\t}"
+      : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+  float2 d;
+  asm("{\n\t.reg .b64 x, y;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmul.rn.f32x2 x, x, y;\n\tmov.b64 {%0, %1}, x;\n\t}"
+      : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
+}
+
 __device__ __forceinline__ void named_bar_sync(int id, int count) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(count) : "memory");
 }
@@ -73,20 +94,26 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   constexpr int kTileBytes = kT * D * 2;
   constexpr int kChunkBytes = kT * 128;     // one 64-column swizzle chunk of a 128-row tile
   constexpr int kDsBytes = kT * kT * 2;
+  constexpr int kOutBytes = D > 64 ? 8 * 4096 : 0;
   constexpr uint32_t kTmemCols = 512;
   constexpr uint32_t kIdescST = umma_idesc_bf16(kT, kT, 0, 0);  // S^T, dP^T: both operands K-major
   constexpr uint32_t kIdescKV = umma_idesc_bf16(kT, D, 0, 1);   // dV, dK: A from TMEM, B MN-major
   constexpr uint32_t kIdescDQ = umma_idesc_bf16(kT, D, 1, 1);   // dQ: A (dS^T in smem) MN-major, B MN-major
 
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  // no slack to align by hand: the tiles, the buffer of dQ and the row statistics fill what a block may have
+  extern __shared__ __align__(1024) uint8_t smem[];
+  if ((smem_u32(smem) & 1023) != 0) {
+    if (threadIdx.x == 0) report_status(p.status, kStatusBadIndex);
+    return;
+  }
   uint8_t* sK = smem;
   uint8_t* sV = sK + kTileBytes;
   uint8_t* sQ = sV + kTileBytes;           // two stages
   uint8_t* sDO = sQ + 2 * kTileBytes;
   uint8_t* sDS = sDO + kTileBytes;
-  float* sLse = reinterpret_cast<float*>(sDS + kDsBytes);  // [2][128]
-  float* sDelta = sLse + 2 * kT;                           // [2][128]
+  uint8_t* sOut = sDS + kDsBytes;           // the later half of dQ on its way out; the earlier half goes through sDS
+  float* sLse = reinterpret_cast<float*>(sOut + kOutBytes);  // [2][128], minus the log-sum
+  float* sDelta = sLse + 2 * kT;                           // [2][128], minus the row product
   uint64_t* bars = reinterpret_cast<uint64_t*>(sDelta + 2 * kT);
   uint64_t* kv_full = bars + 0;
   uint64_t* q_full = bars + 1;   // [2]
@@ -173,10 +200,26 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       bool ok = mbar_wait(kv_full, 0);
       if (!ok) report_status(p.status, kStatusWaitFullTimeout);
       const uint32_t aK = smem_u32(sK), aV = smem_u32(sV), aDO = smem_u32(sDO), aDS = smem_u32(sDS);
+      // dP^T of step `it` into R2: for the next step behind this one's products, while dQ is being read out of R1
+      const auto issue_dp = [&](int it) {
+        if (!mbar_wait(do_full, it & 1)) {
+          report_status(p.status, kStatusWaitFullTimeout);
+          return false;
+        }
+        tc_fence_after();
+#pragma unroll
+        for (int k = 0; k < D / 16; ++k) {
+          const uint32_t off = (k / 4) * kChunkBytes + (k % 4) * 32;
+          tc_mma_f16(tmem_R2, umma_smem_desc(aV + off, 16, 1024), umma_smem_desc(aDO + off, 16, 1024), kIdescST,
+                     k > 0 ? 1u : 0u);
+        }
+        return true;
+      };
+      if (ok && n_it > 0) ok = issue_dp(0);
       for (int it = 0; it < n_it && ok; ++it) {
         const int s = it & 1;
         const uint32_t aQ = smem_u32(sQ + s * kTileBytes);
-        if (!mbar_wait(&q_full[s], (it >> 1) & 1) || !mbar_wait(do_full, it & 1)) {
+        if (!mbar_wait(&q_full[s], (it >> 1) & 1)) {
           report_status(p.status, kStatusWaitFullTimeout);
           break;
         }
@@ -189,12 +232,6 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         for (int k = 0; k < D / 16; ++k) {
           const uint32_t off = (k / 4) * kChunkBytes + (k % 4) * 32;
           tc_mma_f16(tmem_R1, umma_smem_desc(aK + off, 16, 1024), umma_smem_desc(aQ + off, 16, 1024), kIdescST,
-                     k > 0 ? 1u : 0u);
-        }
-#pragma unroll
-        for (int k = 0; k < D / 16; ++k) {
-          const uint32_t off = (k / 4) * kChunkBytes + (k % 4) * 32;
-          tc_mma_f16(tmem_R2, umma_smem_desc(aV + off, 16, 1024), umma_smem_desc(aDO + off, 16, 1024), kIdescST,
                      k > 0 ? 1u : 0u);
         }
         tc_commit(sdp_full);
@@ -221,6 +258,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           tc_mma_f16(tmem_R1, umma_smem_desc(aDS + k * 2048, kChunkBytes, 1024),
                      umma_smem_desc(aK + k * 2048, kChunkBytes, 1024), kIdescDQ, k > 0 ? 1u : 0u);
         tc_commit(dq_full);
+        if (it + 1 < n_it) ok = issue_dp(it + 1);
       }
     }
   } else {
@@ -232,18 +270,20 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     const int kj = k0 + r;
     const uint32_t lane_off = static_cast<uint32_t>(quarter * 32) << 16;
     bool ok = true;
+    // the thread's share of a step's row statistics, requested while the step before is in its products
+    const auto row_stat = [&](int it) {
+      const int hg = it / n_q, qi = k0 + (it - hg * n_q) * kT + r;
+      if (it >= n_it || qi >= seq_len) return part == 0 ? INFINITY : 0.f;
+      return (part == 0 ? p.lse : p.delta)[(long long)(head0 + hg) * p.T + seq_start + qi];
+    };
+    float stat = row_stat(0);
     for (int it = 0; it < n_it; ++it) {
       const int hg = it / n_q, qt = it - hg * n_q;
       const int head = head0 + hg;
       const int q0 = k0 + qt * kT;
       const int b = it & 1;
-      {
-        const int qi = q0 + r;
-        const bool valid = qi < seq_len;
-        const long long idx = (long long)head * p.T + seq_start + qi;
-        if (part == 0) sLse[b * kT + r] = valid ? p.lse[idx] * 1.4426950408889634f : INFINITY;
-        else sDelta[b * kT + r] = valid ? p.delta[idx] : 0.f;
-      }
+      if (part == 0) sLse[b * kT + r] = -(stat * 1.4426950408889634f);
+      else sDelta[b * kT + r] = -stat;
       named_bar_sync(1, 256);
       if (!mbar_wait(sdp_full, it & 1)) {
         report_status(p.status, kStatusWaitTmemFullTimeout);
@@ -259,21 +299,28 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         tmem_ld_32x32(tmem_R2 + lane_off + c * 32, dp);
         tc_wait_ld();
         uint32_t pk[16], dsk[16];
+        const float2 scale2 = make_float2(p.scale, p.scale), scale_log2 = make_float2(p.scale_log2, p.scale_log2);
 #pragma unroll
-        for (int i = 0; i < 32; i += 2) {
-          const int qa = c * 32 + i;
-          float p0 = exp2f(__uint_as_float(sv[i]) * p.scale_log2 - sLse[b * kT + qa]);
-          float p1 = exp2f(__uint_as_float(sv[i + 1]) * p.scale_log2 - sLse[b * kT + qa + 1]);
-          if (diag) {
-            if (kj > q0 + qa) p0 = 0.f;
-            if (kj > q0 + qa + 1) p1 = 0.f;
+        for (int i4 = 0; i4 < 32; i4 += 4) {
+          const float4 ml = *reinterpret_cast<const float4*>(sLse + b * kT + c * 32 + i4);
+          const float4 md = *reinterpret_cast<const float4*>(sDelta + b * kT + c * 32 + i4);
+#pragma unroll
+          for (int i = i4; i < i4 + 4; i += 2) {
+            const int qa = c * 32 + i;
+            const float2 z = fma2(make_float2(__uint_as_float(sv[i]), __uint_as_float(sv[i + 1])), scale_log2,
+                                  i == i4 ? make_float2(ml.x, ml.y) : make_float2(ml.z, ml.w));
+            float2 e = make_float2(exp2f(z.x), exp2f(z.y));
+            if (diag) {
+              if (kj > q0 + qa) e.x = 0.f;
+              if (kj > q0 + qa + 1) e.y = 0.f;
+            }
+            float2 d = mul2(mul2(e, add2(make_float2(__uint_as_float(dp[i]), __uint_as_float(dp[i + 1])),
+                                         i == i4 ? make_float2(md.x, md.y) : make_float2(md.z, md.w))), scale2);
+            if (e.x == 0.f) d.x = 0.f;
+            if (e.y == 0.f) d.y = 0.f;
+            pk[i / 2] = pack_bf16x2(e.x, e.y);
+            dsk[i / 2] = pack_bf16x2(d.x, d.y);
           }
-          float d0 = p0 * (__uint_as_float(dp[i]) - sDelta[b * kT + qa]) * p.scale;
-          float d1 = p1 * (__uint_as_float(dp[i + 1]) - sDelta[b * kT + qa + 1]) * p.scale;
-          if (p0 == 0.f) d0 = 0.f;
-          if (p1 == 0.f) d1 = 0.f;
-          pk[i / 2] = pack_bf16x2(p0, p1);
-          dsk[i / 2] = pack_bf16x2(d0, d1);
         }
         const uint32_t pcol = lane_off + part * 64 + (c & 1) * 16;
         tmem_st_32x16(tmem_R1 + pcol, pk);
@@ -291,6 +338,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(pds_ready);
+      stat = row_stat(it + 1);
 
       if (!mbar_wait(dq_full, it & 1)) {
         report_status(p.status, kStatusWaitTmemFullTimeout);
@@ -309,13 +357,15 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         if (lane == 0) mbar_arrive(dq_read);
         // dS has been consumed: its tile is the staging area, 32 rows x 128 bytes of it per warp. Rows past the sequence go out
         // as zeros: the product has 0 there, or NaN where K is not finite, and the next sequence is not to see it. Cleared
-        // in shared memory: 8 x 4096 tokens take 2043 us (2028 without), 2059 with a select on every value.
-        uint8_t* buf = sDS + (warp - 2) * 4096;
+        // in shared memory, which costs less than a select on every value.
         const bool any = q0 + quarter * 32 < seq_len;
+        static_assert(kMine <= 2, "a buffer for each piece");
 #pragma unroll
         for (int c = 0; c < kMine; ++c) {
-          if (c > 0) {
-            if (lane == 0) bulk_wait_read<0>();
+          // sOut was handed to TMA a step ago, before the wait below let this step's dS be written
+          uint8_t* buf = (c == 0 ? sDS : sOut) + (warp - 2) * 4096;
+          if (c > 0 && it > 0) {
+            if (lane == 0) bulk_wait_read<1>();  // all but the piece just sent
             __syncwarp();
           }
 #pragma unroll
@@ -328,12 +378,12 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           }
           fence_proxy_async_smem();
           __syncwarp();
-          if (lane == 0 && any) {
-            tma_reduce_add_2d(&tmDQ, buf, head * D + (part * kMine + c) * 32, seq_start + q0 + quarter * 32);
-            bulk_commit();
+          if (lane == 0) {
+            if (any) tma_reduce_add_2d(&tmDQ, buf, head * D + (part * kMine + c) * 32, seq_start + q0 + quarter * 32);
+            bulk_commit();  // a group for every piece, so that the waits name the same ones
           }
         }
-        if (lane == 0) bulk_wait_read<0>();  // the barrier at the top lets every warp write dS again
+        if (lane == 0) bulk_wait_read<kMine - 1>();  // sDS: the barrier at the top lets every warp write dS again
         __syncwarp();
       }
     }
@@ -507,7 +557,7 @@ void finalize(const float* acc, long long lda, void* out, long long ld, int T, i
 template <int D>
 void launch_bwd_t(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tdo,
                   const CUtensorMap& tdq, const AttnBwdParams& p, int n_tiles, int Hkv, cudaStream_t s) {
-  constexpr int smem = 5 * kT * D * 2 + kT * kT * 2 + 4 * kT * 4 + 128 + 1024;
+  constexpr int smem = 5 * kT * D * 2 + kT * kT * 2 + (D > 64 ? 8 * 4096 : 0) + 4 * kT * 4 + 128;
   auto kernel = attn_bwd_kernel<D>;
   AGRPO_SET_MAX_DYN_SMEM(kernel, smem, "attn_bwd smem attr");
   dim3 grid(Hkv * p.pieces, n_tiles);
