@@ -94,7 +94,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   constexpr int kTileBytes = kT * D * 2;
   constexpr int kChunkBytes = kT * 128;     // one 64-column swizzle chunk of a 128-row tile
   constexpr int kDsBytes = kT * kT * 2;
-  constexpr int kOutBytes = D > 64 ? 8 * 4096 : 0;
+  constexpr int kOutBytes = 8 * 4096;
   constexpr uint32_t kTmemCols = 512;
   constexpr uint32_t kIdescST = umma_idesc_bf16(kT, kT, 0, 0);  // S^T, dP^T: both operands K-major
   constexpr uint32_t kIdescKV = umma_idesc_bf16(kT, D, 0, 1);   // dV, dK: A from TMEM, B MN-major
@@ -111,7 +111,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   uint8_t* sQ = sV + kTileBytes;           // two stages
   uint8_t* sDO = sQ + 2 * kTileBytes;
   uint8_t* sDS = sDO + kTileBytes;
-  uint8_t* sOut = sDS + kDsBytes;           // the later half of dQ on its way out; the earlier half goes through sDS
+  uint8_t* sOut = sDS + kDsBytes;           // dQ on its way out
   float* sLse = reinterpret_cast<float*>(sOut + kOutBytes);  // [2][128], minus the log-sum
   float* sDelta = sLse + 2 * kT;                           // [2][128], minus the row product
   uint64_t* bars = reinterpret_cast<uint64_t*>(sDelta + 2 * kT);
@@ -119,12 +119,15 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   uint64_t* q_full = bars + 1;   // [2]
   uint64_t* q_empty = bars + 3;  // [2]
   uint64_t* do_full = bars + 5;
-  uint64_t* sdp_full = bars + 6;
-  uint64_t* pds_ready = bars + 7;
-  uint64_t* dv_done = bars + 8;
-  uint64_t* dq_full = bars + 9;
-  uint64_t* dq_read = bars + 10;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 11);
+  uint64_t* s_full = bars + 6;
+  uint64_t* dp_full = bars + 7;
+  uint64_t* p_ready = bars + 8;
+  uint64_t* ds_ready = bars + 9;
+  uint64_t* dv_done = bars + 10;
+  uint64_t* dq_full = bars + 11;
+  uint64_t* dq_read = bars + 12;
+  uint64_t* all_done = bars + 13;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 14);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int kv_head = blockIdx.x / p.pieces, piece = blockIdx.x - kv_head * p.pieces;
@@ -143,8 +146,11 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     mbar_init(&q_empty[0], 1);
     mbar_init(&q_empty[1], 1);
     mbar_init(do_full, 1);
-    mbar_init(sdp_full, 1);
-    mbar_init(pds_ready, 8);
+    mbar_init(s_full, 1);
+    mbar_init(dp_full, 1);
+    mbar_init(p_ready, 8);
+    mbar_init(ds_ready, 8);
+    mbar_init(all_done, 1);
     mbar_init(dv_done, 1);
     mbar_init(dq_full, 1);
     mbar_init(dq_read, 8);
@@ -160,8 +166,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   pdl_wait();
   pdl_launch();
   const uint32_t tmem_base = *tmem_slot;
-  const uint32_t tmem_R1 = tmem_base;        // S^T -> P^T (bf16) -> dQ
-  const uint32_t tmem_R2 = tmem_base + 128;  // dP^T -> dS^T (bf16)
+  const uint32_t tmem_R1 = tmem_base;        // S^T -> P^T (bf16)
+  const uint32_t tmem_R2 = tmem_base + 128;  // dP^T -> dQ
   const uint32_t tmem_dV = tmem_base + 256;
   const uint32_t tmem_dK = tmem_base + 256 + D;
 
@@ -200,66 +206,62 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       bool ok = mbar_wait(kv_full, 0);
       if (!ok) report_status(p.status, kStatusWaitFullTimeout);
       const uint32_t aK = smem_u32(sK), aV = smem_u32(sV), aDO = smem_u32(sDO), aDS = smem_u32(sDS);
-      // dP^T of step `it` into R2: for the next step behind this one's products, while dQ is being read out of R1
-      const auto issue_dp = [&](int it) {
-        if (!mbar_wait(do_full, it & 1)) {
-          report_status(p.status, kStatusWaitFullTimeout);
+      const auto need = [&](uint64_t* bar, uint32_t parity, int code) {
+        if (!mbar_wait(bar, parity)) {
+          report_status(p.status, code);
           return false;
         }
         tc_fence_after();
-#pragma unroll
-        for (int k = 0; k < D / 16; ++k) {
-          const uint32_t off = (k / 4) * kChunkBytes + (k % 4) * 32;
-          tc_mma_f16(tmem_R2, umma_smem_desc(aV + off, 16, 1024), umma_smem_desc(aDO + off, 16, 1024), kIdescST,
-                     k > 0 ? 1u : 0u);
-        }
         return true;
       };
-      if (ok && n_it > 0) ok = issue_dp(0);
-      for (int it = 0; it < n_it && ok; ++it) {
-        const int s = it & 1;
-        const uint32_t aQ = smem_u32(sQ + s * kTileBytes);
-        if (!mbar_wait(&q_full[s], (it >> 1) & 1)) {
-          report_status(p.status, kStatusWaitFullTimeout);
-          break;
-        }
-        if (it >= 1 && !mbar_wait(dq_read, (it - 1) & 1)) {
-          report_status(p.status, kStatusWaitTmemEmptyTimeout);
-          break;
-        }
-        tc_fence_after();
+      const auto score = [&](int it) {  // S^T = K Q^T
+        const uint32_t aQ = smem_u32(sQ + (it & 1) * kTileBytes);
+        if (!need(&q_full[it & 1], (it >> 1) & 1, kStatusWaitFullTimeout)) return false;
 #pragma unroll
         for (int k = 0; k < D / 16; ++k) {
           const uint32_t off = (k / 4) * kChunkBytes + (k % 4) * 32;
-          tc_mma_f16(tmem_R1, umma_smem_desc(aK + off, 16, 1024), umma_smem_desc(aQ + off, 16, 1024), kIdescST,
-                     k > 0 ? 1u : 0u);
+          tc_mma_f16(tmem_R1, umma_smem_desc(aK + off, 16, 1024), umma_smem_desc(aQ + off, 16, 1024), kIdescST, k > 0 ? 1u : 0u);
         }
-        tc_commit(sdp_full);
-        if (!mbar_wait(pds_ready, it & 1)) {
-          report_status(p.status, kStatusWaitTmemFullTimeout);
-          break;
+        tc_commit(s_full);
+        return true;
+      };
+      const auto grad_p = [&](int it) {  // dP^T = V dO^T
+        if (!need(do_full, it & 1, kStatusWaitFullTimeout)) return false;
+#pragma unroll
+        for (int k = 0; k < D / 16; ++k) {
+          const uint32_t off = (k / 4) * kChunkBytes + (k % 4) * 32;
+          tc_mma_f16(tmem_R2, umma_smem_desc(aV + off, 16, 1024), umma_smem_desc(aDO + off, 16, 1024), kIdescST, k > 0 ? 1u : 0u);
         }
-        tc_fence_after();
+        tc_commit(dp_full);
+        return true;
+      };
+      if (ok && n_it > 0) ok = score(0) && grad_p(0);
+      for (int it = 0; it < n_it && ok; ++it) {
+        const uint32_t aQ = smem_u32(sQ + (it & 1) * kTileBytes);
         // dV += P^T dO   (A: P^T packed bf16 in R1, B: dO as [N = D, K = queries], MN-major)
+        if (!need(p_ready, it & 1, kStatusWaitTmemFullTimeout)) break;
 #pragma unroll
         for (int k = 0; k < kT / 16; ++k)
           tc_mma_f16_ts(tmem_dV, tmem_R1 + (k & 3) * 8 + (k >> 2) * 64, umma_smem_desc(aDO + k * 2048, kChunkBytes, 1024), kIdescKV,
                         (it > 0 || k > 0) ? 1u : 0u);
         tc_commit(dv_done);
-        // dK += dS^T Q
-#pragma unroll
-        for (int k = 0; k < kT / 16; ++k)
-          tc_mma_f16_ts(tmem_dK, tmem_R2 + (k & 3) * 8 + (k >> 2) * 64, umma_smem_desc(aQ + k * 2048, kChunkBytes, 1024), kIdescKV,
-                        (it > 0 || k > 0) ? 1u : 0u);
-        tc_commit(&q_empty[s]);
+        if (it + 1 < n_it && !score(it + 1)) break;
         // dQ = dS K      (A: dS^T tile in shared memory read MN-major, B: K as [N = D, K = keys], MN-major)
+        if (!need(ds_ready, it & 1, kStatusWaitTmemFullTimeout)) break;
 #pragma unroll
         for (int k = 0; k < kT / 16; ++k)
-          tc_mma_f16(tmem_R1, umma_smem_desc(aDS + k * 2048, kChunkBytes, 1024),
+          tc_mma_f16(tmem_R2, umma_smem_desc(aDS + k * 2048, kChunkBytes, 1024),
                      umma_smem_desc(aK + k * 2048, kChunkBytes, 1024), kIdescDQ, k > 0 ? 1u : 0u);
         tc_commit(dq_full);
-        if (it + 1 < n_it) ok = issue_dp(it + 1);
+        // dK += dS^T Q   (the same tile read K-major)
+#pragma unroll
+        for (int k = 0; k < kT / 16; ++k)
+          tc_mma_f16(tmem_dK, umma_smem_desc(aDS + (k >> 2) * kChunkBytes + (k & 3) * 32, 16, 1024),
+                     umma_smem_desc(aQ + k * 2048, kChunkBytes, 1024), kIdescKV, (it > 0 || k > 0) ? 1u : 0u);
+        tc_commit(&q_empty[it & 1]);
+        if (it + 1 < n_it) ok = need(dq_read, it & 1, kStatusWaitTmemEmptyTimeout) && grad_p(it + 1);
       }
+      tc_commit(all_done);
     }
   } else {
     // Compute warps: thread = one key row and half of the queries (P^T / dS^T); for the dQ read-out, one query row and half
@@ -277,54 +279,106 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       return (part == 0 ? p.lse : p.delta)[(long long)(head0 + hg) * p.T + seq_start + qi];
     };
     float stat = row_stat(0);
+    constexpr int kMine = D / 64;  // 32-column pieces of dQ that this warp takes out
+    static_assert(kMine <= 2, "the first piece goes out at once, the second behind the next step's exponentials");
+    uint32_t late[32];
+    // Piece c of step it's dQ, from registers through 32 rows x 128 bytes of shared memory per warp. Rows past the sequence go out as
+    // zeros: the product has 0 there, or NaN where K is not finite, and the next sequence is not to see it. Cleared in shared
+    // memory, which costs less than a select on every value.
+    const auto send_dq = [&](const uint32_t (&o)[32], int it, int c) {
+      const int hg = it / n_q, q0 = k0 + (it - hg * n_q) * kT;
+      uint8_t* buf = sOut + (warp - 2) * 4096;
+      if (lane == 0) bulk_wait_read<0>();  // the piece before, sent half a step ago
+      __syncwarp();
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        *reinterpret_cast<uint4*>(buf + lane * 128 + ((u ^ (lane & 7)) << 4)) = make_uint4(o[4 * u], o[4 * u + 1], o[4 * u + 2], o[4 * u + 3]);
+      if (q0 + r >= seq_len) {
+#pragma unroll 1
+        for (int u = 0; u < 8; ++u) *reinterpret_cast<uint4*>(buf + lane * 128 + u * 16) = make_uint4(0, 0, 0, 0);
+      }
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0 && q0 + quarter * 32 < seq_len) {
+        tma_reduce_add_2d(&tmDQ, buf, (head0 + hg) * D + (part * kMine + c) * 32, seq_start + q0 + quarter * 32);
+        bulk_commit();
+      }
+    };
     for (int it = 0; it < n_it; ++it) {
       const int hg = it / n_q, qt = it - hg * n_q;
-      const int head = head0 + hg;
       const int q0 = k0 + qt * kT;
       const int b = it & 1;
       if (part == 0) sLse[b * kT + r] = -(stat * 1.4426950408889634f);
       else sDelta[b * kT + r] = -stat;
       named_bar_sync(1, 256);
-      if (!mbar_wait(sdp_full, it & 1)) {
+      if (!mbar_wait(s_full, it & 1)) {
         report_status(p.status, kStatusWaitTmemFullTimeout);
         ok = false;
         break;
       }
       tc_fence_after();
       const bool diag = (qt == 0);
-#pragma unroll 1
-      for (int c = part * 2; c < part * 2 + 2; ++c) {
-        uint32_t sv[32], dp[32];
+      const float2 scale2 = make_float2(p.scale, p.scale), scale_log2 = make_float2(p.scale_log2, p.scale_log2);
+      float pr[2][32];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int c = part * 2 + h;
+        uint32_t sv[32], pk[16];
         tmem_ld_32x32(tmem_R1 + lane_off + c * 32, sv);
-        tmem_ld_32x32(tmem_R2 + lane_off + c * 32, dp);
         tc_wait_ld();
-        uint32_t pk[16], dsk[16];
-        const float2 scale2 = make_float2(p.scale, p.scale), scale_log2 = make_float2(p.scale_log2, p.scale_log2);
 #pragma unroll
         for (int i4 = 0; i4 < 32; i4 += 4) {
           const float4 ml = *reinterpret_cast<const float4*>(sLse + b * kT + c * 32 + i4);
-          const float4 md = *reinterpret_cast<const float4*>(sDelta + b * kT + c * 32 + i4);
 #pragma unroll
           for (int i = i4; i < i4 + 4; i += 2) {
             const int qa = c * 32 + i;
             const float2 z = fma2(make_float2(__uint_as_float(sv[i]), __uint_as_float(sv[i + 1])), scale_log2,
                                   i == i4 ? make_float2(ml.x, ml.y) : make_float2(ml.z, ml.w));
-            float2 e = make_float2(exp2f(z.x), exp2f(z.y));
+            float e0 = exp2f(z.x), e1 = exp2f(z.y);
             if (diag) {
-              if (kj > q0 + qa) e.x = 0.f;
-              if (kj > q0 + qa + 1) e.y = 0.f;
+              if (kj > q0 + qa) e0 = 0.f;
+              if (kj > q0 + qa + 1) e1 = 0.f;
             }
+            pr[h][i] = e0;
+            pr[h][i + 1] = e1;
+            pk[i / 2] = pack_bf16x2(e0, e1);
+          }
+        }
+        tmem_st_32x16(tmem_R1 + lane_off + part * 64 + h * 16, pk);
+      }
+      tc_wait_st();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(p_ready);
+      if constexpr (kMine > 1) {  // the later half of the step before's dQ
+        if (it > 0) send_dq(late, it - 1, 1);
+      }
+
+      if (!mbar_wait(dp_full, it & 1)) {
+        report_status(p.status, kStatusWaitTmemFullTimeout);
+        ok = false;
+        break;
+      }
+      tc_fence_after();
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int c = part * 2 + h;
+        uint32_t dp[32], dsk[16];
+        tmem_ld_32x32(tmem_R2 + lane_off + c * 32, dp);
+        tc_wait_ld();
+#pragma unroll
+        for (int i4 = 0; i4 < 32; i4 += 4) {
+          const float4 md = *reinterpret_cast<const float4*>(sDelta + b * kT + c * 32 + i4);
+#pragma unroll
+          for (int i = i4; i < i4 + 4; i += 2) {
+            const float2 e = make_float2(pr[h][i], pr[h][i + 1]);
             float2 d = mul2(mul2(e, add2(make_float2(__uint_as_float(dp[i]), __uint_as_float(dp[i + 1])),
                                          i == i4 ? make_float2(md.x, md.y) : make_float2(md.z, md.w))), scale2);
             if (e.x == 0.f) d.x = 0.f;
             if (e.y == 0.f) d.y = 0.f;
-            pk[i / 2] = pack_bf16x2(e.x, e.y);
             dsk[i / 2] = pack_bf16x2(d.x, d.y);
           }
         }
-        const uint32_t pcol = lane_off + part * 64 + (c & 1) * 16;
-        tmem_st_32x16(tmem_R1 + pcol, pk);
-        tmem_st_32x16(tmem_R2 + pcol, dsk);
         // dS^T row r, queries [32c, 32c+32) into the 128-byte-swizzled [keys x queries] tile.
         uint8_t* rowp = sDS + (c >> 1) * kChunkBytes + r * 128;
 #pragma unroll
@@ -333,11 +387,10 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           *reinterpret_cast<uint4*>(rowp + unit * 16) = make_uint4(dsk[u * 4], dsk[u * 4 + 1], dsk[u * 4 + 2], dsk[u * 4 + 3]);
         }
       }
-      tc_wait_st();
       fence_proxy_async_smem();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(pds_ready);
+      if (lane == 0) mbar_arrive(ds_ready);
       stat = row_stat(it + 1);
 
       if (!mbar_wait(dq_full, it & 1)) {
@@ -347,49 +400,26 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       }
       tc_fence_after();
       {
-        constexpr int kMine = D / 64;  // 32-column pieces of dQ that this warp takes out
-        uint32_t o[kMine][32];
-#pragma unroll
-        for (int c = 0; c < kMine; ++c) tmem_ld_32x32(tmem_R1 + lane_off + (part * kMine + c) * 32, o[c]);
+        uint32_t first[32];
+        tmem_ld_32x32(tmem_R2 + lane_off + (part * kMine) * 32, first);
+        if constexpr (kMine > 1) tmem_ld_32x32(tmem_R2 + lane_off + (part * kMine + 1) * 32, late);
         tc_wait_ld();
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(dq_read);
-        // dS has been consumed: its tile is the staging area, 32 rows x 128 bytes of it per warp. Rows past the sequence go out
-        // as zeros: the product has 0 there, or NaN where K is not finite, and the next sequence is not to see it. Cleared
-        // in shared memory, which costs less than a select on every value.
-        const bool any = q0 + quarter * 32 < seq_len;
-        static_assert(kMine <= 2, "a buffer for each piece");
-#pragma unroll
-        for (int c = 0; c < kMine; ++c) {
-          // sOut was handed to TMA a step ago, before the wait below let this step's dS be written
-          uint8_t* buf = (c == 0 ? sDS : sOut) + (warp - 2) * 4096;
-          if (c > 0 && it > 0) {
-            if (lane == 0) bulk_wait_read<1>();  // all but the piece just sent
-            __syncwarp();
-          }
-#pragma unroll
-          for (int u = 0; u < 8; ++u)
-            *reinterpret_cast<uint4*>(buf + lane * 128 + ((u ^ (lane & 7)) << 4)) =
-                make_uint4(o[c][4 * u], o[c][4 * u + 1], o[c][4 * u + 2], o[c][4 * u + 3]);
-          if (q0 + r >= seq_len) {
-#pragma unroll 1
-            for (int u = 0; u < 8; ++u) *reinterpret_cast<uint4*>(buf + lane * 128 + u * 16) = make_uint4(0, 0, 0, 0);
-          }
-          fence_proxy_async_smem();
-          __syncwarp();
-          if (lane == 0) {
-            if (any) tma_reduce_add_2d(&tmDQ, buf, head * D + (part * kMine + c) * 32, seq_start + q0 + quarter * 32);
-            bulk_commit();  // a group for every piece, so that the waits name the same ones
-          }
-        }
-        if (lane == 0) bulk_wait_read<kMine - 1>();  // sDS: the barrier at the top lets every warp write dS again
-        __syncwarp();
+        send_dq(first, it, 0);
       }
+    }
+    if (ok && n_it > 0) {
+      if constexpr (kMine > 1) send_dq(late, n_it - 1, 1);
+      if (!mbar_wait(all_done, 0)) {
+        report_status(p.status, kStatusWaitTmemFullTimeout);
+        ok = false;
+      }
+      tc_fence_after();
     }
     if (lane == 0) bulk_wait_all<0>();
     if (ok && n_it > 0) {
-      // The last dq_full wait also covered the final dV / dK MMAs (commits are cumulative).
       const bool valid = kj < seq_len;
       const long long t = (long long)seq_start + kj;
       const uint32_t acc = (part == 0 ? tmem_dV : tmem_dK) + lane_off;
@@ -557,7 +587,7 @@ void finalize(const float* acc, long long lda, void* out, long long ld, int T, i
 template <int D>
 void launch_bwd_t(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tdo,
                   const CUtensorMap& tdq, const AttnBwdParams& p, int n_tiles, int Hkv, cudaStream_t s) {
-  constexpr int smem = 5 * kT * D * 2 + kT * kT * 2 + (D > 64 ? 8 * 4096 : 0) + 4 * kT * 4 + 128;
+  constexpr int smem = 5 * kT * D * 2 + kT * kT * 2 + 8 * 4096 + 4 * kT * 4 + 128;
   auto kernel = attn_bwd_kernel<D>;
   AGRPO_SET_MAX_DYN_SMEM(kernel, smem, "attn_bwd smem attr");
   dim3 grid(Hkv * p.pieces, n_tiles);
