@@ -871,6 +871,23 @@ void lm_sample(const Tensor& hidden, const Tensor& weight, double temperature, c
                           opt_ptr<int>(status), num_sms(), cur_stream(), (float)softcap);
 }
 
+void feed_back(const Tensor& tokens, const OptTensor& logprobs, int64_t rows, Tensor& last, Tensor& index, Tensor& history, const OptTensor& history_lp) {
+  check_i32(tokens, "tokens"); check_i32(last, "last"); check_i64(index, "index"); check_i32(history, "history");
+  TORCH_CHECK(history.dim() == 2 && history.is_contiguous() && history.size(1) > 0, "feed_back: history [rows, cap]");
+  for (const Tensor& t : {tokens, last, index}) TORCH_CHECK(t.is_contiguous() && t.numel() >= rows, "feed_back: rows");
+  TORCH_CHECK(rows >= 0 && history.size(0) >= rows, "feed_back: rows");
+  if (history_lp.has_value() && history_lp->defined()) {
+    TORCH_CHECK(logprobs.has_value() && logprobs->defined(), "feed_back: log-probabilities");
+    check_f32(*logprobs, "logprobs"); check_f32(*history_lp, "history_lp");
+    TORCH_CHECK(logprobs->is_contiguous() && logprobs->numel() >= rows && history_lp->is_contiguous() && history_lp->sizes() == history.sizes(),
+                "feed_back: history_lp as history");
+  }
+  const c10::cuda::CUDAGuard guard(tokens.device());
+  agrpo::launch_feed_back(tokens.data_ptr<int>(), opt_ptr<float>(logprobs), (int)rows, last.data_ptr<int>(),
+                          reinterpret_cast<long long*>(index.data_ptr<int64_t>()), history.data_ptr<int>(), opt_ptr<float>(history_lp),
+                          history.size(1), cur_stream());
+}
+
 // ---- peer-memory kernels ----
 using PtrList = std::vector<int64_t>;
 inline const long long* lptr(const PtrList& v) { return reinterpret_cast<const long long*>(v.data()); }
@@ -1276,6 +1293,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("lm_sample", &lm_sample, py::arg("hidden"), py::arg("weight"), py::arg("temperature"), py::arg("seeds"),
         py::arg("part_f"), py::arg("part_i"), py::arg("tokens"), py::arg("logprobs") = py::none(),
         py::arg("status") = py::none(), py::arg("softcap") = 0.0, NOGIL);
+  m.def("feed_back", &feed_back, NOGIL);
   m.def("pack_count_tiles", &pack_count_tiles);
   m.def("pack_microbatch", &pack_microbatch);
   m.def("normalize_rewards", &normalize_rewards_cpu);

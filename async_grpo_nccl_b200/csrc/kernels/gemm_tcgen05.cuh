@@ -35,6 +35,8 @@ struct GemmShape {
   // a2; column tiles never straddle n1, and an epilogue sees as N the end of the product that its tile belongs to.
   int n1 = 0;
   int a2 = 0;
+  // B is not written by the kernel before this one (weights): its first tiles are requested before that kernel is complete.
+  bool b_fixed = false;
 
   __host__ __device__ int tiles_n(int BN) const { return n1 > 0 ? (n1 + BN - 1) / BN + (N - n1 + BN - 1) / BN : (N + BN - 1) / BN; }
   __device__ __forceinline__ bool second(int tn, int BN) const { return n1 > 0 && tn >= (n1 + BN - 1) / BN; }
@@ -443,6 +445,42 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     tma_prefetch_desc(&tmA);
     tma_prefetch_desc(&tmB);
   }
+  const auto load_a = [&](int stage, int a0, int m0, int k0) {
+    uint8_t* sa = smem + stage * S::kStageBytes;
+    if constexpr (!A_MN) {
+      tma_load_2d(sa, &tmA, &full_bar[stage], a0 + k0, m0);
+    } else {
+#pragma unroll
+      for (int j = 0; j < kGemmBM / 64; ++j) tma_load_2d(sa + j * 8192, &tmA, &full_bar[stage], m0 + j * 64, k0);
+    }
+  };
+  const auto load_b = [&](int stage, int n0, int k0) {
+    uint8_t* sb = smem + stage * S::kStageBytes + S::kABytes;
+    if constexpr (!B_MN) {
+      if (p.dual_b > 0) {  // the tensor map's box is BN/2 rows high in this mode
+        tma_load_2d(sb, &tmB, &full_bar[stage], k0, n0 / 2);
+        tma_load_2d(sb + (BN / 2) * (kGemmBK * 2), &tmB, &full_bar[stage], k0, p.dual_b + n0 / 2);
+      } else {
+        tma_load_2d(sb, &tmB, &full_bar[stage], k0, n0);
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < BN / 64; ++j) tma_load_2d(sb + j * 8192, &tmB, &full_bar[stage], n0 + j * 64, k0);
+    }
+  };
+  // stages of the first tile whose B comes ahead; that thread of warp 0 alone, right behind its barrier initialisation
+  const int n_ahead = !Gather::kEnabled && !B_MN && p.b_fixed && (int)blockIdx.x < num_items ? min(kStages, num_kb) : 0;
+  if (threadIdx.x == 0 && n_ahead > 0) {
+    int tm, tn0, count;
+    gemm_item_coords((int)blockIdx.x, tiles_m, tiles_n, p.group_n, tm, tn0, count);
+    const int n0 = p.first_col(tn0, BN), a0 = p.second(tn0, BN) ? p.a2 : 0;
+    for (int s = 0; s < n_ahead; ++s) {
+      mbar_expect_tx(&full_bar[s], S::kStageBytes);
+      load_b(s, n0, s * kGemmBK);
+    }
+    pdl_wait();
+    for (int s = 0; s < n_ahead; ++s) load_a(s, a0, tm * kGemmBM, s * kGemmBK);
+  }
   if (warp == 1) {
     tmem_alloc(tmem_slot, kTmemCols);
     tmem_relinquish();
@@ -487,31 +525,16 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
             }
           }
           for (int kb = 0; kb < num_kb; ++kb) {
-            if (!mbar_wait(&empty_bar[stage], phase ^ 1)) {
-              report_status(p.status, kStatusWaitEmptyTimeout);
-              ok = false;
-              break;
-            }
-            uint8_t* sa = smem + stage * S::kStageBytes;
-            uint8_t* sb = sa + S::kABytes;
-            mbar_expect_tx(&full_bar[stage], S::kStageBytes);
-            const int k0 = kb * kGemmBK;
-            if constexpr (!A_MN) {
-              tma_load_2d(sa, &tmA, &full_bar[stage], a0 + k0, m0);
-            } else {
-#pragma unroll
-              for (int j = 0; j < kGemmBM / 64; ++j) tma_load_2d(sa + j * 8192, &tmA, &full_bar[stage], m0 + j * 64, k0);
-            }
-            if constexpr (!B_MN) {
-              if (p.dual_b > 0) {  // the tensor map's box is BN/2 rows high in this mode
-                tma_load_2d(sb, &tmB, &full_bar[stage], k0, n0 / 2);
-                tma_load_2d(sb + (BN / 2) * (kGemmBK * 2), &tmB, &full_bar[stage], k0, p.dual_b + n0 / 2);
-              } else {
-                tma_load_2d(sb, &tmB, &full_bar[stage], k0, n0);
+            if (kb >= n_ahead || t > 0 || item != my_cta) {  // else requested ahead
+              if (!mbar_wait(&empty_bar[stage], phase ^ 1)) {
+                report_status(p.status, kStatusWaitEmptyTimeout);
+                ok = false;
+                break;
               }
-            } else {
-#pragma unroll
-              for (int j = 0; j < BN / 64; ++j) tma_load_2d(sb + j * 8192, &tmB, &full_bar[stage], n0 + j * 64, k0);
+              mbar_expect_tx(&full_bar[stage], S::kStageBytes);
+              const int k0 = kb * kGemmBK;
+              load_a(stage, a0, m0, k0);
+              load_b(stage, n0, k0);
             }
             if (++stage == kStages) {
               stage = 0;

@@ -324,6 +324,9 @@ void launch_cast_f32_bf16(const float* in, void* out, long long n, cudaStream_t 
 // All decoder layers of one decode step in one persistent cooperative launch (csrc/kernels/decode_mega.cu).
 // Per-layer weights sit at constant element strides in flat bf16 buffers; wqkv and wgu are the copies with the RMSNorm
 // weight folded in. Activation buffers have rows_alloc >= the row tile (32 / 64 / 128 / 256) that covers B rows.
+// last[r] = history[r, min(index[r], cap - 1)] = tokens[r] (history_lp alike, unless nullptr), index[r] += 1; histories [rows, cap].
+void launch_feed_back(const int* tokens, const float* logprobs, int rows, int* last, long long* index, int* history, float* history_lp,
+                      long long cap, cudaStream_t s);
 struct DecodeLayersArgs {
   int L, B, rows_alloc, H, Q, QD, F, Hq, Hkv, num_sms, splits;
   const void *wqkv, *wo, *wgu, *wd;

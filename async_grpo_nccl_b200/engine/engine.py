@@ -177,7 +177,6 @@ class RolloutEngine:
         self.gen_index = torch.zeros(S, dtype=torch.int64, device=self.dev)
         self.base_seeds = torch.zeros(S, dtype=torch.int64, device=self.dev)
         self.step_seeds = torch.zeros(S, dtype=torch.int64, device=self.dev)
-        self.row_ids = torch.arange(S, dtype=torch.int64, device=self.dev)
         self.hist_cap = self.max_model_len
         self.history = torch.zeros(S, self.hist_cap, **i32)
         self.b_tokens = torch.zeros(S, **i32)
@@ -504,12 +503,8 @@ class RolloutEngine:
 
     def _feed_back(self, B: int) -> None:
         """The sampled token becomes the next step's input and goes into the history (with its log-probability when kept)."""
-        pos = torch.clamp(self.gen_index[:B], max=self.hist_cap - 1)
-        self.last_tokens[:B].copy_(self.b_tokens[:B])
-        self.history[self.row_ids[:B], pos] = self.b_tokens[:B]
-        if self.record_logprobs:
-            self.history_lp[self.row_ids[:B], pos] = self.b_lp[:B]
-        self.gen_index[:B].add_(1)
+        self.C.feed_back(self.b_tokens, self.b_lp, B, self.last_tokens, self.gen_index, self.history,
+                         self.history_lp if self.record_logprobs else None)
 
     # ---- fused decode path ----
     def _folded(self, i: int) -> Tuple[torch.Tensor, torch.Tensor]:
@@ -642,7 +637,7 @@ class RolloutEngine:
 
     def _launch_count_decode(self, splits: int, B: int = 0) -> int:
         if self.mega_rows and 0 < B <= self.mega_rows:
-            return 1 + 1 + 3
+            return 1 + 1 + 4
         fused = self.fused_decode and 0 < B <= self.fused_rows
         if fused:
             n_chunks = (B + self.fused_chunk - 1) // self.fused_chunk
@@ -650,7 +645,7 @@ class RolloutEngine:
             per_layer = (n_chunks - 1) * (5 if self.fused_chunk <= 128 else 6) + (5 if last <= 128 else 6)
         else:
             per_layer = 9
-        return 1 + per_layer * self.cfg.num_hidden_layers + 3
+        return 1 + per_layer * self.cfg.num_hidden_layers + 4
 
     def _stage_decode(self, active: np.ndarray, upd_slot: np.ndarray, upd_index: np.ndarray, upd_block: np.ndarray) -> None:
         """Brings the inputs of one decode step to the device: every active slot is one token longer."""

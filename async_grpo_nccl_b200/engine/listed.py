@@ -161,7 +161,7 @@ class ListedEngine(RolloutEngine):
         return int(max(1, min(self.max_splits, want, min(max_len, self.dec.reach()) // 128)))
 
     def _launch_count_decode(self, splits: int, B: int = 0) -> int:
-        return self.dec.decode_launches() + 2
+        return self.dec.decode_launches() + 3
 
     # ------------------------------------------------------------------ step-wise driving
     def open_sequence(self) -> int:
