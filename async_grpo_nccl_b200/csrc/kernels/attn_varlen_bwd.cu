@@ -5,12 +5,12 @@
 //
 // One CTA owns one 128-key tile of one kv head and walks over the query heads of its group and the
 // query tiles at or below the diagonal. Per step five tcgen05 GEMMs run with every accumulator in
-// tensor memory (512 columns: S^T/P^T/dQ, dP^T/dS^T, dV, dK):
+// tensor memory (512 columns: R1 = S^T then P^T, R2 = dP^T then dQ, dV, dK):
 //   S^T  = K Q^T          dP^T = V dO^T                 (operands from shared memory, TMA-fed)
-//   dV  += P^T dO         dK  += dS^T Q                 (A operand read back from tensor memory)
-//   dQ   = dS K                                         (dS^T staged in shared memory, MN-major)
-// dK / dV leave as bf16 once per CTA; dQ partial tiles are added to an fp32 accumulator by TMA from the
-// shared memory of dS (whole lines; as 16-byte reductions of single threads, 4096 a step, they were what
+//   dV  += P^T dO                                       (P^T read back from tensor memory)
+//   dQ   = dS K           dK  += dS^T Q                 (one dS^T tile in shared memory, read MN-major and K-major)
+// dK / dV leave as bf16 once per CTA; dQ partial tiles are added to an fp32 accumulator by TMA from a buffer of their own
+// (whole lines; as 16-byte reductions of single threads, 4096 a step, they were what
 // a step waited for) and converted by attn_bwd_finalize_kernel. Where rotary embedding came before the attention,
 // both take its transpose along on the way out.
 //
@@ -18,10 +18,18 @@
 // query heads are dealt to several CTAs. Each stores its fp32 dK / dV, and a second kernel adds them up in order: unlike dQ, whose
 // tiles arrive in any order, dK and dV repeat bit for bit. Only rows of the tiles are written.
 //
-// A step is a chain (S and dP, then the softmax gradient, then three products, then the read-out of dQ), and the
-// 512 columns leave no room for a second tile, so its length is what counts: eight warps share the
-// elementwise part, two per lane quarter with 64 queries each. P^T and dS^T of a warp stay inside the
-// columns that it read S^T and dP^T from (queries 64.. at column 64), so the two need not wait for each other.
+// A step is a chain (S and dP, then the softmax gradient, then three products, then the read-out of dQ), and neither the 512
+// columns nor the 227 KB leave room for a second tile. So the two halves of a step are kept apart and its links run beside each
+// other. The tensor core goes dV(i), S(i+1), dQ(i), dK(i), dP(i+1); dS^T lives in shared memory alone, so R1 is
+// free for S(i+1) as soon as dV(i) is issued, and the exponentials of a step need only S, its gradient only dP. R2 is handed back once
+// dQ is in registers; half of it leaves at once, the other half behind the next step's exponentials, and no step waits for the
+// reduction before the buffer is needed again. Row statistics are loaded a step ahead. Eight warps share the elementwise part,
+// two per lane quarter with 64 queries each; P^T of a warp stays inside the columns that it read S^T from (queries 64.. at column 64).
+//
+// Measured (12 query, 2 kv heads, head_dim 128), before with one chain per step, then as it is: 31287 tokens in 11 sequences
+// 2349 -> 1581 us (714 TFLOP/s), 8 x 4096 2064 -> 1335, 19 x 330 142 -> 125, 1 x 759 69 -> 55; 28 query, 4 kv heads, 25415 tokens
+// 2553 -> 1729. Bound by the elementwise warps between the products: staging dQ for its reduction is 17 % of a step,
+// the exponentials are a small part.
 #include <cuda_bf16.h>
 
 #include "../common/f32x2.cuh"
@@ -578,9 +586,9 @@ void launch_bwd_t(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMa
 
 // CTAs over which the query heads of a (key tile, kv head) are dealt: enough for about four CTAs per SM, so that the longest of them
 // (all query tiles of the longest sequence) is a small part of an SM's share. 12 query and 2 kv heads, us with one piece and with as
-// many as this rule says: one sequence of 759 tokens 210 and 66 (6 pieces), of 8000 1988 and 994 (5), 19 of 330 142 and 136 (6), 11 of up
-// to 8575 2492 and 2342 (2); sequences of one length gain less or nothing: 40 of 330 216 and 232 (3), 8 of 4096 2045 and 2058 (2). 824
-// CTAs (28 and 4 heads, 25415 tokens) are left as they are.
+// many as this rule says: one sequence of 759 tokens 129 and 51 (6 pieces), of 2600 402 and 105 (6), of 8000 1161 and 604 (5), 11 of 250 to
+// 8575 1890 and 1845 (2). Sequences of one length lose: 19 of 330 112 and 124 (6), 40 of 330 175 and 200 (3), 8 of 4096 1278 and 1327 (2);
+// the count of tiles, which is what the host has, does not tell them from the others. From 592 CTAs on nothing is split.
 int attn_bwd_pieces(int n_tiles, int Hq, int Hkv, int num_sms) {
   const long long ctas = (long long)n_tiles * Hkv;
   if (ctas <= 0) return 1;
