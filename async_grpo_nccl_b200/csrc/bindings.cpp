@@ -594,11 +594,12 @@ long long ld_kept(const OptTensor& logits) { return logits.has_value() && logits
 // All of them if torch's allocator holds enough unused memory for both, as it does from the second step of a kind on; else as many as
 // a quarter of what this process could get beyond `reserve` holds, in steps of 256. The device is only asked in the second case:
 // on a machine with other users cudaMemGetInfo takes 0.1 to 100 ms.
-int64_t lmhead_keep_columns(int64_t rows, int64_t V, double reserve) {
+int64_t lmhead_keep_columns(int64_t device, int64_t rows, int64_t V, double reserve) {
   if (rows <= 0) return 0;
+  const c10::cuda::CUDAGuard guard((c10::DeviceIndex)device);
   const int64_t all = (V + 7) / 8 * 8, need = all * rows * 4;
   if (need <= (64 << 20)) return all;
-  const auto st = c10::cuda::CUDACachingAllocator::getDeviceStats(c10::cuda::current_device());
+  const auto st = c10::cuda::CUDACachingAllocator::getDeviceStats((c10::DeviceIndex)device);
   const int64_t cached = st.reserved_bytes[0].current - st.allocated_bytes[0].current;  // [0]: over all pools
   if (cached >= need + (int64_t)(0.6 * reserve)) return all;  // `reserve` is an estimate from above
   size_t free_b = 0, total_b = 0;

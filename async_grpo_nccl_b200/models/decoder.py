@@ -373,6 +373,10 @@ class NativeDecoder:
         layers = 2.0 * T * cfg.hidden_size * cfg.num_hidden_layers + 2 * layer if self.recompute else layer * cfg.num_hidden_layers
         return 1.25 * (layers + layer) + 2.0 * T * vocab_chunk(T, self.lmhead_chunk)
 
+    def _keep_columns(self, rows: int, T: int) -> int:
+        """Columns of the fp32 logits of ``rows`` rows that a training step of T rows may keep on this decoder's device."""
+        return int(self.C.lmhead_keep_columns(self.dev.index or 0, rows, self.cfg.vocab_size, self._activation_bytes(T)))
+
     def _body(self, batch: PackedBatch, saves: Optional[List[dict]]) -> torch.Tensor:
         """Embedding and all layers."""
         cfg, C = self.cfg, self.C
@@ -432,7 +436,7 @@ class NativeDecoder:
         # step then finds the block that the step before gave back whole, where a request behind the activations would find it
         # split and ask the device for another (20 ms).
         n_head = batch.total_out if compact else T
-        keep = int(C.lmhead_keep_columns(n_head, cfg.vocab_size, self._activation_bytes(T)))
+        keep = self._keep_columns(n_head, T)
         logits = self._new(n_head, keep, dtype=torch.float32) if keep > 0 else None
         x_last = self._body(batch, saves)
         labels, advantages, old_logp, old_ent = batch.labels, batch.advantages, batch.old_logprobs, batch.old_entropies
