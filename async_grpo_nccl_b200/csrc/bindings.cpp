@@ -450,6 +450,13 @@ struct LayerSlab {
   }
 };
 
+// What layer_fwd of T rows allocates: activations (kept for the backward pass or not), output.
+int64_t layer_fwd_bytes(const std::vector<int64_t>& dims, int64_t T, bool keep) {
+  LayerArgs a{};
+  a.T = (int)T; a.H = (int)dims.at(0); a.Hq = (int)dims.at(1); a.Hkv = (int)dims.at(2); a.D = (int)dims.at(3); a.F = (int)dims.at(4);
+  return LayerSlab(a, keep).size + T * a.H * 2;
+}
+
 // One layer forward: (output, activations for layer_bwd, launches). `k_cache` given: k and v of every token also go to `slots` of
 // the paged cache (kv heads [kv_head0, kv_head0 + heads of the cache)).
 std::tuple<Tensor, Tensor, int64_t> layer_fwd(const Tensor& params, const std::vector<int64_t>& offs, const std::vector<int64_t>& dims, double eps,
@@ -590,22 +597,26 @@ int kept_cols(const OptTensor& logits, int64_t T, int64_t V) {
   return (int)logits->size(1);
 }
 long long ld_kept(const OptTensor& logits) { return logits.has_value() && logits->defined() ? logits->size(1) : 0; }
-// Columns of [rows, V] fp32 that may be kept from the forward to the backward pass of a step that takes about `reserve` bytes besides.
-// All of them if torch's allocator holds enough unused memory for both, as it does from the second step of a kind on; else as many as
-// a quarter of what this process could get beyond `reserve` holds, in steps of 256. The device is only asked in the second case:
-// on a machine with other users cudaMemGetInfo takes 0.1 to 100 ms.
-int64_t lmhead_keep_columns(int64_t device, int64_t rows, int64_t V, double reserve) {
-  if (rows <= 0) return 0;
-  const c10::cuda::CUDAGuard guard((c10::DeviceIndex)device);
-  const int64_t all = (V + 7) / 8 * 8, need = all * rows * 4;
-  if (need <= (64 << 20)) return all;
-  const auto st = c10::cuda::CUDACachingAllocator::getDeviceStats((c10::DeviceIndex)device);
-  const int64_t cached = st.reserved_bytes[0].current - st.allocated_bytes[0].current;  // [0]: over all pools
-  if (cached >= need + (int64_t)(0.6 * reserve)) return all;  // `reserve` is an estimate from above
-  size_t free_b = 0, total_b = 0;
-  C10_CUDA_CHECK(cudaMemGetInfo(&free_b, &total_b));
-  const int64_t cols = std::max<int64_t>(0, (int64_t)free_b + cached - (int64_t)reserve) / 4 / (rows * 4);
-  return cols >= all ? all : cols / 256 * 256;
+// Memory that torch's allocator holds unused for the current stream of `device`, as far as requests of `piece` bytes and more can have
+// it: segments without a block in use whole (they can also be given back to the device for one of another size), of the others what
+// holds whole pieces. Blocks of other streams and of private pools (captured graphs) are not this stream's to take. Second: the largest
+// of these blocks. Third: all that the allocator holds of the device.
+std::tuple<int64_t, int64_t, int64_t> cached_memory(int64_t device, int64_t piece) {
+  const auto dev = (c10::DeviceIndex)device;
+  const cudaStream_t stream = at::cuda::getCurrentCUDAStream(dev).stream();
+  const c10::cuda::MempoolId_t shared{0, 0};
+  int64_t usable = 0, largest = 0, held = 0;
+  for (const auto& seg : c10::cuda::CUDACachingAllocator::snapshot().segments) {
+    if (seg.device != dev) continue;
+    held += (int64_t)seg.total_size;
+    if (seg.stream != stream || !seg.is_large || seg.owner_private_pool_id != shared) continue;
+    for (const auto& blk : seg.blocks) {
+      if (blk.active || blk.allocated) continue;
+      usable += seg.active_size == 0 ? (int64_t)blk.size : (int64_t)blk.size / piece * piece;
+      largest = std::max(largest, (int64_t)blk.size);
+    }
+  }
+  return {usable, largest, held};
 }
 void lmhead_logprob(const Tensor& hidden, const Tensor& weight, const Tensor& labels, double temperature, Tensor& partials,
                     Tensor& label_logit, const OptTensor& logp, const OptTensor& entropy, const OptTensor& lse,
@@ -1272,7 +1283,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("lmhead_logprob", &lmhead_logprob, py::arg("hidden"), py::arg("weight"), py::arg("labels"), py::arg("temperature"),
         py::arg("partials"), py::arg("label_logit"), py::arg("logp") = py::none(), py::arg("entropy") = py::none(),
         py::arg("lse") = py::none(), py::arg("status") = py::none(), py::arg("logits") = py::none(), NOGIL);
-  m.def("lmhead_keep_columns", &lmhead_keep_columns);
+  m.def("cached_memory", &cached_memory);
+  m.def("layer_fwd_bytes", &layer_fwd_bytes);
   m.def("grpo_token_loss", &grpo_token_loss, py::arg("logp"), py::arg("old_logp"), py::arg("ref_logp"), py::arg("adv"),
         py::arg("labels"), py::arg("entropy"), py::arg("old_entropy"), py::arg("clip_low"), py::arg("clip_high"),
         py::arg("clip_c"), py::arg("kl_beta"), py::arg("grad_weight"), py::arg("dlogp"), py::arg("stats"), NOGIL);

@@ -126,6 +126,13 @@ def vocab_chunk(T: int, asked: Optional[int] = None) -> int:
     return max(4096, min(15360, (1 << 29) // max(T, 1) // 256 * 256))
 
 
+def kept_columns(rows: int, V: int, memory: float) -> int:
+    """Leading columns of [rows, V] fp32 logits that ``memory`` bytes hold: all (rounded up to 8), or a multiple of 256."""
+    cols = max(0, int(memory)) // (4 * rows)
+    every = (V + 7) // 8 * 8
+    return every if cols >= every else cols // 256 * 256
+
+
 class NativeDecoder:
     def __init__(self, cfg: ModelConfig, layout: ParamLayout, params: Optional[torch.Tensor], recompute: bool = False,
                  lmhead_chunk: Optional[int] = None, weights: Any = None):
@@ -155,6 +162,8 @@ class NativeDecoder:
         self._offs = [[layout.segments[f"layers.{i}.{n}"].offset if f"layers.{i}.{n}" in layout.segments else -1
                        for n in ("ln1", "wqkv", "bqkv", "wo", "ln2", "wgu", "wd")] for i in range(cfg.num_hidden_layers)]
         self.launches = 0  # kernels of this package launched (bench bookkeeping)
+        self.memory_share = 1.0  # of the device, what this process's roles are to stay within (kept logits only)
+        self._asked_at = -1  # what the allocator held when the device was last asked for free memory
 
     # ---- helpers ----
     def w(self, name: str) -> torch.Tensor:
@@ -366,16 +375,35 @@ class NativeDecoder:
         self.launches += 1
         return hn, rstd
 
-    def _activation_bytes(self, T: int) -> float:
-        """What a training step of T rows holds at its peak besides kept logits, roughly and from above."""
-        cfg = self.cfg
-        layer = 2.0 * T * (5 * cfg.hidden_size + cfg.qkv_dim + cfg.q_dim + 3 * cfg.intermediate_size)
-        layers = 2.0 * T * cfg.hidden_size * cfg.num_hidden_layers + 2 * layer if self.recompute else layer * cfg.num_hidden_layers
-        return 1.25 * (layers + layer) + 2.0 * T * vocab_chunk(T, self.lmhead_chunk)
+    def _held_bytes(self, T: int, rows: int) -> int:
+        """What a training step of T rows, ``rows`` of them with a loss, holds beside kept logits while it has those: the embedding,
+        the activations of the layers (with recomputation their inputs, and one layer's at a time) and the head's rows, dlogits and dH. As
+        exact as it can be: more, and a step would not find in the allocator what the same step has left there."""
+        L, x, layer = self.cfg.num_hidden_layers, 2 * T * self.cfg.hidden_size, int(self.C.layer_fwd_bytes(self._dims, T, True))
+        head = rows * (2 * min(vocab_chunk(rows, self.lmhead_chunk), (self.cfg.vocab_size + 255) // 256 * 256) + 6 * self.cfg.hidden_size)
+        return x + (L * x + max(layer, head) if self.recompute else L * layer + head)
 
     def _keep_columns(self, rows: int, T: int) -> int:
-        """Columns of the fp32 logits of ``rows`` rows that a training step of T rows may keep on this decoder's device."""
-        return int(self.C.lmhead_keep_columns(self.dev.index or 0, rows, self.cfg.vocab_size, self._activation_bytes(T)))
+        """Columns of the fp32 logits of ``rows`` rows that a training step of T rows may keep on this decoder's device. The allocator is
+        asked first, the device only if this stream's unused blocks do not hold everything, and then not again until the allocator has
+        taken or given back memory: on a machine with other users that question takes 0.1 to 100 ms."""
+        V = self.cfg.vocab_size
+        if rows <= 0 or torch.cuda.is_current_stream_capturing():
+            return 0  # a graph's memory stays taken between its replays
+        if 4 * rows * V <= 64 << 20:
+            return kept_columns(rows, V, 64 << 20)
+        held = self._held_bytes(T, rows)
+        cached, block, reserved = self.C.cached_memory(self.dev.index, 2 * T * self.cfg.hidden_size)
+        cols = kept_columns(rows, V, min(block, cached - held))
+        if cols >= V or reserved == self._asked_at:
+            return cols
+        free, total = torch.cuda.mem_get_info(self.dev)
+        self._asked_at = reserved
+        limit = int(torch.cuda.get_per_process_memory_fraction(self.dev) * total) - reserved
+        free = max(0, min(free - int((1.0 - self.memory_share) * total), limit))
+        # A new block: of what the process could still get a quarter, since other streams and roles grow as well, and not more than the
+        # device has beside what the activations ask it for. Else the allocator would give back all that it holds and begin anew.
+        return max(cols, kept_columns(rows, V, min((cached + free - held) // 4, free - max(0, held - cached))))
 
     def _body(self, batch: PackedBatch, saves: Optional[List[dict]]) -> torch.Tensor:
         """Embedding and all layers."""
@@ -437,7 +465,10 @@ class NativeDecoder:
         # split and ask the device for another (20 ms).
         n_head = batch.total_out if compact else T
         keep = self._keep_columns(n_head, T)
-        logits = self._new(n_head, keep, dtype=torch.float32) if keep > 0 else None
+        try:
+            logits = self._new(n_head, keep, dtype=torch.float32) if keep > 0 else None
+        except torch.OutOfMemoryError:
+            logits = None
         x_last = self._body(batch, saves)
         labels, advantages, old_logp, old_ent = batch.labels, batch.advantages, batch.old_logprobs, batch.old_entropies
         ref = batch.ref_logprobs if (lc.kl_beta > 0 and batch.has_ref) else None
@@ -460,9 +491,6 @@ class NativeDecoder:
         logp = self._new(T, dtype=torch.float32)
         ent = self._new(T, dtype=torch.float32)
         lse = self._new(T, dtype=torch.float32)
-        chunk = min(vocab_chunk(T, self.lmhead_chunk), (V + 255) // 256 * 256)
-        dz = self._new(T, chunk)
-        dh_acc = self._new(T, cfg.hidden_size, dtype=torch.float32)
         C.lmhead_logprob(hn, wl, labels, lc.temperature, partials, ll, logp, ent, lse, self.status, logits)
         del partials
         stats = torch.zeros(self.n_stats, dtype=torch.float32, device=self.dev)
@@ -470,6 +498,9 @@ class NativeDecoder:
         n_valid = max(1.0, batch.scalars.get("num_output_tokens_non_masked", float(batch.total_out)))
         C.grpo_token_loss(logp, old_logp, ref, advantages, labels, ent, old_ent,
                           lc.clip_low, lc.clip_high, lc.clip_ratio_c, lc.kl_beta, loss_scale / n_valid, dlogp, stats)
+        chunk = min(vocab_chunk(T, self.lmhead_chunk), (V + 255) // 256 * 256)
+        dz = self._new(T, chunk)
+        dh_acc = self._new(T, cfg.hidden_size, dtype=torch.float32)
         C.lmhead_backward(hn, wl, labels, lse, dlogp, lc.temperature, dz, dh_acc, sink.view(wl_name), self.status, logits)
         del dz, logits
         dhn = self._new(T, cfg.hidden_size)

@@ -106,6 +106,8 @@ class TrainerCore:
             self._oracle_params = self.params.clone().requires_grad_(True)
             self.decoder = OracleDecoder(mcfg, L, self._oracle_params)
             self.norm_sq = torch.zeros(1, dtype=torch.float32)
+        if self.native:
+            self.decoder.memory_share = cfg.gpu_memory_utilization
         self.loss_cfg = LossConfig(cfg.clip_low, cfg.clip_high, cfg.clip_ratio_c, cfg.kl_beta, cfg.temperature,
                                    cfg.entropy_coeff, cfg.apply_entropy_bonus)
         self.opt_step = 0
