@@ -597,6 +597,10 @@ int kept_cols(const OptTensor& logits, int64_t T, int64_t V) {
   return (int)logits->size(1);
 }
 long long ld_kept(const OptTensor& logits) { return logits.has_value() && logits->defined() ? logits->size(1) : 0; }
+int64_t lmhead_chunk_step(int64_t V, int64_t chunk_cols) {
+  TORCH_CHECK(V > 0 && chunk_cols > 0, "lmhead_chunk_step: sizes");
+  return agrpo::lmhead_chunk_step((int)V, (int)chunk_cols);
+}
 // Memory that torch's allocator holds unused for the current stream of `device`, as far as requests of `piece` bytes and more can have
 // it: segments without a block in use whole (they can also be given back to the device for one of another size), of the others what
 // holds whole pieces. Blocks of other streams and of private pools (captured graphs) are not this stream's to take. Second: the largest
@@ -1283,6 +1287,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("lmhead_logprob", &lmhead_logprob, py::arg("hidden"), py::arg("weight"), py::arg("labels"), py::arg("temperature"),
         py::arg("partials"), py::arg("label_logit"), py::arg("logp") = py::none(), py::arg("entropy") = py::none(),
         py::arg("lse") = py::none(), py::arg("status") = py::none(), py::arg("logits") = py::none(), NOGIL);
+  m.def("lmhead_chunk_step", &lmhead_chunk_step);
   m.def("cached_memory", &cached_memory);
   m.def("layer_fwd_bytes", &layer_fwd_bytes);
   m.def("grpo_token_loss", &grpo_token_loss, py::arg("logp"), py::arg("old_logp"), py::arg("ref_logp"), py::arg("adv"),

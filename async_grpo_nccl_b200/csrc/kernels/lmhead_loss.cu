@@ -367,15 +367,19 @@ void launch_grpo_token_loss(const float* logp, const float* old_logp, const floa
 
 int grpo_num_loss_stats() { return kNumLossStats; }
 
+// Equal chunks, as few as the buffer allows: a short last one would pay for a whole pass over dH.
+int lmhead_chunk_step(int V, int chunk_cols) {
+  const int chunks = (V + chunk_cols - 1) / chunk_cols;
+  return std::min(chunk_cols, ((V + chunks - 1) / chunks + 255) / 256 * 256);
+}
+
 void launch_lmhead_backward(const void* hidden, long long ldh, const void* weight, long long ldw, const int* labels,
                             const float* lse, const float* dlogp, int T, int H, int V, float temperature, void* dz_chunk,
                             int chunk_cols, float* dh_acc, float* dweight, long long ld_dw, const float* logits, long long ld_logits, int keep_cols,
                             int* status, int num_sms, cudaStream_t stream) {
   if (T == 0) return;
   const CUtensorMap ta = make_tmap_2d(hidden, H, T, ldh, 64, kGemmBM);
-  // Equal chunks, as few as the buffer allows: a short last one would pay for a whole pass over dH.
-  const int chunks = (V + chunk_cols - 1) / chunk_cols;
-  const int step = std::min(chunk_cols, ((V + chunks - 1) / chunks + 255) / 256 * 256);
+  const int step = lmhead_chunk_step(V, chunk_cols);
   for (int v0 = 0, ci = 0; v0 < V; v0 += step, ++ci) {
     const int vc = (V - v0) < step ? (V - v0) : step;
     const __nv_bfloat16* wc = reinterpret_cast<const __nv_bfloat16*>(weight) + (long long)v0 * ldw;

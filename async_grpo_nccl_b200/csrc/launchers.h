@@ -249,7 +249,9 @@ void launch_grpo_token_loss(const float* logp, const float* old_logp, const floa
                             cudaStream_t stream);
 int grpo_num_loss_stats();
 // dh_acc (fp32 [T, H]) = d loss / d hidden; dweight (fp32, pitch ld_dw, may be nullptr) += d loss / d weight.
-// dz_chunk: bf16 [T, chunk_cols] scratch, chunk_cols a multiple of 256.
+// dz_chunk: bf16 [T, chunk_cols] scratch, chunk_cols a multiple of 256; the vocabulary is walked in chunks of lmhead_chunk_step
+// columns, of which kept logits serve those that they hold whole.
+int lmhead_chunk_step(int V, int chunk_cols);
 void launch_lmhead_backward(const void* hidden, long long ldh, const void* weight, long long ldw, const int* labels,
                             const float* lse, const float* dlogp, int T, int H, int V, float temperature, void* dz_chunk,
                             int chunk_cols, float* dh_acc, float* dweight, long long ld_dw, const float* logits, long long ld_logits, int keep_cols,

@@ -126,11 +126,12 @@ def vocab_chunk(T: int, asked: Optional[int] = None) -> int:
     return max(4096, min(15360, (1 << 29) // max(T, 1) // 256 * 256))
 
 
-def kept_columns(rows: int, V: int, memory: float) -> int:
-    """Leading columns of [rows, V] fp32 logits that ``memory`` bytes hold: all (rounded up to 8), or a multiple of 256."""
+def kept_columns(rows: int, V: int, memory: float, step: int) -> int:
+    """Leading columns of [rows, V] fp32 logits that ``memory`` bytes hold: all (rounded up to 8), or whole chunks of ``step``, since
+    the backward pass reads no part of one."""
     cols = max(0, int(memory)) // (4 * rows)
     every = (V + 7) // 8 * 8
-    return every if cols >= every else cols // 256 * 256
+    return every if cols >= every else cols // step * step
 
 
 class NativeDecoder:
@@ -375,12 +376,16 @@ class NativeDecoder:
         self.launches += 1
         return hn, rstd
 
+    def _chunk(self, rows: int) -> int:
+        """Columns of the dlogits buffer of ``rows`` rows."""
+        return min(vocab_chunk(rows, self.lmhead_chunk), (self.cfg.vocab_size + 255) // 256 * 256)
+
     def _held_bytes(self, T: int, rows: int) -> int:
         """What a training step of T rows, ``rows`` of them with a loss, holds beside kept logits while it has those: the embedding,
         the activations of the layers (with recomputation their inputs, and one layer's at a time) and the head's rows, dlogits and dH. As
         exact as it can be: more, and a step would not find in the allocator what the same step has left there."""
         L, x, layer = self.cfg.num_hidden_layers, 2 * T * self.cfg.hidden_size, int(self.C.layer_fwd_bytes(self._dims, T, True))
-        head = rows * (2 * min(vocab_chunk(rows, self.lmhead_chunk), (self.cfg.vocab_size + 255) // 256 * 256) + 6 * self.cfg.hidden_size)
+        head = rows * (2 * self._chunk(rows) + 6 * self.cfg.hidden_size)
         return x + (L * x + max(layer, head) if self.recompute else L * layer + head)
 
     def _keep_columns(self, rows: int, T: int) -> int:
@@ -390,11 +395,12 @@ class NativeDecoder:
         V = self.cfg.vocab_size
         if rows <= 0 or torch.cuda.is_current_stream_capturing():
             return 0  # a graph's memory stays taken between its replays
+        step = int(self.C.lmhead_chunk_step(V, self._chunk(rows)))
         if 4 * rows * V <= 64 << 20:
-            return kept_columns(rows, V, 64 << 20)
+            return kept_columns(rows, V, 64 << 20, step)
         held = self._held_bytes(T, rows)
         cached, block, reserved = self.C.cached_memory(self.dev.index, 2 * T * self.cfg.hidden_size)
-        cols = kept_columns(rows, V, min(block, cached - held))
+        cols = kept_columns(rows, V, min(block, cached - held), step)
         if cols >= V or reserved == self._asked_at:
             return cols
         free, total = torch.cuda.mem_get_info(self.dev)
@@ -403,7 +409,7 @@ class NativeDecoder:
         free = max(0, min(free - int((1.0 - self.memory_share) * total), limit))
         # A new block: of what the process could still get a quarter, since other streams and roles grow as well, and not more than the
         # device has beside what the activations ask it for. Else the allocator would give back all that it holds and begin anew.
-        return max(cols, kept_columns(rows, V, min((cached + free - held) // 4, free - max(0, held - cached))))
+        return max(cols, kept_columns(rows, V, min((cached + free - held) // 4, free - max(0, held - cached)), step))
 
     def _body(self, batch: PackedBatch, saves: Optional[List[dict]]) -> torch.Tensor:
         """Embedding and all layers."""
@@ -498,7 +504,7 @@ class NativeDecoder:
         n_valid = max(1.0, batch.scalars.get("num_output_tokens_non_masked", float(batch.total_out)))
         C.grpo_token_loss(logp, old_logp, ref, advantages, labels, ent, old_ent,
                           lc.clip_low, lc.clip_high, lc.clip_ratio_c, lc.kl_beta, loss_scale / n_valid, dlogp, stats)
-        chunk = min(vocab_chunk(T, self.lmhead_chunk), (V + 255) // 256 * 256)
+        chunk = self._chunk(T)
         dz = self._new(T, chunk)
         dh_acc = self._new(T, cfg.hidden_size, dtype=torch.float32)
         C.lmhead_backward(hn, wl, labels, lse, dlogp, lc.temperature, dz, dh_acc, sink.view(wl_name), self.status, logits)

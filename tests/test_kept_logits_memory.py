@@ -5,6 +5,7 @@ import pytest
 import torch
 
 from async_grpo_nccl_b200.models import decoder as D
+from async_grpo_nccl_b200.ops import native
 
 GB = 1 << 30
 
@@ -15,7 +16,8 @@ class Memory:
     def __init__(self, monkeypatch, cached, reserved, free, held=30 * GB, V=151936, total=180 * GB, fraction=1.0, share=1.0):
         self.asked, self.block = [], None
         self.dec = SimpleNamespace(dev=torch.device("cuda", 1), cfg=SimpleNamespace(vocab_size=V, hidden_size=1536), _asked_at=-1, memory_share=share,
-                                   _held_bytes=lambda T, rows: held, C=SimpleNamespace(cached_memory=self.cached_memory))
+                                   _held_bytes=lambda T, rows: held, C=SimpleNamespace(cached_memory=self.cached_memory, lmhead_chunk_step=native().lmhead_chunk_step),
+                                   _chunk=lambda rows: 15360)
         self.cached, self.reserved, self.free, self.total = cached, reserved, free, total
         monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
         monkeypatch.setattr(torch.cuda, "mem_get_info", self.mem_get_info)
@@ -35,10 +37,27 @@ class Memory:
 
 
 def test_columns_that_fit():
-    assert D.kept_columns(100, 1003, 100 * 4 * 1008) == 1008
-    assert D.kept_columns(100, 1003, 100 * 4 * 1008 - 1) == 768
-    assert D.kept_columns(100, 1003, 100 * 4 * 255) == 0
-    assert D.kept_columns(100, 1003, -5.0) == 0
+    assert D.kept_columns(100, 1003, 100 * 4 * 1008, 256) == 1008
+    assert D.kept_columns(100, 1003, 100 * 4 * 1008 - 1, 256) == 768
+    assert D.kept_columns(100, 1003, 100 * 4 * 255, 256) == 0
+    assert D.kept_columns(100, 1003, -5.0, 256) == 0
+
+
+# the fewest chunks of equal width (a multiple of 256) that the buffer allows
+@pytest.mark.parametrize("V,chunk,step", [(151936, 15360, 15360), (152064, 15360, 15360), (2048, 2048, 2048), (1003, 512, 512), (5001, 2048, 1792),
+                                          (100, 256, 256), (256, 256, 256), (257, 256, 256)])
+def test_steps_of_the_backward_pass(V, chunk, step):
+    assert native().lmhead_chunk_step(V, chunk) == step
+    for memory in (0, 3 << 20, 40 << 20, 1 << 40):
+        kept = D.kept_columns(1000, V, memory, step)
+        assert kept % step == 0 or kept == (V + 7) // 8 * 8
+
+
+@pytest.mark.parametrize("cached,free", [(40, 0), (33, 9), (31, 0), (30, 50)])
+def test_only_columns_that_are_read_are_kept(monkeypatch, cached, free):
+    m = Memory(monkeypatch, cached * GB, 60 * GB, free * GB)
+    cols = m.keep(30000, 32768)
+    assert cols % 15360 == 0 and cols < 151936
 
 
 # need: 30000 x 151936 x 4 = 17.0 GB beside 72 GB that the step holds anyway. A cache filled by a larger microbatch without kept logits
