@@ -54,15 +54,33 @@ struct AdamW {
   }
 };
 
+// kVec fp32 values with one access of 32 or 16 bytes.
+template <int kVec>
+__device__ __forceinline__ void ld_vec(const float* p, uint32_t (&r)[kVec]) {
+  if constexpr (kVec == 8) {
+    ld_global_32b(p, r);
+  } else {
+    const uint4 w = *reinterpret_cast<const uint4*>(p);
+    r[0] = w.x; r[1] = w.y; r[2] = w.z; r[3] = w.w;
+  }
+}
+template <int kVec>
+__device__ __forceinline__ void st_vec(float* p, const uint32_t (&r)[kVec]) {
+  if constexpr (kVec == 8) st_global_32b(p, r);
+  else *reinterpret_cast<uint4*>(p) = make_uint4(r[0], r[1], r[2], r[3]);
+}
+
 // norm_sq points at the squared global gradient norm (already scaled by grad_scale^2).
 // clip coefficient = min(1, max_norm / (sqrt(norm_sq) + 1e-6)); max_norm <= 0 disables clipping.
 // Bound by memory: 34 bytes a parameter (p, m, v, g read and written, the bf16 copy written). Eight parameters a thread, every access
 // 32 bytes, and as many blocks as that takes: 607 M parameters took 3.52 ms (5.9 TB/s) with four a thread and 148 x 16 blocks that
 // stride over them, 3.38 ms with eight, 2.99 ms (6.9 TB/s) without the stride: blocks that start in order keep to a few DRAM pages
-// of each of the nine streams.
+// of each of the nine streams. Slices whose buffers keep to 16 bytes (8 for the bf16 copy) but not to 32 take four
+// a thread: 64 M parameters 0.346 ms, 0.341 aligned, 0.683 one by one.
+template <int kVec>  // 1: buffers that no wide access fits
 __global__ void __launch_bounds__(256)
 adamw_kernel(float* __restrict__ p, float* __restrict__ m, float* __restrict__ v, float* __restrict__ g, __nv_bfloat16* __restrict__ p16,
-             long long n, int vec, AdamW k, float bc1, float bc2, const float* __restrict__ norm_sq, float max_norm, int zero_grad) {
+             long long n, AdamW k, float bc1, float bc2, const float* __restrict__ norm_sq, float max_norm, int zero_grad) {
   if (max_norm > 0.f && norm_sq != nullptr) {
     const float nrm = sqrtf(*norm_sq);
     k.coef *= fminf(1.f, max_norm / (nrm + 1e-6f));
@@ -70,34 +88,40 @@ adamw_kernel(float* __restrict__ p, float* __restrict__ m, float* __restrict__ v
   k.inv_bc1 = 1.f / bc1;
   k.inv_sqrt_bc2 = rsqrtf(bc2);
   const long long first = blockIdx.x * (long long)blockDim.x + threadIdx.x, stride = (long long)gridDim.x * blockDim.x;
-  const long long n8 = vec ? n / 8 : 0;
-  if (first < n8) {  // the launcher starts a thread for each
-    const long long at = 8 * first;
-    uint32_t gi[8], pi[8], mi[8], vi[8];
-    ld_global_32b(g + at, gi);
-    ld_global_32b(p + at, pi);
-    ld_global_32b(m + at, mi);
-    ld_global_32b(v + at, vi);
-    float q[8];
+  const long long whole = kVec > 1 ? n / kVec * kVec : 0;
+  if constexpr (kVec > 1) {
+    const long long at = kVec * first;
+    if (at < whole) {  // the launcher starts a thread for each
+      uint32_t gi[kVec], pi[kVec], mi[kVec], vi[kVec];
+      ld_vec(g + at, gi);
+      ld_vec(p + at, pi);
+      ld_vec(m + at, mi);
+      ld_vec(v + at, vi);
+      float q[kVec];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      float mj = __uint_as_float(mi[j]), vj = __uint_as_float(vi[j]);
-      q[j] = __uint_as_float(pi[j]);
-      k.update(__uint_as_float(gi[j]), q[j], mj, vj);
-      pi[j] = __float_as_uint(q[j]);
-      mi[j] = __float_as_uint(mj);
-      vi[j] = __float_as_uint(vj);
-      gi[j] = 0u;
+      for (int j = 0; j < kVec; ++j) {
+        float mj = __uint_as_float(mi[j]), vj = __uint_as_float(vi[j]);
+        q[j] = __uint_as_float(pi[j]);
+        k.update(__uint_as_float(gi[j]), q[j], mj, vj);
+        pi[j] = __float_as_uint(q[j]);
+        mi[j] = __float_as_uint(mj);
+        vi[j] = __float_as_uint(vj);
+        gi[j] = 0u;
+      }
+      st_vec(p + at, pi);
+      st_vec(m + at, mi);
+      st_vec(v + at, vi);
+      if (zero_grad) st_vec(g + at, gi);
+      if (p16 != nullptr) {
+        if constexpr (kVec == 8)
+          *reinterpret_cast<uint4*>(p16 + at) =
+              make_uint4(pack_bf16x2(q[0], q[1]), pack_bf16x2(q[2], q[3]), pack_bf16x2(q[4], q[5]), pack_bf16x2(q[6], q[7]));
+        else
+          *reinterpret_cast<uint2*>(p16 + at) = make_uint2(pack_bf16x2(q[0], q[1]), pack_bf16x2(q[2], q[3]));
+      }
     }
-    st_global_32b(p + at, pi);
-    st_global_32b(m + at, mi);
-    st_global_32b(v + at, vi);
-    if (zero_grad) st_global_32b(g + at, gi);
-    if (p16 != nullptr)
-      *reinterpret_cast<uint4*>(p16 + at) =
-          make_uint4(pack_bf16x2(q[0], q[1]), pack_bf16x2(q[2], q[3]), pack_bf16x2(q[4], q[5]), pack_bf16x2(q[6], q[7]));
   }
-  for (long long i = n8 * 8 + first; i < n; i += stride) {
+  for (long long i = whole + first; i < n; i += stride) {
     k.update(g[i], p[i], m[i], v[i]);
     if (p16 != nullptr) p16[i] = __float2bfloat16(p[i]);
     if (zero_grad) g[i] = 0.f;
@@ -127,12 +151,14 @@ void launch_adamw(float* p, float* m, float* v, float* g, void* p16, long long n
   const float bc1 = 1.f - powf(beta1, (float)step);
   const float bc2 = 1.f - powf(beta2, (float)step);
   const auto aligned = [](const void* q, uintptr_t to) { return (reinterpret_cast<uintptr_t>(q) & (to - 1)) == 0; };
-  const int vec = aligned(p, 32) && aligned(m, 32) && aligned(v, 32) && aligned(g, 32) && aligned(p16, 16) ? 1 : 0;
-  long long blocks = ((vec ? n / 8 : n) + 255) / 256;
+  const auto all = [&](uintptr_t to) { return aligned(p, to) && aligned(m, to) && aligned(v, to) && aligned(g, to) && aligned(p16, to / 2); };
+  const int vec = all(32) ? 8 : all(16) ? 4 : 1;
+  long long blocks = (n / vec + 255) / 256;
   if (blocks < 1) blocks = 1;
-  if (!vec && blocks > 148 * 16) blocks = 148 * 16;
+  if (vec == 1 && blocks > 148 * 16) blocks = 148 * 16;
   const AdamW k{lr, beta1, beta2, eps, wd, 0.f, 0.f, grad_scale};
-  adamw_kernel<<<(int)blocks, 256, 0, s>>>(p, m, v, g, (__nv_bfloat16*)p16, n, vec, k, bc1, bc2, norm_sq, max_norm, zero_grad ? 1 : 0);
+  const auto kernel = vec == 8 ? adamw_kernel<8> : vec == 4 ? adamw_kernel<4> : adamw_kernel<1>;
+  kernel<<<(int)blocks, 256, 0, s>>>(p, m, v, g, (__nv_bfloat16*)p16, n, k, bc1, bc2, norm_sq, max_norm, zero_grad ? 1 : 0);
   check_cuda(cudaGetLastError(), "adamw");
 }
 
