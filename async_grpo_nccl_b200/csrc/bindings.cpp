@@ -423,11 +423,14 @@ void check_tiles(const Tensor& tiles) {
   TORCH_CHECK(tiles.is_contiguous() && tiles.dim() == 2 && tiles.size(1) == 4 && (reinterpret_cast<uintptr_t>(tiles.data_ptr()) & 15) == 0, "layer: tiles [n, 4]");
 }
 // Programmatic dependent launch for the launches of a scope (forward passes): the prologue of a kernel overlaps the tail of the one
-// before.
+// before. Weights may be read early: the kernel ahead of a product is one of the same layer and writes none.
 struct PdlScope {
-  bool before = agrpo::pdl_flag();
-  PdlScope() { agrpo::pdl_flag() = true; }
-  ~PdlScope() { agrpo::pdl_flag() = before; }
+  bool before = agrpo::pdl_flag(), early = agrpo::pdl_early_flag();
+  PdlScope() { agrpo::pdl_flag() = agrpo::pdl_early_flag() = true; }
+  ~PdlScope() {
+    agrpo::pdl_flag() = before;
+    agrpo::pdl_early_flag() = early;
+  }
 };
 // Parts of one allocation, each on a 256-byte boundary.
 struct Carve {
@@ -1233,8 +1236,9 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("embedding_bwd", &embedding_bwd, NOGIL);
   m.def("set_sm_limit", [](int n) { sm_limit() = n; },
         "Cap (0 = none) on the SMs filled by persistent kernels that this THREAD launches.");
-  m.def("set_pdl", [](bool on) { agrpo::pdl_flag() = on; },
-        "Programmatic dependent launch for the kernels this THREAD launches next (used around the decode step).");
+  m.def("set_pdl", [](bool on, bool early) { agrpo::pdl_flag() = on; agrpo::pdl_early_flag() = early; }, py::arg("on"), py::arg("early") = false,
+        "Programmatic dependent launch for the kernels this THREAD launches next (used around the decode step). early: the caller "
+        "vouches that no launch writes the weights, lengths, block tables or older cache entries that the next one reads.");
   m.def("embedding_sumsq", &embedding_sumsq, NOGIL);
   m.def("fold_norm_weight", &fold_norm_weight, NOGIL);
   m.def("gemm_decode", &gemm_decode, py::arg("a"), py::arg("b"), py::arg("d"), py::arg("bias") = py::none(),

@@ -314,7 +314,7 @@ bool launch_gemm_swiglu_bf16(const void* a, long long lda, const void* b, long l
   p.group_n = 1;
   p.status = status;
   p.dual_b = F;
-  p.b_fixed = true;
+  p.b_fixed = pdl_early();
   SwigluEpilogue e;
   e.D = reinterpret_cast<__nv_bfloat16*>(d);
   e.ldd = ldd;

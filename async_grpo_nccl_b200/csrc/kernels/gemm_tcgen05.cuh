@@ -35,7 +35,8 @@ struct GemmShape {
   // a2; column tiles never straddle n1, and an epilogue sees as N the end of the product that its tile belongs to.
   int n1 = 0;
   int a2 = 0;
-  // B is not written by the kernel before this one (weights): its first tiles are requested before that kernel is complete.
+  // B is not written by the kernel before this one (weights, where the caller vouches for that): its first tiles are requested before
+  // that kernel is complete.
   bool b_fixed = false;
 
   __host__ __device__ int tiles_n(int BN) const { return n1 > 0 ? (n1 + BN - 1) / BN + (N - n1 + BN - 1) / BN : (N + BN - 1) / BN; }

@@ -140,7 +140,8 @@ __global__ void __launch_bounds__(kDecWarps * 32)
 paged_decode_attn_kernel(const DecodeParams p) {
   extern __shared__ __align__(256) uint8_t dsm[];
   __shared__ int s_last;
-  // lengths, tables and the pages of older tokens are older than the kernel before this one
+  // `early`: lengths, tables and the pages of older tokens are older than the kernel before this one
+  if (!p.early) pdl_wait();
   paged_decode_attend<2>(p, blockIdx.x, blockIdx.y, blockIdx.z, dsm, threadIdx.x >> 5, threadIdx.x, &s_last, [] {
     pdl_wait();
     pdl_launch();
@@ -436,6 +437,7 @@ void launch_paged_decode_attn(const void* q, long long ldq, int q_col0, const vo
   p.num_cache_blocks = num_cache_blocks;
   p.status = status;
   p.tickets = tickets;
+  p.early = pdl_early();
   constexpr int smem = kDecWarps * 2 * 2 * 4096;  // 64 KB staging (>= merge area of 16.6 KB)
   AGRPO_SET_MAX_DYN_SMEM(paged_decode_attn_kernel, smem, "paged_decode smem attr");
   dim3 grid(splits, Hkv, B);
@@ -464,7 +466,7 @@ void launch_lm_sample(const void* hidden, long long ldh, const void* weight, lon
   p.M = rows; p.N = V; p.K = H;
   p.group_n = group_n;
   p.status = status;
-  p.b_fixed = true;
+  p.b_fixed = pdl_early();
   LmSampleEpilogue e;
   e.seeds = seeds;
   e.greedy = temperature <= 0.f ? 1 : 0;

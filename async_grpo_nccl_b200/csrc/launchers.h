@@ -58,12 +58,20 @@ struct PerDeviceOnce {
 
 // Programmatic dependent launch is a per-thread switch: the rollout engine turns it on around its decode step, whose
 // ~170 short kernels then overlap each prologue (barrier set-up, TMEM allocation, first weight loads) with the tail
-// of the kernel before. Kernels launched through launch_kernel() contain griddepcontrol.wait, so they are correct
-// with the switch on or off.
+// of the kernel before. Every kernel waits (griddepcontrol.wait) before it reads what another kernel writes, so that all are correct with
+// the switch on or off.
 inline bool& pdl_flag() {
   static thread_local bool on = false;
   return on;
 }
+// What the caller vouches for besides: the kernel directly ahead of a launch does not write the launch's weights (the B of a split-K,
+// SwiGLU or sampling product) nor, of an attention step over a paged cache, the lengths, the block tables and the entries older than the
+// newest token. Those are then read before the wait. Also a switch of the thread, without effect where the other is off.
+inline bool& pdl_early_flag() {
+  static thread_local bool on = false;
+  return on;
+}
+inline bool pdl_early() { return pdl_flag() && pdl_early_flag(); }
 template <typename... KArgs, typename... Args>
 inline void launch_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, const char* what,
                           Args&&... args) {

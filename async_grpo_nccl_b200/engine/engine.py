@@ -469,8 +469,9 @@ class RolloutEngine:
         if self.mega_rows and B <= self.mega_rows:
             return self._decode_forward_mega(B, temperature, splits)
         if self.fused_decode and B <= self.fused_rows:
-            # short kernels back to back: let each prologue overlap the tail of the kernel before (this thread only)
-            self.C.set_pdl(self.use_pdl)
+            # short kernels back to back: let each prologue overlap the tail of the kernel before (this thread only). Weights, lengths
+            # and tables are written before the step; a step writes the newest token's cache entry alone
+            self.C.set_pdl(self.use_pdl, True)
             try:
                 return self._decode_forward_fused(B, temperature, splits)
             finally:

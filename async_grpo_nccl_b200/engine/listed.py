@@ -149,7 +149,8 @@ class ListedEngine(RolloutEngine):
 
     def _decode_layers(self, B: int, splits: int) -> None:
         sb = StepBatch(B, self.block_tables, seq_lens=self.seq_lens, splits=splits, scratch=self.b_scratch)
-        self.C.set_pdl(self.use_pdl)  # this thread only: prologues overlap the tail of the kernel before
+        # this thread only: prologues overlap the tail of the kernel before. Weights, lengths and tables are written before the step
+        self.C.set_pdl(self.use_pdl, True)
         try:
             self.dec.forward(self.last_tokens[:B], sb, self.b_buf)
         finally:
