@@ -453,13 +453,6 @@ struct LayerSlab {
   }
 };
 
-// What layer_fwd of T rows allocates: activations (kept for the backward pass or not), output.
-int64_t layer_fwd_bytes(const std::vector<int64_t>& dims, int64_t T, bool keep) {
-  LayerArgs a{};
-  a.T = (int)T; a.H = (int)dims.at(0); a.Hq = (int)dims.at(1); a.Hkv = (int)dims.at(2); a.D = (int)dims.at(3); a.F = (int)dims.at(4);
-  return LayerSlab(a, keep).size + T * a.H * 2;
-}
-
 // One layer forward: (output, activations for layer_bwd, launches). `k_cache` given: k and v of every token also go to `slots` of
 // the paged cache (kv heads [kv_head0, kv_head0 + heads of the cache)).
 std::tuple<Tensor, Tensor, int64_t> layer_fwd(const Tensor& params, const std::vector<int64_t>& offs, const std::vector<int64_t>& dims, double eps,
@@ -1293,7 +1286,6 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         py::arg("lse") = py::none(), py::arg("status") = py::none(), py::arg("logits") = py::none(), NOGIL);
   m.def("lmhead_chunk_step", &lmhead_chunk_step);
   m.def("cached_memory", &cached_memory);
-  m.def("layer_fwd_bytes", &layer_fwd_bytes);
   m.def("grpo_token_loss", &grpo_token_loss, py::arg("logp"), py::arg("old_logp"), py::arg("ref_logp"), py::arg("adv"),
         py::arg("labels"), py::arg("entropy"), py::arg("old_entropy"), py::arg("clip_low"), py::arg("clip_high"),
         py::arg("clip_c"), py::arg("kl_beta"), py::arg("grad_weight"), py::arg("dlogp"), py::arg("stats"), NOGIL);

@@ -164,7 +164,7 @@ class NativeDecoder:
                        for n in ("ln1", "wqkv", "bqkv", "wo", "ln2", "wgu", "wd")] for i in range(cfg.num_hidden_layers)]
         self.launches = 0  # kernels of this package launched (bench bookkeeping)
         self.memory_share = 1.0  # of the device, what this process's roles are to stay within (kept logits only)
-        self._asked_at = -1  # what the allocator held when the device was last asked for free memory
+        self._asked = (-1, 0)  # what the allocator held when the device was last asked, and the free memory then
 
     # ---- helpers ----
     def w(self, name: str) -> torch.Tensor:
@@ -380,36 +380,34 @@ class NativeDecoder:
         """Columns of the dlogits buffer of ``rows`` rows."""
         return min(vocab_chunk(rows, self.lmhead_chunk), (self.cfg.vocab_size + 255) // 256 * 256)
 
-    def _held_bytes(self, T: int, rows: int) -> int:
-        """What a training step of T rows, ``rows`` of them with a loss, holds beside kept logits while it has those: the embedding,
-        the activations of the layers (with recomputation their inputs, and one layer's at a time) and the head's rows, dlogits and dH. As
-        exact as it can be: more, and a step would not find in the allocator what the same step has left there."""
-        L, x, layer = self.cfg.num_hidden_layers, 2 * T * self.cfg.hidden_size, int(self.C.layer_fwd_bytes(self._dims, T, True))
-        head = rows * (2 * self._chunk(rows) + 6 * self.cfg.hidden_size)
-        return x + (L * x + max(layer, head) if self.recompute else L * layer + head)
-
-    def _keep_columns(self, rows: int, T: int) -> int:
-        """Columns of the fp32 logits of ``rows`` rows that a training step of T rows may keep on this decoder's device. The allocator is
-        asked first, the device only if this stream's unused blocks do not hold everything, and then not again until the allocator has
-        taken or given back memory: on a machine with other users that question takes 0.1 to 100 ms."""
-        V = self.cfg.vocab_size
+    def _keep_columns(self, rows: int) -> int:
+        """Columns of the fp32 logits of ``rows`` rows that a training step may keep beside what it holds when it asks (its layers'
+        activations). The allocator is asked first, the device only if this stream's unused blocks do not hold the logits and the head's
+        buffers, and then not again until the allocator has taken or given back memory: on a machine with other users that question
+        takes 0.1 to 100 ms."""
+        V, H = self.cfg.vocab_size, self.cfg.hidden_size
         if rows <= 0 or torch.cuda.is_current_stream_capturing():
             return 0  # a graph's memory stays taken between its replays
-        step = int(self.C.lmhead_chunk_step(V, self._chunk(rows)))
+        chunk = self._chunk(rows)
+        step = int(self.C.lmhead_chunk_step(V, chunk))
         if 4 * rows * V <= 64 << 20:
             return kept_columns(rows, V, 64 << 20, step)
-        held = self._held_bytes(T, rows)
-        cached, block, reserved = self.C.cached_memory(self.dev.index, 2 * T * self.cfg.hidden_size)
-        cols = kept_columns(rows, V, min(block, cached - held), step)
-        if cols >= V or reserved == self._asked_at:
+        # rows of the head, dlogits, dH. As exact as it can be: more, and a step would not find what the same step has left in the allocator
+        head = rows * (2 * chunk + 6 * H)
+        cached, block, reserved = self.C.cached_memory(self.dev.index, 2 * rows * H)
+        cols = kept_columns(rows, V, min(block, cached - head), step)
+        if cols >= V:
             return cols
-        free, total = torch.cuda.mem_get_info(self.dev)
-        self._asked_at = reserved
-        limit = int(torch.cuda.get_per_process_memory_fraction(self.dev) * total) - reserved
-        free = max(0, min(free - int((1.0 - self.memory_share) * total), limit))
-        # A new block: of what the process could still get a quarter, since other streams and roles grow as well, and not more than the
-        # device has beside what the activations ask it for. Else the allocator would give back all that it holds and begin anew.
-        return max(cols, kept_columns(rows, V, min((cached + free - held) // 4, free - max(0, held - cached)), step))
+        if reserved != self._asked[0]:
+            free, total = torch.cuda.mem_get_info(self.dev)
+            limit = int(torch.cuda.get_per_process_memory_fraction(self.dev) * total) - reserved
+            self._asked = (reserved, max(0, min(free - int((1.0 - self.memory_share) * total), limit)))
+        # Of what the process could still get a quarter, since other streams and roles grow as well. For the head's buffers, or for a new
+        # block, which is not more than the device has beside what the head asks it for: else the allocator would give back all that
+        # it holds and begin anew.
+        free = self._asked[1]
+        cols = kept_columns(rows, V, min(block, cached + free // 4 - head), step)
+        return max(cols, kept_columns(rows, V, min((cached + free - head) // 4, free - max(0, head - cached)), step))
 
     def _body(self, batch: PackedBatch, saves: Optional[List[dict]]) -> torch.Tensor:
         """Embedding and all layers."""
@@ -465,17 +463,16 @@ class NativeDecoder:
         # (a third of the rows where answers are short), and their gradient is zero. Work that is saved: logits twice, two gradients.
         compact = (batch.loss_rows and batch.total_out > 0
                    and 8.0 * (T - batch.total_out) * cfg.vocab_size * cfg.hidden_size > LOSS_ROWS_MIN_FLOPS)
+        x_last = self._body(batch, saves)
         # The backward pass needs the logits again: kept in fp32 (31287 x 151936: 19 GB) they are read once, 2 ms, instead of
-        # recomputed, 10 ms. Columns that do not fit into the memory that the activations leave are recomputed. They come first: a
-        # step then finds the block that the step before gave back whole, where a request behind the activations would find it
-        # split and ask the device for another (20 ms).
+        # recomputed, 10 ms. Columns for which there is no memory are recomputed. Decided here, when the activations have what they
+        # need and the device has work: the question takes the host 0.2 ms.
         n_head = batch.total_out if compact else T
-        keep = self._keep_columns(n_head, T)
+        keep = self._keep_columns(n_head)
         try:
             logits = self._new(n_head, keep, dtype=torch.float32) if keep > 0 else None
         except torch.OutOfMemoryError:
             logits = None
-        x_last = self._body(batch, saves)
         labels, advantages, old_logp, old_ent = batch.labels, batch.advantages, batch.old_logprobs, batch.old_entropies
         ref = batch.ref_logprobs if (lc.kl_beta > 0 and batch.has_ref) else None
         rows = None

@@ -8,15 +8,19 @@ from async_grpo_nccl_b200.models import decoder as D
 from async_grpo_nccl_b200.ops import native
 
 GB = 1 << 30
+ROWS, V = 30000, 151936
+NEED = ROWS * V * 4               # 17 GB
+HEAD = ROWS * (2 * 15360 + 6 * 1536)  # 1.1 GB
 
 
 class Memory:
-    """A decoder's view of a device: ``cached`` bytes unused in the allocator, ``free`` on the device, ``fraction`` and ``share`` allowed."""
+    """A decoder's view of a device: ``cached`` bytes unused in the allocator (the largest block ``block``), ``free`` on the device,
+    ``fraction`` and ``share`` allowed."""
 
-    def __init__(self, monkeypatch, cached, reserved, free, held=30 * GB, V=151936, total=180 * GB, fraction=1.0, share=1.0):
+    def __init__(self, monkeypatch, cached, reserved, free, total=180 * GB, fraction=1.0, share=1.0):
         self.asked, self.block = [], None
-        self.dec = SimpleNamespace(dev=torch.device("cuda", 1), cfg=SimpleNamespace(vocab_size=V, hidden_size=1536), _asked_at=-1, memory_share=share,
-                                   _held_bytes=lambda T, rows: held, C=SimpleNamespace(cached_memory=self.cached_memory, lmhead_chunk_step=native().lmhead_chunk_step),
+        self.dec = SimpleNamespace(dev=torch.device("cuda", 1), cfg=SimpleNamespace(vocab_size=V, hidden_size=1536), _asked=(-1, 0), memory_share=share,
+                                   C=SimpleNamespace(cached_memory=self.cached_memory, lmhead_chunk_step=native().lmhead_chunk_step),
                                    _chunk=lambda rows: 15360)
         self.cached, self.reserved, self.free, self.total = cached, reserved, free, total
         monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
@@ -32,8 +36,13 @@ class Memory:
         self.asked.append(dev)
         return self.free, self.total
 
-    def keep(self, rows, T):
-        return D.NativeDecoder._keep_columns(self.dec, rows, T)
+    def keep(self, rows=ROWS):
+        cols = D.NativeDecoder._keep_columns(self.dec, rows)
+        assert cols == V or cols % 15360 == 0  # only columns that are read
+        return cols
+
+    def bytes(self):
+        return self.keep() * 4 * ROWS
 
 
 def test_columns_that_fit():
@@ -53,55 +62,43 @@ def test_steps_of_the_backward_pass(V, chunk, step):
         assert kept % step == 0 or kept == (V + 7) // 8 * 8
 
 
-@pytest.mark.parametrize("cached,free", [(40, 0), (33, 9), (31, 0), (30, 50)])
-def test_only_columns_that_are_read_are_kept(monkeypatch, cached, free):
-    m = Memory(monkeypatch, cached * GB, 60 * GB, free * GB)
-    cols = m.keep(30000, 32768)
-    assert cols % 15360 == 0 and cols < 151936
-
-
-# need: 30000 x 151936 x 4 = 17.0 GB beside 72 GB that the step holds anyway. A cache filled by a larger microbatch without kept logits
-# has room for the step, not for all of its logits: what is short would be an activation's.
-@pytest.mark.parametrize("cached,all_kept", [(72 + 17, True), (85, False), (73, False), (60, False)])
-def test_cached_memory_must_hold_the_step_and_the_logits(monkeypatch, cached, all_kept):
-    m = Memory(monkeypatch, cached * GB, 120 * GB, 0, held=72 * GB)
-    cols = m.keep(30000, 32768)
-    assert (cols == 151936) == all_kept
-    assert cols * 30000 * 4 <= max(0, cached - 72) * GB
+@pytest.mark.parametrize("cached", [0, HEAD, HEAD + NEED // 2, HEAD + NEED - 1, HEAD + NEED])
+def test_the_allocator_must_hold_the_logits_and_the_head(monkeypatch, cached):
+    m = Memory(monkeypatch, cached, 120 * GB, 0)
+    assert (m.keep() == V) == (cached >= HEAD + NEED) and m.bytes() <= max(0, cached - HEAD)
 
 
 def test_device_is_asked_again_only_after_the_allocator_has_changed(monkeypatch):
-    m = Memory(monkeypatch, 33 * GB, 40 * GB, 20 * GB)
-    first = m.keep(30000, 32768)
-    assert len(m.asked) == 1 and 0 < first * 120000 <= 23 * GB // 4
-    m.cached, m.reserved = 36 * GB, 43 * GB
-    m.keep(30000, 32768)
+    m = Memory(monkeypatch, 4 * GB, 40 * GB, 20 * GB)
+    first = m.bytes()
+    assert len(m.asked) == 1 and 0 < first <= (24 * GB - HEAD) // 4
+    m.cached, m.reserved = 9 * GB, 45 * GB
+    m.keep()
     assert len(m.asked) == 2
-    again = m.keep(30000, 32768)
-    assert len(m.asked) == 2 and again * 120000 <= 6 * GB
-    m.cached = 60 * GB  # all of it from here on
-    assert m.keep(30000, 32768) == 151936 and len(m.asked) == 2
+    assert 0 < m.bytes() <= 9 * GB and len(m.asked) == 2  # one cached block, the head from the device
+    m.cached = 40 * GB  # all of it from here on
+    assert m.keep() == V and len(m.asked) == 2
 
 
 def test_one_block_holds_the_logits(monkeypatch):
     m = Memory(monkeypatch, 60 * GB, 70 * GB, 0)
     m.block = 5 * GB  # the rest in smaller ones: a larger block would come from the device, which has nothing left
-    assert 0 < m.keep(30000, 32768) * 120000 <= 5 * GB
-    m.dec._asked_at, m.free = -1, 100 * GB
-    assert m.keep(30000, 32768) == 151936
-    m.dec._asked_at, m.free, m.cached = -1, 25 * GB, 28 * GB  # the activations take 2 GB of it
-    assert 0 < m.keep(30000, 32768) * 120000 <= 23 * GB // 4
+    assert 0 < m.bytes() <= 5 * GB
+    m.dec._asked, m.free = (-1, 0), 100 * GB
+    assert m.keep() == V
+    m.dec._asked, m.free, m.cached, m.block = (-1, 0), 9 * GB, 0, 0  # the head takes 1.1 GB of it
+    assert 0 < m.bytes() <= (9 * GB - HEAD) // 4
 
 
 @pytest.mark.parametrize("kw", [dict(fraction=0.25), dict(share=0.5)])
 def test_limits_of_the_process(monkeypatch, kw):
     # 90 GB free on the device, 45 GB held: a process limit of 45 GB, or a share of the device that others have left half used
-    m = Memory(monkeypatch, 31 * GB, 45 * GB, 90 * GB, **kw)
-    assert m.keep(30000, 32768) * 120000 <= 1 * GB
+    m = Memory(monkeypatch, 5 * GB, 45 * GB, 90 * GB, **kw)
+    assert 0 < m.bytes() <= 5 * GB - HEAD
 
 
 def test_nothing_is_kept_without_rows_or_in_a_graph(monkeypatch):
     m = Memory(monkeypatch, 100 * GB, 120 * GB, 0)
-    assert m.keep(0, 100) == 0
+    assert m.keep(0) == 0
     monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: True)
-    assert m.keep(100, 100) == 0
+    assert m.keep(100) == 0
