@@ -66,12 +66,12 @@ inline bool& pdl_flag() {
 }
 // What the caller vouches for besides: the kernel directly ahead of a launch does not write the launch's weights (the B of a split-K,
 // SwiGLU or sampling product) nor, of an attention step over a paged cache, the lengths, the block tables and the entries older than the
-// newest token. Those are then read before the wait. Also a switch of the thread, without effect where the other is off.
+// newest token. Those are then read before the wait. Also a switch of the thread; with the other off the kernel ahead is complete anyway.
 inline bool& pdl_early_flag() {
   static thread_local bool on = false;
   return on;
 }
-inline bool pdl_early() { return pdl_flag() && pdl_early_flag(); }
+inline bool pdl_early() { return !pdl_flag() || pdl_early_flag(); }
 template <typename... KArgs, typename... Args>
 inline void launch_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, const char* what,
                           Args&&... args) {
