@@ -69,7 +69,6 @@ struct DecodeParams {
   int num_cache_blocks;
   int* status;
   int* tickets;             // [B, Hkv] zero-initialised arrival counters, or nullptr: the last split CTA to finish merges
-  bool early = false;       // stand-alone kernel: reads ahead of the kernel before it
 };
 
 // Shared-memory tile of one 16-token block: 16 rows x 256 bytes, 16-byte chunk c of row r stored at c ^ (r & 7). Tiles start on

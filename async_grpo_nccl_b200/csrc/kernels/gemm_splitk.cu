@@ -78,7 +78,6 @@ struct SkParams {
   float eps;
   int* status;
   long long* trace;  // optional: clock64 stamps of the phases of cluster 0 / CTA 0 (16 slots), nullptr = off
-  bool early;        // the kernel before this one does not write B
 };
 
 #define SK_STAMP(slot)                                                         \
@@ -137,7 +136,7 @@ gemm_splitk_cluster_kernel(const __grid_constant__ CUtensorMap tmA, const __grid
   const int num_kb = (p.K + kBK - 1) / kBK;
   const int kb0 = (int)((long long)num_kb * crank / S);
   const int kb1 = (int)((long long)num_kb * (crank + 1) / S);
-  const int n_pre = !p.early ? 0 : (kb1 - kb0) < STAGES ? (kb1 - kb0) : STAGES;  // loads issued during the prologue
+  const int n_pre = (kb1 - kb0) < STAGES ? (kb1 - kb0) : STAGES;  // loads issued during the prologue
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
@@ -150,7 +149,7 @@ gemm_splitk_cluster_kernel(const __grid_constant__ CUtensorMap tmA, const __grid
     // only warps that hold rows below M push (32 rows each): the inbox expects exactly their bytes
     const int rows_pushed = (((p.M < MT * kBM ? p.M : MT * kBM) + 31) / 32) * 32;
     mbar_expect_tx(inbox_bar, (uint32_t)(BN * 4 * rows_pushed));
-    // The first weight (B) loads depend on nothing that another thread, CTA or (`early`) the preceding kernel produces: issue
+    // The first weight (B) loads depend on nothing that another thread, CTA or the preceding kernel produces: issue
     // them before any synchronisation so that their ~2 us cold latency overlaps the prologue and, under programmatic
     // dependent launch, the tail of the previous kernel. The activation (A) loads follow once that kernel is complete.
     for (int i = 0; i < n_pre; ++i) {
@@ -480,7 +479,7 @@ void launch_sk(const CUtensorMap& ta, const CUtensorMap& tb, const SkParams& p, 
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = pdl_flag() ? 2 : 1;
+  cfg.numAttrs = pdl_on(true) ? 2 : 1;  // reads B ahead of its wait
   check_cuda(cudaLaunchKernelEx(&cfg, kernel, ta, tb, p, S), "gemm_splitk launch");
 }
 
@@ -554,7 +553,6 @@ bool launch_gemm_skinny(const void* a, long long lda, const void* b, long long l
   p.eps = eps;
   p.status = status;
   p.trace = trace;
-  p.early = pdl_early();
   if (MT == 1) launch_sk<128, 1, 4>(ta, tb, p, S, n_tiles, stream);
   else         launch_sk<64, 2, 3>(ta, tb, p, S, n_tiles, stream);
   return true;
@@ -566,7 +564,6 @@ SkParams blank_params(int M, int N, int K, int* status) {
   p.M = M; p.N = N; p.K = K;
   p.inv_k = 1.f / (float)K;
   p.status = status;
-  p.early = pdl_early();
   return p;
 }
 void launch_blank(const void* a, long long lda, int a_cols, const void* b, long long ldb, const SkParams& p, int S, int n_tiles, cudaStream_t s) {

@@ -140,8 +140,7 @@ __global__ void __launch_bounds__(kDecWarps * 32)
 paged_decode_attn_kernel(const DecodeParams p) {
   extern __shared__ __align__(256) uint8_t dsm[];
   __shared__ int s_last;
-  // `early`: lengths, tables and the pages of older tokens are older than the kernel before this one
-  if (!p.early) pdl_wait();
+  // lengths, tables and the pages of older tokens are older than the kernel before this one
   paged_decode_attend<2>(p, blockIdx.x, blockIdx.y, blockIdx.z, dsm, threadIdx.x >> 5, threadIdx.x, &s_last, [] {
     pdl_wait();
     pdl_launch();
@@ -437,12 +436,11 @@ void launch_paged_decode_attn(const void* q, long long ldq, int q_col0, const vo
   p.num_cache_blocks = num_cache_blocks;
   p.status = status;
   p.tickets = tickets;
-  p.early = pdl_early();
   constexpr int smem = kDecWarps * 2 * 2 * 4096;  // 64 KB staging (>= merge area of 16.6 KB)
   AGRPO_SET_MAX_DYN_SMEM(paged_decode_attn_kernel, smem, "paged_decode smem attr");
   dim3 grid(splits, Hkv, B);
   AGRPO_PREFER_SMEM(paged_decode_attn_kernel);
-  launch_kernel(paged_decode_attn_kernel, grid, dim3(kDecWarps * 32), smem, s, "paged_decode_attn", p);
+  launch_kernel<true>(paged_decode_attn_kernel, grid, dim3(kDecWarps * 32), smem, s, "paged_decode_attn", p);
   if (splits > 1 && tickets == nullptr) {
     dim3 g2(Hkv, B);
     AGRPO_PREFER_SMEM(paged_decode_combine_kernel);

@@ -548,8 +548,7 @@ talk_decode_kernel(const __grid_constant__ CUtensorMap tmK, const TalkDecodeArgs
   int* s_last = reinterpret_cast<int*>(empty + 4);
   const int split = blockIdx.x, b = blockIdx.y;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  // `early`: lengths, tables and the keys of earlier tokens were complete before the kernel ahead of this one started.
-  if (!a.early) pdl_wait();
+  // Lengths, tables and the keys of earlier tokens were complete before the kernel ahead of this one started.
   const int pos = p.seq_lens[b] - 1;
   if (pos < 0) {
     pdl_wait();
@@ -985,9 +984,7 @@ void launch_decode_t(const TalkDecodeArgs& a, const DecPlan& d, cudaStream_t s) 
   AGRPO_SET_MAX_DYN_SMEM(kernel, 226 * 1024, "talk_decode smem attr");
   AGRPO_PREFER_SMEM(kernel);
   const CUtensorMap tk = make_tmap_2d(a.k_cache, D, (uint64_t)a.at.num_cache_blocks * a.at.G * 16, D, 64, 16);
-  TalkDecodeArgs args = a;
-  args.early = pdl_early();
-  launch_kernel(kernel, dim3(a.splits, a.at.T), dim3(MW == 1 ? 288 : 512), d.smem, s, "talk_decode", tk, args, d.stages);
+  launch_kernel<true>(kernel, dim3(a.splits, a.at.T), dim3(MW == 1 ? 288 : 512), d.smem, s, "talk_decode", tk, a, d.stages);
 }
 template <int D, int MW, int MTW>
 void launch_decode_n(const TalkDecodeArgs& a, const DecPlan& d, cudaStream_t s) {

@@ -99,7 +99,6 @@ struct TalkDecodeArgs {
   float* part_o;          // [B, splits, H, G, D]
   float* part_ml;         // [B, splits, H, 2]
   int* tickets;           // [B], zero-initialised, re-armed by the kernel
-  bool early = false;     // set by the launcher: lengths, tables and older keys are read ahead of the kernel before
 };
 int talk_decode_ctas_per_sm(int H, int G, int D);  // 0: shape not served
 void launch_talk_attn_decode(const TalkDecodeArgs& a, cudaStream_t s);
