@@ -804,6 +804,7 @@ void decode_layers(int64_t L, int64_t B, const Tensor& wqkv0, int64_t wqkv_strid
   TORCH_CHECK(cache.dim() == 6 && cache.is_contiguous() && cache.size(0) == L && cache.size(1) == 2 && cache.size(3) == Hkv &&
               cache.size(4) == 16 && cache.size(5) == 128, "decode_layers: cache [L, 2, blocks, Hkv, 16, 128]");
   TORCH_CHECK(splits >= 1 && splits <= 64, "decode_layers: splits");
+  // `tickets` is the third of the stand-alone attention's buffers, which the callers pass as they are; this kernel needs none.
   TORCH_CHECK(part_o.numel() >= B * Hkv * splits * 8 * 128 && part_ml.numel() >= B * Hkv * splits * 16 && tickets.numel() >= B * Hkv,
               "decode_layers: split-KV scratch");
   TORCH_CHECK(counters.numel() >= agrpo::decode_layers_counter_words(), "decode_layers: counters");
@@ -821,7 +822,7 @@ void decode_layers(int64_t L, int64_t B, const Tensor& wqkv0, int64_t wqkv_strid
   a.cache = cache.data_ptr(); a.cache_layer_stride = cache.stride(0); a.cache_v_off = cache.stride(1);
   a.num_cache_blocks = (int)cache.size(2);
   a.softmax_scale = (float)softmax_scale;
-  a.part_o = part_o.data_ptr<float>(); a.part_ml = part_ml.data_ptr<float>(); a.att_tickets = tickets.data_ptr<int>();
+  a.part_o = part_o.data_ptr<float>(); a.part_ml = part_ml.data_ptr<float>();
   a.partials = partials.data_ptr<float>(); a.partials_bytes = partials.numel() * 4;
   a.counters = reinterpret_cast<unsigned int*>(counters.data_ptr<int>());
   a.status = opt_ptr<int>(status);

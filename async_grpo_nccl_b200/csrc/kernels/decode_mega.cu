@@ -129,7 +129,6 @@ struct MegaShared {
   uint32_t tmem_slot;
   unsigned int seen;     // the value of `done` that this CTA has observed
   unsigned int xa_free;  // layers whose qkv products have read all that they need from the activation ring
-  int abort;
 };
 
 constexpr int kAttStages = 3;
@@ -268,7 +267,6 @@ decode_layers_kernel(const __grid_constant__ CUtensorMap tmWqkv, const __grid_co
       mbar_init(&sh->tmem_empty[a], 4);  // the compute warps
     }
     mbar_init(&sh->xa_bar, 128);
-    sh->abort = 0;
     sh->seen = 0;
     sh->xa_free = 0;
     fence_mbar_init();
@@ -333,7 +331,6 @@ decode_layers_kernel(const __grid_constant__ CUtensorMap tmWqkv, const __grid_co
             }
           }
         }
-        if (!ok) sh->abort = 1;
       }
     } else if (warp == 1) {
       // ================= activation producer: waits for the phase that writes its operand =================
@@ -387,7 +384,6 @@ decode_layers_kernel(const __grid_constant__ CUtensorMap tmWqkv, const __grid_co
             }
           }
         }
-        if (!ok) sh->abort = 1;
       }
     } else if (warp == 2) {
       // ================= MMA issuer =================
@@ -445,7 +441,6 @@ decode_layers_kernel(const __grid_constant__ CUtensorMap tmWqkv, const __grid_co
             }
           }
         }
-        if (!ok) sh->abort = 1;
       }
     } else if (warp == 3) {
       // ================= watcher: the only thread of the CTA that polls the global counter =================
@@ -694,7 +689,7 @@ decode_layers_kernel(const __grid_constant__ CUtensorMap tmWqkv, const __grid_co
         if (ph == 0 && tid == 0) st_release_cta(&sh->xa_free, (unsigned int)(l + 1));
       }
     }
-    if (!ok && tid == 0) sh->abort = 1;
+    if (!ok && tid == 0) report_status(p.status, kStatusBarrierTimeout);  // the first code stays
   } else {
     // ================= attention warps =================
     asm volatile("setmaxnreg.inc.sync.aligned.u32 240;");
@@ -731,7 +726,6 @@ decode_layers_kernel(const __grid_constant__ CUtensorMap tmWqkv, const __grid_co
       if (tid == 0) MEGA_STAMP(25);
       if (tid == 0) MEGA_STAMP_ALL(1);
     }
-    if (!ok && tid == 0) sh->abort = 1;
   }
 
   tc_fence_before();
@@ -845,10 +839,11 @@ void launch_decode_layers(const DecodeLayersArgs& a, cudaStream_t stream) {
   d.scale_log2 = a.softmax_scale * 1.4426950408889634f;
   d.out = p.attn; d.ldo = a.QD;
   d.part_o = a.part_o; d.part_ml = a.part_ml; d.tickets = nullptr;
-  d.status = a.status;
   p.partials = a.partials;
   p.done = a.counters;
-  p.status = a.status;
+  // A wait that runs out has to end the others, in every CTA: without a status word of the caller's they watch one of the launch's own.
+  p.status = a.status != nullptr ? a.status : reinterpret_cast<int*>(a.counters + 1);
+  d.status = p.status;
   p.trace = a.trace;
   p.trace_layer = a.trace_layer;
   p.trace_all = a.trace_words >= 32 + 4 * a.num_sms ? 1 : 0;

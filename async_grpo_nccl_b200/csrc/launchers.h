@@ -360,7 +360,6 @@ struct DecodeLayersArgs {
   int num_cache_blocks;
   float softmax_scale;
   float *part_o, *part_ml;
-  int* att_tickets;
   float* partials;
   long long partials_bytes;
   unsigned int* counters;  // decode_layers_counter_words() words
