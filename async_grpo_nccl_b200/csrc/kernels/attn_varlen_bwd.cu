@@ -586,9 +586,10 @@ void launch_bwd_t(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMa
 
 // CTAs over which the query heads of a (key tile, kv head) are dealt: enough for about four CTAs per SM, so that the longest of them
 // (all query tiles of the longest sequence) is a small part of an SM's share. 12 query and 2 kv heads, us with one piece and with as
-// many as this rule says: one sequence of 759 tokens 129 and 51 (6 pieces), of 2600 402 and 105 (6), of 8000 1161 and 604 (5), 11 of 250 to
-// 8575 1890 and 1845 (2). Sequences of one length lose: 19 of 330 112 and 124 (6), 40 of 330 175 and 200 (3), 8 of 4096 1278 and 1327 (2);
-// the count of tiles, which is what the host has, does not tell them from the others. From 592 CTAs on nothing is split.
+// many as this rule says, L2 flushed: one sequence of 759 tokens 130 and 52 (6 pieces), of 2600 404 and 105 (6), of 8000 1187 and 618 (5), 11
+// of 250 to 8575 (17341) 841 and 606 (3). Sequences of one length lose: 19 of 330 112 and 122 (6), 40 of 330 169 and 193 (3); 8 of 4096
+// 1281 to 1588 and 1316 to 1710 (2), where runs differ more than the choices. The rule goes by the count of tiles alone, which does not
+// tell these from the others; the packer knows the lengths, a rule by them is not built. From 592 CTAs on nothing is split.
 int attn_bwd_pieces(int n_tiles, int Hq, int Hkv, int num_sms) {
   const long long ctas = (long long)n_tiles * Hkv;
   if (ctas <= 0) return 1;

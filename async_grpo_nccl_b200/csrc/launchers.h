@@ -243,16 +243,17 @@ int attn_bwd_pieces(int n_tiles, int Hq, int Hkv, int num_sms);
 // ---- fused lm_head + GRPO loss (lmhead_loss.cu) ----
 // Number of partial-statistics groups the forward writes for a [T, V] problem.
 int lmhead_num_groups(int V, int T);
-// logits z = hidden . weight^T / temperature never reach memory. labels[t] is the target token of row t
+// logits z = hidden . weight^T / temperature reach memory only where they are kept. labels[t] is the target token of row t
 // (already shifted), negative = masked. partials: fp32 [3 * groups * T] scratch; label_logit: fp32 [T] scratch.
 // Outputs (each may be nullptr): logp[t] = z[label] - lse (0 on masked rows), entropy[t], lse[t].
+// keep_cols > 0: the fp32 logits (before the temperature) of that many leading columns, a multiple of 8 or from V on, also go to
+// logits [T, ld_logits] (rows on 32 bytes, ld_logits >= keep_cols and >= V rounded up to 8 where keep_cols >= V); the backward pass
+// reads them instead of recomputing the product.
 void launch_lmhead_logprob(const void* hidden, long long ldh, const void* weight, long long ldw, const int* labels, int T,
                            int H, int V, float temperature, float* partials, float* label_logit, float* logp,
                            float* entropy, float* lse, float* logits, long long ld_logits, int keep_cols, int* status, int num_sms,
                            cudaStream_t stream);
-// keep_cols > 0: the fp32 logits (before the temperature) of that many leading columns, a multiple of 8 or from V on, also go to
-// logits [T, ld_logits] (rows on 32 bytes, ld_logits >= keep_cols and >= V rounded up to 8 where keep_cols >= V); the backward pass
-// reads them instead of recomputing the product. Per-token dual-clip GRPO objective (+ kl_beta * k3 KL against ref_logp), its derivative w.r.t. logp scaled by
+// Per-token dual-clip GRPO objective (+ kl_beta * k3 KL against ref_logp), its derivative w.r.t. logp scaled by
 // grad_weight, and sums over valid tokens in stats[grpo_num_loss_stats()] (atomic adds; zero it first).
 void launch_grpo_token_loss(const float* logp, const float* old_logp, const float* ref_logp, const float* adv,
                             const int* labels, const float* entropy, const float* old_entropy, int T, float clip_low,
@@ -334,12 +335,13 @@ void launch_adamw(float* p, float* m, float* v, float* g, void* p16, long long n
                   cudaStream_t s);
 void launch_cast_f32_bf16(const float* in, void* out, long long n, cudaStream_t s);
 
-// All decoder layers of one decode step in one persistent cooperative launch (csrc/kernels/decode_mega.cu).
-// Per-layer weights sit at constant element strides in flat bf16 buffers; wqkv and wgu are the copies with the RMSNorm
-// weight folded in. Activation buffers have rows_alloc >= the row tile (32 / 64 / 128 / 256) that covers B rows.
 // last[r] = history[r, min(index[r], cap - 1)] = tokens[r] (history_lp alike, unless nullptr), index[r] += 1; histories [rows, cap].
 void launch_feed_back(const int* tokens, const float* logprobs, int rows, int* last, long long* index, int* history, float* history_lp,
                       long long cap, cudaStream_t s);
+
+// All decoder layers of one decode step in one persistent cooperative launch (csrc/kernels/decode_mega.cu).
+// Per-layer weights sit at constant element strides in flat bf16 buffers; wqkv and wgu are the copies with the RMSNorm
+// weight folded in. Activation buffers have rows_alloc >= the row tile (32 / 64 / 128 / 256) that covers B rows.
 struct DecodeLayersArgs {
   int L, B, rows_alloc, H, Q, QD, F, Hq, Hkv, num_sms, splits;
   const void *wqkv, *wo, *wgu, *wd;
