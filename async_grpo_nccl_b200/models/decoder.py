@@ -386,15 +386,16 @@ class NativeDecoder:
         buffers, and then not again until the allocator has taken or given back memory: on a machine with other users that question
         takes 0.1 to 100 ms."""
         V, H = self.cfg.vocab_size, self.cfg.hidden_size
-        if rows <= 0 or torch.cuda.is_current_stream_capturing():
-            return 0  # a graph's memory stays taken between its replays
+        if rows <= 0 or torch.cuda.is_current_stream_capturing() or torch.cuda.get_allocator_backend() != "native":
+            return 0  # a graph's memory stays taken between its replays; other allocators do not say what they hold
         chunk = self._chunk(rows)
         step = int(self.C.lmhead_chunk_step(V, chunk))
         if 4 * rows * V <= 64 << 20:
             return kept_columns(rows, V, 64 << 20, step)
         # rows of the head, dlogits, dH. As exact as it can be: more, and a step would not find what the same step has left in the allocator
         head = rows * (2 * chunk + 6 * H)
-        cached, block, reserved = self.C.cached_memory(self.dev.index, 2 * rows * H)
+        device = self.dev.index if self.dev.index is not None else torch.cuda.current_device()
+        cached, block, reserved = self.C.cached_memory(device, 2 * rows * H)
         cols = kept_columns(rows, V, min(block, cached - head), step)
         if cols >= V:
             return cols

@@ -24,6 +24,7 @@ class Memory:
                                    _chunk=lambda rows: 15360)
         self.cached, self.reserved, self.free, self.total = cached, reserved, free, total
         monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
+        monkeypatch.setattr(torch.cuda, "get_allocator_backend", lambda: "native")
         monkeypatch.setattr(torch.cuda, "mem_get_info", self.mem_get_info)
         monkeypatch.setattr(torch.cuda, "get_per_process_memory_fraction", lambda dev: fraction)
 
@@ -32,7 +33,7 @@ class Memory:
         return self.cached, self.block if self.block is not None else self.cached, self.reserved
 
     def mem_get_info(self, dev):
-        assert dev == torch.device("cuda", 1)
+        assert dev == self.dec.dev
         self.asked.append(dev)
         return self.free, self.total
 
@@ -97,8 +98,18 @@ def test_limits_of_the_process(monkeypatch, kw):
     assert 0 < m.bytes() <= 5 * GB - HEAD
 
 
-def test_nothing_is_kept_without_rows_or_in_a_graph(monkeypatch):
+def test_device_without_an_index_is_the_current_one(monkeypatch):
+    m = Memory(monkeypatch, 5 * GB, 45 * GB, 9 * GB)
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: 1)
+    m.dec.dev = torch.device("cuda")
+    assert m.keep() > 0 and len(m.asked) == 1
+
+
+def test_nothing_is_kept_without_rows_in_a_graph_or_with_another_allocator(monkeypatch):
     m = Memory(monkeypatch, 100 * GB, 120 * GB, 0)
     assert m.keep(0) == 0
+    with monkeypatch.context() as other:
+        other.setattr(torch.cuda, "get_allocator_backend", lambda: "cudaMallocAsync")
+        assert m.keep() == 0
     monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: True)
     assert m.keep(100) == 0
